@@ -33,9 +33,16 @@
 
 namespace hf {
 
+// The bit pattern of a double and back.  On the device through an opaque register move: from a plain
+// reinterpretation the compiler recognises the masks and compares below as absolute values, negations
+// and NaN tests and puts them back on the FP64 pipe, the stencils' bottleneck (MUSCL-Hancock at 2048^2
+// from the plain reinterpretation: 221 FP64 additions per cell update for the 157 of the scheme,
+// 53.1 M FP64 warp instructions and 3.47 ms a launch; through the move 38.7 M and 2.87 ms).
 HF_HD uint64_t f64_bits(double x) {
 #ifdef __CUDA_ARCH__
-    return (uint64_t)__double_as_longlong(x);
+    uint64_t u;
+    asm("mov.b64 %0, %1;" : "=l"(u) : "d"(x));
+    return u;
 #else
     uint64_t u;
     std::memcpy(&u, &x, 8);
@@ -44,7 +51,9 @@ HF_HD uint64_t f64_bits(double x) {
 }
 HF_HD double f64_from(uint64_t u) {
 #ifdef __CUDA_ARCH__
-    return __longlong_as_double((long long)u);
+    double x;
+    asm("mov.b64 %0, %1;" : "=d"(x) : "l"(u));
+    return x;
 #else
     double x;
     std::memcpy(&x, &u, 8);
