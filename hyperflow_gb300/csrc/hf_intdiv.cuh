@@ -1,24 +1,27 @@
-// Correctly rounded FP64 division on the integer pipes.
+// Correctly rounded FP64 division and square root on the integer pipes.
 //
-// GB300 issues FP64 at 2 lanes per SM per clock -- 1/32 of its integer rate -- and an IEEE
-// FP64 division built from FP64 Newton steps costs about ten FP64 instructions.  This
-// routine computes the same correctly rounded quotient (round to nearest, ties to even)
-// with integer multiplies instead, by the classical scheme of a Newton-Raphson refined
-// fixed-point reciprocal, a quotient by multiplication, and an exact remainder that both
-// corrects the quotient and decides the rounding (see Muller et al., "Handbook of
-// Floating-Point Arithmetic", the chapter on division; Moller & Granlund, "Improved division
-// by invariant integers", IEEE TC 2011, for the fixed-point reciprocal arithmetic):
+// GB300 issues FP64 at 2 lanes per SM per clock: a warp's FP64 instruction holds the SM's pipe for
+// 16 cycles, in which the SM can issue 64 others.  An IEEE division built from FP64 Newton steps
+// costs about ten FP64 instructions; this one costs none, and about 60 others.  It is schoolbook
+// long division with two large digits (see Muller et al., "Handbook of Floating-Point
+// Arithmetic", the chapter on division; Moller & Granlund, "Improved division by invariant
+// integers", IEEE TC 2011, for quotient digits from a truncated reciprocal):
 //
 //   a = ma 2^ea, b = mb 2^eb, ma, mb in [2^52, 2^53) (ma doubled when ma < mb, so that the
 //   quotient mantissa lies in [1, 2));
-//   X ~ 2^116 / mb: an FP32 reciprocal of mb's top 24 bits (about 23 correct bits), then two
-//   Newton steps X += X (2^116 - mb X) / 2^116 in 64-bit fixed point (about 62 bits);
-//   Q ~ floor(ma X / 2^64) = floor(ma 2^52 / mb) to within a few units; the exact remainder
-//   R = ma 2^52 - Q mb (small, so exact modulo 2^64) moves Q to the true floor; 2R against
-//   mb rounds it to nearest even.
+//   X ~ 2^84 / mb, 32 bits: an FP32 reciprocal of mb's top 24 bits and one Newton step, always a
+//   little low;
+//   q1 = ma X / 2^54, 31 bits, and the remainder R1 = ma 2^30 - q1 mb; q2 = R1 X / 2^61, 23 bits
+//   more, and the remainder R2 = R1 2^23 - q2 mb: both remainders are below 2^56, so exact modulo
+//   2^64, and the digits are never too big;
+//   Q = q1 2^23 + q2 is floor(ma 2^53 / mb) or one less, which R2 >= mb decides; the quotient
+//   rounds to nearest at Q's lowest bit.
+//
+// One 32 x 32 -> 64 multiplication per digit and remainder word (9 in all) where a reciprocal
+// refined to 64 bits took 64 x 64 -> 128 products.
 //
 // Every operand outside this fast path -- zero, subnormal, infinite or NaN divisor; a
-// subnormal, infinite or NaN dividend; a quotient whose exponent leaves the normal range --
+// subnormal, infinite or NaN dividend; a quotient whose exponent may leave the normal range --
 // goes to the hardware division, so the result equals `a / b` bit for bit for all inputs.
 // A zero dividend over a normal divisor gives the correctly signed zero directly.
 #pragma once
@@ -69,13 +72,6 @@ HF_HD uint32_t f32_bits(float x) {
     return u;
 #endif
 }
-HF_HD uint64_t umulhi64(uint64_t a, uint64_t b) {
-#ifdef __CUDA_ARCH__
-    return __umul64hi(a, b);
-#else
-    return (uint64_t)(((unsigned __int128)a * b) >> 64);
-#endif
-}
 HF_HD float f32_from(uint32_t u) {
 #ifdef __CUDA_ARCH__
     return __uint_as_float(u);
@@ -110,12 +106,6 @@ HF_HD float rsqrt_f32(float x) {
     const uint32_t b = f32_bits(one / std::sqrt(x));
     return f32_from(b + ((b * 2654435761u) >> 29) - 4u);
 #endif
-}
-// an integer in [2^23, 2^24) as an FP32 value, from its bits (no conversion instruction)
-HF_HD float u24_float(uint32_t m) { return f32_from(0x4B000000u | (m & 0x7FFFFFu)); }
-// an integer in [2^22, 2^24) as an FP32 value
-HF_HD float u22_24_float(uint32_t m) {
-    return (m >> 23) ? f32_from(0x4B000000u | (m & 0x7FFFFFu)) : f32_from(0x4A800000u | ((m << 1) & 0x7FFFFFu));
 }
 // IEEE comparisons on the integer pipes (NaN compares false, -0 equals +0).  A double's
 // sign-magnitude bits map to an order-preserving signed key: key = sign ? -|x| : |x|.
@@ -160,140 +150,120 @@ HF_HD double half(double x) {
 HF_HD double hw_div(double a, double b) { return a / b; }
 HF_HD double hw_sqrt(double x) { return std::sqrt(x); }
 
-// Fixed-point reciprocal X ~ 2^116 / mb of a divisor mantissa mb in (2^52, 2^53) (not a
-// power of two): an FP32 seed of mb's top 24 bits, then two Newton steps.
-HF_HD uint64_t recip_fixed(uint64_t mb) {
-    // FP32 seed: X0 = 2^87 / dh with dh = mb >> 29 in [2^23, 2^24)
-    const uint32_t dh = (uint32_t)(mb >> 29);
-    const float r = rcp_f32(u24_float(dh));
-    const uint32_t rb = f32_bits(r);
-    const uint64_t mr = (uint64_t)((rb & 0x7FFFFFu) | 0x800000u);
-    const int sh = (int)((rb >> 23) & 0xFFu) - 63;   // r = mr 2^(E-150); X0 = mr 2^(E-63)
-    uint64_t X = sh >= 41 ? 0xFFFFFFFFFFFFFFFFull : (mr << sh);
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-        // E = 2^116 - mb X as a signed 128-bit value (small); C = X E / 2^116
-        const uint64_t plo = mb * X, phi = umulhi64(mb, X);
-        const uint64_t elo = 0ull - plo;
-        const uint64_t ehi = (1ull << 52) - phi - (plo != 0 ? 1ull : 0ull);
-        const int64_t e52 = (int64_t)((ehi << 12) | (elo >> 52));     // E >> 52
-        const uint64_t mag = e52 < 0 ? (uint64_t)(-e52) : (uint64_t)e52;
-        const uint64_t c = umulhi64(X, mag);
-        X = e52 < 0 ? X - c : X + c;
-    }
-    return X;
+// hi and lo words of a 64-bit value, their concatenation, and 32-bit helpers
+HF_HD uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
+HF_HD uint32_t lo32(uint64_t x) { return (uint32_t)x; }
+HF_HD uint64_t u64_of(uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; }
+HF_HD uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+HF_HD uint32_t umulhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+// a b modulo 2^64 for a 32-bit a and a 64-bit b
+HF_HD uint64_t mul_low(uint32_t a, uint64_t b) {
+    const uint64_t l = wide(a, lo32(b));
+    return u64_of(hi32(l) + a * hi32(b), lo32(l));
+}
+// y 2^23 for an FP32 value y in (0.5, 1], lowered by a relative 2^-20 so that a seed within a few
+// ulp of the true value never exceeds it; no conversion instruction
+HF_HD uint32_t seed23(float y) {
+    const float low = 1.0f - 9.5367431640625e-7f;
+#ifdef __CUDA_ARCH__
+    const float v = __fmaf_rn(y, low, 1.0f);
+#else
+    const float v = std::fmaf(y, low, 1.0f);
+#endif
+    return f32_bits(v) - 0x3F800000u;
 }
 
-// The quotient of the fast path: a, b as in div_rn with `fast` true and a nonzero; X the
-// reciprocal of b's mantissa (unused when b is a power of two).
-HF_HD double quot_fast(uint64_t A, uint64_t B, uint64_t X) {
-    const uint32_t ea = (uint32_t)(A >> 52) & 0x7FFu, eb = (uint32_t)(B >> 52) & 0x7FFu;
-    const uint64_t sign = (A ^ B) & 0x8000000000000000ull;
-    const uint64_t M52 = 0x000FFFFFFFFFFFFFull, H52 = 0x0010000000000000ull;
-    int e = (int)ea - (int)eb + 1023;
-    uint64_t ma = (A & M52) | H52;
-    const uint64_t mb = (B & M52) | H52;
-    const bool shift = ma < mb;
-    e -= shift ? 1 : 0;
-    if (shift) ma <<= 1;                       // ma / mb in [1, 2)
-    uint64_t Q, R;
-    if ((B & M52) == 0) {                      // divisor a power of two: exact
-        Q = ma;                                // ma in [2^52, 2^53): no shift happened
-        R = 0;
-    } else {
-        Q = umulhi64(ma, X);
-        int64_t Rs = (int64_t)((ma << 52) - Q * mb);   // exact: |R| < 2^55
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (Rs < 0) { Q -= 1; Rs += (int64_t)mb; }
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (Rs >= (int64_t)mb) { Q += 1; Rs -= (int64_t)mb; }
-        R = (uint64_t)Rs;
-    }
-    // round to nearest, ties to even
-    const uint64_t r2 = R << 1;
-    if (r2 > mb || (r2 == mb && (Q & 1ull))) Q += 1;
-    if (Q == (H52 << 1)) { Q = H52; e += 1; }
-    return f64_from(sign | ((uint64_t)e << 52) | (Q & M52));
+constexpr uint32_t kExpHi = 0x7FF00000u, kMantHi = 0x000FFFFFu, kOneHi = 0x00100000u;
+
+// 2^84 / mb rounded down to within 5 units: the 32-bit reciprocal of the 53-bit mantissa mb of a
+// normal B, in (2^31, 2^32).  An FP32 seed (19 bits, low), one Newton step from below, and 3 units
+// off for the mantissa bits it does not see, so that the quotient's digits never come out too big.
+HF_HD uint32_t recip32(uint64_t B) {
+    const uint32_t bh = (uint32_t)(B >> 21) | 0x80000000u;               // mb's top 32 bits
+    const uint32_t x0 = seed23(rcp_f32(f32_from(0x3F800000u | ((bh >> 8) & 0x7FFFFFu))));
+    const uint64_t t = wide(bh, x0);                                     // 2^54 (1 - e)
+    return (x0 << 9) - 3u + umulhi32(x0, ~(uint32_t)(t >> 13));          // x0 (1 + e)
 }
 
-// true when a / b takes the integer path: b normal, and a zero, or a normal with a normal
-// quotient exponent
+// the quotient of the fast path (div_fast) from X = recip32(B)
+HF_HD double quot32(uint64_t A, uint64_t B, uint32_t X) {
+    const uint32_t ha = hi32(A), hb = hi32(B);
+    uint64_t ma = u64_of((ha & kMantHi) | kOneHi, lo32(A));
+    const uint64_t mb = u64_of((hb & kMantHi) | kOneHi, lo32(B));
+    // ma / mb in [1, 2); the exponent field, less the 1 that the mantissa's leading bit adds
+    uint32_t e = (ha & kExpHi) - (hb & kExpHi) + (1022u << 20);
+    if (ma < mb) {
+        ma += ma;
+        e -= kOneHi;
+    }
+    // the first 31 bits, short by at most 6, and their exact remainder below 7 mb
+    const uint32_t q1 = umulhi32((uint32_t)(ma >> 22), X);
+    const uint64_t r1 = (ma << 30) - mul_low(q1, mb);
+    // 23 more bits, short by at most 1; Q = floor(ma 2^53 / mb) or one less, R its remainder
+    const uint32_t q2 = umulhi32((uint32_t)(r1 >> 24), X) >> 5;
+    const uint64_t r2 = (r1 << 23) - mul_low(q2, mb);
+    uint64_t q = wide(q1, 1u << 23) + q2;
+    // round to nearest at the lowest of the 54 bits (a quotient of two 53-bit numbers is never a
+    // halfway case); the carry out of the mantissa lands in the exponent field
+    q = (q + (r2 >= mb ? 2u : 1u)) >> 1;
+    return f64_from(u64_of(hi32(q) + e + ((ha ^ hb) & 0x80000000u), lo32(q)));
+}
+
+// a / b takes the integer path: both normal, and so is every quotient of their exponents
 HF_HD bool div_fast(uint64_t A, uint64_t B) {
-    const uint32_t ea = (uint32_t)(A >> 52) & 0x7FFu, eb = (uint32_t)(B >> 52) & 0x7FFu;
-    const uint64_t M52 = 0x000FFFFFFFFFFFFFull, H52 = 0x0010000000000000ull;
-    const bool a_zero = (A << 1) == 0;
-    int e = (int)ea - (int)eb + 1023;
-    e -= (((A & M52) | H52) < ((B & M52) | H52)) ? 1 : 0;
-    return (eb - 1u < 2046u) && (a_zero || ((ea - 1u < 2046u) && e >= 1 && e <= 2045));
+    const uint32_t ea = hi32(A) & kExpHi, eb = hi32(B) & kExpHi;
+    return (ea - kOneHi < 0x7FE00000u) && (eb - kOneHi < 0x7FE00000u) && (ea - eb + (1021u << 20) < (2044u << 20));
+}
+
+// the other operands: a zero over a normal divisor is a signed zero (velocities at rest), the
+// rest goes to the hardware
+static __host__ __device__ __noinline__ double div_slow(double a, double b) {
+    const uint64_t A = f64_bits(a), B = f64_bits(b);
+    if ((A << 1) == 0 && (hi32(B) & kExpHi) - kOneHi < 0x7FE00000u)
+        return f64_from((A ^ B) & 0x8000000000000000ull);
+    return hw_div(a, b);
 }
 
 // Kept out of line: the stencils call it about 55 times per cell, and one shared copy keeps the
 // kernels inside the instruction cache (measured faster than inlining every call).
 static __host__ __device__ __noinline__ double div_rn(double a, double b) {
     const uint64_t A = f64_bits(a), B = f64_bits(b);
-    if (!div_fast(A, B)) return hw_div(a, b);
-    if ((A << 1) == 0) return f64_from((A ^ B) & 0x8000000000000000ull);
-    const uint64_t M52 = 0x000FFFFFFFFFFFFFull, H52 = 0x0010000000000000ull;
-    const uint64_t X = (B & M52) == 0 ? 0ull : recip_fixed((B & M52) | H52);
-    return quot_fast(A, B, X);
+    if (!div_fast(A, B)) return div_slow(a, b);
+    return quot32(A, B, recip32(B));
 }
 
-}  // namespace hf
-
-namespace hf {
-
-// Correctly rounded FP64 square root on the integer pipes, by the same scheme: x = m 2^E
-// (m doubled when E is odd so the exponent halves exactly), Y ~ 2^90 / sqrt(m) from an FP32
-// reciprocal square root refined by two Newton steps Y += Y (2^180 - m Y^2) / 2^181 in
-// fixed point, S ~ m Y / 2^64 = floor(sqrt(m 2^52)) corrected with the exact remainder
-// R = m 2^52 - S^2, and rounded up when R > S (a square root is never a halfway case).
-// Zero, negative, subnormal, infinite and NaN arguments go to the hardware sqrt.
-// out of line, as div_rn
+// Correctly rounded FP64 square root on the integer pipes, digit by digit as the division:
+// x = z 4^k with z a 64-bit integer in [2^62, 2^64); Y ~ 2^31 / sqrt(z / 2^64) from an FP32
+// reciprocal square root and one Newton step, low by at most 7 units; 32 bits of the root
+// sqrt(z), short by at most 16, and their exact remainder; 22 more bits, short by at most 1;
+// the exact remainder of the 54-bit root decides that 1, and its lowest bit the rounding (a
+// square root is never a halfway case).  Zero, negative, subnormal, infinite and NaN arguments go
+// to the hardware sqrt.  Out of line, as div_rn.
 static __host__ __device__ __noinline__ double sqrt_rn(double x) {
-    const uint64_t X = f64_bits(x);
-    const uint32_t ex = (uint32_t)(X >> 52) & 0x7FFu;
-    if ((X >> 63) != 0 || ex - 1u >= 2046u) return hw_sqrt(x);
-    const uint64_t M52 = 0x000FFFFFFFFFFFFFull, H52 = 0x0010000000000000ull;
-    const int E = (int)ex - 1023;
-    uint64_t m = (X & M52) | H52;
-    int Eh;
-    if (E & 1) { m <<= 1; Eh = (E - 1) / 2; } else { Eh = E / 2; }   // m in [2^52, 2^54)
-    uint64_t S;
-    if (m == H52) {
-        S = H52;                                   // x is an even power of two
-    } else {
-        const uint32_t mh = (uint32_t)(m >> 30);   // [2^22, 2^24), exact in FP32
-        const float rs = rsqrt_f32(u22_24_float(mh));
-        const uint32_t rb = f32_bits(rs);
-        const uint64_t mr = (uint64_t)((rb & 0x7FFFFFu) | 0x800000u);
-        const int sh = (int)((rb >> 23) & 0xFFu) - 75;        // Y0 = 2^75 rs = mr 2^(E_r - 75)
-        uint64_t Y = sh >= 41 ? 0xFFFFFFFFFFFFFFFFull : (sh < 0 ? 0ull : (mr << sh));
-#pragma unroll
-        for (int it = 0; it < 2; ++it) {
-            const uint64_t t = umulhi64(Y, Y);                    // ~ 2^116 / m
-            const uint64_t plo = m * t, phi = umulhi64(m, t);
-            const uint64_t elo = 0ull - plo;
-            const uint64_t ehi = (1ull << 52) - phi - (plo != 0 ? 1ull : 0ull);
-            const int64_t e52 = (int64_t)((ehi << 12) | (elo >> 52));   // (2^116 - m t) >> 52
-            const uint64_t mag = e52 < 0 ? (uint64_t)(-e52) : (uint64_t)e52;
-            const uint64_t c = umulhi64(Y, mag) >> 1;
-            Y = e52 < 0 ? Y - c : Y + c;
-        }
-        S = umulhi64(m, Y);
-        int64_t R = (int64_t)((m << 52) - S * S);                  // exact: |R| small
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (R < 0) { R += (int64_t)(2 * S - 1); S -= 1; }
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-            if (R >= (int64_t)(2 * S + 1)) { R -= (int64_t)(2 * S + 1); S += 1; }
-        if (R > (int64_t)S) S += 1;
-    }
-    int eo = Eh + 1023;
-    if (S == (H52 << 1)) { S = H52; eo += 1; }
-    return f64_from(((uint64_t)eo << 52) | (S & M52));
+    const uint64_t A = f64_bits(x);
+    const uint32_t h = hi32(A);
+    if (h - kOneHi >= 0x7FE00000u) return hw_sqrt(x);
+    const bool odd = (h & kOneHi) == 0;   // an odd exponent: the mantissa doubled
+    uint64_t z = u64_of((h & kMantHi) | kOneHi, lo32(A)) << 10;
+    if (odd) z += z;
+    const uint32_t zh = hi32(z);
+    const uint32_t m23 = (uint32_t)(A >> 29) & 0x7FFFFFu;
+    const uint32_t y0 = seed23(rsqrt_f32(f32_from((odd ? 0x40000000u : 0x3F800000u) | m23)));
+    const uint64_t t = wide(zh, (uint32_t)(wide(y0, y0) >> 14));         // 2^62 (1 - e)
+    const uint32_t Y = (y0 << 9) - 5u + umulhi32(y0, ~(uint32_t)(t >> 22));
+    const uint32_t s1 = (uint32_t)(wide(zh, Y) >> 31);
+    const uint64_t r1 = z - wide(s1, s1);
+    uint64_t s = wide(s1, 1u << 22) + (umulhi32((uint32_t)(r1 >> 5), Y) >> 5);
+    const uint64_t sq = wide(lo32(s), lo32(s));
+    const uint64_t r2 = u64_of((lo32(z) << 12) - hi32(sq) - 2u * lo32(s) * hi32(s), 0u) - lo32(sq);
+    s = (s + (r2 > s + s ? 2u : 1u)) >> 1;
+    return f64_from(u64_of(hi32(s) + (((h >> 20) + 1021u) >> 1 << 20), lo32(s)));
 }
 
 }  // namespace hf
