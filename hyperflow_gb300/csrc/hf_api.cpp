@@ -66,6 +66,7 @@ struct hf_ctx {
     hf::MeshDev hmesh{};
     hf::MeshDev* dmesh = nullptr;
     hf::Ctrl* dctrl = nullptr;
+    hf::TileShape tile{};       // the stencils' tile, for the whole mesh
     CUtensorMap tmap[HF_MAXB][2];
     hf::StepPlan plan{};        // the all-blocks MUSCL-Hancock launch (plan.nb = 0: not usable)
     bool block_launches = false;   // hf_set_block_launches: one stencil launch per block instead
@@ -436,32 +437,33 @@ bool step_kernel(const hf_ctx* ctx) { return ctx->scheme == 1 && ctx->plan.nb > 
 // mesh of one block gains nothing from it unless the block fills many waves (measured: a 264^2
 // block 341 Mcell-updates/s against 448 with one launch per block, 1010^2 999 against 986, 4096^2
 // 1173 against 1163).
-constexpr int kStepMinTilesOneBlock = 1024;
+constexpr long long kStepMinCellsOneBlock = 393216;
 
 void make_plan(hf_ctx* ctx) {
     ctx->plan = hf::StepPlan{};
     if (ctx->scheme != 1 || ctx->nblocks > hf::kStepMaxBlocks) return;
     hf::StepPlan plan{};
+    plan.tile = ctx->tile;
     for (int b = 0; b < ctx->nblocks; ++b) {
         plan.tm[b][0] = ctx->tmap[b][0];
         plan.tm[b][1] = ctx->tmap[b][1];
         hf::step_plan_tiles(plan, b, ctx->blocks[b].nx, ctx->blocks[b].ny);
     }
     plan.nb = ctx->nblocks;
-    if (ctx->nblocks == 1 && plan.tile_start[1] < kStepMinTilesOneBlock) return;
+    if (ctx->nblocks == 1 && (long long)ctx->blocks[0].nx * ctx->blocks[0].ny < kStepMinCellsOneBlock) return;
     ctx->plan = plan;
 }
 
 int make_tmaps(hf_ctx* ctx) {
     PFN_encodeTiled enc = get_encode();
     if (!enc) return fail(ctx, HF_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-    hf::StencilTiles t = hf::stencil_tiles(ctx->scheme);
+    const int halo = 2 * ctx->ghost;
     for (int b = 0; b < ctx->nblocks; ++b) {
         const BlockHost& B = ctx->blocks[b];
         for (int k = 0; k < 2; ++k) {
             cuuint64_t dims[3] = {(cuuint64_t)B.tx, (cuuint64_t)B.ty, 4};
             cuuint64_t strides[2] = {(cuuint64_t)B.pitch * 8, (cuuint64_t)B.pitch * B.ty * 8};
-            cuuint32_t box[3] = {(cuuint32_t)t.box_x, (cuuint32_t)t.box_y, 4};
+            cuuint32_t box[3] = {(cuuint32_t)(ctx->tile.tx + halo), (cuuint32_t)(ctx->tile.ty + halo), 4};
             cuuint32_t es[3] = {1, 1, 1};
             CUresult r = enc(&ctx->tmap[b][k], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
                              ctx->hmesh.b[b].buf[k], dims, strides, box, es,
@@ -525,7 +527,7 @@ int enqueue_step(hf_ctx* ctx, bool profiled) {
         } else {
             for (int b = 0; b < ctx->nblocks; ++b)
                 CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].nx, ctx->blocks[b].ny,
-                                      ctx->scheme, ctx->limiter, &ctx->tmap[b][0], &ctx->tmap[b][1],
+                                      ctx->scheme, ctx->limiter, ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1],
                                       ctx->stream));
         }
     }
@@ -648,6 +650,15 @@ int hf_create(const char* case_json, size_t len, hf_ctx** out) {
     C.first_nonpos = ~0ull;
     CK(cudaMalloc(&ctx->dctrl, sizeof(hf::Ctrl)));
     CK(cudaMemcpyAsync(ctx->dctrl, &C, sizeof C, cudaMemcpyHostToDevice, ctx->stream));
+    {
+        int nx[HF_MAXB], ny[HF_MAXB], sms = 0;
+        for (int b = 0; b < ctx->nblocks; ++b) {
+            nx[b] = ctx->blocks[b].nx;
+            ny[b] = ctx->blocks[b].ny;
+        }
+        CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        ctx->tile = hf::choose_tile(ctx->scheme, nx, ny, ctx->nblocks, sms);
+    }
     int r = make_tmaps(ctx);
     if (r != HF_OK) return r;
     make_plan(ctx);
@@ -805,7 +816,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         CK(hf::launch_set_dt(ctx->dctrl, dt, ctx->stream));
     }
     CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].nx, ctx->blocks[b].ny,
-                          ctx->scheme, ctx->limiter, &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream));
+                          ctx->scheme, ctx->limiter, ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream));
     if (b == ctx->nblocks - 1) {
         CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
         ctx->next_block = 0;
@@ -916,7 +927,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
             for (int b = 0; b < ctx->nblocks; ++b) {
                 const BlockHost& B = ctx->blocks[b];
                 CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, B.nx, B.ny, ctx->scheme, ctx->limiter,
-                                      &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream, out[b]));
+                                      ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream, out[b]));
             }
         }
         CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
@@ -942,7 +953,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
     for (int b = 0; b < ctx->nblocks; ++b) {
         const BlockHost& B = ctx->blocks[b];
         CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, B.nx, B.ny, ctx->scheme, ctx->limiter,
-                              &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream));
+                              ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream));
         CK(cudaEventRecord(ctx->block_done[b], ctx->stream));
         CK(cudaStreamWaitEvent(ctx->copy_stream, ctx->block_done[b], 0));
         CK(cudaMemcpy2DAsync(out[b], (size_t)B.tx * 8, ctx->hmesh.b[b].buf[p ^ 1], (size_t)B.pitch * 8,

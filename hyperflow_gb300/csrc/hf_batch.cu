@@ -149,7 +149,7 @@ template <int TX, int TY>
 struct BatchTile<1, TX, TY> {   // MUSCL-Hancock: 2-cell halo; evolved states, face fluxes
     using T = MhTile<TX, TY>;
     static constexpr int H = 2, UX = T::UX, UY = T::UY, U_SIZE = T::U_SIZE;
-    static constexpr int WORK = T::A_SIZE + T::F_SIZE + T::G_SIZE;
+    static constexpr int WORK = T::A_SIZE;
 };
 
 // stage tile `t`'s state + mirrored halo into sU (cp.async, one commit group)
@@ -219,8 +219,8 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps)
 #pragma unroll
     for (int k = 0; k < STAGES; ++k) sUb[k] = smem + k * BT::U_SIZE;
     double* sW = smem + STAGES * BT::U_SIZE;   // MUSCL-Hancock: sA; Godunov: sQ
-    double* sF = sW + (SCHEME == 1 ? MhTile<TX, TY>::A_SIZE : GoTile<TX, TY>::Q_SIZE);
-    double* sG = sF + (SCHEME == 1 ? MhTile<TX, TY>::F_SIZE : GoTile<TX, TY>::F_SIZE);
+    double* sF = sW + GoTile<TX, TY>::Q_SIZE;   // Godunov only
+    double* sG = sF + GoTile<TX, TY>::F_SIZE;
     __shared__ double sdt[5];
 
     BatchCtrl* c = d.ctrl;
@@ -313,9 +313,9 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps)
             if (SCHEME == 0)
                 herr += go_tile_fluxes<TX, TY, NT>(sU, sW, sF, sG, g, g1, x0, y0, I.n, I.n);
             else if (lim == 0)
-                herr += mh_tile_fluxes<TX, TY, NT, 0>(sU, sW, sF, sG, g, g1, hdx, hdy, x0, y0, I.n, I.n);
+                herr += mh_tile_fluxes<NT, 0>(MhTile<TX, TY>(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
             else
-                herr += mh_tile_fluxes<TX, TY, NT, 1>(sU, sW, sF, sG, g, g1, hdx, hdy, x0, y0, I.n, I.n);
+                herr += mh_tile_fluxes<NT, 1>(MhTile<TX, TY>(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
             double mx = 0.0, my = 0.0;
             double* __restrict__ out = Un + I.off;
             const size_t plane = (size_t)I.pitch * I.n;
@@ -324,10 +324,10 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps)
                 const int gx = x0 + ox, gy = y0 + oy;
                 if (gx < I.n && gy < I.n) {
                     double un[4];
+                    if (SCHEME == 1) mh_update(MhTile<TX, TY>(), sU, sW, ox, oy, dt, one_dx, one_dy, un);
 #pragma unroll
                     for (int v = 0; v < 4; ++v) {
-                        un[v] = SCHEME == 0 ? go_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy)
-                                            : mh_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy);
+                        if (SCHEME == 0) un[v] = go_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy);
                         out[v * plane + (size_t)gy * I.pitch + gx] = un[v];
                     }
                     double sx, sy;
@@ -399,8 +399,8 @@ struct BatchConfig {
 // tile shape, threads, halo staging buffers, CTAs per SM the registers are budgeted for
 // (the last, 32x4 tiles of 128 threads at four CTAs per SM, is for batches too small to give
 // every SM several large tiles per step, such as a single 256^2 case)
-constexpr BatchConfig kConfigs[] = {{32, 14, 256, 1, 2}, {32, 14, 256, 2, 2}, {32, 16, 256, 1, 2},
-                                    {32, 12, 256, 1, 3}, {32, 12, 256, 2, 2}, {32, 4, 128, 1, 4}};
+constexpr BatchConfig kConfigs[] = {{32, 14, 256, 1, 2}, {32, 14, 256, 2, 2}, {32, 19, 448, 1, 2},
+                                    {32, 12, 256, 1, 3}, {24, 25, 448, 1, 2}, {32, 4, 128, 1, 4}};
 constexpr int kNumConfigs = 6;
 
 template <int SCHEME, int TX, int TY, int ST>
@@ -443,9 +443,9 @@ cudaError_t launch_scheme_config(int k, const BatchDev& d, int nsteps, int sms, 
     switch (k) {
         case 0: return launch_batch<SCHEME, 32, 14, 256, 1, 2>(d, nsteps, sms, s, cfl_only);
         case 1: return launch_batch<SCHEME, 32, 14, 256, 2, 2>(d, nsteps, sms, s, cfl_only);
-        case 2: return launch_batch<SCHEME, 32, 16, 256, 1, 2>(d, nsteps, sms, s, cfl_only);
+        case 2: return launch_batch<SCHEME, 32, 19, 448, 1, 2>(d, nsteps, sms, s, cfl_only);
         case 3: return launch_batch<SCHEME, 32, 12, 256, 1, 3>(d, nsteps, sms, s, cfl_only);
-        case 4: return launch_batch<SCHEME, 32, 12, 256, 2, 2>(d, nsteps, sms, s, cfl_only);
+        case 4: return launch_batch<SCHEME, 24, 25, 448, 1, 2>(d, nsteps, sms, s, cfl_only);
         default: return launch_batch<SCHEME, 32, 4, 128, 1, 4>(d, nsteps, sms, s, cfl_only);
     }
 }

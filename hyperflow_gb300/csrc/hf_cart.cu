@@ -352,19 +352,11 @@ __global__ void finalize_kernel(Ctrl* c) {
 // ------------------------------------------------------------------------------------
 // shared helpers for the stencils
 // ------------------------------------------------------------------------------------
-// issue the tile's TMA load and wait for it (bounded); false if the wait gave up
-template <int NBYTES>
-__device__ __forceinline__ bool load_tile(double* sU, uint64_t* bar, const CUtensorMap* tm, int x0,
-                                          int y0, Ctrl* c) {
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        mbar_expect_tx(bar, NBYTES);
-        tma_load_3d(sU, tm, bar, x0, y0, 0);
-    }
+// wait (bounded) for the tile's first TMA load, which thread 0 issued; false if the wait gave up
+__device__ __forceinline__ bool wait_tile(uint64_t* bar, Ctrl* c) {
     __syncthreads();
-    bool ok = mbar_wait_bounded(bar, 0, kWaitLimit);
-    int bad = __syncthreads_or(!ok);
-    if (bad) {
+    const bool ok = mbar_wait_bounded(bar, 0, kWaitLimit);
+    if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) {
             raise_error(c, HF_DEV_TIMEOUT);
             mbar_wait_bounded(bar, 0, kWaitLimit);   // let an in-flight copy land before exit
@@ -379,63 +371,86 @@ __device__ __forceinline__ bool load_tile(double* sU, uint64_t* bar, const CUten
 // step's output buffer, so the updated state carries the ghost values the reference's mesh holds
 // after the step (its update leaves ghost cells as filled) and the next fill finds this fill's
 // values in its other buffer.  Each ghost cell is stored by the one tile holding its nearest
-// interior cell; only tiles on the block's edge hold any.  sU is [4][TY + 2G][TX + 2G].
-template <int TX, int TY, int G, int NT>
-__device__ __forceinline__ void store_ghosts(const double* __restrict__ sU, const BlockDev& B, int x0, int y0,
-                                             double* __restrict__ out, int* err) {
-    if (x0 > 0 && y0 > 0 && x0 + TX < B.nx && y0 + TY < B.ny) return;
-    constexpr int UX = TX + 2 * G, UY = TY + 2 * G;
+// interior cell; only tiles on the block's edge hold any.  sU is [4][ty + 2G][tx + 2G].
+template <int G, int NT>
+__device__ __forceinline__ void store_ghosts(const double* __restrict__ sU, const BlockDev& B, int tx, int ty, int x0,
+                                             int y0, double* __restrict__ out, int* err) {
+    if (x0 > 0 && y0 > 0 && x0 + tx < B.nx && y0 + ty < B.ny) return;
+    const int ux = tx + 2 * G, uy = ty + 2 * G;
     const size_t plane = (size_t)B.ty * B.pitch;
-    for (int it = threadIdx.x; it < UX * UY; it += NT) {
-        const int lx = it % UX, ly = it / UX;
+    for (int it = threadIdx.x; it < ux * uy; it += NT) {
+        const int lx = it % ux, ly = it / ux;
         const int x = x0 - G + lx, y = y0 - G + ly;   // interior coordinates
         if (x < -G || y < -G || x >= B.nx + G || y >= B.ny + G) continue;
         if (x >= 0 && y >= 0 && x < B.nx && y < B.ny) continue;
         const int cx = x < 0 ? 0 : (x >= B.nx ? B.nx - 1 : x);
         const int cy = y < 0 ? 0 : (y >= B.ny ? B.ny - 1 : y);
-        if (cx < x0 || cx >= x0 + TX || cy < y0 || cy >= y0 + TY) continue;
+        if (cx < x0 || cx >= x0 + tx || cy < y0 || cy >= y0 + ty) continue;
         const size_t o = (size_t)(y + G) * B.pitch + (x + G);
         if (!hf_in((long long)o, (long long)plane, err)) continue;
 #pragma unroll
-        for (int v = 0; v < 4; ++v) out[v * plane + o] = sU[(v * UY + ly) * UX + lx];
+        for (int v = 0; v < 4; ++v) out[v * plane + o] = sU[(v * uy + ly) * ux + lx];
+    }
+}
+
+// The tile's update: conservative update + forward Euler of its cells into out (and hout), the next
+// step's TimeStep terms into mx and my, the earliest non-positive cell into *nonpos.
+template <int NT>
+__device__ __forceinline__ void mh_store(const MhShape& S, const double* sU, const double* sA, const BlockDev& B, int x0,
+                                         int y0, double* __restrict__ out, double* __restrict__ hout, double dt,
+                                         double one_dx, double one_dy, double g, double g1, unsigned long long* nonpos,
+                                         unsigned long long key, double& mx, double& my, int* err) {
+    const int tx = S.tx(), n = tx * S.ty();
+    const size_t plane = (size_t)B.ty * B.pitch;
+    for (int it = threadIdx.x; it < n; it += NT) {
+        const int oy = S.row0(it), ox = it - oy * tx;
+        const int gxx = x0 + ox, gyy = y0 + oy;
+        if (gxx < B.nx && gyy < B.ny) {
+            double un[4];
+            const size_t o = (size_t)(gyy + 2) * B.pitch + (gxx + 2);
+            const size_t h = (size_t)(gyy + 2) * B.tx + gxx + 2;
+            if (!hf_in((long long)o, (long long)plane, err) || !hf_in((long long)h, (long long)B.ty * B.tx, err)) continue;
+            mh_update(S, sU, sA, ox, oy, dt, one_dx, one_dy, un);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+                out[v * plane + o] = un[v];
+                if (hout) __stcs(&hout[(size_t)v * B.ty * B.tx + h], un[v]);
+            }
+            double sx, sy;
+            if (!wave_terms(g, g1, un[0], un[1], un[2], un[3], sx, sy)) atomicMin(nonpos, key | face_key(0, 0, 0, gyy, gxx));
+            mx = nmax(mx, sx);
+            my = nmax(my, sy);
+        }
     }
 }
 
 // ------------------------------------------------------------------------------------
 // MUSCL-Hancock, fused
 // ------------------------------------------------------------------------------------
-template <int TX, int TY>
-struct MhLayout {
-    using T = MhTile<TX, TY>;
-    static constexpr int U_OFF = 0;
-    static constexpr int A_OFF = U_OFF + T::U_SIZE;
-    static constexpr int F_OFF = A_OFF + T::A_SIZE;
-    static constexpr int G_OFF = F_OFF + T::F_SIZE;
-    static constexpr int END = G_OFF + T::G_SIZE;
-    static constexpr size_t BYTES = (size_t)END * 8 + 16;   // + mbarrier
-    static constexpr int TMA_BYTES = T::U_SIZE * 8;
-};
+// Two 448-thread CTAs per SM (72 registers; 110.9 KB of shared memory each, which a 32 x 19 tile fills):
+// the tile's 42 warp-items of predictor cells are three rounds of the 14 warps, its 40 of faces too.
+// Measured at 2048^2 (Mcell-updates/s): 1973; 512 threads and 64 registers 1962, 320 threads and 32 x 18
+// tiles 1933, 256 threads and 32 x 14 1880, three CTAs of 256 threads and 32 x 12 tiles 1751.
+constexpr int kMhNT = 448, kMhDoubles = 13856;
+constexpr size_t kMhBytes = (size_t)kMhDoubles * 8;
 
-template <int TX, int TY, int LIM, int NT>
-// three 256-thread CTAs per SM (80 registers, 73 KB of shared memory each): 24 warps hide more
-// of the integer sequences' latency than 16 (measured faster despite a few spilled registers)
-__global__ void __launch_bounds__(NT, 3) mh_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                                int b, const __grid_constant__ CUtensorMap tm0,
-                                                const __grid_constant__ CUtensorMap tm1,
-                                                double* __restrict__ hout) {
-    using L = MhLayout<TX, TY>;
+template <int LIM>
+__global__ void __launch_bounds__(kMhNT, 2) mh_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
+                                                      const TileShape tile, const __grid_constant__ CUtensorMap tm0,
+                                                      const __grid_constant__ CUtensorMap tm1,
+                                                      double* __restrict__ hout) {
     extern __shared__ __align__(1024) double smem[];
-    double* sU = smem + L::U_OFF;
-    double* sA = smem + L::A_OFF;
-    double* sF = smem + L::F_OFF;
-    double* sG = smem + L::G_OFF;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::END);
+    __shared__ uint64_t bar;
+    const MhShape S{tile};
+    const int tx = tile.tx, ty = tile.ty, usize = 4 * (tx + 4) * (ty + 4);
+    double* sU = smem;
+    double* sA = smem + usize;
     if (c->done) return;
 
     const BlockDev& B = m->b[b];
     const int p = (int)(c->step & 1);
-    const int tiles_x = (B.nx + TX - 1) / TX;
-    const int x0 = (blockIdx.x % tiles_x) * TX, y0 = (blockIdx.x / tiles_x) * TY;
+    const int tiles_x = (B.nx + tx - 1) / tx;
+    const int x0 = (blockIdx.x % tiles_x) * tx, y0 = (blockIdx.x / tiles_x) * ty;
 
     // scalars of this step, formed once per CTA by thread 0 while the tile is in flight and
     // published by the barrier in load_tile
@@ -443,50 +458,28 @@ __global__ void __launch_bounds__(NT, 3) mh_kernel(Ctrl* __restrict__ c, const M
     const double g = c->gamma, g1 = c->g1;
     const double dt = c->dt;
     if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, usize * 8);
+        tma_load_3d(sU, p ? &tm1 : &tm0, &bar, x0, y0, 0);
         // the predictor's own TimeStep call (muscl_hancock.cpp:246): blocks < b already advanced
         const double dtp = cfl_dt(c, c->calls + b, b, p, p ^ 1);
         const double dx = c->dx[b], dy = c->dy[b];
-        sc[0] = 0.5 * dtp / dx;   // 248-249
-        sc[1] = 0.5 * dtp / dy;
-        sc[2] = 1.0 / dx;         // 352-353
-        sc[3] = 1.0 / dy;
+        sc[0] = div_rn(0.5 * dtp, dx);   // 248-249
+        sc[1] = div_rn(0.5 * dtp, dy);
+        sc[2] = div_rn(1.0, dx);         // 352-353
+        sc[3] = div_rn(1.0, dy);
         if (blockIdx.x == 0) c->dt_pred[b] = dtp;
     }
-
-    if (!load_tile<L::TMA_BYTES>(sU, bar, p ? &tm1 : &tm0, x0, y0, c)) return;
+    if (!wait_tile(&bar, c)) return;
     const double hdx = sc[0], hdy = sc[1], one_dx = sc[2], one_dy = sc[3];
 
-    const int herr = mh_tile_fluxes<TX, TY, NT, LIM>(sU, sA, sF, sG, g, g1, hdx, hdy, x0, y0, B.nx, B.ny,
-                                                     &c->first_bad, face_key(c->step, b, 0, 0, 0));
-    // conservative update + forward Euler, and the next step's TimeStep terms
-    double* __restrict__ out = B.buf[p ^ 1];
-    const size_t plane = (size_t)B.ty * B.pitch;
+    const int herr = mh_tile_fluxes<kMhNT, LIM>(S, sU, sA, g, g1, hdx, hdy, x0, y0, B.nx, B.ny, &c->first_bad,
+                                                face_key(c->step, b, 0, 0, 0));
     double mx = 0.0, my = 0.0;
-    for (int it = threadIdx.x; it < TX * TY; it += NT) {
-        const int ox = it % TX, oy = it / TX;
-        const int gxx = x0 + ox, gyy = y0 + oy;
-        if (gxx < B.nx && gyy < B.ny) {
-            double un[4];
-            const size_t o = (size_t)(gyy + 2) * B.pitch + (gxx + 2);
-            const size_t h = (size_t)(gyy + 2) * B.tx + gxx + 2;
-            if (!hf_in((long long)o, (long long)plane, &c->err) ||
-                !hf_in((long long)h, (long long)B.ty * B.tx, &c->err))
-                continue;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                un[v] = mh_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy);
-                out[v * plane + o] = un[v];
-                if (hout) __stcs(&hout[(size_t)v * B.ty * B.tx + h], un[v]);
-            }
-            double sx, sy;
-            if (!wave_terms(g, g1, un[0], un[1], un[2], un[3], sx, sy))
-                atomicMin(&c->first_nonpos, face_key(c->step, b, 0, gyy, gxx));
-            mx = nmax(mx, sx);
-            my = nmax(my, sy);
-        }
-    }
-    store_ghosts<TX, TY, 2, NT>(sU, B, x0, y0, out, &c->err);
-    block_max2_atomic<NT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
+    mh_store<kMhNT>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], hout, dt, one_dx, one_dy, g, g1, &c->first_nonpos,
+                    face_key(c->step, b, 0, 0, 0), mx, my, &c->err);
+    store_ghosts<2, kMhNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
+    block_max2_atomic<kMhNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
 
@@ -547,23 +540,26 @@ __device__ bool step_grid_barrier(Ctrl* c) {
 
 // this launch's predictor scalars per block: 0.5 dtp / dx, 0.5 dtp / dy, 1 / dx, 1 / dy, and dtp
 __shared__ double s_step_sc[kStepMaxBlocks][5];
+__shared__ uint64_t s_step_bar;   // the tiles' TMA loads
 
 // One tile of block b (local tile index `local`): its TMA load (mbarrier phase `phase`), the
 // fused fluxes with the block's predictor scalars, the update and the block's records.  False if
 // the load's bounded wait gave up.  Out of line: the tile loop and the re-run loop share one copy.
-template <int TX, int TY, int LIM, int NT>
+template <int LIM>
 __device__ __noinline__ bool mh_step_tile(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                           const StepPlan& plan, int b, int local, int p, uint32_t phase) {
-    using L = MhLayout<TX, TY>;
     extern __shared__ __align__(1024) double smem[];
-    double* sU = smem + L::U_OFF;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::END);
+    const MhShape S{plan.tile};
+    const int tx = plan.tile.tx, ty = plan.tile.ty, usize = 4 * (tx + 4) * (ty + 4);
+    double* sU = smem;
+    double* sA = smem + usize;
+    uint64_t* bar = &s_step_bar;
     const BlockDev& B = m->b[b];
-    const int x0 = (local % plan.tiles_x[b]) * TX, y0 = (local / plan.tiles_x[b]) * TY;
+    const int x0 = (local % plan.tiles_x[b]) * tx, y0 = (local / plan.tiles_x[b]) * ty;
     if (threadIdx.x == 0) {
         // the previous tile's reads of sU (generic proxy) are ordered before this copy's writes
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(bar, L::TMA_BYTES);
+        mbar_expect_tx(bar, usize * 8);
         tma_load_3d(sU, &plan.tm[b][p], bar, x0, y0, 0);
     }
     const bool ok = mbar_wait_bounded(bar, phase, kWaitLimit);
@@ -576,41 +572,14 @@ __device__ __noinline__ bool mh_step_tile(Ctrl* __restrict__ c, const MeshDev* _
         return false;
     }
     const double g = c->gamma, g1 = c->g1;
-    const int herr = mh_tile_fluxes<TX, TY, NT, LIM>(sU, smem + L::A_OFF, smem + L::F_OFF, smem + L::G_OFF, g, g1,
-                                                     s_step_sc[b][0], s_step_sc[b][1], x0, y0, B.nx, B.ny,
-                                                     &c->step_bad[b], face_key(c->step, b, 0, 0, 0));
-    const double* sF = smem + L::F_OFF;
-    const double* sG = smem + L::G_OFF;
-    const double dt = c->dt, one_dx = s_step_sc[b][2], one_dy = s_step_sc[b][3];
-    double* __restrict__ out = B.buf[p ^ 1];
-    double* __restrict__ hout = plan.hout[b];
-    const size_t plane = (size_t)B.ty * B.pitch;
+    const unsigned long long key = face_key(c->step, b, 0, 0, 0);
+    const int herr = mh_tile_fluxes<kMhNT, LIM>(S, sU, sA, g, g1, s_step_sc[b][0], s_step_sc[b][1], x0, y0, B.nx, B.ny,
+                                                &c->step_bad[b], key);
     double mx = 0.0, my = 0.0;
-    for (int it = threadIdx.x; it < TX * TY; it += NT) {
-        const int ox = it % TX, oy = it / TX;
-        const int gxx = x0 + ox, gyy = y0 + oy;
-        if (gxx < B.nx && gyy < B.ny) {
-            double un[4];
-            const size_t o = (size_t)(gyy + 2) * B.pitch + (gxx + 2);
-            const size_t h = (size_t)(gyy + 2) * B.tx + gxx + 2;
-            if (!hf_in((long long)o, (long long)plane, &c->err) ||
-                !hf_in((long long)h, (long long)B.ty * B.tx, &c->err))
-                continue;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                un[v] = mh_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy);
-                out[v * plane + o] = un[v];
-                if (hout) __stcs(&hout[(size_t)v * B.ty * B.tx + h], un[v]);
-            }
-            double sx, sy;
-            if (!wave_terms(g, g1, un[0], un[1], un[2], un[3], sx, sy))
-                atomicMin(&c->step_nonpos[b], face_key(c->step, b, 0, gyy, gxx));
-            mx = nmax(mx, sx);
-            my = nmax(my, sy);
-        }
-    }
-    store_ghosts<TX, TY, 2, NT>(sU, B, x0, y0, out, &c->err);
-    block_max2_atomic<NT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
+    mh_store<kMhNT>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], plan.hout[b], c->dt, s_step_sc[b][2], s_step_sc[b][3], g, g1,
+                    &c->step_nonpos[b], key, mx, my, &c->err);
+    store_ghosts<2, kMhNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
+    block_max2_atomic<kMhNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->step_hllc[b]), (unsigned long long)herr);
     return true;
 }
@@ -624,12 +593,9 @@ __device__ __forceinline__ void step_scalars(const Ctrl* c, int b, double dtp) {
     s_step_sc[b][4] = dtp;
 }
 
-template <int TX, int TY, int LIM, int NT>
-__global__ void __launch_bounds__(NT, 3) mh_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                                     const __grid_constant__ StepPlan plan) {
-    using L = MhLayout<TX, TY>;
-    extern __shared__ __align__(1024) double smem[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::END);
+template <int LIM>
+__global__ void __launch_bounds__(kMhNT, 2) mh_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+                                                           const __grid_constant__ StepPlan plan) {
     if (c->done) return;   // set before this launch: every CTA leaves, no barrier is entered
 
     const int p = (int)(c->step & 1);
@@ -638,7 +604,7 @@ __global__ void __launch_bounds__(NT, 3) mh_step_kernel(Ctrl* __restrict__ c, co
     __shared__ int s_tile, s_redo;
     if (threadIdx.x == 0) {
         for (int b = 0; b < nb; ++b) step_scalars(c, b, cfl_dt(c, calls + b, 0, p, p ^ 1));   // starting state
-        mbar_init(bar, 1);
+        mbar_init(&s_step_bar, 1);
     }
     __syncthreads();
     uint32_t phase = 0u;
@@ -650,7 +616,7 @@ __global__ void __launch_bounds__(NT, 3) mh_step_kernel(Ctrl* __restrict__ c, co
         if (t >= total) break;
         int b = 0;
         while (t >= plan.tile_start[b + 1]) ++b;
-        if (!mh_step_tile<TX, TY, LIM, NT>(c, m, plan, b, t - plan.tile_start[b], p, phase)) return;
+        if (!mh_step_tile<LIM>(c, m, plan, b, t - plan.tile_start[b], p, phase)) return;
         phase ^= 1u;
     }
     for (int b = 1; b < nb; ++b) {
@@ -673,7 +639,7 @@ __global__ void __launch_bounds__(NT, 3) mh_step_kernel(Ctrl* __restrict__ c, co
         if (!step_grid_barrier(c)) return;   // the cleared records are in place before the re-run
         const int ntiles = plan.tile_start[b + 1] - plan.tile_start[b];
         for (int local = blockIdx.x; local < ntiles; local += gridDim.x) {
-            if (!mh_step_tile<TX, TY, LIM, NT>(c, m, plan, b, local, p, phase)) return;
+            if (!mh_step_tile<LIM>(c, m, plan, b, local, p, phase)) return;
             phase ^= 1u;
         }
     }
@@ -733,11 +699,14 @@ __global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c,
     const double dt = c->dt;
     __shared__ double sc[2];
     if (threadIdx.x == 0) {
-        sc[0] = 1.0 / c->dx[b];   // godunov.cpp:97-98
-        sc[1] = 1.0 / c->dy[b];
+        mbar_init(bar, 1);
+        mbar_expect_tx(bar, L::TMA_BYTES);
+        tma_load_3d(sU, p ? &tm1 : &tm0, bar, x0, y0, 0);
+        sc[0] = div_rn(1.0, c->dx[b]);   // godunov.cpp:97-98
+        sc[1] = div_rn(1.0, c->dy[b]);
     }
 
-    if (!load_tile<L::TMA_BYTES>(sU, bar, p ? &tm1 : &tm0, x0, y0, c)) return;
+    if (!wait_tile(bar, c)) return;
     const double one_dx = sc[0], one_dy = sc[1];
 
     const int herr = go_tile_fluxes<TX, TY, NT>(sU, sQ, sF, sG, g, g1, x0, y0, B.nx, B.ny, &c->first_bad,
@@ -768,7 +737,7 @@ __global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c,
             my = nmax(my, sy);
         }
     }
-    store_ghosts<TX, TY, 1, NT>(sU, B, x0, y0, out, &c->err);
+    store_ghosts<1, NT>(sU, B, TX, TY, x0, y0, out, &c->err);
     block_max2_atomic<NT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
@@ -776,16 +745,52 @@ __global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c,
 // ------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------
-constexpr int kMhTX = 32, kMhTY = 12, kMhNT = 256;
 constexpr int kGoTX = 32, kGoTY = 10, kGoNT = 256;
 
-StencilTiles stencil_tiles(int scheme) {
-    return scheme == 0 ? StencilTiles{kGoTX + 2, kGoTY + 2} : StencilTiles{kMhTX + 4, kMhTY + 4};
+TileShape tile_shape(int tx, int ty) {
+    TileShape t;
+    t.tx = tx;
+    t.ty = ty;
+    for (int k = 0; k < 3; ++k) t.m[k] = ((1u << 21) + (unsigned)(tx + k) - 1) / (unsigned)(tx + k);
+    return t;
+}
+
+// The MUSCL-Hancock tile: of the even widths (a TMA copy starts on 16 bytes) and heights that fit a CTA's
+// shared memory, the one whose tiles take the least time by the model below -- the rounds of a CTA's
+// 14 warps over the tile's predictor cells, faces and cells, at their measured instruction counts,
+// times the waves of the 2 x sms resident CTAs.  A mesh of many tiles gets the shape with the fewest
+// wasted lanes and halo items (32 x 19); a small one a shape that fills the GPU once: 256^2 in 32 x 19
+// tiles would leave 44 of 152 SMs without work.
+TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms) {
+    if (scheme == 0) return tile_shape(kGoTX, kGoTY);
+    constexpr int W = kMhNT / 32;
+    auto warps = [](int items) { return (items + 31) / 32; };
+    auto rounds = [](int w) { return (w + W - 1) / W; };
+    double best = 0.0;
+    int bx = 32, by = 19;
+    for (int tx = 8; tx <= 64; tx += 2)
+        for (int ty = 2; ty <= 32; ++ty) {
+            if (mh_tile_doubles(tx, ty) > kMhDoubles) continue;
+            long long n = 0;
+            for (int b = 0; b < nb; ++b) n += (long long)((nx[b] + tx - 1) / tx) * ((ny[b] + ty - 1) / ty);
+            const double tile = 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) +
+                                2200.0 * rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))) +
+                                800.0 * rounds(warps(tx * ty)) + 600.0;
+            const long long rest = n % (2 * sms);
+            // one CTA alone on its SM runs faster than beside a second one, but not twice as fast
+            const double waves = (double)(n / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
+            if (best == 0.0 || tile * waves < best) {
+                best = tile * waves;
+                bx = tx;
+                by = ty;
+            }
+        }
+    return tile_shape(bx, by);
 }
 
 void step_plan_tiles(StepPlan& plan, int b, int nx, int ny) {
-    plan.tiles_x[b] = (nx + kMhTX - 1) / kMhTX;
-    plan.tile_start[b + 1] = plan.tile_start[b] + plan.tiles_x[b] * ((ny + kMhTY - 1) / kMhTY);
+    plan.tiles_x[b] = (nx + plan.tile.tx - 1) / plan.tile.tx;
+    plan.tile_start[b + 1] = plan.tile_start[b] + plan.tiles_x[b] * ((ny + plan.tile.ty - 1) / plan.tile.ty);
 }
 
 // CTAs of the all-blocks launch: as many as are resident at once (the grid barrier needs every
@@ -794,8 +799,8 @@ static int g_step_grid[2][64];
 
 template <int LIM>
 static cudaError_t launch_mh_step_lim(Ctrl* c, const MeshDev* m, const StepPlan& plan, cudaStream_t s) {
-    auto k = mh_step_kernel<kMhTX, kMhTY, LIM, kMhNT>;
-    const size_t smem = MhLayout<kMhTX, kMhTY>::BYTES;
+    auto k = mh_step_kernel<LIM>;
+    const size_t smem = kMhBytes;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -827,21 +832,11 @@ cudaError_t launch_mh_step(Ctrl* c, const MeshDev* m, const StepPlan& plan, int 
 }
 
 cudaError_t stencil_prepare() {
-    cudaError_t e;
-    e = cudaFuncSetAttribute(mh_step_kernel<kMhTX, kMhTY, 0, kMhNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)MhLayout<kMhTX, kMhTY>::BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(mh_step_kernel<kMhTX, kMhTY, 1, kMhNT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)MhLayout<kMhTX, kMhTY>::BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(mh_kernel<kMhTX, kMhTY, 0, kMhNT>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)MhLayout<kMhTX, kMhTY>::BYTES);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(mh_kernel<kMhTX, kMhTY, 1, kMhNT>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)MhLayout<kMhTX, kMhTY>::BYTES);
-    if (e != cudaSuccess) return e;
+    for (const void* k : {(const void*)mh_step_kernel<0>, (const void*)mh_step_kernel<1>, (const void*)mh_kernel<0>,
+                          (const void*)mh_kernel<1>}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMhBytes);
+        if (e != cudaSuccess) return e;
+    }
     return cudaFuncSetAttribute(godunov_kernel<kGoTX, kGoTY, kGoNT>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)GoLayout<kGoTX, kGoTY>::BYTES);
@@ -925,20 +920,16 @@ cudaError_t launch_finalize(Ctrl* c, cudaStream_t s) {
 }
 
 cudaError_t launch_stencil(Ctrl* c, const MeshDev* m, int b, int nx, int ny, int scheme, int limiter,
-                           const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s, double* hout) {
-    if (scheme == 0) {
-        int tiles = ((nx + kGoTX - 1) / kGoTX) * ((ny + kGoTY - 1) / kGoTY);
+                           const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
+                           double* hout) {
+    const int tiles = ((nx + tile.tx - 1) / tile.tx) * ((ny + tile.ty - 1) / tile.ty);
+    if (scheme == 0)
         godunov_kernel<kGoTX, kGoTY, kGoNT>
             <<<tiles, kGoNT, GoLayout<kGoTX, kGoTY>::BYTES, s>>>(c, m, b, *tm0, *tm1, hout);
-    } else {
-        int tiles = ((nx + kMhTX - 1) / kMhTX) * ((ny + kMhTY - 1) / kMhTY);
-        if (limiter == 0)
-            mh_kernel<kMhTX, kMhTY, 0, kMhNT>
-                <<<tiles, kMhNT, MhLayout<kMhTX, kMhTY>::BYTES, s>>>(c, m, b, *tm0, *tm1, hout);
-        else
-            mh_kernel<kMhTX, kMhTY, 1, kMhNT>
-                <<<tiles, kMhNT, MhLayout<kMhTX, kMhTY>::BYTES, s>>>(c, m, b, *tm0, *tm1, hout);
-    }
+    else if (limiter == 0)
+        mh_kernel<0><<<tiles, kMhNT, kMhBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
+    else
+        mh_kernel<1><<<tiles, kMhNT, kMhBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
     return cudaGetLastError();
 }
 

@@ -56,9 +56,15 @@ struct FrameRing {
     long long off[HF_MAXB];
 };
 
-struct StencilTiles {
-    int box_x, box_y;   // the stencil's TMA box per variable plane (tile + halo)
+// The tile a stencil CTA updates: tx x ty cells (its TMA box adds the halo), and the multipliers that
+// give an item's row: 2^21 / (tx + k) rounded up, exact for the items of any tile that fits a CTA.
+struct TileShape {
+    int tx, ty;
+    unsigned int m[3];
 };
+TileShape tile_shape(int tx, int ty);
+// the tile for a mesh of nb blocks of nx x ny cells under the scheme, on a GPU of sms SMs
+TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms);
 
 // launchers (all asynchronous on `s`)
 // The ghost fill of every block in one launch from the fill program (m->fill), written into the
@@ -90,7 +96,7 @@ cudaError_t launch_frame_copy(Ctrl* c, const MeshDev* m, const FrameRing& ring, 
 // hout (optional): host memory the GPU maps, [4][total_y][total_x]; the stencil also stores its
 // updated interior cells there
 cudaError_t launch_stencil(Ctrl* c, const MeshDev* m, int b, int nx, int ny, int scheme, int limiter,
-                           const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
+                           const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
                            double* hout = nullptr);
 // host-buffer steps over mapped host memory: block b's state [4][total_y][total_x] into both
 // buffers with the interior TimeStep terms (int_s[parity][b] zeroed before), and, after the
@@ -107,11 +113,12 @@ constexpr int kStepMaxBlocks = 4;
 struct StepPlan {
     CUtensorMap tm[kStepMaxBlocks][2];   // per block, per state parity
     double* hout[kStepMaxBlocks];        // host-buffer stores of the updated cells, or null
+    TileShape tile;
     int tiles_x[kStepMaxBlocks];
     int tile_start[kStepMaxBlocks + 1];  // prefix sums of the blocks' tile counts
     int nb;
 };
-// the tile grid of block b (nx x ny interior cells) in the plan
+// the tile grid of block b (nx x ny interior cells) in the plan (plan.tile set)
 void step_plan_tiles(StepPlan& plan, int b, int nx, int ny);
 cudaError_t launch_mh_step(Ctrl* c, const MeshDev* m, const StepPlan& plan, int limiter, cudaStream_t s);
 
@@ -121,8 +128,6 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn tensor_map_encoder();
 
-// TMA box of the stencil for the scheme
-StencilTiles stencil_tiles(int scheme);
 cudaError_t stencil_prepare();   // sets the large dynamic shared-memory opt-ins once
 
 // geometry of one block as the initial condition needs it

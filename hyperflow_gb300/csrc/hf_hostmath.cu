@@ -5,6 +5,7 @@
 #include <cstdint>
 
 #include "hf_device.cuh"
+#include "hf_fast.cuh"
 
 extern "C" {
 
@@ -42,6 +43,40 @@ int hm_compare(double a, double b, double* out) {
 
 void hm_wave_terms(double gamma, const double* u, double* s2) {
     hf::wave_terms(gamma, gamma - 1.0, u[0], u[1], u[2], u[3], s2[0], s2[1]);
+}
+
+// The straight-through functions of hf_fast.cuh and the general ones on the same n items: c [n][3][4] the
+// states around a cell (normal, tangential order), each item along x (y = 0) or y.  ok[k] is 1 where the
+// item stayed in the window; fast and any get [n][8] evolved states.
+void hm_predict(int lim, int y, const double* c, double g1, double h, int64_t n, int* ok, double* fast, double* any) {
+    for (int64_t k = 0; k < n; ++k) {
+        const double* a = c + 12 * k;
+        double *f = fast + 8 * k, *s = any + 8 * k;
+        if (lim == 0) {
+            ok[k] = hf::predict_fast<0>(y != 0, a, a + 4, a + 8, g1, h, f, f + 4);
+            hf::predict_any<0>(y != 0, a, a + 4, a + 8, g1, h, s, s + 4);
+        } else {
+            ok[k] = hf::predict_fast<1>(y != 0, a, a + 4, a + 8, g1, h, f, f + 4);
+            hf::predict_any<1>(y != 0, a, a + 4, a + 8, g1, h, s, s + 4);
+        }
+    }
+}
+
+// the face between c[k][0] and c[k][2]; [n][4] fluxes (normal, tangential order), bad: zero-flux fallbacks
+void hm_face(int y, const double* c, double g, double g1, int64_t n, int* ok, int* bad, double* fast, double* any) {
+    for (int64_t k = 0; k < n; ++k) {
+        ok[k] = hf::hllc_fast(y != 0, g, g1, c + 12 * k, c + 12 * k + 8, fast + 4 * k);
+        bad[k] = hf::hllc_any(y != 0, g, g1, c + 12 * k, c + 12 * k + 8, any + 4 * k);
+    }
+}
+
+// the update of c[k][1] with c[k][0] and c[k][2] as the flux differences
+void hm_update(const double* c, double dt, double one_dx, double one_dy, int64_t n, int* ok, double* fast, double* any) {
+    for (int64_t k = 0; k < n; ++k) {
+        const double* a = c + 12 * k;
+        ok[k] = hf::update_fast(a, a + 8, a + 4, dt, one_dx, one_dy, fast + 4 * k);
+        for (int v = 0; v < 4; ++v) any[4 * k + v] = hf::update_any(a[v], a[8 + v], a[4 + v], dt, one_dx, one_dy);
+    }
 }
 
 }  // extern "C"

@@ -162,6 +162,14 @@ HF_HD uint32_t umulhi32(uint32_t a, uint32_t b) {
     return (uint32_t)(((uint64_t)a * b) >> 32);
 #endif
 }
+// the upper word of (hi:lo) << s, s in 1..31
+HF_HD uint32_t fshl32(uint32_t hi, uint32_t lo, uint32_t s) {
+#ifdef __CUDA_ARCH__
+    return __funnelshift_l(lo, hi, s);
+#else
+    return (hi << s) | (lo >> (32 - s));
+#endif
+}
 // a b modulo 2^64 for a 32-bit a and a 64-bit b
 HF_HD uint64_t mul_low(uint32_t a, uint64_t b) {
     const uint64_t l = wide(a, lo32(b));
@@ -245,10 +253,8 @@ static __host__ __device__ __noinline__ double div_rn(double a, double b) {
 // the exact remainder of the 54-bit root decides that 1, and its lowest bit the rounding (a
 // square root is never a halfway case).  Zero, negative, subnormal, infinite and NaN arguments go
 // to the hardware sqrt.  Out of line, as div_rn.
-static __host__ __device__ __noinline__ double sqrt_rn(double x) {
-    const uint64_t A = f64_bits(x);
+HF_HD double root32(uint64_t A) {   // A normal and positive
     const uint32_t h = hi32(A);
-    if (h - kOneHi >= 0x7FE00000u) return hw_sqrt(x);
     const bool odd = (h & kOneHi) == 0;   // an odd exponent: the mantissa doubled
     uint64_t z = u64_of((h & kMantHi) | kOneHi, lo32(A)) << 10;
     if (odd) z += z;
@@ -264,6 +270,11 @@ static __host__ __device__ __noinline__ double sqrt_rn(double x) {
     const uint64_t r2 = u64_of((lo32(z) << 12) - hi32(sq) - 2u * lo32(s) * hi32(s), 0u) - lo32(sq);
     s = (s + (r2 > s + s ? 2u : 1u)) >> 1;
     return f64_from(u64_of(hi32(s) + (((h >> 20) + 1021u) >> 1 << 20), lo32(s)));
+}
+static __host__ __device__ __noinline__ double sqrt_rn(double x) {
+    const uint64_t A = f64_bits(x);
+    if (hi32(A) - kOneHi >= 0x7FE00000u) return hw_sqrt(x);
+    return root32(A);
 }
 
 }  // namespace hf
