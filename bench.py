@@ -650,9 +650,8 @@ def main():
     achieved = BYTES_PER_CELL * cells * args.steps / (stencil_ms / 1e3) / 1e9
     traffic = None
     tr = ncu_traffic()
-    tiles = sum(-(-b["x_cells"] // 32) * -(-b["y_cells"] // 12) for b in case["mesh"]["blocks"])
-    all_blocks = (args.scheme == "MUSCLHancock" and nb <= 4 and not args.per_block_launches
-                  and (nb > 1 or tiles >= 1024))
+    all_blocks = nb <= 4 and not args.per_block_launches
+    all_mh = args.scheme == "MUSCLHancock"
     per_launch = 1 if all_blocks else nb           # stencil launches per step
     if tr and tr.get("workload") == workload_name(args):
         traffic = tr["dram_bytes_per_cell_update"] * cells / per_launch
@@ -692,9 +691,10 @@ def main():
     if rank == 0 and ws == 1 and args.workload == "ffs" and args.cpu_seconds > 0:
         cpu_ref = reference_cpu_baseline(args.limiter)
 
-    # step start, the ghost fill + ghost CFL + dt, the stencils (one launch for every block of a
-    # MUSCL-Hancock mesh of up to 4 blocks, else one per block), finalize
-    launches_per_step = 3 + per_launch
+    # the ghost fill + ghost CFL + dt, then one launch for every block of a mesh of up to 4 blocks (with
+    # MUSCL-Hancock one more for each block but the first, which re-runs it where its predictor dt
+    # changed), else one per block and the step's end
+    launches_per_step = (2 + (nb - 1 if all_mh else 0)) if all_blocks else 2 + nb
     if rank == 0:
         line = {
             "metric": "Mcell-updates/s", "value": value, "unit": "Mcell-updates/s",

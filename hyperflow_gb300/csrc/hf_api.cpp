@@ -68,7 +68,9 @@ struct hf_ctx {
     hf::Ctrl* dctrl = nullptr;
     hf::TileShape tile{};       // the stencils' tile, for the whole mesh
     CUtensorMap tmap[HF_MAXB][2];
-    hf::StepPlan plan{};        // the all-blocks MUSCL-Hancock launch (plan.nb = 0: not usable)
+    hf::StepPlan plan{};        // the all-blocks launch (plan.nb = 0: not usable)
+    hf::StepState* dstep = nullptr;
+    bool clean = false;         // the step's accumulators are cleared (by the end of the last step)
     bool block_launches = false;   // hf_set_block_launches: one stencil launch per block instead
     std::vector<double*> allocs;
     double* pinned = nullptr;   // staging for layout conversion
@@ -430,18 +432,12 @@ int build_fill_program(hf_ctx* ctx, std::vector<hf::FillOp>& ops) {
     return HF_OK;
 }
 
-// every block of a MUSCL-Hancock step in one launch, where the mesh has few enough blocks
-bool step_kernel(const hf_ctx* ctx) { return ctx->scheme == 1 && ctx->plan.nb > 0 && !ctx->block_launches; }
-
-// The all-blocks launch pays a grid barrier per block and the start-up of every resident CTA; a
-// mesh of one block gains nothing from it unless the block fills many waves (measured: a 264^2
-// block 341 Mcell-updates/s against 448 with one launch per block, 1010^2 999 against 986, 4096^2
-// 1173 against 1163).
-constexpr long long kStepMinCellsOneBlock = 393216;
+// every block of a step in one launch, where the mesh has few enough blocks
+bool step_kernel(const hf_ctx* ctx) { return ctx->plan.nb > 0 && !ctx->block_launches; }
 
 void make_plan(hf_ctx* ctx) {
     ctx->plan = hf::StepPlan{};
-    if (ctx->scheme != 1 || ctx->nblocks > hf::kStepMaxBlocks) return;
+    if (ctx->nblocks > hf::kStepMaxBlocks) return;
     hf::StepPlan plan{};
     plan.tile = ctx->tile;
     for (int b = 0; b < ctx->nblocks; ++b) {
@@ -450,7 +446,6 @@ void make_plan(hf_ctx* ctx) {
         hf::step_plan_tiles(plan, b, ctx->blocks[b].nx, ctx->blocks[b].ny);
     }
     plan.nb = ctx->nblocks;
-    if (ctx->nblocks == 1 && (long long)ctx->blocks[0].nx * ctx->blocks[0].ny < kStepMinCellsOneBlock) return;
     ctx->plan = plan;
 }
 
@@ -511,29 +506,45 @@ void ev_record(hf_ctx* ctx, int kind, bool start) {
     }
 }
 
-// one step's kernels after the ghost fill: dt, then every block, then finalize
+// the block updates of a step, in one launch or one per block; hout: host buffers that also take the
+// updated cells, or null.  With frames off the one launch ends the step too.
+int enqueue_blocks(hf_ctx* ctx, double* const* hout) {
+    hf::TraceRange trace_("block stencils");
+    if (step_kernel(ctx)) {
+        hf::StepPlan plan = ctx->plan;
+        plan.finish = ctx->ring_slots == 0;
+        for (int b = 0; b < ctx->nblocks; ++b) plan.hout[b] = hout ? hout[b] : nullptr;
+        CK(hf::launch_step(ctx->dctrl, ctx->dmesh, ctx->dstep, plan, ctx->scheme, ctx->limiter, ctx->stream));
+        return HF_OK;
+    }
+    for (int b = 0; b < ctx->nblocks; ++b)
+        CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].nx, ctx->blocks[b].ny, ctx->scheme,
+                              ctx->limiter, ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream,
+                              hout ? hout[b] : nullptr));
+    return HF_OK;
+}
+
+// the accumulators of the next step cleared, where the last step did not end normally before it
+int ensure_clean(hf_ctx* ctx) {
+    if (!ctx->clean) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
+    ctx->clean = true;
+    return HF_OK;
+}
+
+// A step's kernels from its ghost fill on (ensure_clean before): fill and dt, every block, the end of the
+// step.  The two launches of a step of one block were four: its start and its end were kernels of one thread.
 int enqueue_step(hf_ctx* ctx, bool profiled) {
     if (profiled) ev_record(ctx, 1, true);
     {
         hf::TraceRange trace_("ghost fill + dt");
-        CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-        CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
+        CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 1, ctx->dstep));
     }
     if (profiled) { ev_record(ctx, 1, false); ev_record(ctx, 0, true); }
-    {
-        hf::TraceRange trace_("block stencils");
-        if (step_kernel(ctx)) {
-            CK(hf::launch_mh_step(ctx->dctrl, ctx->dmesh, ctx->plan, ctx->limiter, ctx->stream));
-        } else {
-            for (int b = 0; b < ctx->nblocks; ++b)
-                CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].nx, ctx->blocks[b].ny,
-                                      ctx->scheme, ctx->limiter, ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1],
-                                      ctx->stream));
-        }
-    }
+    int r = enqueue_blocks(ctx, nullptr);
+    if (r != HF_OK) return r;
     if (profiled) ev_record(ctx, 0, false);
     if (ctx->ring_slots > 0) CK(hf::launch_frame_copy(ctx->dctrl, ctx->dmesh, ctx->ring, ctx->stream));
-    CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
+    if (ctx->ring_slots > 0 || !step_kernel(ctx)) CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
     ctx->step_started = ctx->ghost_fresh = false;
     return HF_OK;
 }
@@ -648,6 +659,8 @@ int hf_create(const char* case_json, size_t len, hf_ctx** out) {
     C.t_end = ctx->t_end;
     C.first_bad = ~0ull;
     C.first_nonpos = ~0ull;
+    CK(cudaMalloc(&ctx->dstep, sizeof(hf::StepState)));
+    CK(cudaMemsetAsync(ctx->dstep, 0, sizeof(hf::StepState), ctx->stream));
     CK(cudaMalloc(&ctx->dctrl, sizeof(hf::Ctrl)));
     CK(cudaMemcpyAsync(ctx->dctrl, &C, sizeof C, cudaMemcpyHostToDevice, ctx->stream));
     {
@@ -691,6 +704,7 @@ void hf_destroy(hf_ctx* ctx) {
     if (ctx->coarse) cudaFree(ctx->coarse);
     if (ctx->dmesh) cudaFree(ctx->dmesh);
     if (ctx->dctrl) cudaFree(ctx->dctrl);
+    if (ctx->dstep) cudaFree(ctx->dstep);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (int b = 0; b < HF_MAXB; ++b)
@@ -777,6 +791,7 @@ int hf_apply_bcs(hf_ctx* ctx) {
     hf::TraceRange trace_("hf_apply_bcs");
     if (!ctx) return HF_ERR_ARG;
     if (ctx->next_block != 0) return fail(ctx, HF_ERR_STATE, "apply_bcs in the middle of a step");
+    ctx->clean = false;
     CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
     CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 0));
     CK(hf::launch_ghost_mirror(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
@@ -792,6 +807,7 @@ int hf_time_step(hf_ctx* ctx, double* dt) {
     if (r != HF_OK) return r;
     // a step's accumulators start from zero whether or not the ghost fill ran on the device
     // (a caller that fills the ghosts on the host uploads them and calls this directly)
+    ctx->clean = false;
     CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
     CK(hf::launch_ghost_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
     ctx->step_started = true;
@@ -810,6 +826,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
     if (b == 0) {
         // a caller that gives dt itself may have skipped hf_time_step: start the step, and give
         // the MUSCL-Hancock predictor's TimeStep call the ghost maxima of the current fields
+        ctx->clean = false;
         if (!ctx->step_started) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
         if (ctx->scheme == 1 && !ctx->ghost_fresh)
             CK(hf::launch_ghost_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 0));
@@ -821,6 +838,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
         ctx->next_block = 0;
         ctx->step_started = ctx->ghost_fresh = false;
+        ctx->clean = true;
     } else {
         ctx->next_block = b + 1;
     }
@@ -913,24 +931,15 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
             CK(hf::launch_upload(ctx->dctrl, ctx->dmesh, b, B.tx, B.ty, p, in[b], ctx->stream));
         }
         int r = set_clamp(ctx, 0);
+        if (r == HF_OK) r = ensure_clean(ctx);
         if (r != HF_OK) return r;
-        CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-        CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
+        CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 1, ctx->dstep));
         for (int b = 0; b < ctx->nblocks; ++b)
             CK(hf::launch_ghost_store(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].tx, ctx->blocks[b].ny, ctx->ghost,
                                       p, out[b], ctx->stream));
-        if (step_kernel(ctx)) {
-            hf::StepPlan plan = ctx->plan;
-            for (int b = 0; b < ctx->nblocks; ++b) plan.hout[b] = out[b];
-            CK(hf::launch_mh_step(ctx->dctrl, ctx->dmesh, plan, ctx->limiter, ctx->stream));
-        } else {
-            for (int b = 0; b < ctx->nblocks; ++b) {
-                const BlockHost& B = ctx->blocks[b];
-                CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, B.nx, B.ny, ctx->scheme, ctx->limiter,
-                                      ctx->tile, &ctx->tmap[b][0], &ctx->tmap[b][1], ctx->stream, out[b]));
-            }
-        }
-        CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
+        r = enqueue_blocks(ctx, out);
+        if (r != HF_OK) return r;
+        if (ctx->ring_slots > 0 || !step_kernel(ctx)) CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
         ctx->step_started = ctx->ghost_fresh = false;
         if (dt) CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
@@ -947,9 +956,9 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
         CK(hf::launch_interior_cfl(ctx->dctrl, ctx->dmesh, b, B.nx, B.ny, p, ctx->stream));
     }
     int r = set_clamp(ctx, 0);
+    if (r == HF_OK) r = ensure_clean(ctx);
     if (r != HF_OK) return r;
-    CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-    CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
+    CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 1, ctx->dstep));
     for (int b = 0; b < ctx->nblocks; ++b) {
         const BlockHost& B = ctx->blocks[b];
         CK(hf::launch_stencil(ctx->dctrl, ctx->dmesh, b, B.nx, B.ny, ctx->scheme, ctx->limiter,
@@ -972,6 +981,7 @@ int hf_step(hf_ctx* ctx, double* dt) {
     if (!ctx) return HF_ERR_ARG;
     if (ctx->next_block != 0) return fail(ctx, HF_ERR_STATE, "step in the middle of a step");
     int r = set_clamp(ctx, 0);
+    if (r == HF_OK) r = ensure_clean(ctx);
     if (r != HF_OK) return r;
     r = enqueue_step(ctx, ctx->profile);
     if (r != HF_OK) return r;
@@ -990,6 +1000,7 @@ int hf_run(hf_ctx* ctx, int64_t n, int clamp_t_end, int use_graph, int64_t* step
     long long s0 = steps_done ? read_step(ctx) : 0;
     int clamp = clamp_t_end ? 1 : 0;
     int r = set_clamp(ctx, clamp);
+    if (r == HF_OK) r = ensure_clean(ctx);
     if (r != HF_OK) return r;
     if (use_graph && !ctx->profile) {
         if (!ctx->graph[clamp]) {
@@ -1295,7 +1306,7 @@ int hf_checkpoint_load(hf_ctx* ctx, const void* buf, size_t bytes) {
     C.err = 0;
     C.strict = cur.strict;
     ctx->drained = 0;
-    ctx->step_started = ctx->ghost_fresh = false;
+    ctx->step_started = ctx->ghost_fresh = ctx->clean = false;
     for (int b = 0; b < ctx->nblocks; ++b)
         for (int k = 0; k < 2; ++k) {
             size_t n = (size_t)4 * ctx->blocks[b].ty * ctx->blocks[b].pitch * sizeof(double);

@@ -23,25 +23,33 @@ namespace hf {
 
 constexpr unsigned kWaitLimit = 1u << 22;   // bounded mbarrier polls before giving up
 
-// start of a step: stop at t_end (device loop), clear this step's accumulators
-__global__ void step_begin_kernel(Ctrl* __restrict__ c) {
-    const int p = (int)(c->step & 1);
-    int done = c->clamp && (c->t == c->t_end);
-    if (c->strict && (c->first_bad != ~0ull || c->first_nonpos != ~0ull)) done = 1;   // strict mode
-    // a step takes at most two frames: pause the loop while the ring lacks room for them
-    if (c->clamp && c->frames && c->captured - c->drained > c->ring_slots - 2) done = 1;
-    c->done = done;
-    c->snap_pre = c->snap_post = 0;
-    if (done) return;
-    for (int b = 0; b < HF_MAXB; ++b) {
+// stop the device loop before this step?  At t_end; in strict mode once a failure is recorded; while the
+// frame ring lacks room for the two frames a step takes at most.
+__device__ __forceinline__ bool loop_done(const Ctrl* c) {
+    if (c->clamp && c->t == c->t_end) return true;
+    if (c->strict && (c->first_bad != ~0ull || c->first_nonpos != ~0ull)) return true;
+    return c->clamp && c->frames && c->captured - c->drained > c->ring_slots - 2;
+}
+
+// the accumulators of a step whose starting state has parity p, cleared
+__device__ void clear_step(Ctrl* __restrict__ c, int p) {
+    for (int b = 0; b < c->nblocks; ++b) {
         c->ghost_s[b][0] = c->ghost_s[b][1] = 0ull;
         c->int_s[p ^ 1][b][0] = c->int_s[p ^ 1][b][1] = 0ull;
         c->step_hllc[b] = 0;
         c->step_bad[b] = c->step_nonpos[b] = ~0ull;
     }
     c->ticket = 0u;
-    c->tile_ctr = 0u;
-    c->bar_count = 0u;
+}
+
+// Start of a step that no finished step prepared (after an upload, a restore, a ghost fill on its own): its
+// stop flag, and its accumulators cleared.  A finished step clears the next one's itself (finish_step) and
+// the fill takes the stop flag, so a loop's steps need no launch for this.
+__global__ void step_begin_kernel(Ctrl* __restrict__ c) {
+    const int done = loop_done(c);
+    c->done = done;
+    c->snap_pre = c->snap_post = 0;
+    if (!done) clear_step(c, (int)(c->step & 1));
 }
 
 // ------------------------------------------------------------------------------------
@@ -64,7 +72,23 @@ __device__ __forceinline__ void ghost_cell_ij(const BlockDev& B, int g, long lon
 
 constexpr int kRedThreads = 256;
 
-__device__ void form_step_dt(Ctrl* __restrict__ c, int p);
+__device__ void form_step_dt(Ctrl* __restrict__ c, int p, StepState* __restrict__ ss);
+
+// block b's dx / max(|u| + c) and dy / max(|v| + c), ghost cells and the interior of parity p, read past L1
+__device__ __forceinline__ void block_dt(const Ctrl* c, int b, int p, double& dtx, double& dty) {
+    const volatile Ctrl* vc = c;
+    dtx = div_rn(c->dx[b], smax(bitsd(vc->ghost_s[b][0]), bitsd(vc->int_s[p][b][0])));
+    dty = div_rn(c->dy[b], smax(bitsd(vc->ghost_s[b][1]), bitsd(vc->int_s[p][b][1])));
+}
+
+// the predictor scalars of block b from its predictor dt (muscl_hancock.cpp:248-249, 352-353)
+__device__ __forceinline__ void step_scalars(const Ctrl* c, StepState* ss, int b, double dtp) {
+    ss->sc[b][0] = div_rn(0.5 * dtp, c->dx[b]);
+    ss->sc[b][1] = div_rn(0.5 * dtp, c->dy[b]);
+    ss->sc[b][2] = div_rn(1.0, c->dx[b]);
+    ss->sc[b][3] = div_rn(1.0, c->dy[b]);
+    ss->sc[b][4] = dtp;
+}
 
 // form_dt = 0: the ghost maxima only (for a predictor TimeStep in a step whose dt the caller gave)
 __global__ void __launch_bounds__(kRedThreads) ghost_cfl_kernel(Ctrl* __restrict__ c,
@@ -92,37 +116,61 @@ __global__ void __launch_bounds__(kRedThreads) ghost_cfl_kernel(Ctrl* __restrict
         block_max2_atomic<kRedThreads>(mx, my, &c->ghost_s[b][0], &c->ghost_s[b][1]);
         __syncthreads();
     }
-    if (form_dt) form_step_dt(c, p);
+    if (form_dt) form_step_dt(c, p, nullptr);
 }
 
 // The last CTA of a ghost-maxima launch to finish forms the step's dt: TimeStep call number
 // `calls` over every block (timestep.cpp:29-68), then Simulation::solve's clamps and frame points.
-__device__ void form_step_dt(Ctrl* __restrict__ c, int p) {
+// With ss, also the all-blocks launch's scalars: each block's predictor dt from the same maxima (the
+// predictor's TimeStep call, muscl_hancock.cpp:246-249, over the step's starting state).  A block per
+// thread: the quotients take about 300 cycles each, one after the other on one thread more than the fill.
+__device__ void form_step_dt(Ctrl* __restrict__ c, int p, StepState* __restrict__ ss) {
     __shared__ bool last;
+    __shared__ double s_dt[HF_MAXB][2], s_min;
     __threadfence();
     if (threadIdx.x == 0) last = (atomicAdd(&c->ticket, 1u) == gridDim.x - 1);
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
+    if (!last) return;
     __threadfence();
-    volatile Ctrl* vc = c;
-    long long call = vc->calls;
-    double dt = cfl_dt_fresh(c, call, 0, p, p);
-    c->dt_cfl = dt;
-    const double t = c->t;
-    if (c->clamp && t + dt > c->t_end) dt = c->t_end - t;        // simulation.cpp:88-90
-    if (c->clamp && c->frames) {
-        const double cur = c->frame_next;
-        c->snap_pre = (cur == 0.0);                              // simulation.cpp:93-96
-        if ((t + dt > cur) && (cur > 0.0)) dt = cur - t;         // simulation.cpp:98-102
-        if (fabs(t - cur) < 1e-12) {                             // simulation.cpp:106-113
-            c->snap_post = 1;
-            c->frame_next = cur + c->frame_interval;
+    const int nb = c->nblocks;
+    const long long call = c->calls;
+    const double cfl = c->cfl;
+    if ((int)threadIdx.x < nb) block_dt(c, threadIdx.x, p, s_dt[threadIdx.x][0], s_dt[threadIdx.x][1]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double dtx = 1e16, dty = 1e16;
+        for (int b = 0; b < nb; ++b) {
+            dtx = smin(dtx, s_dt[b][0]);
+            dty = smin(dty, s_dt[b][1]);
         }
-        c->snap_t = t;
+        s_min = smin(dtx, dty);
+        double dt = ((call + 1 <= 10) ? 0.2 * cfl : cfl) * s_min;
+        c->dt_cfl = dt;
+        const double t = c->t;
+        c->snap_pre = c->snap_post = 0;
+        if (c->clamp && t + dt > c->t_end) dt = c->t_end - t;        // simulation.cpp:88-90
+        if (c->clamp && c->frames) {
+            const double cur = c->frame_next;
+            c->snap_pre = (cur == 0.0);                              // simulation.cpp:93-96
+            if ((t + dt > cur) && (cur > 0.0)) dt = cur - t;         // simulation.cpp:98-102
+            if (fabs(t - cur) < 1e-12) {                             // simulation.cpp:106-113
+                c->snap_post = 1;
+                c->frame_next = cur + c->frame_interval;
+            }
+            c->snap_t = t;
+        }
+        c->dt = dt;
+        c->done = 0;
+        c->calls = call + 1;
+        c->ticket = 0u;
     }
-    c->dt = dt;
-    c->calls = call + 1;
-    c->ticket = 0u;
+    if (!ss) return;
+    __syncthreads();
+    if ((int)threadIdx.x < nb) {
+        const int b = threadIdx.x;
+        const double dtp = ((call + 1 + b + 1 <= 10) ? 0.2 * cfl : cfl) * s_min;
+        step_scalars(c, ss, b, dtp);
+    }
 }
 
 // the block of ghost cell k of the all-blocks enumeration
@@ -136,10 +184,17 @@ __device__ __forceinline__ int ghost_block(const MeshDev* __restrict__ m, long l
 // value from the fill program (a copy of one cell's pre-fill value or of a Dirichlet side's state,
 // with the reflective sides' negations: transmissive_boundary.cpp, reflective_boundary.cpp,
 // dirichlet_boundary.cpp, internal_boundary.cpp replayed in the reference's order on the host),
-// then its TimeStep terms feed the block's ghost maxima.
+// then its TimeStep terms feed the block's ghost maxima.  With ss (a step of the loop) the stop flag is
+// taken here: nothing it depends on changes before the last CTA forms the dt.
 __global__ void __launch_bounds__(kRedThreads) fill_cfl_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                                               int form_dt) {
-    if (c->done) return;
+                                                               int form_dt, StepState* __restrict__ ss) {
+    if (ss ? loop_done(c) : c->done != 0) {
+        if (ss && blockIdx.x == 0 && threadIdx.x == 0) {
+            c->done = 1;
+            c->snap_pre = c->snap_post = 0;
+        }
+        return;
+    }
     const int p = (int)(c->step & 1);
     const double g = c->gamma, g1 = c->g1;
     const int gh = m->ghost;
@@ -190,7 +245,7 @@ __global__ void __launch_bounds__(kRedThreads) fill_cfl_kernel(Ctrl* __restrict_
     for (int bb = b0; bb <= b1; ++bb)
         block_max2_atomic<kRedThreads>(b == bb ? sx : 0.0, b == bb ? sy : 0.0, &c->ghost_s[bb][0],
                                        &c->ghost_s[bb][1]);
-    if (form_dt) form_step_dt(c, p);
+    if (form_dt) form_step_dt(c, p, ss);
 }
 
 // the current buffer's ghost cells into the other buffer (after a fill no stencil follows)
@@ -331,9 +386,8 @@ __global__ void __launch_bounds__(256) frame_copy_kernel(const Ctrl* __restrict_
 }
 
 // end of step: t += dt; the MUSCL-Hancock predictor calls advance the counter; record this
-// step's frames; flip parity
-__global__ void finalize_kernel(Ctrl* c) {
-    if (c->done) return;
+// step's frames; flip parity; clear the next step's accumulators
+__device__ void finish_step(Ctrl* __restrict__ c) {
     if (c->clamp && c->frames) {
         for (int which = 0; which < 2; ++which) {
             if (which == 0 ? !c->snap_pre : !c->snap_post) continue;
@@ -346,7 +400,13 @@ __global__ void finalize_kernel(Ctrl* c) {
     }
     c->t = c->t + c->dt;
     if (c->scheme == 1) c->calls = c->calls + c->nblocks;
-    c->step = c->step + 1;
+    const long long step = c->step + 1;
+    c->step = step;
+    clear_step(c, (int)(step & 1));
+}
+
+__global__ void finalize_kernel(Ctrl* c) {
+    if (!c->done) finish_step(c);
 }
 
 // ------------------------------------------------------------------------------------
@@ -484,76 +544,81 @@ __global__ void __launch_bounds__(kMhNT, 2) mh_kernel(Ctrl* __restrict__ c, cons
 }
 
 // ------------------------------------------------------------------------------------
-// MUSCL-Hancock, every block of a step in one persistent launch
+// MUSCL-Hancock, every block of a step in one launch
 // ------------------------------------------------------------------------------------
 // The reference updates the blocks one after the other, and block b's half-step predictor takes
 // its dt from a TimeStep call over a mesh whose blocks < b are already updated
 // (muscl_hancock.cpp:246, called from simulation.cpp:106-110).  One launch per block leaves a
-// partly filled last wave of CTAs at the end of every block.  Here one cooperative launch (all
-// CTAs resident) walks the tiles of all blocks, in block order, from a shared counter, so one
-// block's tail overlaps the next block's start, and runs every block with the predictor dt of a
-// TimeStep call over the step's starting state.  For block 0 that is the reference's value.  For
-// block b > 0 it is the reference's value whenever updating blocks 0..b-1 leaves the largest wave
-// speed TimeStep sees unchanged, the usual case.  After all tiles, block by block: a grid barrier,
-// then every CTA forms block b's true predictor dt (the reference's call: blocks < b from their
-// updated state) from the same data; where its bits differ from the value used, the grid runs
-// block b again with it.  A step never writes a block's input buffer, so the second run gives
-// exactly the sequential result; a block's wave-speed maxima and numerical-failure records are
-// kept per block and folded into the totals only when every block is final, so a discarded run
-// leaves nothing behind.
-// grid-wide barrier with a bounded wait (10 s of the global timer); false after a timeout or
-// once another CTA raised the error word
-__device__ bool step_grid_barrier(Ctrl* c) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned int* gen = &c->bar_gen;
-        const unsigned int g0 = *gen;
-        __threadfence();
-        const unsigned int arrived = atomicAdd(&c->bar_count, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            c->bar_count = 0u;
-            __threadfence();
-            atomicAdd(&c->bar_gen, 1u);
-            ok = 1;
-        } else {
-            ok = 0;
-            unsigned long long t0;
-            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
-            for (;;) {
-                if (*gen != g0) { ok = 1; break; }
-                if (*(volatile int*)&c->err != 0) break;
-                unsigned long long t1;
-                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-                if (t1 - t0 > 10000000000ull) {
-                    raise_error(c, HF_DEV_TIMEOUT);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
+// partly filled last wave of CTAs at the end of every block, and its launches.  Here one launch
+// holds the tiles of all blocks, in block order, so one block's tail overlaps the next block's
+// start, and runs every block with the predictor dt of a TimeStep call over the step's starting
+// state.  For block 0 that is the reference's value.  For block b > 0 it is the reference's value
+// whenever updating blocks 0..b-1 leaves the largest wave speed TimeStep sees unchanged, the usual
+// case.  The last CTA to finish forms the true predictor dt block by block (the reference's call:
+// blocks < b from their updated state); at the first whose bits differ from the value used it
+// leaves that block to the re-run launch that follows (one for every block but the first; with
+// nothing to do it leaves at once), whose last CTA goes on from there.  A step never writes a
+// block's input buffer, so the second run gives exactly the sequential result; a block's
+// wave-speed maxima and numerical-failure records are kept per block and folded into the totals
+// only when every block is final, so a discarded run leaves nothing behind.  The CTA that finds
+// every block final also ends the step, so a step is this launch, the fill and the re-runs.
+//
+// (It was a persistent cooperative launch with a grid barrier per block, tiles from a counter:
+// 1958 Mcell-updates/s at 2048^2 where a CTA per tile gives 2062, and two launches more a step.)
+
+// the last CTA's thread 0: the next block from b on whose predictor dt was not the reference's, its
+// scalars and records made ready; the step's end when there is none.
+__device__ void settle_step(Ctrl* __restrict__ c, StepState* __restrict__ ss, int b, int finish) {
+    const int p = (int)(c->step & 1), nb = c->nblocks;
+    for (; b < nb; ++b) {
+        const double dtp = cfl_dt_fresh(c, c->calls + b, b, p, p ^ 1);
+        if (f64_bits(dtp) == f64_bits(ss->sc[b][4])) continue;
+        step_scalars(c, ss, b, dtp);
+        c->int_s[p ^ 1][b][0] = c->int_s[p ^ 1][b][1] = 0ull;   // forget the first run's records
+        c->step_hllc[b] = 0;
+        c->step_bad[b] = c->step_nonpos[b] = ~0ull;
+        c->blocks_rerun = c->blocks_rerun + 1;
+        ss->rerun = b;
+        return;
     }
-    __syncthreads();
-    return ok != 0;
+    ss->rerun = 0;
+    const volatile Ctrl* vc = c;
+    long long herr = 0;
+    for (b = 0; b < nb; ++b) {   // every block final: fold this step's records
+        herr += vc->step_hllc[b];
+        const unsigned long long fb = vc->step_bad[b], fn = vc->step_nonpos[b];
+        if (fb < c->first_bad) c->first_bad = fb;
+        if (fn < c->first_nonpos) c->first_nonpos = fn;
+        c->dt_pred[b] = ss->sc[b][4];
+    }
+    c->hllc_errors = c->hllc_errors + herr;
+    if (finish) finish_step(c);
 }
 
-// this launch's predictor scalars per block: 0.5 dtp / dx, 0.5 dtp / dy, 1 / dx, 1 / dy, and dtp
-__shared__ double s_step_sc[kStepMaxBlocks][5];
-__shared__ uint64_t s_step_bar;   // the tiles' TMA loads
+// this CTA's work is done; true in thread 0 of the last of the launch's CTAs
+__device__ __forceinline__ bool last_cta(unsigned int* ctr) {
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+    __threadfence();
+    const bool last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+    if (last) {
+        *ctr = 0u;
+        __threadfence();
+    }
+    return last;
+}
 
 // One tile of block b (local tile index `local`): its TMA load (mbarrier phase `phase`), the
-// fused fluxes with the block's predictor scalars, the update and the block's records.  False if
-// the load's bounded wait gave up.  Out of line: the tile loop and the re-run loop share one copy.
+// fused fluxes with the block's predictor scalars, the update and the block's records.
 template <int LIM>
-__device__ __noinline__ bool mh_step_tile(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                          const StepPlan& plan, int b, int local, int p, uint32_t phase) {
+__device__ __forceinline__ void mh_plan_tile(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, const StepState* ss,
+                                             const StepPlan& plan, int b, int local, uint64_t* bar, uint32_t phase) {
     extern __shared__ __align__(1024) double smem[];
+    const int p = (int)(c->step & 1);
     const MhShape S{plan.tile};
     const int tx = plan.tile.tx, ty = plan.tile.ty, usize = 4 * (tx + 4) * (ty + 4);
     double* sU = smem;
     double* sA = smem + usize;
-    uint64_t* bar = &s_step_bar;
     const BlockDev& B = m->b[b];
     const int x0 = (local % plan.tiles_x[b]) * tx, y0 = (local / plan.tiles_x[b]) * ty;
     if (threadIdx.x == 0) {
@@ -562,6 +627,7 @@ __device__ __noinline__ bool mh_step_tile(Ctrl* __restrict__ c, const MeshDev* _
         mbar_expect_tx(bar, usize * 8);
         tma_load_3d(sU, &plan.tm[b][p], bar, x0, y0, 0);
     }
+    const double hdx = ss->sc[b][0], hdy = ss->sc[b][1];
     const bool ok = mbar_wait_bounded(bar, phase, kWaitLimit);
     if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0) {
@@ -569,93 +635,50 @@ __device__ __noinline__ bool mh_step_tile(Ctrl* __restrict__ c, const MeshDev* _
             mbar_wait_bounded(bar, phase, kWaitLimit);   // let an in-flight copy land before exit
         }
         __syncthreads();
-        return false;
+        return;
     }
     const double g = c->gamma, g1 = c->g1;
     const unsigned long long key = face_key(c->step, b, 0, 0, 0);
-    const int herr = mh_tile_fluxes<kMhNT, LIM>(S, sU, sA, g, g1, s_step_sc[b][0], s_step_sc[b][1], x0, y0, B.nx, B.ny,
-                                                &c->step_bad[b], key);
+    const int herr = mh_tile_fluxes<kMhNT, LIM>(S, sU, sA, g, g1, hdx, hdy, x0, y0, B.nx, B.ny, &c->step_bad[b], key);
     double mx = 0.0, my = 0.0;
-    mh_store<kMhNT>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], plan.hout[b], c->dt, s_step_sc[b][2], s_step_sc[b][3], g, g1,
+    mh_store<kMhNT>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], plan.hout[b], c->dt, ss->sc[b][2], ss->sc[b][3], g, g1,
                     &c->step_nonpos[b], key, mx, my, &c->err);
     store_ghosts<2, kMhNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
     block_max2_atomic<kMhNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->step_hllc[b]), (unsigned long long)herr);
-    return true;
-}
-
-// the predictor scalars of block b from its predictor dt (muscl_hancock.cpp:248-249, 352-353)
-__device__ __forceinline__ void step_scalars(const Ctrl* c, int b, double dtp) {
-    s_step_sc[b][0] = div_rn(0.5 * dtp, c->dx[b]);
-    s_step_sc[b][1] = div_rn(0.5 * dtp, c->dy[b]);
-    s_step_sc[b][2] = div_rn(1.0, c->dx[b]);
-    s_step_sc[b][3] = div_rn(1.0, c->dy[b]);
-    s_step_sc[b][4] = dtp;
 }
 
 template <int LIM>
 __global__ void __launch_bounds__(kMhNT, 2) mh_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+                                                           StepState* __restrict__ ss,
                                                            const __grid_constant__ StepPlan plan) {
-    if (c->done) return;   // set before this launch: every CTA leaves, no barrier is entered
+    if (c->done) return;   // set before this launch: every CTA leaves
+    __shared__ uint64_t bar;
+    if (threadIdx.x == 0) mbar_init(&bar, 1);
+    __syncthreads();
+    int b = 0;
+    while (b + 1 < plan.nb && (int)blockIdx.x >= plan.tile_start[b + 1]) ++b;
+    mh_plan_tile<LIM>(c, m, ss, plan, b, blockIdx.x - plan.tile_start[b], &bar, 0u);
+    if (last_cta(&ss->tiles)) settle_step(c, ss, 1, plan.finish);
+}
 
-    const int p = (int)(c->step & 1);
-    const int nb = plan.nb;
-    const long long calls = c->calls;
-    __shared__ int s_tile, s_redo;
-    if (threadIdx.x == 0) {
-        for (int b = 0; b < nb; ++b) step_scalars(c, b, cfl_dt(c, calls + b, 0, p, p ^ 1));   // starting state
-        mbar_init(&s_step_bar, 1);
-    }
+// the block a launch before this one left to be run again, if any, on the resident CTAs
+template <int LIM>
+__global__ void __launch_bounds__(kMhNT, 2) mh_rerun_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+                                                            StepState* __restrict__ ss,
+                                                            const __grid_constant__ StepPlan plan) {
+    const int b = c->done ? 0 : ss->rerun;
+    if (b == 0) return;
+    __shared__ uint64_t bar;
+    if (threadIdx.x == 0) mbar_init(&bar, 1);
     __syncthreads();
     uint32_t phase = 0u;
-    const int total = plan.tile_start[nb];
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = (int)atomicAdd(&c->tile_ctr, 1u);
-        __syncthreads();
-        const int t = s_tile;
-        if (t >= total) break;
-        int b = 0;
-        while (t >= plan.tile_start[b + 1]) ++b;
-        if (!mh_step_tile<LIM>(c, m, plan, b, t - plan.tile_start[b], p, phase)) return;
+    for (int t = plan.tile_start[b] + blockIdx.x; t < plan.tile_start[b + 1]; t += gridDim.x) {
+        mh_plan_tile<LIM>(c, m, ss, plan, b, t - plan.tile_start[b], &bar, phase);
         phase ^= 1u;
+        __syncthreads();   // the tile's last reads of shared memory come before the next one's load
     }
-    for (int b = 1; b < nb; ++b) {
-        if (!step_grid_barrier(c)) return;   // blocks < b final
-        if (threadIdx.x == 0) {
-            const double dtp = cfl_dt_fresh(c, calls + b, b, p, p ^ 1);
-            s_redo = f64_bits(dtp) != f64_bits(s_step_sc[b][4]);
-            if (s_redo) {
-                step_scalars(c, b, dtp);
-                if (blockIdx.x == 0) {   // forget the first run's records of block b
-                    c->int_s[p ^ 1][b][0] = c->int_s[p ^ 1][b][1] = 0ull;
-                    c->step_hllc[b] = 0;
-                    c->step_bad[b] = c->step_nonpos[b] = ~0ull;
-                    c->blocks_rerun = c->blocks_rerun + 1;
-                }
-            }
-        }
-        __syncthreads();
-        if (!s_redo) continue;
-        if (!step_grid_barrier(c)) return;   // the cleared records are in place before the re-run
-        const int ntiles = plan.tile_start[b + 1] - plan.tile_start[b];
-        for (int local = blockIdx.x; local < ntiles; local += gridDim.x) {
-            if (!mh_step_tile<LIM>(c, m, plan, b, local, p, phase)) return;
-            phase ^= 1u;
-        }
-    }
-    if (!step_grid_barrier(c)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {   // every block final: fold this step's records
-        const volatile Ctrl* vc = c;
-        long long herr = 0;
-        for (int b = 0; b < nb; ++b) {
-            herr += vc->step_hllc[b];
-            const unsigned long long fb = vc->step_bad[b], fn = vc->step_nonpos[b];
-            if (fb < c->first_bad) c->first_bad = fb;
-            if (fn < c->first_nonpos) c->first_nonpos = fn;
-            c->dt_pred[b] = s_step_sc[b][4];
-        }
-        c->hllc_errors = c->hllc_errors + herr;
-    }
+    if (last_cta(&ss->tiles)) settle_step(c, ss, b + 1, plan.finish);
 }
 
 // ------------------------------------------------------------------------------------
@@ -677,11 +700,8 @@ struct GoLayout {
 // three 256-thread CTAs per SM (80 registers, 74 KB of shared memory with 32x10 tiles): measured
 // 3 % faster than two CTAs of 32x14 tiles at 110 registers, and than 32x8 or 32x6 tiles
 template <int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c,
-                                                     const MeshDev* __restrict__ m, int b,
-                                                     const __grid_constant__ CUtensorMap tm0,
-                                                     const __grid_constant__ CUtensorMap tm1,
-                                                     double* __restrict__ hout) {
+__device__ __forceinline__ void godunov_tile(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b, int local,
+                                             const CUtensorMap* tm, double* __restrict__ hout) {
     using L = GoLayout<TX, TY>;
     extern __shared__ __align__(1024) double smem[];
     double* sU = smem + L::U_OFF;
@@ -689,23 +709,21 @@ __global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c,
     double* sF = smem + L::F_OFF;
     double* sG = smem + L::G_OFF;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::END);
-    if (c->done) return;
 
     const BlockDev& B = m->b[b];
     const int p = (int)(c->step & 1);
     const int tiles_x = (B.nx + TX - 1) / TX;
-    const int x0 = (blockIdx.x % tiles_x) * TX, y0 = (blockIdx.x / tiles_x) * TY;
+    const int x0 = (local % tiles_x) * TX, y0 = (local / tiles_x) * TY;
     const double g = c->gamma, g1 = c->g1;
     const double dt = c->dt;
     __shared__ double sc[2];
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         mbar_expect_tx(bar, L::TMA_BYTES);
-        tma_load_3d(sU, p ? &tm1 : &tm0, bar, x0, y0, 0);
+        tma_load_3d(sU, tm, bar, x0, y0, 0);
         sc[0] = div_rn(1.0, c->dx[b]);   // godunov.cpp:97-98
         sc[1] = div_rn(1.0, c->dy[b]);
     }
-
     if (!wait_tile(bar, c)) return;
     const double one_dx = sc[0], one_dy = sc[1];
 
@@ -740,6 +758,28 @@ __global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c,
     store_ghosts<1, NT>(sU, B, TX, TY, x0, y0, out, &c->err);
     block_max2_atomic<NT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
+}
+
+// one block (hf_advance_block, meshes of many blocks)
+template <int TX, int TY, int NT>
+__global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
+                                                        const __grid_constant__ CUtensorMap tm0,
+                                                        const __grid_constant__ CUtensorMap tm1,
+                                                        double* __restrict__ hout) {
+    if (c->done) return;
+    godunov_tile<TX, TY, NT>(c, m, b, blockIdx.x, (c->step & 1) ? &tm1 : &tm0, hout);
+}
+
+// every block of a step in one launch, whose last CTA ends the step
+template <int TX, int TY, int NT>
+__global__ void __launch_bounds__(NT, 3) godunov_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+                                                             StepState* __restrict__ ss,
+                                                             const __grid_constant__ StepPlan plan) {
+    if (c->done) return;
+    int b = 0;
+    while (b + 1 < plan.nb && (int)blockIdx.x >= plan.tile_start[b + 1]) ++b;
+    godunov_tile<TX, TY, NT>(c, m, b, blockIdx.x - plan.tile_start[b], &plan.tm[b][c->step & 1], plan.hout[b]);
+    if (last_cta(&ss->tiles) && plan.finish) finish_step(c);
 }
 
 // ------------------------------------------------------------------------------------
@@ -793,50 +833,35 @@ void step_plan_tiles(StepPlan& plan, int b, int nx, int ny) {
     plan.tile_start[b + 1] = plan.tile_start[b] + plan.tiles_x[b] * ((ny + plan.tile.ty - 1) / plan.tile.ty);
 }
 
-// CTAs of the all-blocks launch: as many as are resident at once (the grid barrier needs every
-// CTA running), found once per limiter and device
-static int g_step_grid[2][64];
-
-template <int LIM>
-static cudaError_t launch_mh_step_lim(Ctrl* c, const MeshDev* m, const StepPlan& plan, cudaStream_t s) {
-    auto k = mh_step_kernel<LIM>;
-    const size_t smem = kMhBytes;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    int& grid = g_step_grid[LIM][dev];
-    if (grid == 0) {
-        int per_sm = 0, sms = 0;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kMhNT, smem)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        grid = per_sm * sms;
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kMhNT);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;   // all CTAs resident: the grid barrier is safe
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, c, m, plan);
-}
-
-cudaError_t launch_mh_step(Ctrl* c, const MeshDev* m, const StepPlan& plan, int limiter, cudaStream_t s) {
+cudaError_t launch_step(Ctrl* c, const MeshDev* m, StepState* ss, const StepPlan& plan, int scheme, int limiter,
+                        cudaStream_t s) {
     if (plan.nb < 1 || plan.nb > kStepMaxBlocks) return cudaErrorInvalidValue;
-    return limiter == 0 ? launch_mh_step_lim<0>(c, m, plan, s) : launch_mh_step_lim<1>(c, m, plan, s);
+    const int tiles = plan.tile_start[plan.nb];
+    if (scheme == 0) {
+        godunov_step_kernel<kGoTX, kGoTY, kGoNT><<<tiles, kGoNT, GoLayout<kGoTX, kGoTY>::BYTES, s>>>(c, m, ss, plan);
+        return cudaGetLastError();
+    }
+    if (limiter == 0) mh_step_kernel<0><<<tiles, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
+    else mh_step_kernel<1><<<tiles, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
+    // a block run again on a fixed grid: with nothing to do (nearly always) few CTAs come and go
+    const int again = tiles < 2 * 152 ? tiles : 2 * 152;
+    for (int b = 1; b < plan.nb; ++b) {
+        if (limiter == 0) mh_rerun_kernel<0><<<again, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
+        else mh_rerun_kernel<1><<<again, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
+    }
+    return cudaGetLastError();
 }
 
 cudaError_t stencil_prepare() {
-    for (const void* k : {(const void*)mh_step_kernel<0>, (const void*)mh_step_kernel<1>, (const void*)mh_kernel<0>,
-                          (const void*)mh_kernel<1>}) {
+    for (const void* k : {(const void*)mh_step_kernel<0>, (const void*)mh_step_kernel<1>, (const void*)mh_rerun_kernel<0>,
+                          (const void*)mh_rerun_kernel<1>, (const void*)mh_kernel<0>, (const void*)mh_kernel<1>}) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMhBytes);
         if (e != cudaSuccess) return e;
     }
+    const cudaError_t e = cudaFuncSetAttribute(godunov_step_kernel<kGoTX, kGoTY, kGoNT>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)GoLayout<kGoTX, kGoTY>::BYTES);
+    if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(godunov_kernel<kGoTX, kGoTY, kGoNT>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)GoLayout<kGoTX, kGoTY>::BYTES);
@@ -847,9 +872,10 @@ cudaError_t launch_step_begin(Ctrl* c, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_fill_cfl(Ctrl* c, const MeshDev* m, long long total_ghost, cudaStream_t s, int form_dt) {
+cudaError_t launch_fill_cfl(Ctrl* c, const MeshDev* m, long long total_ghost, cudaStream_t s, int form_dt,
+                            StepState* ss) {
     long long grid = (total_ghost + kRedThreads - 1) / kRedThreads;
-    fill_cfl_kernel<<<(unsigned)(grid < 1 ? 1 : grid), kRedThreads, 0, s>>>(c, m, form_dt);
+    fill_cfl_kernel<<<(unsigned)(grid < 1 ? 1 : grid), kRedThreads, 0, s>>>(c, m, form_dt, ss);
     return cudaGetLastError();
 }
 

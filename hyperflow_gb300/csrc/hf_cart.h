@@ -66,19 +66,29 @@ TileShape tile_shape(int tx, int ty);
 // the tile for a mesh of nb blocks of nx x ny cells under the scheme, on a GPU of sms SMs
 TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms);
 
+// What the all-blocks launch keeps between its kernels, beside the checkpointed control block.
+struct StepState {
+    double sc[HF_MAXB][5];   // per block: 0.5 dtp / dx, 0.5 dtp / dy, 1 / dx, 1 / dy, the predictor dt dtp
+    int rerun;               // the block to be run again (0: none)
+    unsigned int tiles;      // CTAs of a launch that are done
+};
+
 // launchers (all asynchronous on `s`)
 // The ghost fill of every block in one launch from the fill program (m->fill), written into the
 // current buffer only, with the ghost cells' TimeStep terms; with form_dt the last CTA forms the
 // step's dt (a TimeStep call: counter, clamps, frame points).  Its ghost-cell sources are read
 // from the other buffer, whose ghost cells equal the current buffer's before the fill: every
 // stencil stores the ghost cells it loaded into its output buffer, and launch_ghost_mirror does
-// the same after a fill that no stencil follows.  Launch after launch_step_begin.
-cudaError_t launch_fill_cfl(Ctrl* c, const MeshDev* m, long long total_ghost, cudaStream_t s, int form_dt = 1);
+// the same after a fill that no stencil follows.  Launch after launch_step_begin; with ss (a step of the
+// loop, its accumulators cleared by the step before) it takes the stop flag itself and forms the
+// all-blocks launch's scalars.
+cudaError_t launch_fill_cfl(Ctrl* c, const MeshDev* m, long long total_ghost, cudaStream_t s, int form_dt = 1,
+                            StepState* ss = nullptr);
 // the current buffer's ghost cells into the other buffer
 cudaError_t launch_ghost_mirror(Ctrl* c, const MeshDev* m, long long total_ghost, cudaStream_t s);
 // start of a step (before its ghost fill, or before a TimeStep call when the caller filled the
-// ghosts): stop flags; the ghost and next-state maxima, the reduction ticket and the all-blocks
-// launch's counters and records reset
+// ghosts): stop flags; the ghost and next-state maxima, the reduction ticket and the step's
+// records reset
 cudaError_t launch_step_begin(Ctrl* c, cudaStream_t s);
 // wave-speed maxima over the ghost cells; with form_dt the last CTA forms the step's dt (a
 // TimeStep call: counter, clamps, frame points)
@@ -105,10 +115,10 @@ cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int 
                           cudaStream_t s);
 cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int b, int tx, int ny, int ghost, int parity,
                                double* hout, cudaStream_t s);
-// Every block of a MUSCL-Hancock step in one cooperative launch (mh_step_kernel in hf_cart.cu:
-// the blocks' tiles from one counter, each block's predictor dt verified against the reference's
-// TimeStep call and the block run again where it differs), for meshes of at most
-// kStepMaxBlocks blocks.
+// Every block of a step in one launch, for meshes of at most kStepMaxBlocks blocks, and the end of the
+// step by its last CTA (hf_cart.cu; MUSCL-Hancock: each block's predictor dt verified against the
+// reference's TimeStep call, a block whose dt differs run again by one of the launches that follow).
+// After launch_fill_cfl with ss.
 constexpr int kStepMaxBlocks = 4;
 struct StepPlan {
     CUtensorMap tm[kStepMaxBlocks][2];   // per block, per state parity
@@ -117,10 +127,12 @@ struct StepPlan {
     int tiles_x[kStepMaxBlocks];
     int tile_start[kStepMaxBlocks + 1];  // prefix sums of the blocks' tile counts
     int nb;
+    int finish;                          // the last CTA ends the step (else launch_finalize does)
 };
 // the tile grid of block b (nx x ny interior cells) in the plan (plan.tile set)
 void step_plan_tiles(StepPlan& plan, int b, int nx, int ny);
-cudaError_t launch_mh_step(Ctrl* c, const MeshDev* m, const StepPlan& plan, int limiter, cudaStream_t s);
+cudaError_t launch_step(Ctrl* c, const MeshDev* m, StepState* ss, const StepPlan& plan, int scheme, int limiter,
+                        cudaStream_t s);
 
 // the driver's cuTensorMapEncodeTiled, or null where the driver lacks it
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

@@ -284,9 +284,9 @@ class CartSolver:
         return s.value or 0
 
     def set_block_launches(self, per_block: bool):
-        """True: one stencil launch per block, in order.  False (default): a MUSCL-Hancock step
-        of up to 4 blocks is one launch that checks each block's predictor dt against the
-        reference's and runs a block again where it differs; the results are identical."""
+        """True: one stencil launch per block, in order.  False (default): a step of up to 4 blocks
+        is one launch; with MUSCL-Hancock each block's predictor dt is then checked against the
+        reference's and the block run again where it differs; the results are identical."""
         check(lib().hf_set_block_launches(self._h, int(bool(per_block))), self._h)
 
     def blocks_rerun(self) -> int:

@@ -141,17 +141,15 @@ int hf_clear_error_cell(hf_ctx* ctx);
 /* the context's CUDA stream (a cudaStream_t), for callers that time or order work on it */
 int hf_stream(hf_ctx* ctx, void** stream);
 
-/* How a step's MUSCL-Hancock block updates are launched.  No counterpart in the reference,
- * whose Simulation::solve updates the blocks in order (simulation.cpp:106-110).  By default a
- * mesh of 2 to 4 blocks (or one block of at least 1024 tiles of 32 x 12 cells) is updated by one
- * cooperative launch that takes the blocks' tiles in
- * order from one counter (no partly filled last wave per block) and runs every block with the
- * predictor dt of a TimeStep call over the step's starting state; each block b > 0 is then
- * checked against the predictor dt the reference forms (muscl_hancock.cpp:246: blocks < b
- * already updated) and run again where the two differ, so results are the reference's bit for
- * bit either way.  per_block = 1 selects one launch per block in order instead (also used for
- * Godunov, for meshes of more blocks and by hf_advance_block).  hf_blocks_rerun counts the
- * block runs redone since creation. */
+/* How a step's block updates are launched.  No counterpart in the reference, whose
+ * Simulation::solve updates the blocks in order (simulation.cpp:106-110).  By default a mesh of up
+ * to 4 blocks is updated by one launch over the tiles of all blocks (no partly filled last wave per
+ * block), whose last CTA also ends the step.  With MUSCL-Hancock every block runs with the predictor
+ * dt of a TimeStep call over the step's starting state; each block b > 0 is then checked against the
+ * predictor dt the reference forms (muscl_hancock.cpp:246: blocks < b already updated) and run again
+ * where the two differ, so results are the reference's bit for bit either way.  per_block = 1 selects
+ * one launch per block in order instead (also used for meshes of more blocks and by
+ * hf_advance_block).  hf_blocks_rerun counts the block runs redone since creation. */
 int hf_set_block_launches(hf_ctx* ctx, int per_block);
 int hf_blocks_rerun(hf_ctx* ctx, int64_t* count);
 
