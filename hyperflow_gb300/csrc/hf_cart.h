@@ -113,6 +113,8 @@ cudaError_t launch_stencil(Ctrl* c, const MeshDev* m, int b, int nx, int ny, int
 // ghost fill, the updated buffer's ghost cells back out
 cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, const double* hin,
                           cudaStream_t s);
+// block b's whole state of one parity into mapped host memory [4][total_y][total_x]
+cudaError_t launch_download(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, double* hout, cudaStream_t s);
 cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int b, int tx, int ny, int ghost, int parity,
                                double* hout, cudaStream_t s);
 // Every block of a step in one launch, for meshes of at most kStepMaxBlocks blocks, and the end of the
