@@ -140,16 +140,12 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 template <int SCHEME, int TX, int TY>
 struct BatchTile;
 template <int TX, int TY>
-struct BatchTile<0, TX, TY> {   // Godunov: 1-cell halo; per-cell primitives/fluxes, face fluxes
-    using T = GoTile<TX, TY>;
-    static constexpr int H = 1, UX = T::UX, UY = T::UY, U_SIZE = T::U_SIZE;
-    static constexpr int WORK = T::Q_SIZE + T::F_SIZE + T::G_SIZE;
+struct BatchTile<0, TX, TY> : GoTile<TX, TY> {   // Godunov: 1-cell halo; the cells' values, face fluxes
+    static constexpr int H = 1;
 };
 template <int TX, int TY>
-struct BatchTile<1, TX, TY> {   // MUSCL-Hancock: 2-cell halo; evolved states, face fluxes
-    using T = MhTile<TX, TY>;
-    static constexpr int H = 2, UX = T::UX, UY = T::UY, U_SIZE = T::U_SIZE;
-    static constexpr int WORK = T::A_SIZE;
+struct BatchTile<1, TX, TY> : MhTile<TX, TY> {   // MUSCL-Hancock: 2-cell halo; evolved states, face fluxes
+    static constexpr int H = 2;
 };
 
 // stage tile `t`'s state + mirrored halo into sU (cp.async, one commit group)
@@ -218,9 +214,7 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps)
     double* sUb[STAGES];
 #pragma unroll
     for (int k = 0; k < STAGES; ++k) sUb[k] = smem + k * BT::U_SIZE;
-    double* sW = smem + STAGES * BT::U_SIZE;   // MUSCL-Hancock: sA; Godunov: sQ
-    double* sF = sW + GoTile<TX, TY>::Q_SIZE;   // Godunov only
-    double* sG = sF + GoTile<TX, TY>::F_SIZE;
+    double* sW = smem + STAGES * BT::U_SIZE;
     __shared__ double sdt[5];
 
     BatchCtrl* c = d.ctrl;
@@ -311,11 +305,11 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps)
             __syncthreads();
             const double dt = sdt[0], hdx = sdt[1], hdy = sdt[2], one_dx = sdt[3], one_dy = sdt[4];
             if (SCHEME == 0)
-                herr += go_tile_fluxes<TX, TY, NT>(sU, sW, sF, sG, g, g1, x0, y0, I.n, I.n);
+                herr += go_tile_fluxes<NT>(BT(), sU, sW, g, g1, x0, y0, I.n, I.n);
             else if (lim == 0)
-                herr += mh_tile_fluxes<NT, 0>(MhTile<TX, TY>(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
+                herr += mh_tile_fluxes<NT, 0>(BT(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
             else
-                herr += mh_tile_fluxes<NT, 1>(MhTile<TX, TY>(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
+                herr += mh_tile_fluxes<NT, 1>(BT(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
             double mx = 0.0, my = 0.0;
             double* __restrict__ out = Un + I.off;
             const size_t plane = (size_t)I.pitch * I.n;
@@ -324,14 +318,12 @@ __global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps)
                 const int gx = x0 + ox, gy = y0 + oy;
                 if (gx < I.n && gy < I.n) {
                     double un[4];
-                    if (SCHEME == 1) mh_update(MhTile<TX, TY>(), sU, sW, ox, oy, dt, one_dx, one_dy, un);
+                    if (SCHEME == 0) go_update(BT(), sU, sW, ox, oy, dt, one_dx, one_dy, un);
+                    else mh_update(BT(), sU, sW, ox, oy, dt, one_dx, one_dy, un);
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) {
-                        if (SCHEME == 0) un[v] = go_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy);
-                        out[v * plane + (size_t)gy * I.pitch + gx] = un[v];
-                    }
+                    for (int v = 0; v < 4; ++v) out[v * plane + (size_t)gy * I.pitch + gx] = un[v];
                     double sx, sy;
-                    if (!wave_terms(g, g1, un[0], un[1], un[2], un[3], sx, sy))
+                    if (!speeds(g, g1, un, sx, sy))
                         atomicMin(&c->first_nonpos, batch_key(step, I.off + (long long)gy * I.pitch + gx));
                     mx = nmax(mx, sx);
                     my = nmax(my, sy);

@@ -480,10 +480,10 @@ __device__ __forceinline__ void store_ghosts(const double* __restrict__ sU, cons
     }
 }
 
-// The tile's update: conservative update + forward Euler of its cells into out (and hout), the next
+// The tile's update (G ghost layers: 1 Godunov, 2 MUSCL-Hancock) of its cells into out (and hout), the next
 // step's TimeStep terms into mx and my, the earliest non-positive cell into *nonpos.
-template <int NT>
-__device__ __forceinline__ void mh_store(const MhShape& S, const double* sU, const double* sA, const BlockDev& B, int x0,
+template <int NT, int G>
+__device__ __forceinline__ void store_tile(const RowShape& S, const double* sU, const double* sA, const BlockDev& B, int x0,
                                          int y0, double* __restrict__ out, double* __restrict__ hout, double dt,
                                          double one_dx, double one_dy, double g, double g1, unsigned long long* nonpos,
                                          unsigned long long key, double& mx, double& my, int* err) {
@@ -494,17 +494,18 @@ __device__ __forceinline__ void mh_store(const MhShape& S, const double* sU, con
         const int gxx = x0 + ox, gyy = y0 + oy;
         if (gxx < B.nx && gyy < B.ny) {
             double un[4];
-            const size_t o = (size_t)(gyy + 2) * B.pitch + (gxx + 2);
-            const size_t h = (size_t)(gyy + 2) * B.tx + gxx + 2;
+            const size_t o = (size_t)(gyy + G) * B.pitch + (gxx + G);
+            const size_t h = (size_t)(gyy + G) * B.tx + gxx + G;
             if (!hf_in((long long)o, (long long)plane, err) || !hf_in((long long)h, (long long)B.ty * B.tx, err)) continue;
-            mh_update(S, sU, sA, ox, oy, dt, one_dx, one_dy, un);
+            if (G == 1) go_update(S, sU, sA, ox, oy, dt, one_dx, one_dy, un);
+            else mh_update(S, sU, sA, ox, oy, dt, one_dx, one_dy, un);
 #pragma unroll
             for (int v = 0; v < 4; ++v) {
                 out[v * plane + o] = un[v];
                 if (hout) __stcs(&hout[(size_t)v * B.ty * B.tx + h], un[v]);
             }
             double sx, sy;
-            if (!wave_terms(g, g1, un[0], un[1], un[2], un[3], sx, sy)) atomicMin(nonpos, key | face_key(0, 0, 0, gyy, gxx));
+            if (!speeds(g, g1, un, sx, sy)) atomicMin(nonpos, key | face_key(0, 0, 0, gyy, gxx));
             mx = nmax(mx, sx);
             my = nmax(my, sy);
         }
@@ -518,17 +519,17 @@ __device__ __forceinline__ void mh_store(const MhShape& S, const double* sU, con
 // the tile's 42 warp-items of predictor cells are three rounds of the 14 warps, its 40 of faces too.
 // Measured at 2048^2 (Mcell-updates/s): 1973; 512 threads and 64 registers 1962, 320 threads and 32 x 18
 // tiles 1933, 256 threads and 32 x 14 1880, three CTAs of 256 threads and 32 x 12 tiles 1751.
-constexpr int kMhNT = 448, kMhDoubles = 13856;
-constexpr size_t kMhBytes = (size_t)kMhDoubles * 8;
+constexpr int kNT = 448, kTileDoubles = 13856;
+constexpr size_t kTileBytes = (size_t)kTileDoubles * 8;
 
 template <int LIM>
-__global__ void __launch_bounds__(kMhNT, 2) mh_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
+__global__ void __launch_bounds__(kNT, 2) mh_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
                                                       const TileShape tile, const __grid_constant__ CUtensorMap tm0,
                                                       const __grid_constant__ CUtensorMap tm1,
                                                       double* __restrict__ hout) {
     extern __shared__ __align__(1024) double smem[];
     __shared__ uint64_t bar;
-    const MhShape S{tile};
+    const RowShape S{tile};
     const int tx = tile.tx, ty = tile.ty, usize = 4 * (tx + 4) * (ty + 4);
     double* sU = smem;
     double* sA = smem + usize;
@@ -560,13 +561,13 @@ __global__ void __launch_bounds__(kMhNT, 2) mh_kernel(Ctrl* __restrict__ c, cons
     if (!wait_tile(&bar, c)) return;
     const double hdx = sc[0], hdy = sc[1], one_dx = sc[2], one_dy = sc[3];
 
-    const int herr = mh_tile_fluxes<kMhNT, LIM>(S, sU, sA, g, g1, hdx, hdy, x0, y0, B.nx, B.ny, &c->first_bad,
+    const int herr = mh_tile_fluxes<kNT, LIM>(S, sU, sA, g, g1, hdx, hdy, x0, y0, B.nx, B.ny, &c->first_bad,
                                                 face_key(c->step, b, 0, 0, 0));
     double mx = 0.0, my = 0.0;
-    mh_store<kMhNT>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], hout, dt, one_dx, one_dy, g, g1, &c->first_nonpos,
+    store_tile<kNT, 2>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], hout, dt, one_dx, one_dy, g, g1, &c->first_nonpos,
                     face_key(c->step, b, 0, 0, 0), mx, my, &c->err);
-    store_ghosts<2, kMhNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
-    block_max2_atomic<kMhNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
+    store_ghosts<2, kNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
+    block_max2_atomic<kNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
 
@@ -642,7 +643,7 @@ __device__ __forceinline__ void mh_plan_tile(Ctrl* __restrict__ c, const MeshDev
                                              const StepPlan& plan, int b, int local, uint64_t* bar, uint32_t phase) {
     extern __shared__ __align__(1024) double smem[];
     const int p = (int)(c->step & 1);
-    const MhShape S{plan.tile};
+    const RowShape S{plan.tile};
     const int tx = plan.tile.tx, ty = plan.tile.ty, usize = 4 * (tx + 4) * (ty + 4);
     double* sU = smem;
     double* sA = smem + usize;
@@ -666,17 +667,17 @@ __device__ __forceinline__ void mh_plan_tile(Ctrl* __restrict__ c, const MeshDev
     }
     const double g = c->gamma, g1 = c->g1;
     const unsigned long long key = face_key(c->step, b, 0, 0, 0);
-    const int herr = mh_tile_fluxes<kMhNT, LIM>(S, sU, sA, g, g1, hdx, hdy, x0, y0, B.nx, B.ny, &c->step_bad[b], key);
+    const int herr = mh_tile_fluxes<kNT, LIM>(S, sU, sA, g, g1, hdx, hdy, x0, y0, B.nx, B.ny, &c->step_bad[b], key);
     double mx = 0.0, my = 0.0;
-    mh_store<kMhNT>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], plan.hout[b], c->dt, ss->sc[b][2], ss->sc[b][3], g, g1,
+    store_tile<kNT, 2>(S, sU, sA, B, x0, y0, B.buf[p ^ 1], plan.hout[b], c->dt, ss->sc[b][2], ss->sc[b][3], g, g1,
                     &c->step_nonpos[b], key, mx, my, &c->err);
-    store_ghosts<2, kMhNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
-    block_max2_atomic<kMhNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
+    store_ghosts<2, kNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
+    block_max2_atomic<kNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->step_hllc[b]), (unsigned long long)herr);
 }
 
 template <int LIM>
-__global__ void __launch_bounds__(kMhNT, 2) mh_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+__global__ void __launch_bounds__(kNT, 2) mh_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                            StepState* __restrict__ ss,
                                                            const __grid_constant__ StepPlan plan) {
     if (c->done) return;   // set before this launch: every CTA leaves
@@ -691,7 +692,7 @@ __global__ void __launch_bounds__(kMhNT, 2) mh_step_kernel(Ctrl* __restrict__ c,
 
 // the block a launch before this one left to be run again, if any, on the resident CTAs
 template <int LIM>
-__global__ void __launch_bounds__(kMhNT, 2) mh_rerun_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+__global__ void __launch_bounds__(kNT, 2) mh_rerun_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                             StepState* __restrict__ ss,
                                                             const __grid_constant__ StepPlan plan) {
     const int b = c->done ? 0 : ss->rerun;
@@ -709,111 +710,66 @@ __global__ void __launch_bounds__(kMhNT, 2) mh_rerun_kernel(Ctrl* __restrict__ c
 }
 
 // ------------------------------------------------------------------------------------
-// Godunov, fused: per-cell primitives/fluxes once, then x/y HLLC, then update
+// Godunov, fused: per-cell primitives once, then x/y HLLC, then update
 // ------------------------------------------------------------------------------------
-template <int TX, int TY>
-struct GoLayout {
-    using T = GoTile<TX, TY>;
-    static constexpr int NC = T::NC;
-    static constexpr int U_OFF = 0;
-    static constexpr int Q_OFF = U_OFF + T::U_SIZE;
-    static constexpr int F_OFF = Q_OFF + T::Q_SIZE;
-    static constexpr int G_OFF = F_OFF + T::F_SIZE;
-    static constexpr int END = G_OFF + T::G_SIZE;
-    static constexpr size_t BYTES = (size_t)END * 8 + 16;   // + mbarrier
-    static constexpr int TMA_BYTES = T::U_SIZE * 8;
-};
-
-// three 256-thread CTAs per SM (80 registers, 74 KB of shared memory with 32x10 tiles): measured
-// 3 % faster than two CTAs of 32x14 tiles at 110 registers, and than 32x8 or 32x6 tiles
-template <int TX, int TY, int NT>
 __device__ __forceinline__ void godunov_tile(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b, int local,
-                                             const CUtensorMap* tm, double* __restrict__ hout) {
-    using L = GoLayout<TX, TY>;
+                                             const TileShape& tile, const CUtensorMap* tm, double* __restrict__ hout) {
     extern __shared__ __align__(1024) double smem[];
-    double* sU = smem + L::U_OFF;
-    double* sQ = smem + L::Q_OFF;
-    double* sF = smem + L::F_OFF;
-    double* sG = smem + L::G_OFF;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::END);
+    __shared__ uint64_t bar;
+    const RowShape S{tile};
+    const int tx = tile.tx, ty = tile.ty, usize = 4 * (tx + 2) * (ty + 2);
+    double* sU = smem;
+    double* sW = smem + usize;
 
     const BlockDev& B = m->b[b];
     const int p = (int)(c->step & 1);
-    const int tiles_x = (B.nx + TX - 1) / TX;
-    const int x0 = (local % tiles_x) * TX, y0 = (local / tiles_x) * TY;
+    const int tiles_x = (B.nx + tx - 1) / tx;
+    const int x0 = (local % tiles_x) * tx, y0 = (local / tiles_x) * ty;
     const double g = c->gamma, g1 = c->g1;
     const double dt = c->dt;
     __shared__ double sc[2];
     if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        mbar_expect_tx(bar, L::TMA_BYTES);
-        tma_load_3d(sU, tm, bar, x0, y0, 0);
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, usize * 8);
+        tma_load_3d(sU, tm, &bar, x0, y0, 0);
         sc[0] = div_rn(1.0, c->dx[b]);   // godunov.cpp:97-98
         sc[1] = div_rn(1.0, c->dy[b]);
     }
-    if (!wait_tile(bar, c)) return;
-    const double one_dx = sc[0], one_dy = sc[1];
+    if (!wait_tile(&bar, c)) return;
 
-    const int herr = go_tile_fluxes<TX, TY, NT>(sU, sQ, sF, sG, g, g1, x0, y0, B.nx, B.ny, &c->first_bad,
-                                                face_key(c->step, b, 0, 0, 0));
-    double* __restrict__ out = B.buf[p ^ 1];
-    const size_t plane = (size_t)B.ty * B.pitch;
+    const int herr = go_tile_fluxes<kNT>(S, sU, sW, g, g1, x0, y0, B.nx, B.ny, &c->first_bad,
+                                         face_key(c->step, b, 0, 0, 0));
     double mx = 0.0, my = 0.0;
-    for (int it = threadIdx.x; it < TX * TY; it += NT) {
-        const int ox = it % TX, oy = it / TX;
-        const int gxx = x0 + ox, gyy = y0 + oy;
-        if (gxx < B.nx && gyy < B.ny) {
-            double un[4];
-            const size_t o = (size_t)(gyy + 1) * B.pitch + (gxx + 1);
-            const size_t h = (size_t)(gyy + 1) * B.tx + gxx + 1;
-            if (!hf_in((long long)o, (long long)plane, &c->err) ||
-                !hf_in((long long)h, (long long)B.ty * B.tx, &c->err))
-                continue;
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                un[v] = go_update<TX, TY>(sU, sF, sG, v, ox, oy, dt, one_dx, one_dy);
-                out[v * plane + o] = un[v];
-                if (hout) __stcs(&hout[(size_t)v * B.ty * B.tx + h], un[v]);
-            }
-            double sx, sy;
-            if (!wave_terms(g, g1, un[0], un[1], un[2], un[3], sx, sy))
-                atomicMin(&c->first_nonpos, face_key(c->step, b, 0, gyy, gxx));
-            mx = nmax(mx, sx);
-            my = nmax(my, sy);
-        }
-    }
-    store_ghosts<1, NT>(sU, B, TX, TY, x0, y0, out, &c->err);
-    block_max2_atomic<NT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
+    store_tile<kNT, 1>(S, sU, sW, B, x0, y0, B.buf[p ^ 1], hout, dt, sc[0], sc[1], g, g1, &c->first_nonpos,
+                       face_key(c->step, b, 0, 0, 0), mx, my, &c->err);
+    store_ghosts<1, kNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
+    block_max2_atomic<kNT>(mx, my, &c->int_s[p ^ 1][b][0], &c->int_s[p ^ 1][b][1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
 
 // one block (hf_advance_block, meshes of many blocks)
-template <int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT, 3) godunov_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
-                                                        const __grid_constant__ CUtensorMap tm0,
-                                                        const __grid_constant__ CUtensorMap tm1,
-                                                        double* __restrict__ hout) {
+__global__ void __launch_bounds__(kNT, 2) godunov_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
+                                                         const TileShape tile, const __grid_constant__ CUtensorMap tm0,
+                                                         const __grid_constant__ CUtensorMap tm1,
+                                                         double* __restrict__ hout) {
     if (c->done) return;
-    godunov_tile<TX, TY, NT>(c, m, b, blockIdx.x, (c->step & 1) ? &tm1 : &tm0, hout);
+    godunov_tile(c, m, b, blockIdx.x, tile, (c->step & 1) ? &tm1 : &tm0, hout);
 }
 
 // every block of a step in one launch, whose last CTA ends the step
-template <int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT, 3) godunov_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                                             StepState* __restrict__ ss,
-                                                             const __grid_constant__ StepPlan plan) {
+__global__ void __launch_bounds__(kNT, 2) godunov_step_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+                                                              StepState* __restrict__ ss,
+                                                              const __grid_constant__ StepPlan plan) {
     if (c->done) return;
     int b = 0;
     while (b + 1 < plan.nb && (int)blockIdx.x >= plan.tile_start[b + 1]) ++b;
-    godunov_tile<TX, TY, NT>(c, m, b, blockIdx.x - plan.tile_start[b], &plan.tm[b][c->step & 1], plan.hout[b]);
+    godunov_tile(c, m, b, blockIdx.x - plan.tile_start[b], plan.tile, &plan.tm[b][c->step & 1], plan.hout[b]);
     if (last_cta(&ss->tiles) && plan.finish) finish_step(c);
 }
 
 // ------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------
-constexpr int kGoTX = 32, kGoTY = 10, kGoNT = 256;
-
 TileShape tile_shape(int tx, int ty) {
     TileShape t;
     t.tx = tx;
@@ -822,27 +778,26 @@ TileShape tile_shape(int tx, int ty) {
     return t;
 }
 
-// The MUSCL-Hancock tile: of the even widths (a TMA copy starts on 16 bytes) and heights that fit a CTA's
-// shared memory, the one whose tiles take the least time by the model below -- the rounds of a CTA's
-// 14 warps over the tile's predictor cells, faces and cells, at their measured instruction counts,
-// times the waves of the 2 x sms resident CTAs.  A mesh of many tiles gets the shape with the fewest
-// wasted lanes and halo items (32 x 19); a small one a shape that fills the GPU once: 256^2 in 32 x 19
-// tiles would leave 44 of 152 SMs without work.
+// The tile: of the even widths (a TMA copy starts on 16 bytes) and heights that fit a CTA's shared memory,
+// the one whose tiles take the least time by the model below -- the rounds of a CTA's 14 warps over the
+// tile's cells and faces, at their instruction counts, times the waves of the 2 x sms resident CTAs.
+// A mesh of many tiles gets the shape with the fewest wasted lanes and halo items; a small one a shape that
+// fills the GPU once: 256^2 in 32 x 19 tiles would leave 44 of 152 SMs without work.
 TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms) {
-    if (scheme == 0) return tile_shape(kGoTX, kGoTY);
-    constexpr int W = kMhNT / 32;
+    constexpr int W = kNT / 32;
     auto warps = [](int items) { return (items + 31) / 32; };
     auto rounds = [](int w) { return (w + W - 1) / W; };
     double best = 0.0;
-    int bx = 32, by = 19;
+    int bx = 8, by = 2;
     for (int tx = 8; tx <= 64; tx += 2)
         for (int ty = 2; ty <= 32; ++ty) {
-            if (mh_tile_doubles(tx, ty) > kMhDoubles) continue;
+            if ((scheme == 0 ? go_tile_doubles(tx, ty) : mh_tile_doubles(tx, ty)) > kTileDoubles) continue;
             long long n = 0;
             for (int b = 0; b < nb; ++b) n += (long long)((nx[b] + tx - 1) / tx) * ((ny[b] + ty - 1) / ty);
-            const double tile = 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) +
-                                2200.0 * rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))) +
-                                800.0 * rounds(warps(tx * ty)) + 600.0;
+            const int faces = rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))), cells = rounds(warps(tx * ty));
+            const double tile = scheme == 0
+                ? 550.0 * rounds(warps((tx + 2) * (ty + 2))) + 950.0 * faces + 750.0 * cells + 400.0
+                : 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) + 2200.0 * faces + 800.0 * cells + 600.0;
             const long long rest = n % (2 * sms);
             // one CTA alone on its SM runs faster than beside a second one, but not twice as fast
             const double waves = (double)(n / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
@@ -865,33 +820,28 @@ cudaError_t launch_step(Ctrl* c, const MeshDev* m, StepState* ss, const StepPlan
     if (plan.nb < 1 || plan.nb > kStepMaxBlocks) return cudaErrorInvalidValue;
     const int tiles = plan.tile_start[plan.nb];
     if (scheme == 0) {
-        godunov_step_kernel<kGoTX, kGoTY, kGoNT><<<tiles, kGoNT, GoLayout<kGoTX, kGoTY>::BYTES, s>>>(c, m, ss, plan);
+        godunov_step_kernel<<<tiles, kNT, kTileBytes, s>>>(c, m, ss, plan);
         return cudaGetLastError();
     }
-    if (limiter == 0) mh_step_kernel<0><<<tiles, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
-    else mh_step_kernel<1><<<tiles, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
+    if (limiter == 0) mh_step_kernel<0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, plan);
+    else mh_step_kernel<1><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, plan);
     // a block run again on a fixed grid: with nothing to do (nearly always) few CTAs come and go
     const int again = tiles < 2 * 152 ? tiles : 2 * 152;
     for (int b = 1; b < plan.nb; ++b) {
-        if (limiter == 0) mh_rerun_kernel<0><<<again, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
-        else mh_rerun_kernel<1><<<again, kMhNT, kMhBytes, s>>>(c, m, ss, plan);
+        if (limiter == 0) mh_rerun_kernel<0><<<again, kNT, kTileBytes, s>>>(c, m, ss, plan);
+        else mh_rerun_kernel<1><<<again, kNT, kTileBytes, s>>>(c, m, ss, plan);
     }
     return cudaGetLastError();
 }
 
 cudaError_t stencil_prepare() {
     for (const void* k : {(const void*)mh_step_kernel<0>, (const void*)mh_step_kernel<1>, (const void*)mh_rerun_kernel<0>,
-                          (const void*)mh_rerun_kernel<1>, (const void*)mh_kernel<0>, (const void*)mh_kernel<1>}) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMhBytes);
+                          (const void*)mh_rerun_kernel<1>, (const void*)mh_kernel<0>, (const void*)mh_kernel<1>,
+                          (const void*)godunov_step_kernel, (const void*)godunov_kernel}) {
+        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes);
         if (e != cudaSuccess) return e;
     }
-    const cudaError_t e = cudaFuncSetAttribute(godunov_step_kernel<kGoTX, kGoTY, kGoNT>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)GoLayout<kGoTX, kGoTY>::BYTES);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(godunov_kernel<kGoTX, kGoTY, kGoNT>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)GoLayout<kGoTX, kGoTY>::BYTES);
+    return cudaSuccess;
 }
 
 cudaError_t launch_step_begin(Ctrl* c, cudaStream_t s) {
@@ -977,12 +927,11 @@ cudaError_t launch_stencil(Ctrl* c, const MeshDev* m, int b, int nx, int ny, int
                            double* hout) {
     const int tiles = ((nx + tile.tx - 1) / tile.tx) * ((ny + tile.ty - 1) / tile.ty);
     if (scheme == 0)
-        godunov_kernel<kGoTX, kGoTY, kGoNT>
-            <<<tiles, kGoNT, GoLayout<kGoTX, kGoTY>::BYTES, s>>>(c, m, b, *tm0, *tm1, hout);
+        godunov_kernel<<<tiles, kNT, kTileBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
     else if (limiter == 0)
-        mh_kernel<0><<<tiles, kMhNT, kMhBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
+        mh_kernel<0><<<tiles, kNT, kTileBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
     else
-        mh_kernel<1><<<tiles, kMhNT, kMhBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
+        mh_kernel<1><<<tiles, kNT, kTileBytes, s>>>(c, m, b, tile, *tm0, *tm1, hout);
     return cudaGetLastError();
 }
 

@@ -173,14 +173,13 @@ HF_HD bool predict_fast(bool y, const double* um, const double* u0, const double
 // a < b for values that are not NaN
 HF_HD bool less(double a, double b) { return order_key(a) < order_key(b); }
 
-// The HLLC flux (n, t order) between ordinary states; false: some value is outside the window
-HF_HD bool hllc_fast(bool y, double g, double g1, const double* UL, const double* UR, double* F) {
-    Window w;
-    see(w, g);
-    see(w, g1);
-    const PrimN L = prim_n(w, g1, UL), R = prim_n(w, g1, UR);
-    const double aL = root32(f64_bits(quot(mulw(g, L.p), L.r, L.X)));
-    const double aR = root32(f64_bits(quot(mulw(g, R.p), R.r, R.X)));
+HF_HD double sound_n(double g, const PrimN& a) { return root32(f64_bits(quot(mulw(g, a.p), a.r, a.X))); }
+
+// The HLLC flux (n, t order) from the two sides' primitives and sound speeds (E: and total energies, in
+// place of the reciprocals); only the side the branches select forms its energy, flux and star state.
+template <bool E>
+HF_HD bool hllc_sides(Window& w, bool y, double g1, const PrimN& L, const PrimN& R, double aL, double aR, double EL,
+                      double ER, const double* UL, const double* UR, double* F) {
     const double l0 = L.n - aL, r0 = R.n - aR, l1 = L.n + aL, r1 = R.n + aR;
     const double SL = less(r0, l0) ? r0 : l0, SR = less(l1, r1) ? r1 : l1;
     if (outside(w)) return false;
@@ -198,7 +197,8 @@ HF_HD bool hllc_fast(bool y, double g, double g1, const double* UL, const double
         see(w, den);
         if (outside(w)) return false;
         Ss = quotz(num, den, rcp32(den), z);
-        left = ge0(Ss);                         // SL < 0
+        // the branches of riemann_hllc.cpp:179-211 with SL < 0 and no NaN: star left, star right, right
+        left = ge0(Ss);
         star = left || ge0(SR);
     }
     PrimN a;
@@ -209,8 +209,8 @@ HF_HD bool hllc_fast(bool y, double g, double g1, const double* UL, const double
     a.q = left ? L.q : R.q;
     a.zn = left ? L.zn : R.zn;
     a.zt = left ? L.zt : R.zt;
-    a.X = left ? L.X : R.X;
-    const double Et = energy_n(w, g1, a);
+    if (!E) a.X = left ? L.X : R.X;
+    const double Et = E ? (left ? EL : ER) : energy_n(w, g1, a);
     double f[4];
     flux_n(w, y, a, Et, f);
     if (star) {
@@ -225,7 +225,7 @@ HF_HD bool hllc_fast(bool y, double g, double g1, const double* UL, const double
         see(w, c);
         const double k = Ss + quot(a.p, rd, rcp32(rd));
         see(w, k);
-        const double m = quot(Et, a.r, a.X) + mulz(sn, k, zsn);
+        const double m = quot(Et, a.r, E ? rcp32(a.r) : a.X) + mulz(sn, k, zsn);
         see(w, m);
         const double us[4] = {c, mulz(c, Ss, zs), mulz(c, a.t, a.zt), mulw(c, m)};
 #pragma unroll
@@ -239,6 +239,117 @@ HF_HD bool hllc_fast(bool y, double g, double g1, const double* UL, const double
 #pragma unroll
     for (int v = 0; v < 4; ++v) F[v] = f[v];
     return !outside(w);
+}
+
+// The HLLC flux (n, t order) between ordinary states; false: some value is outside the window
+HF_HD bool hllc_fast(bool y, double g, double g1, const double* UL, const double* UR, double* F) {
+    Window w;
+    see(w, g);
+    see(w, g1);
+    const PrimN L = prim_n(w, g1, UL), R = prim_n(w, g1, UR);
+    return hllc_sides<false>(w, y, g1, L, R, sound_n(g, L), sound_n(g, R), 0.0, 0.0, UL, UR, F);
+}
+
+// TimeStep's terms |u| + c and |v| + c of an ordinary state (wave_terms); its density and pressure are positive
+HF_HD bool speeds_fast(double g, double g1, const double* U, double& sx, double& sy) {
+    Window w;
+    see(w, g);
+    see(w, g1);
+    const PrimN a = prim_n(w, g1, U);
+    const double c = sound_n(g, a);
+    sx = f64_from(f64_bits(a.n) & kAbs) + c;
+    sy = f64_from(f64_bits(a.t) & kAbs) + c;
+    return !outside(w);
+}
+static __host__ __device__ __noinline__ bool speeds_any(double g, double g1, double r, double ru, double rv, double E,
+                                                        double* s) {
+    return wave_terms(g, g1, r, ru, rv, E, s[0], s[1]);
+}
+// false: density or pressure not positive
+HF_HD bool speeds(double g, double g1, const double* U, double& sx, double& sy) {
+    if (speeds_fast(g, g1, U, sx, sy)) return true;
+    double s[2];
+    const bool ok = speeds_any(g, g1, U[0], U[1], U[2], U[3], s);
+    sx = s[0];
+    sy = s[1];
+    return ok;
+}
+
+// A Godunov cell: q = u, v, p, Et, a (its primitives, total energy and sound speed), formed once for its
+// four faces
+HF_HD bool cell_fast(double g, double g1, const double* U, double* q) {
+    Window w;
+    see(w, g);
+    see(w, g1);
+    const PrimN a = prim_n(w, g1, U);
+    q[0] = a.n;
+    q[1] = a.t;
+    q[2] = a.p;
+    q[3] = energy_n(w, g1, a);
+    q[4] = sound_n(g, a);
+    return !outside(w);
+}
+static __host__ __device__ __noinline__ void cell_any(double g, double g1, double r, double ru, double rv, double E,
+                                                      double* q) {
+    const Prim w = to_prim(g1, r, ru, rv, E);
+    q[0] = w.u;
+    q[1] = w.v;
+    q[2] = w.p;
+    q[3] = w.Et;
+    q[4] = sound(g, w.r, w.p);
+}
+// the sides of a Godunov face from their cells' values (n, t order)
+HF_HD PrimN prim_of(Window& w, const double* U, const double* q) {
+    PrimN a;
+    a.r = U[0];
+    a.n = q[0];
+    a.t = q[1];
+    a.p = q[2];
+    a.q = 0.0;
+    a.X = 0u;
+    a.zn = zero(a.n);
+    a.zt = zero(a.t);
+    see_pos(w, a.r);
+    see0(w, a.n, a.zn);
+    see0(w, a.t, a.zt);
+    see_pos(w, a.p);
+    see_pos(w, q[3]);
+    see_pos(w, q[4]);
+    return a;
+}
+HF_HD bool face_fast(bool y, const double* UL, const double* qL, const double* UR, const double* qR, double* F) {
+    Window w;
+    const PrimN L = prim_of(w, UL, qL), R = prim_of(w, UR, qR);
+    return hllc_sides<true>(w, y, 0.0, L, R, qL[4], qR[4], qL[3], qR[3], UL, UR, F);
+}
+static __host__ __device__ __noinline__ int face_any(bool y, const double* UL, const double* qL, const double* UR,
+                                                     const double* qR, double* F) {
+    const double* const U[2] = {UL, UR};
+    const double* const q[2] = {qL, qR};
+    const int n = y ? 2 : 1, t = 3 - n;
+    Prim w[2];
+    double V[2][4], f[2][4], G[4];
+    for (int k = 0; k < 2; ++k) {
+        V[k][0] = U[k][0];
+        V[k][n] = U[k][1];
+        V[k][t] = U[k][2];
+        V[k][3] = U[k][3];
+        w[k].r = U[k][0];
+        w[k].u = y ? q[k][1] : q[k][0];
+        w[k].v = y ? q[k][0] : q[k][1];
+        w[k].p = q[k][2];
+        w[k].Et = q[k][3];
+        w[k].q = 0.0;
+        if (y) flux<1>(w[k], f[k]);
+        else flux<0>(w[k], f[k]);
+    }
+    const int bad = y ? hllc<1>(V[0], w[0], qL[4], f[0], V[1], w[1], qR[4], f[1], G)
+                      : hllc<0>(V[0], w[0], qL[4], f[0], V[1], w[1], qR[4], f[1], G);
+    F[0] = G[0];
+    F[1] = G[n];
+    F[2] = G[t];
+    F[3] = G[3];
+    return bad;
 }
 
 // dt (one_dx (F_l - F_r) + one_dy (G_b - G_t)) + U of four variables; false: outside the window

@@ -1,112 +1,138 @@
-// The first-order Godunov tile computation shared by the per-block stencil (hf_cart.cu) and the
+// The first-order Godunov tile computation shared by the Cartesian stencils (hf_cart.cu) and the
 // batched persistent kernel (hf_batch.cu): GodunovScheme::calculate_fluxes_{x,y} +
 // calculate_spatial_update (src/fvm_2d_cart/scheme/godunov/godunov.cpp:27-118) with the
 // forward-Euler update (forward_euler.cpp:19-29).
 //
-// Input: sU, the tile's conservative state plus a 1-cell halo in shared memory,
-// [4][TY+2][TX+2].  Each cell's primitives, sound speed and x/y fluxes are formed once (sQ) and
-// shared by the two faces that use them.  Output: sF / sG, the HLLC fluxes of the tile's x faces
-// [4][TY][TX+1] and y faces [4][TY+1][TX].
+// Input: sU, the tile's conservative state plus a 1-cell halo in shared memory, [4][ty+2][tx+2].  Each
+// cell's primitives, total energy and sound speed are formed once (sQ [5][cells]) for the faces that use
+// them.  Output: sF / sG, the HLLC fluxes of the tile's x faces [4][ty][tx+1] and y faces [4][ty+1][tx].
+//
+// As the MUSCL-Hancock tile: FP64 issue bounds it, the products go to the integer pipes (hf_fast.cuh) and
+// both directions run one copy of the code.  A face forms the flux of the one side it uses: with both
+// fluxes of every cell in sQ (12 values) a CTA's tile was 32 x 10 cells and a quarter of its cells halo.
 #pragma once
 
-#include "hf_ctrl.h"
+#include "hf_cart.h"
 #include "hf_device.cuh"
-#include "hf_mh_tile.cuh"   // owned_face
+#include "hf_fast.cuh"
+#include "hf_mh_tile.cuh"   // tile shapes, owned_face
 
 namespace hf {
 
 template <int TX, int TY>
-struct GoTile {
-    static constexpr int UX = TX + 2, UY = TY + 2, NC = UX * UY;
-    static constexpr int NQ = 12;   // u v p Et a fx0 fx1 fx2 fx3 fy0 fy2 fy3 (fy1 == fx2)
-    static constexpr int U_SIZE = 4 * NC;
-    static constexpr int Q_SIZE = NQ * NC;
-    static constexpr int F_SIZE = 4 * TY * (TX + 1);
-    static constexpr int G_SIZE = 4 * (TY + 1) * TX;
+struct GoTile : TileRows<TX, TY> {
+    static constexpr int UX = TX + 2, UY = TY + 2;
+    static constexpr int U_SIZE = 4 * UX * UY;                                               // doubles
+    static constexpr int WORK = 5 * UX * UY + 4 * TY * (TX + 1) + 4 * (TY + 1) * TX;
 };
+// doubles of shared memory a tile takes: the state with its halo, the cells' values, the fluxes
+inline int go_tile_doubles(int tx, int ty) {
+    return 9 * (tx + 2) * (ty + 2) + 4 * ty * (tx + 1) + 4 * (ty + 1) * tx;
+}
 
-// Computes sF and sG from sU (tile origin x0, y0 in interior cells of an nx x ny block).  Ends
-// with __syncthreads().  Returns the number of owned faces whose HLLC took the zero-flux branch;
-// with first_bad, each such face's face_key (key_base: its step and block bits) is min-reduced
-// there.  Cells beyond the first ghost layer and faces beyond the last face are skipped: no
-// in-block cell reads them, and zero-filled states would only take the slow division paths.
-template <int TX, int TY, int NT>
-__device__ __forceinline__ int go_tile_fluxes(const double* __restrict__ sU, double* __restrict__ sQ,
-                                              double* __restrict__ sF, double* __restrict__ sG, double g,
-                                              double g1, int x0, int y0, int nx, int ny,
-                                              unsigned long long* first_bad = nullptr,
+// One face between the tile cells l and r = l + step (nc cells a plane); its flux, in the variables'
+// order, to f[v * fs].  Returns 1 for the zero-flux fallback.
+__device__ __forceinline__ int go_face(bool y, const double* sU, const double* sQ, int l, int step, int nc, double* f,
+                                       int fs) {
+    const int pn = y ? 2 * nc : nc, pt = 3 * nc - pn, qn = y ? nc : 0, qt = nc - qn;
+    double U[2][4], q[2][5], F[4];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const double* u = sU + l + k * step;
+        const double* w = sQ + l + k * step;
+        U[k][0] = u[0]; U[k][1] = u[pn]; U[k][2] = u[pt]; U[k][3] = u[3 * nc];
+        q[k][0] = w[qn]; q[k][1] = w[qt]; q[k][2] = w[2 * nc]; q[k][3] = w[3 * nc]; q[k][4] = w[4 * nc];
+    }
+    int bad = 0;
+    if (!face_fast(y, U[0], q[0], U[1], q[1], F)) {
+        double V[2][4], r[2][5], G[4];   // copies, so that the fast path's stay in registers
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const double* u = sU + l + k * step;
+            const double* w = sQ + l + k * step;
+            V[k][0] = u[0]; V[k][1] = u[pn]; V[k][2] = u[pt]; V[k][3] = u[3 * nc];
+            r[k][0] = w[qn]; r[k][1] = w[qt]; r[k][2] = w[2 * nc]; r[k][3] = w[3 * nc]; r[k][4] = w[4 * nc];
+        }
+        bad = face_any(y, V[0], r[0], V[1], r[1], G);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) F[v] = G[v];
+    }
+    f[0] = F[0];
+    f[(y ? 2 : 1) * fs] = F[1];
+    f[(y ? 1 : 2) * fs] = F[2];
+    f[3 * fs] = F[3];
+    return bad;
+}
+
+// Computes the fluxes in sW (after the cells' values there) from sU (tile origin x0, y0 in interior cells
+// of an nx x ny block).  Ends with __syncthreads().  Returns the number of owned faces whose HLLC took
+// the zero-flux branch; with first_bad, each such face's face_key (key_base: its step and block bits) is
+// min-reduced there.  Cells beyond the first ghost layer and faces beyond the last face are skipped: no
+// in-block cell reads them, and zero-filled states would only take the general path.
+template <int NT, class S>
+__device__ __forceinline__ int go_tile_fluxes(const S& s, const double* sU, double* sW, double g, double g1, int x0, int y0,
+                                              int nx, int ny, unsigned long long* first_bad = nullptr,
                                               unsigned long long key_base = 0) {
-    using L = GoTile<TX, TY>;
-#define Q(k, cell) sQ[(k) * L::NC + (cell)]
-    for (int cell = threadIdx.x; cell < L::NC; cell += NT) {
-        if (x0 - 1 + cell % L::UX > nx || y0 - 1 + cell / L::UX > ny) continue;
-        Prim w = to_prim(g1, sU[cell], sU[L::NC + cell], sU[2 * L::NC + cell], sU[3 * L::NC + cell]);
-        double fx[4], fy[4];
-        flux<0>(w, fx);
-        flux<1>(w, fy);
-        Q(0, cell) = w.u; Q(1, cell) = w.v; Q(2, cell) = w.p; Q(3, cell) = w.Et;
-        Q(4, cell) = sound(g, w.r, w.p);
-        Q(5, cell) = fx[0]; Q(6, cell) = fx[1]; Q(7, cell) = fx[2]; Q(8, cell) = fx[3];
-        Q(9, cell) = fy[0]; Q(10, cell) = fy[2]; Q(11, cell) = fy[3];
+    const int tx = s.tx(), ty = s.ty(), ux = tx + 2, nc = ux * (ty + 2);
+    const int nfx = (tx + 1) * ty, nfy = tx * (ty + 1);
+    double* const sQ = sW;
+    double* const sF = sW + 5 * nc;
+    double* const sG = sF + 4 * nfx;
+#pragma unroll 1
+    for (int cell = threadIdx.x; cell < nc; cell += NT) {
+        const int row = s.row2(cell);
+        if (x0 - 1 + cell - row * ux > nx || y0 - 1 + row > ny) continue;
+        const double U[4] = {sU[cell], sU[nc + cell], sU[2 * nc + cell], sU[3 * nc + cell]};
+        double q[5];
+        if (!cell_fast(g, g1, U, q)) {
+            double r[5];
+            cell_any(g, g1, U[0], U[1], U[2], U[3], r);
+#pragma unroll
+            for (int k = 0; k < 5; ++k) q[k] = r[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 5; ++k) sQ[k * nc + cell] = q[k];
     }
     __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int fx = (nfx + 31) >> 5, fxy = fx + ((nfy + 31) >> 5);
     int herr = 0;
-    auto load = [&](int cell, double* U, Prim& w, double& a, double* fx, double* fy) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v) U[v] = sU[v * L::NC + cell];
-        w.r = U[0]; w.u = Q(0, cell); w.v = Q(1, cell); w.p = Q(2, cell); w.Et = Q(3, cell); w.q = 0.0;
-        a = Q(4, cell);
-        if (fx) { fx[0] = Q(5, cell); fx[1] = Q(6, cell); fx[2] = Q(7, cell); fx[3] = Q(8, cell); }
-        if (fy) { fy[0] = Q(9, cell); fy[1] = Q(7, cell); fy[2] = Q(10, cell); fy[3] = Q(11, cell); }
-    };
-    // x faces: face f of row r sits between tile cells (f-1, r) and (f, r)
-    for (int it = threadIdx.x; it < (TX + 1) * TY; it += NT) {
-        const int fx = it % (TX + 1), fy = it / (TX + 1);
-        if (x0 + fx > nx || y0 + fy >= ny) continue;
-        const int cl = (fy + 1) * L::UX + fx, cr = cl + 1;
-        double UL[4], UR[4], FL[4], FR[4], F[4], aL, aR;
-        Prim wL, wR;
-        load(cl, UL, wL, aL, FL, nullptr);
-        load(cr, UR, wR, aR, FR, nullptr);
-        const int bad = hllc<0>(UL, wL, aL, FL, UR, wR, aR, FR, F);
-        if (bad && owned_face(x0 + fx, fx, TX, nx, y0 + fy, ny)) {
+#pragma unroll 1
+    for (int w = warp; w < fxy; w += NT / 32) {
+        const bool y = w >= fx;
+        const int it = (y ? w - fx : w) * 32 + lane, row = y ? s.row0(it) : s.row1(it), col = it - row * (y ? tx : tx + 1);
+        if (it >= (y ? nfy : nfx) || x0 + col >= nx + (y ? 0 : 1) || y0 + row >= ny + (y ? 1 : 0)) continue;
+        // face f of row r sits between tile cells (f-1, r) and (f, r), or (r, f-1) and (r, f)
+        const int l = (row + (y ? 0 : 1)) * ux + col + (y ? 1 : 0);
+        const int bad = go_face(y, sU, sQ, l, y ? ux : 1, nc, (y ? sG : sF) + it, y ? nfy : nfx);
+        if (bad && (y ? owned_face(y0 + row, row, ty, ny, x0 + col, nx) : owned_face(x0 + col, col, tx, nx, y0 + row, ny))) {
             ++herr;
-            if (first_bad) atomicMin(first_bad, key_base | face_key(0, 0, 0, y0 + fy, x0 + fx));
+            if (first_bad) atomicMin(first_bad, key_base | face_key(0, 0, y ? 1 : 0, y0 + row, x0 + col));
         }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) sF[(v * TY + fy) * (TX + 1) + fx] = F[v];
     }
-    for (int it = threadIdx.x; it < TX * (TY + 1); it += NT) {
-        const int gx = it % TX, gy = it / TX;
-        if (x0 + gx >= nx || y0 + gy > ny) continue;
-        const int cb = gy * L::UX + gx + 1, ct = cb + L::UX;
-        double UB[4], UT[4], FB[4], FT[4], F[4], aB, aT;
-        Prim wB, wT;
-        load(cb, UB, wB, aB, nullptr, FB);
-        load(ct, UT, wT, aT, nullptr, FT);
-        const int bad = hllc<1>(UB, wB, aB, FB, UT, wT, aT, FT, F);
-        if (bad && owned_face(y0 + gy, gy, TY, ny, x0 + gx, nx)) {
-            ++herr;
-            if (first_bad) atomicMin(first_bad, key_base | face_key(0, 0, 1, y0 + gy, x0 + gx));
-        }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) sG[(v * (TY + 1) + gy) * TX + gx] = F[v];
-    }
-#undef Q
     __syncthreads();
     return herr;
 }
 
-// Conservative update + forward Euler of output cell (ox, oy) of the tile, variable v
+// Conservative update + forward Euler of output cell (ox, oy) of the tile
 // (godunov.cpp:97-113; forward_euler.cpp:19-29)
-template <int TX, int TY>
-__device__ __forceinline__ double go_update(const double* __restrict__ sU, const double* __restrict__ sF,
-                                            const double* __restrict__ sG, int v, int ox, int oy, double dt,
-                                            double one_dx, double one_dy) {
-    using L = GoTile<TX, TY>;
-    const double Lv = (one_dx * (sF[(v * TY + oy) * (TX + 1) + ox] - sF[(v * TY + oy) * (TX + 1) + ox + 1])) +
-                      (one_dy * (sG[(v * (TY + 1) + oy) * TX + ox] - sG[(v * (TY + 1) + oy + 1) * TX + ox]));
-    return dt * Lv + sU[v * L::NC + (oy + 1) * L::UX + ox + 1];
+template <class S>
+__device__ __forceinline__ void go_update(const S& s, const double* sU, const double* sW, int ox, int oy, double dt,
+                                          double one_dx, double one_dy, double* un) {
+    const int tx = s.tx(), ty = s.ty(), nc = (tx + 2) * (ty + 2), nfx = (tx + 1) * ty, nfy = tx * (ty + 1);
+    const double* F = sW + 5 * nc + oy * (tx + 1) + ox;
+    const double* G = sW + 5 * nc + 4 * nfx + oy * tx + ox;
+    const double* U = sU + (oy + 1) * (tx + 2) + ox + 1;
+    double a[4], b[4], u[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        a[v] = F[v * nfx] - F[v * nfx + 1];
+        b[v] = G[v * nfy] - G[v * nfy + tx];
+        u[v] = U[v * nc];
+    }
+    if (!update_fast(a, b, u, dt, one_dx, one_dy, un))
+#pragma unroll
+        for (int v = 0; v < 4; ++v) un[v] = update_any(a[v], b[v], u[v], dt, one_dx, one_dy);
 }
 
 }  // namespace hf

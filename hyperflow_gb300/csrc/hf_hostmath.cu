@@ -79,4 +79,21 @@ void hm_update(const double* c, double dt, double one_dx, double one_dy, int64_t
     }
 }
 
+// Godunov: the cells c[k][0] and c[k][2] (n, t order; q [n][2][5]) and the face between them; and TimeStep's
+// terms of c[k][0] (s [n][2]).  Bits of ok: 1 both cells, 2 the face (from the general cells), 4 the terms.
+void hm_godunov(int y, const double* c, double g, double g1, int64_t n, int* ok, int* bad, double* fq, double* aq,
+                double* ff, double* af, double* fs, double* as) {
+    for (int64_t k = 0; k < n; ++k) {
+        const double *l = c + 12 * k, *r = l + 8;
+        double *f = fq + 10 * k, *a = aq + 10 * k;
+        ok[k] = hf::cell_fast(g, g1, l, f) & hf::cell_fast(g, g1, r, f + 5) ? 1 : 0;
+        hf::cell_any(g, g1, l[0], l[1], l[2], l[3], a);
+        hf::cell_any(g, g1, r[0], r[1], r[2], r[3], a + 5);
+        ok[k] |= hf::face_fast(y != 0, l, a, r, a + 5, ff + 4 * k) ? 2 : 0;
+        bad[k] = hf::face_any(y != 0, l, a, r, a + 5, af + 4 * k);
+        ok[k] |= hf::speeds_fast(g, g1, l, fs[2 * k], fs[2 * k + 1]) ? 4 : 0;
+        hf::speeds_any(g, g1, l[0], l[1], l[2], l[3], as + 2 * k);
+    }
+}
+
 }  // extern "C"

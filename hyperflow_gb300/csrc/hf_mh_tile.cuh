@@ -22,19 +22,22 @@
 namespace hf {
 
 // A tile of tx x ty cells: the shape's sizes, and the row of item `it` of a list whose rows are tx, tx + 1
-// or tx + 2 long.  Of fixed size (the batch's configurations) or chosen for a block (MhShape).
+// or tx + 2 long.  Of fixed size (the batch's configurations) or chosen for a block (RowShape).
 template <int TX, int TY>
-struct MhTile {
-    static constexpr int UX = TX + 4, UY = TY + 4;
-    static constexpr int U_SIZE = 4 * UY * UX;                                  // doubles
-    static constexpr int A_SIZE = 8 * ((TX + 2) * TY + TX * (TY + 2));
+struct TileRows {
     __device__ static constexpr int tx() { return TX; }
     __device__ static constexpr int ty() { return TY; }
     __device__ static constexpr int row0(int it) { return it / TX; }
     __device__ static constexpr int row1(int it) { return it / (TX + 1); }
     __device__ static constexpr int row2(int it) { return it / (TX + 2); }
 };
-struct MhShape {
+template <int TX, int TY>
+struct MhTile : TileRows<TX, TY> {
+    static constexpr int UX = TX + 4, UY = TY + 4;
+    static constexpr int U_SIZE = 4 * UY * UX;                                  // doubles
+    static constexpr int WORK = 8 * ((TX + 2) * TY + TX * (TY + 2));
+};
+struct RowShape {
     TileShape t;
     __device__ int tx() const { return t.tx; }
     __device__ int ty() const { return t.ty; }

@@ -23,6 +23,7 @@ def hm():
     L.hm_predict.argtypes = [I, I, P, D, D, N, P, P, P]
     L.hm_face.argtypes = [I, P, D, D, N, P, P, P, P]
     L.hm_update.argtypes = [P, D, D, D, N, P, P, P]
+    L.hm_godunov.argtypes = [I, P, D, D, N, P, P, P, P, P, P, P, P]
     return L
 
 
@@ -80,6 +81,26 @@ def test_fast_functions_equal_the_general_ones(hm, kind, y):
         assert ok.mean() > 0.99
     hm.hm_update(c.ctypes.data, 1.7e-4, 1365.0, 1000.3, n, ok.ctypes.data, fast.ctypes.data, gen.ctypes.data)
     assert same(fast, gen)[ok == 1].all()
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "faint", "unphysical", "scaled", "special"])
+@pytest.mark.parametrize("y", [0, 1])
+def test_godunov_functions_equal_the_general_ones(hm, kind, y):
+    """cells, faces and TimeStep terms; and the faces against hllc on the conservative states"""
+    c = states(kind)
+    n = len(c)
+    g, g1 = 1.4, 1.4 - 1.0
+    ok, bad = np.empty(n, np.int32), np.empty(n, np.int32)
+    out = [np.zeros((n, k)) for k in (10, 10, 4, 4, 2, 2)]
+    hm.hm_godunov(y, c.ctypes.data, g, g1, n, ok.ctypes.data, bad.ctypes.data, *[o.ctypes.data for o in out])
+    for bit, fast, gen in ((1, out[0], out[1]), (2, out[2], out[3]), (4, out[4], out[5])):
+        assert same(fast, gen)[(ok & bit) != 0].all()
+        if kind == "ordinary":
+            assert ((ok & bit) != 0).mean() > 0.99
+    assert not bad[(ok & 2) != 0].any()
+    ok2, bad2, fast, gen = np.empty(n, np.int32), np.empty(n, np.int32), np.zeros((n, 4)), np.empty((n, 4))
+    hm.hm_face(y, c.ctypes.data, g, g1, n, ok2.ctypes.data, bad2.ctypes.data, fast.ctypes.data, gen.ctypes.data)
+    assert same(out[3], gen).all() and (bad == bad2).all()
 
 
 def test_fast_functions_leave_the_window_for_odd_constants(hm):
