@@ -414,4 +414,57 @@ static __host__ __device__ __noinline__ int hllc_any(bool y, double g, double g1
     return bad;
 }
 
+// A state's momentum turned by an angle (euler_ideal_gas.cpp:152-165): (c m1 + s m2, c m2 - s m1)
+HF_HD void turn_fast(Window& w, double c, double s, const double* f, double* o) {
+    const bool zc = zero(c), zs = zero(s), z1 = zero(f[1]), z2 = zero(f[2]);
+    see0(w, c, zc);
+    see0(w, s, zs);
+    see0(w, f[1], z1);
+    see0(w, f[2], z2);
+    o[0] = f[0];
+    o[1] = mulz(c, f[1], zc || z1) + mulz(s, f[2], zs || z2);
+    o[2] = mulz(c, f[2], zc || z2) - mulz(s, f[1], zs || z1);
+    o[3] = f[3];
+}
+// The flux through an unstructured edge of length len between the states U and V: turned into the edge's
+// frame (c, s), the HLLC flux there, turned back (cn, sn) and scaled
+HF_HD bool edge_fast(double c, double s, double cn, double sn, double len, double g, double g1, const double* U,
+                     const double* V, double* f) {
+    Window w;
+    double a[4], b[4], F[4], t[4];
+    turn_fast(w, c, s, U, a);
+    turn_fast(w, c, s, V, b);
+    if (outside(w) || !hllc_fast(false, g, g1, a, b, F)) return false;
+    turn_fast(w, cn, sn, F, t);
+    see(w, len);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const bool z = zero(t[v]);
+        see0(w, t[v], z);
+        f[v] = mulz(len, t[v], z);
+    }
+    return !outside(w);
+}
+// The unstructured update dt (-(inv acc)) + U of a cell, and its TimeStep term r_in / (|V| + c)
+HF_HD bool uns_update_fast(double g, double g1, double dt, double inv, double rin, const double* acc, const double* U,
+                           double* un, double& term) {
+    Window w;
+    see(w, g);
+    see(w, g1);
+    see(w, dt);
+    see(w, inv);
+    see_pos(w, rin);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const bool z = zero(acc[v]);
+        see0(w, acc[v], z);
+        un[v] = U[v] - mulz(dt, mulz(inv, acc[v], z), z);
+    }
+    const PrimN a = prim_n(w, g1, un);
+    const double c = sound_n(g, a), sp = (a.zn && a.zt ? 0.0 : root32(f64_bits(a.q))) + c;
+    see_pos(w, sp);
+    term = quot(rin, sp, rcp32(sp));
+    return !outside(w);
+}
+
 }  // namespace hf

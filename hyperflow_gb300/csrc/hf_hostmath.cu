@@ -96,4 +96,33 @@ void hm_godunov(int y, const double* c, double g, double g1, int64_t n, int* ok,
     }
 }
 
+// The flux through an unstructured edge between c[k][0] and c[k][2], geo [n][5] = cos, sin, cos and sin of the
+// opposite angle, length; and the update of c[k][1] with c[k][0] as the flux sum: [n][5] with the TimeStep
+// term.  Bits of ok: 1 the edge, 2 the update.
+void hm_uns(const double* c, const double* geo, double g, double g1, double dt, double rin, int64_t n, int* ok,
+            int* bad, double* ff, double* af, double* fu, double* au) {
+    auto rot = [](double a, double b, const double* f, double* o) {
+        o[0] = f[0];
+        o[1] = a * f[1] + b * f[2];
+        o[2] = (-b) * f[1] + a * f[2];
+        o[3] = f[3];
+    };
+    for (int64_t k = 0; k < n; ++k) {
+        const double *l = c + 12 * k, *m = l + 4, *r = l + 8, *q = geo + 5 * k;
+        ok[k] = hf::edge_fast(q[0], q[1], q[2], q[3], q[4], g, g1, l, r, ff + 4 * k) ? 1 : 0;
+        double a[4], b[4], F[4];
+        rot(q[0], q[1], l, a);
+        rot(q[0], q[1], r, b);
+        bad[k] = hf::hllc_cons<0>(g, g1, a, b, F);
+        rot(q[2], q[3], F, a);
+        for (int v = 0; v < 4; ++v) af[4 * k + v] = q[4] * a[v];
+        double* u = au + 5 * k;
+        ok[k] |= hf::uns_update_fast(g, g1, dt, q[4], rin, l, m, fu + 5 * k, fu[5 * k + 4]) ? 2 : 0;
+        for (int v = 0; v < 4; ++v) u[v] = dt * (-(q[4] * l[v])) + m[v];
+        double uu, vv, p;
+        hf::to_prim_short(g1, u[0], u[1], u[2], u[3], uu, vv, p);
+        u[4] = hf::div_rn(rin, std::fabs(hf::sqrt_rn(uu * uu + vv * vv)) + hf::sound(g, u[0], p));
+    }
+}
+
 }  // extern "C"

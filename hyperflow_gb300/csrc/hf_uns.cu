@@ -29,6 +29,7 @@
 #include "../../include/hyperflow_gb300_uns.h"
 #include "hf_ctrl.h"
 #include "hf_device.cuh"
+#include "hf_fast.cuh"
 #include "hf_trace.h"
 #include "hf_json.hpp"
 
@@ -77,6 +78,7 @@ struct UnsMesh {
     // cells are held in a locality order (Morton order of their vertex centroids); orig[i] is
     // the mesh file's index of device cell i, used in the failure records' keys
     const int* __restrict__ orig;
+    unsigned int* ticket;                   // CTAs of a step kernel that are done
 };
 
 // rotate_flow_values (euler_ideal_gas.cpp:152-165) with precomputed cos/sin
@@ -96,8 +98,21 @@ __device__ __forceinline__ double uns_dt_term(double g, double g1, double rin, c
     return div_rn(rin, fabs(sqrt_rn(uu * uu + vv * vv)) + c);
 }
 
-// NaN-skipping min of non-negative values
-__device__ __forceinline__ double nmin(double m, double s) { return (s < m) ? s : m; }
+// a cell's update (un[0..3]) and its TimeStep term (un[4]), the general form; false: density or pressure
+// not positive
+__device__ __noinline__ bool uns_update_any(double g, double g1, double dt, double inv, double rin, const double* acc,
+                                            const double* cv, double* un) {
+    for (int v = 0; v < 4; ++v) {
+        const double L = -(inv * acc[v]);   // -1.0 * (...) of godunov.cpp, exactly
+        un[v] = dt * L + cv[v];
+    }
+    bool pos;
+    un[4] = uns_dt_term(g, g1, rin, un, pos);
+    return pos;
+}
+
+// NaN-skipping min of non-negative values, on the bit patterns (they order as the values; NaN is above all)
+__device__ __forceinline__ double nmin(double m, double s) { return f64_bits(s) < f64_bits(m) ? s : m; }
 
 template <int NT>
 __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* acc) {
@@ -111,11 +126,13 @@ __device__ __forceinline__ void block_min_atomic(double v, unsigned long long* a
         v = l < NT / 32 ? red[l] : 1e16;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v = nmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-        if (l == 0 && v < 1e16) atomicMin(acc, dbits(v));
+        if (l == 0 && f64_bits(v) < f64_bits(1e16)) atomicMin(acc, dbits(v));
     }
 }
 
-constexpr int kUnsNT = 256;
+// Small CTAs: on 120k cells, 1.5 waves of 256-thread CTAs, 128 threads take 6 - 10 % off a step (4000 cells
+// 15 %); on 1M cells they cost 1 %.
+constexpr int kUnsNT = 128;
 
 // key of a cell in the error records (a zero-flux pair's cell, a non-positive cell): step (24
 // bits), then cell (40 bits)
@@ -124,8 +141,36 @@ __device__ __forceinline__ unsigned long long uns_key(long long step, long long 
     return (s << 40) | ((unsigned long long)cell & 0xFFFFFFFFFFull);
 }
 
+// length x rotated-back HLLC flux between the states cv and nb (given as it is, before the rotation into
+// the edge's frame), the general form; returns 1 for the zero-flux fallback
+__device__ __noinline__ int edge_any(double ca, double sa, double cn, double sn, double len, double g, double g1,
+                                     const double* cv, const double* nb, double* f) {
+    double rc[4], rn[4], rf[4], fr[4];
+    rot(ca, sa, cv, rc);
+    rot(ca, sa, nb, rn);
+    const int bad = hllc_cons<0>(g, g1, rc, rn, rf);
+    rot(cn, sn, rf, fr);
+    for (int v = 0; v < 4; ++v) f[v] = len * fr[v];
+    return bad;
+}
+
+// the flux of an edge with geometry geo[k * stride], k = 0 .. 4 (cos, sin, cos and sin of the opposite
+// angle, length): the integer-pipe path, or the general one for states outside its window
+__device__ __forceinline__ int geo_flux(const double* __restrict__ geo, size_t stride, double g, double g1,
+                                        const double* cv, const double* nb, double* f) {
+    const double ca = geo[0], sa = geo[stride], cn = geo[2 * stride], sn = geo[3 * stride], len = geo[4 * stride];
+    if (edge_fast(ca, sa, cn, sn, len, g, g1, cv, nb, f)) return 0;
+    const double c4[4] = {cv[0], cv[1], cv[2], cv[3]}, n4[4] = {nb[0], nb[1], nb[2], nb[3]};
+    double x[4];   // copies, so that the fast path's stay in registers
+    const int bad = edge_any(ca, sa, cn, sn, len, g, g1, c4, n4, x);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) f[v] = x[v];
+    return bad;
+}
+
 // length x rotated-back HLLC flux of the pair (owner cell c, neighbour cell k); in checked
 // builds a pair or neighbour index outside the mesh raises the error word and gives a zero flux
+template <bool RARE>
 __device__ __forceinline__ int pair_flux(const UnsMesh& m, const double* __restrict__ U, size_t N, double g,
                                          double g1, int e, const double* cv, double* f, int* err) {
     if (!hf_in(e, m.npairs, err) || (m.nbr[e] >= 0 && !hf_in(m.nbr[e], m.ncells, err))) {
@@ -133,31 +178,32 @@ __device__ __forceinline__ int pair_flux(const UnsMesh& m, const double* __restr
         for (int v = 0; v < 4; ++v) f[v] = 0.0;
         return 0;
     }
-    const double ca = m.geo[e], sa = m.geo[m.npairs + e];
-    const double cn = m.geo[2 * m.npairs + e], sn = m.geo[3 * m.npairs + e];
-    const double len = m.geo[4 * m.npairs + e];
     const int k = m.nbr[e];
-    double rc[4], rn[4];
-    rot(ca, sa, cv, rc);
+    double nb[4];
     if (k >= 0) {
-        double nb[4] = {U[k], U[N + k], U[2 * N + k], U[3 * N + k]};
-        rot(ca, sa, nb, rn);
+        nb[0] = U[k]; nb[1] = U[N + k]; nb[2] = U[2 * N + k]; nb[3] = U[3 * N + k];
     } else if (k == -1) {   // reflective: rotate, negate normal momentum, rotate back
-        double r1[4], nb[4];
-        r1[0] = rc[0]; r1[1] = rc[1] * -1.0; r1[2] = rc[2]; r1[3] = rc[3];
-        rot(cn, sn, r1, nb);
-        rot(ca, sa, nb, rn);
+        double rc[4];
+        rot(m.geo[e], m.geo[m.npairs + e], cv, rc);
+        rc[1] = rc[1] * -1.0;
+        rot(m.geo[2 * m.npairs + e], m.geo[3 * m.npairs + e], rc, nb);
     } else if (k == -2) {   // transmissive: the cell's own state
-        rot(ca, sa, cv, rn);
-    } else {                // inlet
-        rot(ca, sa, m.inlet, rn);
-    }
-    double rf[4], fr[4];
-    const int bad = hllc_cons<0>(g, g1, rc, rn, rf);
-    rot(cn, sn, rf, fr);
 #pragma unroll
-    for (int v = 0; v < 4; ++v) f[v] = len * fr[v];
-    return bad;
+        for (int v = 0; v < 4; ++v) nb[v] = cv[v];
+    } else {                // inlet
+#pragma unroll
+        for (int v = 0; v < 4; ++v) nb[v] = m.inlet[v];
+    }
+    if (RARE) {   // the boundary pairs of edge mode: the general form alone, out of line
+        const double* q = m.geo + e;
+        const double c4[4] = {cv[0], cv[1], cv[2], cv[3]};
+        double x[4];
+        const int bad = edge_any(q[0], q[m.npairs], q[2 * m.npairs], q[3 * m.npairs], q[4 * m.npairs], g, g1, c4, nb, x);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) f[v] = x[v];
+        return bad;
+    }
+    return geo_flux(m.geo + e, (size_t)m.npairs, g, g1, cv, nb, f);
 }
 
 // pair_flux of an interior edge's owning pair from the per-edge arrays (the same arithmetic):
@@ -170,24 +216,25 @@ __device__ __forceinline__ int edge_flux(const UnsMesh& m, const double* __restr
         for (int v = 0; v < 4; ++v) f[v] = 0.0;
         return 0;
     }
-    const size_t E = (size_t)m.nedges;
-    const double ca = m.edge_geo[e], sa = m.edge_geo[E + e];
-    const double cn = m.edge_geo[2 * E + e], sn = m.edge_geo[3 * E + e];
-    const double len = m.edge_geo[4 * E + e];
-    double rc[4], rn[4], nb[4] = {U[k], U[N + k], U[2 * N + k], U[3 * N + k]};
-    rot(ca, sa, cv, rc);
-    rot(ca, sa, nb, rn);
-    double rf[4], fr[4];
-    const int bad = hllc_cons<0>(g, g1, rc, rn, rf);
-    rot(cn, sn, rf, fr);
-#pragma unroll
-    for (int v = 0; v < 4; ++v) f[v] = len * fr[v];
-    return bad;
+    const double nb[4] = {U[k], U[N + k], U[2 * N + k], U[3 * N + k]};
+    return geo_flux(m.edge_geo + e, (size_t)m.nedges, g, g1, cv, nb, f);
+}
+
+// A step of the loop without frames and strict mode takes its stop flag and dt (a TimeStep call, timestep.cpp:29-62, clamped
+// as simulation.cpp:85-88) from the control block itself, in every CTA alike -- nothing they depend on
+// changes before the step's last CTA has ended the step (kStepForms | kStepEnds): one or two launches a
+// step where its start and its end were kernels of one thread beside them.
+enum { kStepForms = 1, kStepEnds = 2 };
+__device__ __forceinline__ bool uns_loop_done(const UnsCtrl* c) { return c->clamp && c->t == c->t_end; }
+__device__ __forceinline__ double uns_loop_dt(const UnsCtrl* c) {
+    const double dtr = smin(1e16, bitsd(c->min_dt[(int)(c->step & 1)]));
+    const double dt = ((c->calls + 1 <= 10) ? 0.2 * c->cfl : c->cfl) * dtr;
+    return c->clamp && c->t + dt > c->t_end ? c->t_end - c->t : dt;
 }
 
 // edge-based mode, pass 1: one flux per unique interior edge, from its owner's side
-__global__ void __launch_bounds__(kUnsNT, 3) uns_edge_flux_kernel(UnsCtrl* __restrict__ c, UnsMesh m) {
-    if (c->done) return;
+__global__ void __launch_bounds__(kUnsNT, 6) uns_edge_flux_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int mode) {
+    if (mode & kStepForms ? uns_loop_done(c) : c->done != 0) return;
     const int p = (int)(c->step & 1);
     const double g = c->gamma, g1 = c->g1;
     const size_t N = (size_t)m.ncells;
@@ -207,15 +254,35 @@ __global__ void __launch_bounds__(kUnsNT, 3) uns_edge_flux_kernel(UnsCtrl* __res
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
 
-__global__ void __launch_bounds__(kUnsNT) uns_cfl_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int parity) {
+// a state in the mesh file's order (the other buffer) into the device's order, with its TimeStep terms
+__global__ void __launch_bounds__(kUnsNT) uns_load_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int parity) {
     double mn = 1e16;
-    const double* U = m.U[parity];
+    const size_t N = (size_t)m.ncells;
+    const double* __restrict__ F = m.U[parity ^ 1];
+    double* __restrict__ U = m.U[parity];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.ncells; i += gridDim.x * blockDim.x) {
-        double u[4] = {U[i], U[m.ncells + i], U[2 * (size_t)m.ncells + i], U[3 * (size_t)m.ncells + i]};
+        const int o = m.orig[i];
+        if (!hf_in(o, m.ncells, &c->err)) continue;
+        const double u[4] = {F[o], F[N + o], F[2 * N + o], F[3 * N + o]};
+#pragma unroll
+        for (int v = 0; v < 4; ++v) U[v * N + i] = u[v];
         bool pos;
         mn = nmin(mn, uns_dt_term(c->gamma, c->g1, m.rin[i], u, pos));
     }
     block_min_atomic<kUnsNT>(mn, &c->min_dt[parity]);
+}
+
+// the state into the mesh file's order, in the other buffer (the next step overwrites it)
+__global__ void __launch_bounds__(kUnsNT) uns_store_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int parity) {
+    const size_t N = (size_t)m.ncells;
+    const double* __restrict__ U = m.U[parity];
+    double* __restrict__ F = m.U[parity ^ 1];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.ncells; i += gridDim.x * blockDim.x) {
+        const int o = m.orig[i];
+        if (!hf_in(o, m.ncells, &c->err)) continue;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) F[v * N + o] = U[v * N + i];
+    }
 }
 
 // start of a device-loop step: stop at t_end, form dt (TimeStep call), reset the accumulator
@@ -273,6 +340,16 @@ __global__ void __launch_bounds__(256) uns_frame_copy_kernel(const UnsCtrl* __re
     }
 }
 
+// t and the step counted; the next step's minimum starts over
+__device__ __forceinline__ void uns_end_step(UnsCtrl* c) {
+    const int p = (int)(c->step & 1);
+    c->t = c->t + c->dt;
+    c->step = c->step + 1;
+    c->min_dt[p] = dbits(1e16);
+}
+// the same for a step that no ended step came before
+__global__ void uns_clean_kernel(UnsCtrl* c) { c->min_dt[(int)(c->step & 1) ^ 1] = dbits(1e16); }
+
 __global__ void uns_finalize_kernel(UnsCtrl* c) {
     if (c->done) return;
     if (c->clamp && c->frames) {
@@ -285,18 +362,24 @@ __global__ void uns_finalize_kernel(UnsCtrl* c) {
             c->captured = c->captured + 1;
         }
     }
-    c->t = c->t + c->dt;
-    c->step = c->step + 1;
+    uns_end_step(c);
 }
 
-// MINB: CTAs per SM the registers are budgeted for -- three in edge mode (the per-cell work is a
-// gather of precomputed edge fluxes, and more warps hide its latency), two in the per-pair mode
-// (its HLLC needs the registers: 128 per thread; at 148 only one CTA fits and it runs 27 % slower)
-template <int MINB>
-__global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restrict__ c, UnsMesh m) {
-    if (c->done) return;
+// The products, quotients and roots of a pair on the integer pipes (hf_fast.cuh), as the stencils': per pair
+// 40 FP64 instructions of 83, and no out-of-line calls.  Measured (Mcell-updates/s, 1M triangles): 1232 ->
+// 2550 with a flux per pair, 1992 -> 3450 with a flux per edge (of these two the long division alone 1650
+// and 2500).
+// MINB: CTAs per SM the registers are budgeted for -- six in edge mode (the per-cell work is a
+// gather of precomputed edge fluxes, and more warps hide its latency), four in the per-pair mode
+// (its HLLC needs the registers: 128 per thread)
+template <int MINB, bool EDGES>
+__global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int mode) {
+    if (mode & kStepForms ? uns_loop_done(c) : c->done != 0) {
+        if ((mode & kStepForms) && blockIdx.x == 0 && threadIdx.x == 0) c->done = 1;
+        return;
+    }
     const int p = (int)(c->step & 1);
-    const double g = c->gamma, g1 = c->g1, dt = c->dt;
+    const double g = c->gamma, g1 = c->g1, dt = mode & kStepForms ? uns_loop_dt(c) : c->dt;
     const size_t N = (size_t)m.ncells;
     const double* __restrict__ U = m.U[p];
     double* __restrict__ Un = m.U[p ^ 1];
@@ -308,7 +391,7 @@ __global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restr
         const int e0 = m.pair_start[i], e1 = m.pair_start[i + 1];
         for (int e = e0; e < e1; ++e) {
             double f[4];
-            const int ed = m.pair_edge && hf_in(e, m.npairs, &c->err) ? m.pair_edge[e] : -1;
+            const int ed = EDGES && hf_in(e, m.npairs, &c->err) ? m.pair_edge[e] : -1;
             if (ed >= 0 && hf_in(ed, m.nedges, &c->err)) {   // edge-based mode: the owner's flux, negated on the other side
                 // (a sign flip, not a multiplication by -1.0: the same value, off the FP64 pipe)
                 const bool neg = m.pair_sign[e] < 0;
@@ -317,27 +400,43 @@ __global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restr
                     const double x = m.edge_flux[(size_t)v * m.nedges + ed];
                     f[v] = neg ? -x : x;
                 }
-            } else if (pair_flux(m, U, N, g, g1, e, cv, f, &c->err)) {
+            } else if (pair_flux<EDGES>(m, U, N, g, g1, e, cv, f, &c->err)) {
                 ++herr;
                 atomicMin(&c->first_bad, uns_key(c->step, m.orig[i]));
             }
 #pragma unroll
             for (int v = 0; v < 4; ++v) acc[v] = acc[v] + f[v];
         }
-        const double inv = m.inv_area[i];
-        double un[4];
+        double un[4], term;
+        bool pos = true;   // the fast path's states are
+        if (!uns_update_fast(g, g1, dt, m.inv_area[i], m.rin[i], acc, cv, un, term)) {
+            const double a4[4] = {acc[0], acc[1], acc[2], acc[3]}, c4[4] = {cv[0], cv[1], cv[2], cv[3]};
+            double x[5];   // copies, so that the fast path's stay in registers
+            pos = uns_update_any(g, g1, dt, m.inv_area[i], m.rin[i], a4, c4, x);
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const double L = -(inv * acc[v]);   // -1.0 * (...) of godunov.cpp, exactly
-            un[v] = dt * L + cv[v];
-            Un[v * N + i] = un[v];
+            for (int v = 0; v < 4; ++v) un[v] = x[v];
+            term = x[4];
         }
-        bool pos;
-        mn = nmin(mn, uns_dt_term(g, g1, m.rin[i], un, pos));
+#pragma unroll
+        for (int v = 0; v < 4; ++v) Un[v * N + i] = un[v];
+        mn = nmin(mn, term);
         if (!pos) atomicMin(&c->first_nonpos, uns_key(c->step, m.orig[i]));
     }
     block_min_atomic<kUnsNT>(mn, &c->min_dt[p ^ 1]);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
+    if (!(mode & kStepEnds)) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(m.ticket, 1u) != gridDim.x - 1) return;
+    *m.ticket = 0u;   // every other CTA has read what the end of the step changes
+    if (mode & kStepForms) {
+        c->done = 0;
+        c->snap_pre = c->snap_post = 0;
+        c->dt = dt;
+        c->calls = c->calls + 1;
+    }
+    uns_end_step(c);
 }
 
 }  // namespace hf
@@ -372,6 +471,7 @@ struct hf_uns {
     int strict = 0;                     // hf_uns_set_strict
     bool has_anim = false;
     double anim_duration = 0.0, anim_fps = 0.0;
+    bool clean = false;                 // the next step's minimum starts over (an ended step came before)
     double* ring = nullptr;             // device frame ring
     int ring_slots = 0;
     long long drained = 0;
@@ -717,12 +817,7 @@ void build_geometry(hf_uns* u) {
     }
 }
 
-// a [4][ncells] state in the mesh file's cell order into u->stage in device order, and back
-void to_device_order(hf_uns* u, const double* cons) {
-    const size_t n = (size_t)u->ncells;
-    for (int v = 0; v < 4; ++v)
-        for (size_t d = 0; d < n; ++d) u->stage[v * n + d] = cons[v * n + (size_t)u->perm[d]];
-}
+// the [4][ncells] state in u->stage (device order) into the mesh file's cell order
 void to_file_order(const hf_uns* u, double* cons) {
     const size_t n = (size_t)u->ncells;
     for (int v = 0; v < 4; ++v)
@@ -802,7 +897,6 @@ int finish_create(hf_uns* u, const Json& cfg) {
             u->perm[d] = (int)(key[d] & 0xFFFFFFFFu);
             u->iperm[u->perm[d]] = d;
         }
-        u->stage.resize((size_t)4 * n);
     }
     const std::vector<int>& perm = u->perm;
     const std::vector<int>& iperm = u->iperm;
@@ -900,6 +994,9 @@ int finish_create(hf_uns* u, const Json& cfg) {
         u->allocs.push_back(p);
         u->dm.U[k] = p;
     }
+    UCK(cudaMalloc(&u->dm.ticket, sizeof(unsigned int)));
+    u->allocs.push_back(u->dm.ticket);
+    UCK(cudaMemset(u->dm.ticket, 0, sizeof(unsigned int)));
     hf::UnsCtrl C{};
     C.gamma = u->gamma;
     C.g1 = u->gamma - 1.0;
@@ -913,24 +1010,26 @@ int finish_create(hf_uns* u, const Json& cfg) {
     return hf_uns_set_state(u, u->init.data());
 }
 
+// A step's kernels.  prep: a step of the loop, which forms its own dt; else c->dt is given.  With frames
+// on, or in strict mode (whose records change during a step), a kernel before it forms the stop flag, dt
+// and frame points, and one after it ends the step.
 int enqueue_uns_step(hf_uns* u, bool prep) {
-    int grid = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
-    if (prep) hf::uns_prep_kernel<<<1, 1, 0, u->stream>>>(u->dctrl);
+    const int grid = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
+    const bool frames = u->ring_slots > 0, fused = !frames && !u->strict;
+    if (prep && !fused) hf::uns_prep_kernel<<<1, 1, 0, u->stream>>>(u->dctrl);
+    const int mode = !fused ? 0 : (prep ? hf::kStepForms | hf::kStepEnds : hf::kStepEnds);
     hf::UnsMesh m = u->dm;
     if (u->edge_mode) {
         m.pair_edge = u->d_pair_edge;
         m.pair_sign = u->d_pair_sign;
-        int eg = (m.nedges + hf::kUnsNT - 1) / hf::kUnsNT;
-        hf::uns_edge_flux_kernel<<<eg < 1 ? 1 : eg, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m);
+        const int eg = (m.nedges + hf::kUnsNT - 1) / hf::kUnsNT;
+        hf::uns_edge_flux_kernel<<<eg < 1 ? 1 : eg, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
+        hf::uns_step_kernel<6, true><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
     } else {
-        m.pair_edge = nullptr;
+        hf::uns_step_kernel<4, false><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
     }
-    if (u->edge_mode)
-        hf::uns_step_kernel<3><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m);
-    else
-        hf::uns_step_kernel<2><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m);
-    if (u->ring_slots > 0) hf::uns_frame_copy_kernel<<<4 * 152, 256, 0, u->stream>>>(u->dctrl, m, u->ring);
-    hf::uns_finalize_kernel<<<1, 1, 0, u->stream>>>(u->dctrl);
+    if (frames) hf::uns_frame_copy_kernel<<<4 * 152, 256, 0, u->stream>>>(u->dctrl, m, u->ring);
+    if (!fused) hf::uns_finalize_kernel<<<1, 1, 0, u->stream>>>(u->dctrl);
     UCK(cudaGetLastError());
     return HF_OK;
 }
@@ -1094,15 +1193,15 @@ int hf_uns_set_state(hf_uns* u, const double* cons) {
     if (r) return r;
     int p = (int)(s & 1);
     size_t bytes = (size_t)4 * u->ncells * sizeof(double);
-    to_device_order(u, cons);
-    UCK(cudaMemcpyAsync(u->dm.U[p], u->stage.data(), bytes, cudaMemcpyHostToDevice, u->stream));
+    // in the file's order into the other buffer, and from there by a kernel into the device's order
+    UCK(cudaMemcpyAsync(u->dm.U[p ^ 1], cons, bytes, cudaMemcpyHostToDevice, u->stream));
     unsigned long long init = 0;
     double big = 1e16;
     std::memcpy(&init, &big, 8);
     UCK(cudaMemcpyAsync(&u->dctrl->min_dt[p], &init, 8, cudaMemcpyHostToDevice, u->stream));
     int grid = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
     if (grid > 8 * 152) grid = 8 * 152;
-    hf::uns_cfl_kernel<<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, u->dm, p);
+    hf::uns_load_kernel<<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, u->dm, p);
     UCK(cudaGetLastError());
     UCK(cudaStreamSynchronize(u->stream));
     return HF_OK;
@@ -1113,8 +1212,12 @@ int hf_uns_get_state(hf_uns* u, double* cons) {
     long long s;
     int r = read_step(u, &s);
     if (r) return r;
-    UCK(cudaMemcpy(u->stage.data(), u->dm.U[s & 1], (size_t)4 * u->ncells * sizeof(double), cudaMemcpyDeviceToHost));
-    to_file_order(u, cons);
+    // a kernel writes it in the file's order into the other buffer; the host's scatter of 1M cells took 7 ms
+    const int p = (int)(s & 1), want = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
+    hf::uns_store_kernel<<<want > 8 * 152 ? 8 * 152 : want, hf::kUnsNT, 0, u->stream>>>(u->dctrl, u->dm, p);
+    UCK(cudaGetLastError());
+    UCK(cudaMemcpyAsync(cons, u->dm.U[p ^ 1], (size_t)4 * u->ncells * sizeof(double), cudaMemcpyDeviceToHost, u->stream));
+    UCK(cudaStreamSynchronize(u->stream));
     return HF_OK;
 }
 
@@ -1145,6 +1248,11 @@ int hf_uns_sync(hf_uns* u) {
 
 int hf_uns_set_strict(hf_uns* u, int on) {
     if (!u || !u->dctrl) return HF_ERR_ARG;
+    if (u->strict != (on ? 1 : 0)) {
+        UCK(cudaStreamSynchronize(u->stream));
+        for (int k = 0; k < 2; ++k)   // the captured steps are the other mode's
+            if (u->graph[k]) { cudaGraphExecDestroy(u->graph[k]); u->graph[k] = nullptr; }
+    }
     u->strict = on ? 1 : 0;
     UCK(cudaMemcpyAsync(&u->dctrl->strict, &u->strict, sizeof(int), cudaMemcpyHostToDevice, u->stream));
     UCK(cudaStreamSynchronize(u->stream));
@@ -1212,6 +1320,8 @@ int hf_uns_run(hf_uns* u, int64_t n, int clamp_t_end, int use_graph, int64_t* st
     if (r) return r;
     int clamp = clamp_t_end ? 1 : 0;
     UCK(cudaMemcpyAsync(&u->dctrl->clamp, &clamp, sizeof clamp, cudaMemcpyHostToDevice, u->stream));
+    if (!u->clean) hf::uns_clean_kernel<<<1, 1, 0, u->stream>>>(u->dctrl);
+    u->clean = true;
     if (use_graph) {
         if (!u->graph[clamp]) {
             cudaGraph_t g;
@@ -1372,6 +1482,7 @@ int hf_uns_checkpoint_load(hf_uns* u, const void* buf, size_t bytes) {
     C.err = 0;
     C.strict = cur.strict;
     u->drained = 0;
+    u->clean = false;
     const size_t n = (size_t)4 * u->ncells * sizeof(double);
     for (int k = 0; k < 2; ++k) {
         UCK(cudaMemcpy(u->dm.U[k], p, n, cudaMemcpyHostToDevice));
@@ -1390,6 +1501,7 @@ int hf_uns_frame_pop(hf_uns* u, double* cons, double* t, int64_t* index) {
     if (C.captured == u->drained) return ufail(u, HF_ERR_STATE, "no frame pending");
     const long long slot = u->drained % u->ring_slots, len = 4LL * u->ncells;
     if (cons) {
+        u->stage.resize((size_t)len);
         UCK(cudaMemcpy(u->stage.data(), u->ring + slot * len, (size_t)len * sizeof(double), cudaMemcpyDeviceToHost));
         to_file_order(u, cons);
     }

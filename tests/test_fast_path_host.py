@@ -23,6 +23,7 @@ def hm():
     L.hm_predict.argtypes = [I, I, P, D, D, N, P, P, P]
     L.hm_face.argtypes = [I, P, D, D, N, P, P, P, P]
     L.hm_update.argtypes = [P, D, D, D, N, P, P, P]
+    L.hm_uns.argtypes = [P, P, D, D, D, D, N, P, P, P, P, P, P]
     L.hm_godunov.argtypes = [I, P, D, D, N, P, P, P, P, P, P, P, P]
     return L
 
@@ -101,6 +102,26 @@ def test_godunov_functions_equal_the_general_ones(hm, kind, y):
     ok2, bad2, fast, gen = np.empty(n, np.int32), np.empty(n, np.int32), np.zeros((n, 4)), np.empty((n, 4))
     hm.hm_face(y, c.ctypes.data, g, g1, n, ok2.ctypes.data, bad2.ctypes.data, fast.ctypes.data, gen.ctypes.data)
     assert same(out[3], gen).all() and (bad == bad2).all()
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "faint", "unphysical", "scaled", "special"])
+def test_unstructured_functions_equal_the_general_ones(hm, kind):
+    """edges at any angle (along the axes among them, where a sine or cosine is zero) and cell updates"""
+    c = states(kind)
+    n = len(c)
+    rng = np.random.default_rng(5)
+    a = rng.uniform(-np.pi, np.pi, n)
+    a[::5] = rng.integers(-2, 3, len(a[::5])) * (np.pi / 2)
+    geo = np.stack([np.cos(a), np.sin(a), np.cos(-a), np.sin(-a), 10.0 ** rng.uniform(-4, 0, n)], 1)
+    geo[::10, :4] = np.round(geo[::10, :4])
+    ok, bad = np.empty(n, np.int32), np.empty(n, np.int32)
+    out = [np.zeros((n, k)) for k in (4, 4, 5, 5)]
+    hm.hm_uns(c.ctypes.data, geo.ctypes.data, 1.4, 1.4 - 1.0, 1e-3, 0.01, n, ok.ctypes.data, bad.ctypes.data,
+              *[o.ctypes.data for o in out])
+    assert same(out[0], out[1])[(ok & 1) != 0].all() and not bad[(ok & 1) != 0].any()
+    assert same(out[2], out[3])[(ok & 2) != 0].all()
+    if kind == "ordinary":
+        assert ((ok & 1) != 0).mean() > 0.98 and ((ok & 2) != 0).mean() > 0.95
 
 
 def test_fast_functions_leave_the_window_for_odd_constants(hm):
