@@ -768,6 +768,139 @@ __global__ void __launch_bounds__(kNT, 2) godunov_step_kernel(Ctrl* __restrict__
 }
 
 // ------------------------------------------------------------------------------------
+// a step of one block in one launch
+// ------------------------------------------------------------------------------------
+// Where every ghost cell takes an interior cell's value (transmissive and reflective sides, up to the sign of
+// a momentum) or a Dirichlet state, TimeStep's largest wave speed over the ghost cells is one of the
+// interior's or of those states, so dt is known before any ghost is filled: every CTA forms it from the
+// maxima the last step left, writes the ghosts of its own tile's halo in shared memory, and stores them with
+// its update.  The fill, a chain of dependent loads, quotients and a reduction over few cells, took 9 to
+// 11 us a step beside 20 to 25 us for the stencil of a small mesh (100 x 5, 256^2).  Steps with frames,
+// strict mode (whose records change during a step) or one launch per block keep the fill.
+__global__ void prepare_solo_kernel(Ctrl* c, const MeshDev* m, StepState* ss) {
+    double mx = 0.0, my = 0.0;
+    for (int side = 0; side < 4; ++side) {
+        if (m->b[0].bc_type[side] != BC_DIRICHLET) continue;
+        const double* u = m->b[0].bc_state[side];
+        double sx, sy;
+        wave_terms(c->gamma, c->g1, u[0], u[1], u[2], u[3], sx, sy);
+        mx = nmax(mx, sx);
+        my = nmax(my, sy);
+    }
+    ss->solo[0] = mx;
+    ss->solo[1] = my;
+    ss->solo[2] = div_rn(1.0, c->dx[0]);
+    ss->solo[3] = div_rn(1.0, c->dy[0]);
+}
+
+// the ghost cells in the tile's halo by the fill program, from the interior cells of U
+template <int G>
+__device__ __forceinline__ void tile_ghosts(double* sU, const MeshDev* __restrict__ m, const double* __restrict__ U,
+                                            int tx, int ty, int x0, int y0, int* err) {
+    const BlockDev& B = m->b[0];
+    if (x0 >= G && y0 >= G && x0 + tx + G <= B.nx && y0 + ty + G <= B.ny) return;
+    const int ux = tx + 2 * G, uy = ty + 2 * G;
+    const size_t plane = (size_t)B.ty * B.pitch;
+    for (int it = threadIdx.x; it < ux * uy; it += kNT) {
+        const int ly = it / ux, lx = it - ly * ux, i = x0 + lx, j = y0 + ly;   // in the block, ghosts included
+        if (i >= B.tx || j >= B.ty || (i >= G && i < B.tx - G && j >= G && j < B.ty - G)) continue;
+        const long long k = j < G ? (long long)j * B.tx + i
+                          : j >= B.ty - G ? (long long)(G + j - (B.ty - G)) * B.tx + i
+                          : 2LL * G * B.tx + (long long)(j - G) * (2 * G) + (i < G ? i : i - (B.tx - 2 * G));
+        const FillOp op = m->fill[k];
+        double u[4];
+        if (op.kind == 2) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) u[v] = B.bc_state[op.side][v];
+        } else {
+            if (!hf_in(op.src, (long long)plane, err)) continue;
+#pragma unroll
+            for (int v = 0; v < 4; ++v) u[v] = U[v * plane + op.src];
+        }
+        if (op.neg & 1) u[1] = -1.0 * u[1];
+        if (op.neg & 2) u[2] = -1.0 * u[2];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) sU[v * ux * uy + it] = u[v];
+    }
+    __syncthreads();
+}
+
+// SCHEME 0 Godunov, 1 MUSCL-Hancock with limiter LIM
+template <int SCHEME, int LIM>
+__global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
+                                                      StepState* __restrict__ ss, const TileShape tile,
+                                                      const __grid_constant__ CUtensorMap tm0,
+                                                      const __grid_constant__ CUtensorMap tm1) {
+    constexpr int G = SCHEME == 0 ? 1 : 2;
+    extern __shared__ __align__(1024) double smem[];
+    __shared__ uint64_t bar;
+    // the step's scalars live here, not in registers across the stencil: dx and dy quotients, 0.5 dtp / dx, 0.5 dtp / dy, dt, dt before its clamp, dtp
+    __shared__ double s_v[7];
+    if (c->clamp && c->t == c->t_end) {   // the loop stops here
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            c->done = 1;
+            c->snap_pre = c->snap_post = 0;
+        }
+        return;
+    }
+    const RowShape S{tile};
+    const int tx = tile.tx, ty = tile.ty, usize = 4 * (tx + 2 * G) * (ty + 2 * G);
+    double* sU = smem;
+    double* sW = smem + usize;
+    const BlockDev& B = m->b[0];
+    const int p = (int)(c->step & 1);
+    const int tiles_x = (B.nx + tx - 1) / tx;
+    const int x0 = (blockIdx.x % tiles_x) * tx, y0 = (blockIdx.x / tiles_x) * ty;
+    // TimeStep (timestep.cpp:29-68), its clamp (simulation.cpp:88-90) and the predictor's call
+    // (muscl_hancock.cpp:246-249) while the tile is in flight; a direction's quotients per thread
+    const bool forms = threadIdx.x == 0 || threadIdx.x == 32;
+    const int d = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar, 1);
+        mbar_expect_tx(&bar, usize * 8);
+        tma_load_3d(sU, p ? &tm1 : &tm0, &bar, x0, y0, 0);
+    }
+    if (forms) s_v[d] = div_rn(d ? c->dy[0] : c->dx[0], smax(ss->solo[d], bitsd(c->int_s[p][0][d])));
+    __syncthreads();
+    if (forms) {
+        const double least = smin(smin(1e16, s_v[0]), smin(1e16, s_v[1])), cfl = c->cfl;
+        const long long call = c->calls;
+        if (SCHEME == 1) {
+            const double dtp = ((call + 2 <= 10) ? 0.2 * cfl : cfl) * least;
+            s_v[2 + d] = div_rn(0.5 * dtp, d ? c->dy[0] : c->dx[0]);
+            if (d == 0) s_v[6] = dtp;
+        }
+        if (d == 0) {
+            const double dt = ((call + 1 <= 10) ? 0.2 * cfl : cfl) * least;
+            s_v[4] = c->clamp && c->t + dt > c->t_end ? c->t_end - c->t : dt;
+            s_v[5] = dt;
+        }
+    }
+    if (wait_tile(&bar, c)) {
+        tile_ghosts<G>(sU, m, B.buf[p], tx, ty, x0, y0, &c->err);
+        const double g = c->gamma, g1 = c->g1;
+        const int herr = SCHEME == 0
+            ? go_tile_fluxes<kNT>(S, sU, sW, g, g1, x0, y0, B.nx, B.ny, &c->first_bad, face_key(c->step, 0, 0, 0, 0))
+            : mh_tile_fluxes<kNT, LIM>(S, sU, sW, g, g1, s_v[2], s_v[3], x0, y0, B.nx, B.ny, &c->first_bad,
+                                       face_key(c->step, 0, 0, 0, 0));
+        double mx = 0.0, my = 0.0;
+        store_tile<kNT, G>(S, sU, sW, B, x0, y0, B.buf[p ^ 1], nullptr, s_v[4], ss->solo[2], ss->solo[3], g, g1,
+                           &c->first_nonpos, face_key(c->step, 0, 0, 0, 0), mx, my, &c->err);
+        store_ghosts<G, kNT>(sU, B, tx, ty, x0, y0, B.buf[p ^ 1], &c->err);
+        block_max2_atomic<kNT>(mx, my, &c->int_s[p ^ 1][0][0], &c->int_s[p ^ 1][0][1]);
+        if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
+    }
+    if (!last_cta(&ss->tiles)) return;
+    c->done = 0;
+    c->snap_pre = c->snap_post = 0;
+    c->dt_cfl = s_v[5];
+    c->dt = s_v[4];
+    if (SCHEME == 1) c->dt_pred[0] = s_v[6];
+    c->calls = c->calls + 1;
+    finish_step(c);
+}
+
+// ------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------
 TileShape tile_shape(int tx, int ty) {
@@ -834,10 +967,25 @@ cudaError_t launch_step(Ctrl* c, const MeshDev* m, StepState* ss, const StepPlan
     return cudaGetLastError();
 }
 
+cudaError_t prepare_solo(Ctrl* c, const MeshDev* m, StepState* ss, cudaStream_t s) {
+    prepare_solo_kernel<<<1, 1, 0, s>>>(c, m, ss);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_solo(Ctrl* c, const MeshDev* m, StepState* ss, int nx, int ny, int scheme, int limiter,
+                        const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s) {
+    const int tiles = ((nx + tile.tx - 1) / tile.tx) * ((ny + tile.ty - 1) / tile.ty);
+    if (scheme == 0) solo_kernel<0, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1);
+    else if (limiter == 0) solo_kernel<1, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1);
+    else solo_kernel<1, 1><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1);
+    return cudaGetLastError();
+}
+
 cudaError_t stencil_prepare() {
     for (const void* k : {(const void*)mh_step_kernel<0>, (const void*)mh_step_kernel<1>, (const void*)mh_rerun_kernel<0>,
                           (const void*)mh_rerun_kernel<1>, (const void*)mh_kernel<0>, (const void*)mh_kernel<1>,
-                          (const void*)godunov_step_kernel, (const void*)godunov_kernel}) {
+                          (const void*)godunov_step_kernel, (const void*)godunov_kernel, (const void*)solo_kernel<0, 0>,
+                          (const void*)solo_kernel<1, 0>, (const void*)solo_kernel<1, 1>}) {
         const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes);
         if (e != cudaSuccess) return e;
     }

@@ -69,6 +69,8 @@ TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms)
 // What the all-blocks launch keeps between its kernels, beside the checkpointed control block.
 struct StepState {
     double sc[HF_MAXB][5];   // per block: 0.5 dtp / dx, 0.5 dtp / dy, 1 / dx, 1 / dy, the predictor dt dtp
+    double solo[4];          // one-launch steps: the wave-speed maxima |u| + c, |v| + c of the Dirichlet sides'
+                             // states, 1 / dx, 1 / dy
     int rerun;               // the block to be run again (0: none)
     unsigned int tiles;      // CTAs of a launch that are done
 };
@@ -135,6 +137,12 @@ struct StepPlan {
 void step_plan_tiles(StepPlan& plan, int b, int nx, int ny);
 cudaError_t launch_step(Ctrl* c, const MeshDev* m, StepState* ss, const StepPlan& plan, int scheme, int limiter,
                         cudaStream_t s);
+
+// A step of a mesh of one block in one launch (hf_cart.cu), where every ghost cell's value is an interior
+// cell's or a Dirichlet state: no fill before it, the step ended by its last CTA.  prepare_solo once.
+cudaError_t prepare_solo(Ctrl* c, const MeshDev* m, StepState* ss, cudaStream_t s);
+cudaError_t launch_solo(Ctrl* c, const MeshDev* m, StepState* ss, int nx, int ny, int scheme, int limiter,
+                        const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s);
 
 // the driver's cuTensorMapEncodeTiled, or null where the driver lacks it
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
