@@ -128,6 +128,17 @@ __device__ __forceinline__ float slopef(int lim, float um, float u0, float up) {
     return limf(lim, dlc / drc) * (0.5f * dl + 0.5f * dr);
 }
 
+// The run loop on the device (hf_lc_run_to): the step to take next, formed by the last CTA of the update
+// before it.  Kernels given a loop take dt and dt / dx from it and leave at once when it has ended; given
+// none they take them as arguments.
+struct Loop {
+    double t, t_end, dt, cfl_dx, dx;   // cfl_dx = cfl dx; dt: the next step's
+    float dtf, r;                      // (float)dt, (float)(dt / dx)
+    int done, failed;                  // t_end reached, or dt not positive and finite
+    long long steps, taken, rejected;  // steps since time 0, steps and rejected cells of this run
+    unsigned int ticket;
+};
+
 struct Grid {
     int n;
     float dx, g, g1;
@@ -188,8 +199,14 @@ __device__ __forceinline__ void plain_face_flux(const float* __restrict__ U, con
     }
 }
 
-// plain MUSCL-Hancock HLLC flux of every face (FP32)
-__global__ void plain_flux_kernel(const float* __restrict__ U, Grid G, float dt, float* __restrict__ F) {
+// plain MUSCL-Hancock HLLC flux of every face (FP32); maxs (optional): the step's wave-speed maximum, zeroed
+__global__ void plain_flux_kernel(const float* __restrict__ U, Grid G, float dt, float* __restrict__ F,
+                                  const Loop* __restrict__ loop, float* __restrict__ maxs) {
+    if (loop) {
+        if (loop->done) return;
+        dt = loop->dtf;
+    }
+    if (maxs && blockIdx.x == 0 && threadIdx.x == 0) *maxs = 0.0f;
     const int nf = 2 * (G.n + 1) * G.n;
     const float hdt = 0.5f * dt / G.dx;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
@@ -676,7 +693,11 @@ __global__ void __launch_bounds__(kTcThreads, 3)
 face_kernel(const float* __restrict__ U, const float4* __restrict__ W, Grid G, float dt,
             const __nv_bfloat16* __restrict__ Wb, const float* __restrict__ P, float* __restrict__ F,
             float* __restrict__ dF, unsigned char* __restrict__ ok, unsigned long long* __restrict__ rejected,
-            float* __restrict__ maxs, int* __restrict__ err) {
+            float* __restrict__ maxs, int* __restrict__ err, const Loop* __restrict__ loop) {
+    if (loop) {
+        if (loop->done) return;
+        dt = loop->dtf;
+    }
     extern __shared__ unsigned char smem_raw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     if (blockIdx.x == 0 && threadIdx.x == 0) {   // the step's counters, read by the guard and the update
@@ -1113,7 +1134,12 @@ __device__ __forceinline__ bool guard_bad(const float* __restrict__ U, const flo
 // keeps every cell's update with all its corrections for pass 2
 __global__ void guard_kernel(const float* __restrict__ U, const float* __restrict__ F, const float* __restrict__ dF,
                              Grid G, float r, float bound, int mode, unsigned char* __restrict__ ok,
-                             unsigned long long* __restrict__ rejected, float4* __restrict__ Uc) {
+                             unsigned long long* __restrict__ rejected, float4* __restrict__ Uc,
+                             const Loop* __restrict__ loop) {
+    if (loop) {
+        if (loop->done) return;
+        r = loop->r;
+    }
     const int n = G.n;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n * n; c += gridDim.x * blockDim.x) {
         const int i = c % n, j = c / n;
@@ -1129,6 +1155,24 @@ __global__ void guard_kernel(const float* __restrict__ U, const float* __restric
     }
 }
 
+// the loop's next dt from the state's wave-speed maximum, or its end.  The reference's TimeStep uses 0.2 x
+// CFL for its first 10 calls; a MUSCL-Hancock step makes two (step and predictor), so the first 5
+// steps are reduced.
+__device__ void form_step(Loop* loop, float m) {
+    loop->done = !(loop->t < loop->t_end);
+    if (loop->done) return;
+    double dt = loop->cfl_dx / (double)m;
+    if (loop->steps < 5) dt *= 0.2;
+    if (!(dt > 0.0) || isinf(dt)) {
+        loop->failed = loop->done = 1;
+        return;
+    }
+    if (loop->t + dt > loop->t_end) dt = loop->t_end - loop->t;
+    loop->dt = dt;
+    loop->dtf = (float)dt;
+    loop->r = (float)(dt / loop->dx);
+}
+
 // pass 2: the update (corrections where accepted); a cell still violating takes its plain update
 // Wn (optional): the primitives of the new state, as prims_kernel forms them, for the next step's
 // features.  Uc (optional, with dF and ok): pass 1's fully corrected updates -- a cell whose four
@@ -1137,7 +1181,12 @@ __global__ void guard_kernel(const float* __restrict__ U, const float* __restric
 __global__ void update_kernel(const float* __restrict__ U, const float* __restrict__ F, const float* __restrict__ dF,
                               const unsigned char* __restrict__ ok, Grid G, float r, float bound, int mode,
                               float* __restrict__ Un, float* __restrict__ maxs, float4* __restrict__ Wn,
-                              const float4* __restrict__ Uc) {
+                              const float4* __restrict__ Uc, Loop* __restrict__ loop,
+                              const unsigned long long* __restrict__ rejected) {
+    if (loop) {
+        if (loop->done) return;
+        r = loop->r;
+    }
     const int n = G.n;
     float m = 0.0f;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n * n; c += gridDim.x * blockDim.x) {
@@ -1172,7 +1221,20 @@ __global__ void update_kernel(const float* __restrict__ U, const float* __restri
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
         if (threadIdx.x == 0 && m > 0.0f) atomicMax(reinterpret_cast<int*>(maxs), __float_as_int(m));
     }
+    if (!loop || threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd(&loop->ticket, 1u) != gridDim.x - 1) return;
+    __threadfence();   // the last CTA: the step is done
+    loop->ticket = 0u;
+    loop->t = loop->t + loop->dt;
+    loop->steps = loop->steps + 1;
+    loop->taken = loop->taken + 1;
+    if (rejected) loop->rejected = loop->rejected + (long long)*(const volatile unsigned long long*)rejected;
+    form_step(loop, *(const volatile float*)maxs);
 }
+
+// the first step of a run
+__global__ void loop_begin_kernel(Loop* __restrict__ loop, const float* __restrict__ maxs) { form_step(loop, *maxs); }
 
 // dL/dY for L = (1/N) sum_cells sum_v w_v (U^{n+1}_v - T_v)^2, U^{n+1} with every correction
 __global__ void loss_grad_kernel(const float* __restrict__ Un, const float* __restrict__ T, const float* __restrict__ scale,
@@ -1253,6 +1315,7 @@ struct hf_lc {
     unsigned long long* rejected = nullptr;
     double* loss = nullptr;
     int* derr = nullptr;       // device error word (a bounded wait gave up)
+    Loop* loop = nullptr;      // the device run loop
     int cur = 0;
     long long steps = 0;       // steps since time 0 (TimeStep's start-up multiplier)
     long long adam_t = 0;
@@ -1357,7 +1420,7 @@ void launch_features(hf_lc* L) {
 // plain fluxes F, and (use_mlp) the corrections dF for state U[cur].  Inference (no saved
 // activations) with the fused kernel also sets the guard's face mask and zeroes the step's
 // counters; returns through *mask_set whether it did.
-int fluxes(hf_lc* L, float dt, bool use_mlp, bool save_acts, bool* mask_set = nullptr) {
+int fluxes(hf_lc* L, float dt, bool use_mlp, bool save_acts, bool* mask_set = nullptr, Loop* loop = nullptr) {
     hf::lc::Grid G = grid(L);
     const int nf = nfaces(L);
     if (mask_set) *mask_set = false;
@@ -1370,7 +1433,7 @@ int fluxes(hf_lc* L, float dt, bool use_mlp, bool save_acts, bool* mask_set = nu
         if (L->fused == 2) {
             face_kernel<true><<<mlp_grid(L, L->fit_face[1], units, L->face_ctas_per_sm),
                                 hf::lc::kTcThreads, sm, L->stream>>>(L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F,
-                                                                     L->dF, L->ok, L->rejected, L->maxs, L->derr);
+                                                                     L->dF, L->ok, L->rejected, L->maxs, L->derr, loop);
         } else {
             // the plain fluxes on the side stream, running beside the face kernel (independent
             // work: the face kernel is latency-bound, the flux kernel arithmetic-bound); the face
@@ -1379,9 +1442,10 @@ int fluxes(hf_lc* L, float dt, bool use_mlp, bool save_acts, bool* mask_set = nu
             face_kernel<false><<<mlp_grid(L, L->fit_face[0], units,
                                           L->face_ctas_per_sm > 0 ? L->face_ctas_per_sm : 2),
                                  hf::lc::kTcThreads, sm, L->stream>>>(L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F,
-                                                                      L->dF, L->ok, L->rejected, L->maxs, L->derr);
+                                                                      L->dF, L->ok, L->rejected, L->maxs, L->derr,
+                                                                      loop);
             LCK(cudaStreamWaitEvent(L->side, L->fork, 0));
-            plain_flux_kernel<<<blocks_for(nf, 256), 256, 0, L->side>>>(L->U[L->cur], G, dt, L->F);
+            plain_flux_kernel<<<blocks_for(nf, 256), 256, 0, L->side>>>(L->U[L->cur], G, dt, L->F, loop, nullptr);
             LCK(cudaEventRecord(L->join, L->side));
             LCK(cudaStreamWaitEvent(L->stream, L->join, 0));
         }
@@ -1389,7 +1453,8 @@ int fluxes(hf_lc* L, float dt, bool use_mlp, bool save_acts, bool* mask_set = nu
         if (mask_set) *mask_set = true;
         return HF_OK;
     }
-    plain_flux_kernel<<<blocks_for(nf, 256), 256, 0, L->stream>>>(L->U[L->cur], G, dt, L->F);
+    plain_flux_kernel<<<blocks_for(nf, 256), 256, 0, L->stream>>>(L->U[L->cur], G, dt, L->F, loop,
+                                                                  save_acts ? nullptr : L->maxs);
     if (use_mlp) {
         launch_features(L);
         launch_forward(L, nf, save_acts);
@@ -1450,7 +1515,7 @@ int hf_lc_create(int n, double dx, double gamma, double cfl, int limiter, hf_lc*
         (r = alloc(L, &L->grad, (size_t)NPARAM)) || (r = alloc(L, &L->m1, (size_t)NPARAM)) ||
         (r = alloc(L, &L->m2, (size_t)NPARAM)) || (r = alloc(L, &L->maxs, 4)) || (r = alloc(L, &L->ok, nf)) ||
         (r = alloc(L, &L->rejected, 1)) || (r = alloc(L, &L->loss, 1)) || (r = alloc(L, &L->derr, 1)) ||
-        (r = alloc(L, &L->Wp, cells)) || (r = alloc(L, &L->Uc, cells)))
+        (r = alloc(L, &L->Wp, cells)) || (r = alloc(L, &L->Uc, cells)) || (r = alloc(L, &L->loop, 1)))
         return r;
     return HF_OK;
 }
@@ -1513,7 +1578,8 @@ static int enqueue_max_speed(hf_lc* L) {
     LCK(cudaMemsetAsync(L->maxs, 0, 4, L->stream));
     LCK(cudaMemsetAsync(L->F, 0, (size_t)4 * nfaces(L) * sizeof(float), L->stream));
     update_kernel<<<blocks_for((long long)L->n * L->n, 256), 256, 0, L->stream>>>(
-        L->U[L->cur], L->F, nullptr, nullptr, G, 0.0f, 0.0f, 0, L->U[L->cur ^ 1], L->maxs, nullptr, nullptr);
+        L->U[L->cur], L->F, nullptr, nullptr, G, 0.0f, 0.0f, 0, L->U[L->cur ^ 1], L->maxs, nullptr, nullptr, nullptr,
+        nullptr);
     LCK(cudaGetLastError());
     L->maxs_valid = true;
     return HF_OK;
@@ -1528,37 +1594,42 @@ int hf_lc_cfl_dt(hf_lc* L, double* dt) {
     return HF_OK;
 }
 
-// one coarse step with the given dt; use_mlp adds the guarded correction
-int hf_lc_step(hf_lc* L, double dt, int use_mlp, int64_t* rejected_cells) {
-    hf::TraceRange trace_("hf_lc_step");
-    if (!L || dt <= 0) return HF_ERR_ARG;
+// The kernels of one coarse step: with the given dt, or (loop) with the device loop's.
+static int enqueue_lc_step(hf_lc* L, double dt, int use_mlp, Loop* loop) {
     hf::lc::Grid G = grid(L);
     bool mask_set = false;
-    int r = fluxes(L, (float)dt, use_mlp != 0, false, &mask_set);
+    int r = fluxes(L, (float)dt, use_mlp != 0, false, &mask_set, loop);
     if (r) return r;
     const float rr = (float)(dt / L->dx);
     const int nf = nfaces(L);
-    if (!mask_set) {   // else the fused kernel set the mask and zeroed the counters
-        LCK(cudaMemsetAsync(L->maxs, 0, 4, L->stream));
-        if (use_mlp) {
-            LCK(cudaMemsetAsync(L->ok, 1, nf, L->stream));
-            LCK(cudaMemsetAsync(L->rejected, 0, 8, L->stream));
-        }
+    if (!mask_set && use_mlp) {   // else the fused kernel set the mask and zeroed the counters
+        LCK(cudaMemsetAsync(L->ok, 1, nf, L->stream));
+        LCK(cudaMemsetAsync(L->rejected, 0, 8, L->stream));
     }
     if (use_mlp)
         guard_kernel<<<blocks_for((long long)L->n * L->n, 256), 256, 0, L->stream>>>(
             L->U[L->cur], L->F, L->dF, G, rr, (float)L->bound, L->guard_mode, L->ok, L->rejected,
-            L->fused ? L->Uc : nullptr);
+            L->fused ? L->Uc : nullptr, loop);
     // an MLP step also leaves the primitives of the new state for the next one's features; with
     // the fused kernels the update takes the guard pass's corrected states where no face was
     // rejected (the separate kernels recompute them all: the same values)
     update_kernel<<<blocks_for((long long)L->n * L->n, 256), 256, 0, L->stream>>>(
         L->U[L->cur], L->F, use_mlp ? L->dF : nullptr, use_mlp ? L->ok : nullptr, G, rr, (float)L->bound,
-        L->guard_mode, L->U[L->cur ^ 1], L->maxs, use_mlp ? L->Wp : nullptr, use_mlp && L->fused ? L->Uc : nullptr);
+        L->guard_mode, L->U[L->cur ^ 1], L->maxs, use_mlp ? L->Wp : nullptr, use_mlp && L->fused ? L->Uc : nullptr, loop,
+        use_mlp ? L->rejected : nullptr);
     LCK(cudaGetLastError());
     L->cur ^= 1;
     L->wp_valid = use_mlp != 0;
     L->maxs_valid = true;   // the update formed the new state's maximum wave speed
+    return HF_OK;
+}
+
+// one coarse step with the given dt; use_mlp adds the guarded correction
+int hf_lc_step(hf_lc* L, double dt, int use_mlp, int64_t* rejected_cells) {
+    hf::TraceRange trace_("hf_lc_step");
+    if (!L || dt <= 0) return HF_ERR_ARG;
+    int r = enqueue_lc_step(L, dt, use_mlp, nullptr);
+    if (r) return r;
     L->t += dt;
     L->steps += 1;
     if (rejected_cells) {
@@ -1571,42 +1642,46 @@ int hf_lc_step(hf_lc* L, double dt, int use_mlp, int64_t* rejected_cells) {
     return HF_OK;
 }
 
-// runs until t_end with CFL dt (host loop, one sync per step for dt); returns steps
+// Runs until t_end with CFL dt; returns steps.  The loop is the device's: every step's update forms the
+// next dt, and a step after the end leaves its buffers alone.  The host enqueues as many steps as the
+// last dt it read suggests are left and reads the loop's state once for all of them (it read the wave-speed
+// maximum back for every step's dt: 112 us a step at 512^2 for 72 of kernels).
 int hf_lc_run_to(hf_lc* L, double t_end, int use_mlp, int64_t* steps, int64_t* rejected_cells) {
     hf::TraceRange trace_("hf_lc_run_to");
     if (!L) return HF_ERR_ARG;
-    // one wait per step: the step's wave-speed maximum (the next dt) and rejection count are read
-    // together; the device error word once at the end
-    int64_t k = 0, rej = 0;
     int r = enqueue_max_speed(L);
     if (r) return r;
-    while (L->t < t_end) {
-        float m = 0.0f;
-        unsigned long long rc = 0;
-        LCK(cudaMemcpyAsync(&m, L->maxs, sizeof m, cudaMemcpyDeviceToHost, L->stream));
-        if (use_mlp && k > 0) LCK(cudaMemcpyAsync(&rc, L->rejected, sizeof rc, cudaMemcpyDeviceToHost, L->stream));
+    Loop S{};
+    S.t = L->t;
+    S.t_end = t_end;
+    S.cfl_dx = L->cfl * L->dx;
+    S.dx = L->dx;
+    S.steps = L->steps;
+    LCK(cudaMemcpyAsync(L->loop, &S, sizeof S, cudaMemcpyHostToDevice, L->stream));
+    loop_begin_kernel<<<1, 1, 0, L->stream>>>(L->loop, L->maxs);
+    LCK(cudaGetLastError());
+    const int cur = L->cur;
+    const bool wp = L->wp_valid;
+    for (;;) {
+        LCK(cudaMemcpyAsync(&S, L->loop, sizeof S, cudaMemcpyDeviceToHost, L->stream));
         LCK(cudaStreamSynchronize(L->stream));
-        rej += (int64_t)rc;
-        double dt = L->cfl * L->dx / (double)m;
-        // the reference's TimeStep uses 0.2 x CFL for its first 10 calls; a MUSCL-Hancock
-        // step makes two (step and predictor), so the first 5 steps are reduced
-        if (L->steps < 5) dt *= 0.2;
-        if (!(dt > 0.0) || !std::isfinite(dt))
-            return lfail(L, HF_ERR_DEVICE, "coarse run stopped advancing (non-positive or non-finite dt)");
-        if (L->t + dt > t_end) dt = t_end - L->t;
-        r = hf_lc_step(L, dt, use_mlp, nullptr);
-        if (r) return r;
-        ++k;
+        L->cur = cur ^ (int)(S.taken & 1);   // steps past the end did nothing
+        // (the separate kernels form the primitives anew in every step, those past the end too)
+        L->wp_valid = S.taken > 0 ? use_mlp && L->fused : wp && L->fused;
+        L->t = S.t;
+        L->steps = S.steps;
+        if (S.done) break;
+        const int slow = S.steps < 5 ? (int)(5 - S.steps) : 0;   // steps at 0.2 CFL left
+        const double full = slow ? 5.0 * S.dt : S.dt;
+        const double left = (S.t_end - S.t - slow * S.dt) / full;
+        const double want = slow + (left > 0.0 ? std::ceil(left) : 0.0);
+        const int k = want < 1.0 ? 1 : (want > 64.0 ? 64 : (int)want);
+        for (int i = 0; i < k; ++i)
+            if ((r = enqueue_lc_step(L, S.dt, use_mlp, L->loop))) return r;
     }
-    if (use_mlp && k > 0) {
-        unsigned long long rc = 0;
-        LCK(cudaMemcpyAsync(&rc, L->rejected, sizeof rc, cudaMemcpyDeviceToHost, L->stream));
-        LCK(cudaStreamSynchronize(L->stream));
-        rej += (int64_t)rc;
-    }
-    LCK(cudaStreamSynchronize(L->stream));
-    if (steps) *steps = k;
-    if (rejected_cells) *rejected_cells = rej;
+    if (steps) *steps = S.taken;
+    if (rejected_cells) *rejected_cells = S.rejected;
+    if (S.failed) return lfail(L, HF_ERR_DEVICE, "coarse run stopped advancing (non-positive or non-finite dt)");
     return check_derr(L);
 }
 
@@ -1658,13 +1733,14 @@ int hf_lc_train_step(hf_lc* L, const float* U0, const float* T, const float* w, 
         LCK(cudaMemsetAsync(L->ok, 1, nf, L->stream));
         LCK(cudaMemsetAsync(L->rejected, 0, 8, L->stream));
         guard_kernel<<<blocks_for((long long)L->n * L->n, 256), 256, 0, L->stream>>>(
-            L->U[L->cur], L->F, L->dF, G, rr, (float)L->bound, L->guard_mode, L->ok, L->rejected, nullptr);
+            L->U[L->cur], L->F, L->dF, G, rr, (float)L->bound, L->guard_mode, L->ok, L->rejected, nullptr, nullptr);
         update_kernel<<<blocks_for((long long)L->n * L->n, 256), 256, 0, L->stream>>>(
             L->U[L->cur], L->F, L->dF, L->ok, G, rr, (float)L->bound, L->guard_mode, L->U[L->cur ^ 1], L->maxs,
-            nullptr, nullptr);
+            nullptr, nullptr, nullptr, nullptr);
     } else {
         update_kernel<<<blocks_for((long long)L->n * L->n, 256), 256, 0, L->stream>>>(
-            L->U[L->cur], L->F, L->dF, nullptr, G, rr, 0.0f, 0, L->U[L->cur ^ 1], L->maxs, nullptr, nullptr);
+            L->U[L->cur], L->F, L->dF, nullptr, G, rr, 0.0f, 0, L->U[L->cur ^ 1], L->maxs, nullptr, nullptr, nullptr,
+            nullptr);
     }
     LCK(cudaMemsetAsync(L->loss, 0, 8, L->stream));
     loss_grad_kernel<<<blocks_for(nf, 256), 256, 0, L->stream>>>(L->U[L->cur ^ 1], L->T, L->scale, L->n, rr, L->wv,
