@@ -680,27 +680,34 @@ mlp_forward_kernel(const __nv_bfloat16* __restrict__ X, int nf, const __nv_bfloa
     mlp_teardown(S);
 }
 
-// The inference path of a learned step in one kernel, per 128-face tile of a group: the features of every
+// The network's path of a learned step in one kernel, per 128-face tile of a group: the features of every
 // face formed straight into the MLP's first operand, the three layers on the tensor cores, and
 // (FLUX) the plain MUSCL-Hancock HLLC flux computed on the CUDA cores while the first layer
 // runs.  Out go the correction dF [4][nf] (the correction kernel's formula), the guard's face
 // mask set to 1, the step's rejection count and maximum wave speed zeroed, and (FLUX) the plain
-// flux F [4][nf].  The results equal those of features +
+// flux F [4][nf]; (SAVE, training) what the backward reads: the features X, the scales and the hidden
+// pre-activations Z1, Z2, in place of the mask and the counters.  The results equal those of features +
 // mlp_forward + correction (+ plain_flux) bit for bit: the same device functions.  Failure
 // handling as mlp_forward_kernel's.
-template <bool FLUX>
+enum { FACE_INFER = 0, FACE_FLUX = 1, FACE_SAVE = 2 };
+struct FaceSaved {
+    __nv_bfloat16* X;
+    float *scale, *Z1, *Z2;
+};
+template <int MODE>
 __global__ void __launch_bounds__(kTcThreads, 3)
 face_kernel(const float* __restrict__ U, const float4* __restrict__ W, Grid G, float dt,
             const __nv_bfloat16* __restrict__ Wb, const float* __restrict__ P, float* __restrict__ F,
             float* __restrict__ dF, unsigned char* __restrict__ ok, unsigned long long* __restrict__ rejected,
-            float* __restrict__ maxs, int* __restrict__ err, const Loop* __restrict__ loop) {
+            float* __restrict__ maxs, int* __restrict__ err, const Loop* __restrict__ loop, FaceSaved saved) {
+    constexpr bool FLUX = MODE == FACE_FLUX, SAVE = MODE == FACE_SAVE;
     if (loop) {
         if (loop->done) return;
         dt = loop->dtf;
     }
     extern __shared__ unsigned char smem_raw[];
     TcSmem& S = *reinterpret_cast<TcSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    if (blockIdx.x == 0 && threadIdx.x == 0) {   // the step's counters, read by the guard and the update
+    if (!SAVE && blockIdx.x == 0 && threadIdx.x == 0) {   // the step's counters, read by the guard and the update
         *rejected = 0ull;
         *maxs = 0.0f;
     }
@@ -720,8 +727,13 @@ face_kernel(const float* __restrict__ U, const float4* __restrict__ W, Grid G, f
         {
             uint32_t pk[32] = {};
             if (valid) face_features(W, G, dir, i, j, pk, rr, cref);
+            uint4* const xo = SAVE ? reinterpret_cast<uint4*>(saved.X + (size_t)(valid ? f : 0) * NIN) : nullptr;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) *a_chunk(S, q) = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+            for (int q = 0; q < 8; ++q) {
+                const uint4 x = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
+                *a_chunk(S, q) = x;
+                if (SAVE && valid) xo[q] = x;
+            }
         }
         mlp_issue(S, 0);
         if (valid) {
@@ -731,13 +743,14 @@ face_kernel(const float* __restrict__ U, const float4* __restrict__ W, Grid G, f
 #pragma unroll
                 for (int v = 0; v < 4; ++v) F[(size_t)v * nf + f] = fl[v];
             }
-            ok[f] = 1;
+            if (SAVE) *reinterpret_cast<float2*>(saved.scale + 2 * (size_t)f) = make_float2(rr, cref);
+            else ok[f] = 1;
         }
         if (!mlp_wait(S, phase, err)) break;
-        mlp_hidden(S, tl, nullptr, f, valid);
+        mlp_hidden(S, tl, SAVE ? saved.Z1 : nullptr, f, valid);
         mlp_issue(S, 1);
         if (!mlp_wait(S, phase, err)) break;
-        mlp_hidden(S, tl, nullptr, f, valid);
+        mlp_hidden(S, tl, SAVE ? saved.Z2 : nullptr, f, valid);
         mlp_issue(S, 2);
         if (!mlp_wait(S, phase, err)) break;
         float o[NOUT];
@@ -1036,7 +1049,12 @@ __global__ void adam_kernel(float* __restrict__ P, const float* __restrict__ G, 
         const float mk = b1 * m[k] + (1.f - b1) * g, vk = b2 * v[k] + (1.f - b2) * g * g;
         m[k] = mk;
         v[k] = vk;
-        P[k] -= lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+        const float w = P[k] - lr * (mk / c1) / (sqrtf(vk / c2) + eps);
+        P[k] = w;
+        // the BF16 copies of W1, W2, W3, contiguous
+        const int b = k < OFF_B1 ? k : k >= OFF_W2 && k < OFF_B2 ? H * NIN + k - OFF_W2
+                    : k >= OFF_W3 && k < OFF_B3 ? H * NIN + H * H + k - OFF_W3 : -1;
+        if (b >= 0) Wb[b] = __float2bfloat16_rn(w);
     }
 }
 
@@ -1238,10 +1256,11 @@ __global__ void loop_begin_kernel(Loop* __restrict__ loop, const float* __restri
 
 // dL/dY for L = (1/N) sum_cells sum_v w_v (U^{n+1}_v - T_v)^2, U^{n+1} with every correction
 __global__ void loss_grad_kernel(const float* __restrict__ Un, const float* __restrict__ T, const float* __restrict__ scale,
-                                 int n, float r, const float* __restrict__ wv, const unsigned char* __restrict__ ok,
+                                 int n, float r, float4 w4, const unsigned char* __restrict__ ok,
                                  float* __restrict__ dY, double* __restrict__ loss) {
     const int nf = 2 * (n + 1) * n;
     const float invN = 1.0f / ((float)n * n);
+    const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
     double ls = 0.0;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < nf; f += gridDim.x * blockDim.x) {
         int dir, i, j;
@@ -1277,8 +1296,16 @@ __global__ void loss_grad_kernel(const float* __restrict__ Un, const float* __re
             const float d = Un[(size_t)v * n * n + c] - T[(size_t)v * n * n + c];
             ls += (double)(wv[v] * d * d * invN);
         }
+    // one addition per CTA: one per warp queued for 8 us at 256^2
+    __shared__ double part[32];
     for (int o = 16; o > 0; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(loss, ls);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ls;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        ls = threadIdx.x < (blockDim.x >> 5) ? part[threadIdx.x] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) ls += __shfl_xor_sync(0xffffffffu, ls, o);
+        if (threadIdx.x == 0) atomicAdd(loss, ls);
+    }
 }
 
 }  // namespace lc
@@ -1298,12 +1325,12 @@ struct hf_lc {
                                // plain flux too, 0 the separate kernels
     int face_ctas_per_sm = 0;  // face_kernel CTAs per SM (0: as many as fit)
     int sms = 152;             // the device's SMs, and how many CTAs of each MLP kernel fit on one
-    int fit_fwd = 1, fit_face[2] = {1, 1};
+    int fit_fwd = 1, fit_face[3] = {1, 1, 1};   // (face_kernel by mode)
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr;           // the plain fluxes, beside the fused face kernel
     cudaEvent_t fork = nullptr, join = nullptr;
     float *U[2] = {nullptr, nullptr}, *F = nullptr, *dF = nullptr, *scale = nullptr, *Y = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *dY = nullptr, *T = nullptr, *wv = nullptr;
+    float *Z1 = nullptr, *Z2 = nullptr, *dY = nullptr, *T = nullptr;
     __nv_bfloat16 *X = nullptr, *Wb = nullptr;
     float4* Wp = nullptr;      // per-cell primitives (rho, u, v, p) for the feature stencils
     bool wp_valid = false;     // Wp holds the primitives of U[cur] (written by the last step)
@@ -1314,8 +1341,15 @@ struct hf_lc {
     unsigned char* ok = nullptr;
     unsigned long long* rejected = nullptr;
     double* loss = nullptr;
+    struct Out { double loss; int derr, pad; };
+    Out* out = nullptr;        // pinned: a training iteration's loss and the error word
     int* derr = nullptr;       // device error word (a bounded wait gave up)
     Loop* loop = nullptr;      // the device run loop
+    cudaGraphExec_t pair = nullptr;   // two steps of it, captured for the settings in pair_key
+    struct PairKey {
+        int cur, use_mlp, guard_mode, fused, ctas;
+        double bound;
+    } pair_key{};
     int cur = 0;
     long long steps = 0;       // steps since time 0 (TimeStep's start-up multiplier)
     long long adam_t = 0;
@@ -1417,40 +1451,42 @@ void launch_features(hf_lc* L) {
     features_kernel<<<blocks_for(nf, hf::lc::kFeatNT), hf::lc::kFeatNT, 0, L->stream>>>(L->Wp, G, L->X, L->scale);
 }
 
-// plain fluxes F, and (use_mlp) the corrections dF for state U[cur].  Inference (no saved
-// activations) with the fused kernel also sets the guard's face mask and zeroes the step's
-// counters; returns through *mask_set whether it did.
+// plain fluxes F, and (use_mlp) the corrections dF for state U[cur]; save_acts keeps what the backward
+// reads.  Inference with the fused kernel also sets the guard's face mask and zeroes the step's counters;
+// returns through *mask_set whether it did.
 int fluxes(hf_lc* L, float dt, bool use_mlp, bool save_acts, bool* mask_set = nullptr, Loop* loop = nullptr) {
     hf::lc::Grid G = grid(L);
     const int nf = nfaces(L);
     if (mask_set) *mask_set = false;
-    if (use_mlp && !save_acts && L->fused) {
+    if (use_mlp && L->fused) {
         if (!L->wp_valid)   // else the previous step's update wrote them
             prims_kernel<<<blocks_for(L->n * L->n, 256), 256, 0, L->stream>>>(L->U[L->cur], L->n, G.g1, L->Wp);
         L->wp_valid = true;
         const size_t sm = hf::lc::mlp_forward_smem();
-        const int units = nf;
-        if (L->fused == 2) {
-            face_kernel<true><<<mlp_grid(L, L->fit_face[1], units, L->face_ctas_per_sm),
-                                hf::lc::kTcThreads, sm, L->stream>>>(L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F,
-                                                                     L->dF, L->ok, L->rejected, L->maxs, L->derr, loop);
+        const FaceSaved none{nullptr, nullptr, nullptr, nullptr}, saved{L->X, L->scale, L->Z1, L->Z2};
+        if (L->fused == 2 && !save_acts) {
+            face_kernel<FACE_FLUX><<<mlp_grid(L, L->fit_face[1], nf, L->face_ctas_per_sm), hf::lc::kTcThreads, sm,
+                                     L->stream>>>(L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F, L->dF, L->ok,
+                                                  L->rejected, L->maxs, L->derr, loop, none);
         } else {
             // the plain fluxes on the side stream, running beside the face kernel (independent
             // work: the face kernel is latency-bound, the flux kernel arithmetic-bound); the face
             // kernel at 2 CTAs per SM by default leaves the flux kernel room on every SM
+            const int per = L->face_ctas_per_sm > 0 ? L->face_ctas_per_sm : 2;
             LCK(cudaEventRecord(L->fork, L->stream));
-            face_kernel<false><<<mlp_grid(L, L->fit_face[0], units,
-                                          L->face_ctas_per_sm > 0 ? L->face_ctas_per_sm : 2),
-                                 hf::lc::kTcThreads, sm, L->stream>>>(L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F,
-                                                                      L->dF, L->ok, L->rejected, L->maxs, L->derr,
-                                                                      loop);
+            if (save_acts)
+                face_kernel<FACE_SAVE><<<mlp_grid(L, L->fit_face[2], nf, per), hf::lc::kTcThreads, sm, L->stream>>>(
+                    L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F, L->dF, L->ok, L->rejected, L->maxs, L->derr, loop, saved);
+            else
+                face_kernel<FACE_INFER><<<mlp_grid(L, L->fit_face[0], nf, per), hf::lc::kTcThreads, sm, L->stream>>>(
+                    L->U[L->cur], L->Wp, G, dt, L->Wb, L->P, L->F, L->dF, L->ok, L->rejected, L->maxs, L->derr, loop, none);
             LCK(cudaStreamWaitEvent(L->side, L->fork, 0));
             plain_flux_kernel<<<blocks_for(nf, 256), 256, 0, L->side>>>(L->U[L->cur], G, dt, L->F, loop, nullptr);
             LCK(cudaEventRecord(L->join, L->side));
             LCK(cudaStreamWaitEvent(L->stream, L->join, 0));
         }
         LCK(cudaGetLastError());
-        if (mask_set) *mask_set = true;
+        if (mask_set) *mask_set = !save_acts;
         return HF_OK;
     }
     plain_flux_kernel<<<blocks_for(nf, 256), 256, 0, L->stream>>>(L->U[L->cur], G, dt, L->F, loop,
@@ -1485,16 +1521,15 @@ int hf_lc_create(int n, double dx, double gamma, double cfl, int limiter, hf_lc*
     LCK(cudaStreamCreateWithFlags(&L->side, cudaStreamNonBlocking));
     LCK(cudaEventCreateWithFlags(&L->fork, cudaEventDisableTiming));
     LCK(cudaEventCreateWithFlags(&L->join, cudaEventDisableTiming));
-    LCK(cudaFuncSetAttribute(hf::lc::face_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)hf::lc::mlp_forward_smem()));
-    LCK(cudaFuncSetAttribute(hf::lc::face_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)hf::lc::mlp_forward_smem()));
+    const void* const face[3] = {(const void*)face_kernel<FACE_INFER>, (const void*)face_kernel<FACE_FLUX>,
+                                 (const void*)face_kernel<FACE_SAVE>};
+    for (const void* k : face)
+        LCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hf::lc::mlp_forward_smem()));
     LCK(cudaFuncSetAttribute(hf::lc::mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)hf::lc::mlp_forward_smem()));
     LCK(cudaFuncSetAttribute(hf::lc::mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)hf::lc::mlp_backward_smem()));
-    for (const void* k : {(const void*)hf::lc::face_kernel<false>, (const void*)hf::lc::face_kernel<true>,
-                          (const void*)hf::lc::mlp_forward_kernel})
+    for (const void* k : {face[0], face[1], face[2], (const void*)hf::lc::mlp_forward_kernel})
         LCK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
     {
         int dev = 0;
@@ -1502,21 +1537,25 @@ int hf_lc_create(int n, double dx, double gamma, double cfl, int limiter, hf_lc*
             cudaDeviceGetAttribute(&L->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || L->sms < 1)
             L->sms = 152;
         L->fit_fwd = mlp_fit((const void*)hf::lc::mlp_forward_kernel);
-        L->fit_face[0] = mlp_fit((const void*)hf::lc::face_kernel<false>);
-        L->fit_face[1] = mlp_fit((const void*)hf::lc::face_kernel<true>);
+        for (int k = 0; k < 3; ++k) L->fit_face[k] = mlp_fit(face[k]);
     }
     const size_t cells = (size_t)n * n, nf = nfaces(L);
     int r;
     if ((r = alloc(L, &L->U[0], 4 * cells)) || (r = alloc(L, &L->U[1], 4 * cells)) || (r = alloc(L, &L->F, 4 * nf)) ||
         (r = alloc(L, &L->dF, 4 * nf)) || (r = alloc(L, &L->scale, 2 * nf)) || (r = alloc(L, &L->Y, 4 * nf)) ||
         (r = alloc(L, &L->Z1, (size_t)H * nf)) || (r = alloc(L, &L->Z2, (size_t)H * nf)) || (r = alloc(L, &L->dY, 4 * nf)) ||
-        (r = alloc(L, &L->T, 4 * cells)) || (r = alloc(L, &L->wv, 4)) || (r = alloc(L, &L->X, (size_t)NIN * nf)) ||
+        (r = alloc(L, &L->T, 4 * cells)) || (r = alloc(L, &L->X, (size_t)NIN * nf)) ||
         (r = alloc(L, &L->Wb, (size_t)(H * NIN + H * H + NOUT * H))) || (r = alloc(L, &L->P, (size_t)NPARAM)) ||
-        (r = alloc(L, &L->grad, (size_t)NPARAM)) || (r = alloc(L, &L->m1, (size_t)NPARAM)) ||
+        (r = alloc(L, &L->grad, (size_t)NPARAM + 4)) || (r = alloc(L, &L->m1, (size_t)NPARAM)) ||
         (r = alloc(L, &L->m2, (size_t)NPARAM)) || (r = alloc(L, &L->maxs, 4)) || (r = alloc(L, &L->ok, nf)) ||
-        (r = alloc(L, &L->rejected, 1)) || (r = alloc(L, &L->loss, 1)) || (r = alloc(L, &L->derr, 1)) ||
+        (r = alloc(L, &L->rejected, 1)) ||
         (r = alloc(L, &L->Wp, cells)) || (r = alloc(L, &L->Uc, cells)) || (r = alloc(L, &L->loop, 1)))
         return r;
+    // the loss and the error word behind the gradient: cleared, and read back, in one piece each
+    static_assert(NPARAM % 2 == 0, "the loss follows the gradient");
+    L->loss = reinterpret_cast<double*>(L->grad + NPARAM);
+    L->derr = reinterpret_cast<int*>(L->loss + 1);
+    LCK(cudaMallocHost(&L->out, sizeof(hf_lc::Out)));
     return HF_OK;
 }
 
@@ -1525,6 +1564,8 @@ void hf_lc_destroy(hf_lc* L) {
     if (L->stream) cudaStreamSynchronize(L->stream);
     if (L->side) cudaStreamSynchronize(L->side);
     for (void* p : L->allocs) cudaFree(p);
+    if (L->out) cudaFreeHost(L->out);
+    if (L->pair) cudaGraphExecDestroy(L->pair);
     if (L->fork) cudaEventDestroy(L->fork);
     if (L->join) cudaEventDestroy(L->join);
     if (L->side) cudaStreamDestroy(L->side);
@@ -1642,6 +1683,30 @@ int hf_lc_step(hf_lc* L, double dt, int use_mlp, int64_t* rejected_cells) {
     return HF_OK;
 }
 
+// Two steps of the device loop as a graph: a step is four launches on two streams with their events, and
+// the host needed 85 to 100 us for what the GPU does in 73 (512^2).  Captured once for its settings.
+static int lc_pair_graph(hf_lc* L, int use_mlp) {
+    const hf_lc::PairKey key{L->cur, use_mlp != 0, L->guard_mode, L->fused, L->face_ctas_per_sm, L->bound};
+    const hf_lc::PairKey& k = L->pair_key;
+    if (L->pair && k.cur == key.cur && k.use_mlp == key.use_mlp && k.guard_mode == key.guard_mode && k.fused == key.fused &&
+        k.ctas == key.ctas && k.bound == key.bound)
+        return HF_OK;
+    if (L->pair) cudaGraphExecDestroy(L->pair);
+    L->pair = nullptr;
+    cudaGraph_t g;
+    LCK(cudaStreamBeginCapture(L->stream, cudaStreamCaptureModeThreadLocal));
+    int r = enqueue_lc_step(L, 0.0, use_mlp, L->loop);
+    if (r == HF_OK) r = enqueue_lc_step(L, 0.0, use_mlp, L->loop);
+    const cudaError_t e = cudaStreamEndCapture(L->stream, &g);
+    if (r) return r;
+    if (e != cudaSuccess) return lfail(L, HF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+    const cudaError_t ei = cudaGraphInstantiate(&L->pair, g, 0);
+    cudaGraphDestroy(g);
+    if (ei != cudaSuccess) return lfail(L, HF_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ei));
+    L->pair_key = key;
+    return HF_OK;
+}
+
 // Runs until t_end with CFL dt; returns steps.  The loop is the device's: every step's update forms the
 // next dt, and a step after the end leaves its buffers alone.  The host enqueues as many steps as the
 // last dt it read suggests are left and reads the loop's state once for all of them (it read the wave-speed
@@ -1661,7 +1726,13 @@ int hf_lc_run_to(hf_lc* L, double t_end, int use_mlp, int64_t* steps, int64_t* r
     loop_begin_kernel<<<1, 1, 0, L->stream>>>(L->loop, L->maxs);
     LCK(cudaGetLastError());
     const int cur = L->cur;
+    if (use_mlp && L->fused && !L->wp_valid) {   // the steps find the primitives of the state before them
+        prims_kernel<<<blocks_for(L->n * L->n, 256), 256, 0, L->stream>>>(L->U[cur], L->n, grid(L).g1, L->Wp);
+        LCK(cudaGetLastError());
+        L->wp_valid = true;
+    }
     const bool wp = L->wp_valid;
+    if ((r = lc_pair_graph(L, use_mlp))) return r;
     for (;;) {
         LCK(cudaMemcpyAsync(&S, L->loop, sizeof S, cudaMemcpyDeviceToHost, L->stream));
         LCK(cudaStreamSynchronize(L->stream));
@@ -1676,8 +1747,8 @@ int hf_lc_run_to(hf_lc* L, double t_end, int use_mlp, int64_t* steps, int64_t* r
         const double left = (S.t_end - S.t - slow * S.dt) / full;
         const double want = slow + (left > 0.0 ? std::ceil(left) : 0.0);
         const int k = want < 1.0 ? 1 : (want > 64.0 ? 64 : (int)want);
-        for (int i = 0; i < k; ++i)
-            if ((r = enqueue_lc_step(L, S.dt, use_mlp, L->loop))) return r;
+        // (pairs: the state before one is in the buffer it was captured with)
+        for (int i = 0; i < k; i += 2) LCK(cudaGraphLaunch(L->pair, L->stream));
     }
     if (steps) *steps = S.taken;
     if (rejected_cells) *rejected_cells = S.rejected;
@@ -1724,10 +1795,11 @@ int hf_lc_train_step(hf_lc* L, const float* U0, const float* T, const float* w, 
         LCK(cudaMemcpyAsync(L->U[L->cur], U0, bytes, cudaMemcpyHostToDevice, L->stream));
         L->wp_valid = false;
     }
-    LCK(cudaMemcpyAsync(L->T, T, bytes, cudaMemcpyHostToDevice, L->stream));
-    LCK(cudaMemcpyAsync(L->wv, w, 4 * sizeof(float), cudaMemcpyHostToDevice, L->stream));
     int r = fluxes(L, (float)dt, true, true);
     if (r) return r;
+    LCK(cudaMemcpyAsync(L->T, T, bytes, cudaMemcpyHostToDevice, L->side));   // beside the forward
+    LCK(cudaEventRecord(L->join, L->side));
+    LCK(cudaStreamWaitEvent(L->stream, L->join, 0));
     const float rr = (float)(dt / L->dx);
     if (L->train_guard) {   // the guard of inference: rejected faces take the plain flux
         LCK(cudaMemsetAsync(L->ok, 1, nf, L->stream));
@@ -1742,22 +1814,22 @@ int hf_lc_train_step(hf_lc* L, const float* U0, const float* T, const float* w, 
             L->U[L->cur], L->F, L->dF, nullptr, G, rr, 0.0f, 0, L->U[L->cur ^ 1], L->maxs, nullptr, nullptr, nullptr,
             nullptr);
     }
-    LCK(cudaMemsetAsync(L->loss, 0, 8, L->stream));
-    loss_grad_kernel<<<blocks_for(nf, 256), 256, 0, L->stream>>>(L->U[L->cur ^ 1], L->T, L->scale, L->n, rr, L->wv,
+    LCK(cudaMemsetAsync(L->grad, 0, NPARAM * sizeof(float) + sizeof(double), L->stream));   // and the loss
+    loss_grad_kernel<<<blocks_for(nf, 256), 256, 0, L->stream>>>(L->U[L->cur ^ 1], L->T, L->scale, L->n, rr,
+                                                                  make_float4(w[0], w[1], w[2], w[3]),
                                                                   L->train_guard ? L->ok : nullptr, L->dY, L->loss);
-    LCK(cudaMemsetAsync(L->grad, 0, NPARAM * sizeof(float), L->stream));
     launch_backward(L, nf);
     L->adam_t += 1;
     const float b1 = 0.9f, b2 = 0.999f;
     const float c1 = 1.f - powf(b1, (float)L->adam_t), c2 = 1.f - powf(b2, (float)L->adam_t);
-    adam_kernel<<<16, 256, 0, L->stream>>>(L->P, L->grad, L->m1, L->m2, L->Wb, (float)lr, b1, b2, 1e-8f, c1, c2);
-    to_bf16_kernel<<<16, 256, 0, L->stream>>>(L->P, L->Wb);
+    adam_kernel<<<(NPARAM + 255) / 256, 256, 0, L->stream>>>(L->P, L->grad, L->m1, L->m2, L->Wb, (float)lr, b1, b2, 1e-8f,
+                                                             c1, c2);
     LCK(cudaGetLastError());
-    if (loss) {
-        LCK(cudaMemcpyAsync(loss, L->loss, 8, cudaMemcpyDeviceToHost, L->stream));
-    }
+    LCK(cudaMemcpyAsync(L->out, L->loss, sizeof(hf_lc::Out), cudaMemcpyDeviceToHost, L->stream));
     LCK(cudaStreamSynchronize(L->stream));
-    return check_derr(L);
+    if (loss) *loss = L->out->loss;
+    if (L->out->derr) return lfail(L, HF_ERR_DEVICE, "a bounded device wait gave up (tensor-core MLP)");
+    return HF_OK;
 }
 
 // ---- test entry points: the MLP alone on given inputs ----
