@@ -17,7 +17,7 @@ independent replica (the path does not shard across GPUs) and `value` sums the r
 
 Other workloads (`--workload`, one JSON line each, not the headline):
     square    one N x N four-quadrant block (--n, --scheme, --limiter)
-    batch     512 batched Riemann problems in one persistent launch (autotuned)
+    batch     512 batched Riemann problems, one launch per step of all (autotuned)
     uns       the ~1M-triangle channel, edge-based (or --uns-per-side) fluxes
     quad256   the 256^2 Godunov problem as a batch of one (the whole run one launch)
     learned   the 512^2 learned coarse step (FP32 + the tcgen05 MLP on every face)
@@ -225,7 +225,7 @@ def timed_device(stream, fn):
 def bench_batch(args):
     """The batched workload: 512 seeded four-quadrant Riemann problems (sides log-uniform in
     64..1024), MUSCL-Hancock MinBee, per-instance dt, autotuned launch shape, the run of
-    `steps` steps in one persistent launch captured in a CUDA graph."""
+    `steps` steps captured in a CUDA graph."""
     import numpy as np  # noqa: F401
     import torch
     from hyperflow_gb300 import BatchSolver, cases
@@ -268,19 +268,18 @@ def bench_batch(args):
                    "l2": "state 2 x %.0f MB > 129 MB L2, no flush needed" % (cells * 32 / 1e6)},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm, "traffic": None, "peak_kind": peak_kind,
-                     "kernel": "batch_kernel<MUSCL-Hancock> (persistent, all instances, one launch per run)"},
+                     "kernel": "batch_kernel<MUSCL-Hancock> (all instances, one launch per step)"},
         "cpu_baseline": {"value": sample_cells / cpu_s / 1e6, "unit": "Mcell-updates/s", "cores": nth,
                          "kind": "port", "sample": f"every 16th instance ({len(sample)}), 20 steps each"},
-        "e2e": None, "gpu_launches": 1, "clocks": clk.summary()}), flush=True)
+        "e2e": None, "gpu_launches": args.steps, "clocks": clk.summary()}), flush=True)
     b.close()
 
 
 def bench_quad256(args):
     """The reference's first configuration: the 256^2 four-quadrant Riemann problem, Godunov +
-    HLLC, CFL 0.8, `steps` steps (200 in the reference's run).  At 65,536 cells a step is too
-    small to fill the GPU through per-step launches, so the whole run goes through the batched
-    path as a batch of one: one persistent launch, grid barriers between steps.  The per-block
-    solver's device loop (CUDA graph of the per-step launches) is timed beside it."""
+    HLLC, CFL 0.8, `steps` steps (200 in the reference's run).  The run goes
+    through the batched path as a batch of one: a CUDA graph of one launch per step.  The per-block
+    solver's device loop (a CUDA graph too) is timed beside it."""
     import torch
     from hyperflow_gb300 import BatchSolver, CartSolver, cases
     from oracle.oracle import Oracle, build_port
@@ -313,15 +312,15 @@ def bench_quad256(args):
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f64",
         "data": "synthetic (the case's own initial condition)",
         "config": {"workload": "quadrant_riemann_256x256_godunov_hllc_fp64", "cells": cells, "cfl": 0.8,
-                   "path": "batch of one: one persistent launch for the whole run", "autotuned_config": best,
-                   "l2": "state 2 x 2 MB, L2-resident by nature across the steps of the one launch"},
+                   "path": "batch of one: one launch per step", "autotuned_config": best,
+                   "l2": "state 2 x 2 MB, L2-resident by nature across the steps"},
         "per_block_device_loop_value": cells * args.steps / (ms_pb / 1e3) / 1e6,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm, "traffic": None, "peak_kind": peak_kind,
-                     "kernel": "batch_kernel<Godunov> (persistent)"},
+                     "kernel": "batch_kernel<Godunov>"},
         "cpu_baseline": {"value": cells * args.steps / cpu_s / 1e6, "unit": "Mcell-updates/s", "cores": nth,
                          "kind": "port", "sample": f"the whole run ({args.steps} steps)"},
-        "e2e": None, "gpu_launches": 1, "clocks": clk.summary()}), flush=True)
+        "e2e": None, "gpu_launches": args.steps, "clocks": clk.summary()}), flush=True)
     b.close()
     s.close()
 

@@ -1,6 +1,6 @@
 """Python host mirror of the batched MUSCL-Hancock entry points
-(include/hyperflow_gb300_batch.h): many independent single-block cases, one persistent
-cooperative kernel per run of steps, optional CUDA graph, autotuned launch shape."""
+(include/hyperflow_gb300_batch.h): many independent single-block cases, one launch per
+step of all of them, optional CUDA graph, autotuned launch shape."""
 from __future__ import annotations
 
 import ctypes as C

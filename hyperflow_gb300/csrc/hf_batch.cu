@@ -1,5 +1,5 @@
 // Batched single-block cases: hundreds of independent, all-transmissive cases of different
-// sizes advanced together by one persistent cooperative kernel per run of steps, captured in a
+// sizes advanced together, one launch per step, a run of steps captured in a
 // CUDA graph, each case with its own CFL dt.  C ABI in include/hyperflow_gb300_batch.h.
 //
 // Each case is the reference's single-block MUSCL-Hancock step
@@ -9,24 +9,28 @@
 // four sides every ghost value is a mirror copy of an interior value
 // (transmissive_boundary.cpp:25-104; the fill order makes corner ghosts mirror in x and in y).
 // So the tile loader reads the mirrored interior cell directly and the state is stored without
-// ghosts, and the CFL maximum over ghost cells equals the maximum over the interior.  A single
-// small case (the 256^2 Godunov quadrant problem) runs as a batch of one: its whole run of steps
-// is one launch, with no per-step launch chain.
+// ghosts, and the CFL maximum over ghost cells equals the maximum over the interior.
 //
-// Work decomposition: every case is cut into TX x TY tiles; the tiles of all cases form
-// one list that the persistent CTAs walk round-robin.  A step ends at a grid barrier
-// (bounded wait; a timeout raises the error word and stops the kernel).  The CFL maxima
-// rotate through three slots per case: read (this step's dt), write (the next step's, by
-// the update epilogue), and cleared (for the step after).
+// Work decomposition: every case is cut into tiles; the tiles of all cases form one list, the
+// dearest first, a CTA each.  The CFL maxima rotate through three slots: read (this step's
+// dt), write (the next step's, by the update epilogue), and one that the step before cleared; the
+// last CTA of a step clears the slot just read and counts the step.
 //
-// Autotuning: the tile shape, threads per CTA and the number of halo staging buffers
-// (1 = load then compute; 2 = the next tile's halo is fetched with cp.async while the
-// current tile computes) come from a small set of compiled configurations; the autotuner
-// times each on the real batch and keeps the fastest.
+// (A step was a round of a persistent cooperative kernel: one launch per run, a grid barrier per
+// step.  The loop's state cost the tile computation registers, and a CTA's next tile waited for its
+// descriptor: with the same tiles 54.3 against 52.6 ms for 100 steps of 24 cases of 64^2 .. 385^2,
+// Godunov 22.7 against 21.0, and 2.39 against 2.23 for two cases of 16^2 and 81^2.  Letting the next
+// step's CTAs take their places during a step's tail gave nothing on large batches and put two on
+// one SM where there are fewer tiles than SMs: 9.7 against 6.0 ms for one case of 256^2.)
+//
+// Autotuning: two configurations give each case a tile shape of its own (case_tiles), the others one
+// shape for all; the autotuner times each on the real batch and keeps the fastest.
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <memory>
+#include <queue>
 #include <string>
 #include <vector>
 
@@ -43,8 +47,18 @@ struct BatchInst {
     int n;                 // cells per side
     int pitch;             // doubles per row: n rounded up to even (a TMA row stride is a multiple of 16 bytes)
     long long off;         // offset (doubles) of the case's [4][n][pitch] state
-    double dx, dy;
+    double dx, dy, one_dx, one_dy;   // and 1 / dx, 1 / dy
 };
+
+// One tile of the batch
+struct __align__(16) BatchTile {
+    int inst, x0, y0;        // interior cells
+    int n, pitch;            // the case's
+    int tx, ty;
+    unsigned int m[3];       // TileShape's
+    long long off;           // the case's
+};
+static_assert(sizeof(BatchTile) == 48, "a tile is copied in 16-byte pieces");
 
 struct BatchCtrl {
     double gamma, g1, cfl;
@@ -54,8 +68,7 @@ struct BatchCtrl {
     int scheme;             // 0 Godunov, 1 MUSCL-Hancock
     int ninst;
     int err;
-    unsigned int bar_count;
-    unsigned int bar_gen;
+    unsigned int tiles_done;           // of the running step
     long long hllc_errors;
     unsigned long long first_nonpos;   // least batch_key of a cell a step left with density or
                                        // pressure not positive, ~0 when none
@@ -74,53 +87,13 @@ struct BatchDev {
     const BatchInst* inst;
     const CUtensorMap* maps;       // MUSCL-Hancock: per state parity, per case, [2][ninst]
     int ninst;
-    const int* tile_inst;
-    const int* tile_xy;            // x0 | (y0 << 16), interior cells
+    const BatchTile* tiles;        // [ntiles]
     long long ntiles;
     double* U[2];
     unsigned long long* acc;       // [3][ninst][2]
     double* t;                     // [ninst]
     double* last_dt;               // [ninst]
 };
-
-__device__ __forceinline__ unsigned long long gtimer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// grid-wide barrier with a bounded wait (10 s); false after a timeout
-__device__ bool grid_barrier(BatchCtrl* c) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned int* gen = &c->bar_gen;
-        const unsigned int g0 = *gen;
-        __threadfence();
-        const unsigned int arrived = atomicAdd(&c->bar_count, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            c->bar_count = 0u;
-            __threadfence();
-            atomicAdd(&c->bar_gen, 1u);
-            ok = 1;
-        } else {
-            ok = 0;
-            const unsigned long long t0 = gtimer_ns();
-            for (;;) {
-                if (*gen != g0) { ok = 1; break; }
-                if (c->err != 0) break;
-                if (gtimer_ns() - t0 > 10000000000ull) {
-                    atomicCAS(&c->err, 0, HF_DEV_TIMEOUT);
-                    break;
-                }
-                __nanosleep(128);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return ok != 0;
-}
 
 __device__ __forceinline__ int mirror(int x, int n) {
     x = x < 0 ? -1 - x : (x >= n ? 2 * n - 1 - x : x);
@@ -132,320 +105,315 @@ constexpr unsigned kBatchWaitLimit = 1u << 22;   // bounded mbarrier polls befor
 __device__ __forceinline__ void cp_async8(void* dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// shared-memory tiles of the two schemes: halo H cells, the staged state, the scratch after it
-template <int SCHEME, int TX, int TY>
-struct BatchTile;
-template <int TX, int TY>
-struct BatchTile<0, TX, TY> : GoTile<TX, TY> {   // Godunov: 1-cell halo; the cells' values, face fluxes
-    static constexpr int H = 1;
-};
-template <int TX, int TY>
-struct BatchTile<1, TX, TY> : MhTile<TX, TY> {   // MUSCL-Hancock: 2-cell halo; evolved states, face fluxes
-    static constexpr int H = 2;
-};
-
-// stage tile `t`'s state + mirrored halo into sU (cp.async, one commit group)
-template <int SCHEME, int TX, int TY, int NT>
-__device__ __forceinline__ void stage_tile(const BatchDev& d, const double* __restrict__ U, long long t,
-                                           double* sU) {
-    using T = BatchTile<SCHEME, TX, TY>;
-    const int inst = d.tile_inst[t];
-    const int xy = d.tile_xy[t];
-    const int x0 = xy & 0xffff, y0 = xy >> 16;
-    const BatchInst I = d.inst[inst];
-    const double* __restrict__ base = U + I.off;
-    const size_t plane = (size_t)I.pitch * I.n;
-    for (int k = threadIdx.x; k < T::U_SIZE; k += NT) {
-        const int v = k / (T::UY * T::UX);
-        const int r = k - v * (T::UY * T::UX);
-        const int ly = r / T::UX, lx = r - ly * T::UX;
-        const int gx = mirror(x0 + lx - T::H, I.n), gy = mirror(y0 + ly - T::H, I.n);
-        cp_async8(sU + k, base + v * plane + (size_t)gy * I.pitch + gx);
-    }
-    cp_async_commit();
-}
-
-// MUSCL-Hancock tiles by TMA: one 3-D box (the tile and its 2-cell halo, all four variables) of
-// the case's state per tile, issued by thread 0 on `bar`; positions outside the case arrive as
-// zeros and mirror_halo then writes the transmissive ghosts there.  (The box's x start, x0 - 2, is
-// even, as a TMA copy of FP64 needs; Godunov's 1-cell halo would start at an odd x, so Godunov
-// batches keep the element-wise loader.)
-template <int TX, int TY>
-__device__ __forceinline__ void tma_tile(const BatchDev& d, int p, long long t, double* sU, uint64_t* bar) {
-    using T = BatchTile<1, TX, TY>;
-    const int inst = d.tile_inst[t];
-    const int xy = d.tile_xy[t];
-    const int x0 = xy & 0xffff, y0 = xy >> 16;
-    // the previous tile's reads and writes of this buffer (generic proxy) come before the copy
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(bar, T::U_SIZE * 8);
-    tma_load_3d(sU, &d.maps[(size_t)p * d.ninst + inst], bar, x0 - T::H, y0 - T::H, 0);
-}
 
 // The halo positions outside the case (within 2 cells of it) take the mirrored interior values,
 // the transmissive ghosts (transmissive_boundary.cpp:25-104; corners mirrored in x and in y).
 // Every source is an interior cell inside the same box.  Positions further out are never read.
-template <int TX, int TY, int NT>
-__device__ __forceinline__ void mirror_halo(double* sU, int x0, int y0, int n) {
-    using T = BatchTile<1, TX, TY>;
-    constexpr int H = T::H;
-    if (x0 >= H && y0 >= H && x0 + TX + H <= n && y0 + TY + H <= n) return;   // the box lies inside the case
-    for (int k = threadIdx.x; k < T::U_SIZE; k += NT) {
-        const int v = k / (T::UY * T::UX);
-        const int r = k - v * (T::UY * T::UX);
-        const int ly = r / T::UX, lx = r - ly * T::UX;
-        const int gx = x0 + lx - H, gy = y0 + ly - H;
-        if (gx >= 0 && gx < n && gy >= 0 && gy < n) continue;
-        if (gx < -H || gy < -H || gx >= n + H || gy >= n + H) continue;
-        const int sx = mirror(gx, n) - x0 + H, sy = mirror(gy, n) - y0 + H;
-        sU[k] = sU[(v * T::UY + sy) * T::UX + sx];
+// A warp's row at a time; ends with __syncthreads() where there was something to write.
+template <int NT>
+__device__ __forceinline__ void mirror_halo(double* sU, int tx, int ty, int x0, int y0, int n) {
+    constexpr int H = 2;
+    if (x0 >= H && y0 >= H && x0 + tx + H <= n && y0 + ty + H <= n) return;   // the box lies inside the case
+    const int ux = tx + 2 * H, uy = ty + 2 * H;
+    for (int r = threadIdx.x >> 5; r < 4 * uy; r += NT / 32) {
+        const int ly = r % uy, gy = y0 + ly - H;
+        if (gy < -H || gy >= n + H) continue;
+        double* const row = sU + r * ux;
+        const double* const from = row + (mirror(gy, n) - gy) * ux;
+        for (int lx = threadIdx.x & 31; lx < ux; lx += 32) {
+            const int gx = x0 + lx - H;
+            if (gx < -H || gx >= n + H || (gx >= 0 && gx < n && gy >= 0 && gy < n)) continue;
+            row[lx] = from[lx + mirror(gx, n) - gx];
+        }
     }
+    __syncthreads();
 }
 
-template <int SCHEME, int TX, int TY, int NT, int STAGES, int MINB>
-__global__ void __launch_bounds__(NT, MINB) batch_kernel(BatchDev d, int nsteps) {
-    using BT = BatchTile<SCHEME, TX, TY>;
+// One step of every case, a CTA per tile.
+// What bounds it: the FP64 and integer pipes of the tile computation, as in the Cartesian step kernel,
+// whose CTA it shares (two per SM, any tile that fits 110.9 KB); beyond that the lanes a
+// tile wastes on the part of it outside its case, and the tail of a step.  So a case has a tile that
+// divides it well, and the dearest tiles are dispatched first.  Measured (Mcell-updates/s, 100 steps;
+// before: the best of the fixed shapes, in a persistent kernel): 24 cases of 64^2 .. 385^2 1902 (1738),
+// Godunov 4753 (4036); 64 of 48^2 .. 97^2 1729 (1148); 8 of 128^2 1526 (1327); 40 of 83^2 .. 501^2 1963.
+// One block of 2048^2 on the Cartesian path, without a tail or partial tiles to speak of, has 2108.
+//
+// MUSCL-Hancock tiles come by TMA: one 3-D box (the tile and its 2-cell halo, all four variables) of
+// the case's state, issued by thread 0; positions outside the case arrive as zeros and mirror_halo
+// then writes the transmissive ghosts there.  (The box's x start, x0 - 2, is even, as a TMA copy of
+// FP64 needs; Godunov's 1-cell halo would start at an odd x, so Godunov batches load by element.)
+template <int NT, int SCHEME, int LIM>
+__global__ void __launch_bounds__(NT, 2) batch_kernel(const __grid_constant__ BatchDev d) {
+    constexpr int H = SCHEME == 1 ? 2 : 1;
     constexpr int CALLS = SCHEME == 1 ? 2 : 1;   // TimeStep calls per step (+ the predictor's)
     extern __shared__ __align__(1024) double smem[];
-    double* sUb[STAGES];
-#pragma unroll
-    for (int k = 0; k < STAGES; ++k) sUb[k] = smem + k * BT::U_SIZE;
-    double* sW = smem + STAGES * BT::U_SIZE;
-    __shared__ double sdt[5];
-
-    BatchCtrl* c = d.ctrl;
-    const long long step0 = c->step, calls0 = c->calls;
-    const double g = c->gamma, g1 = c->g1, cfl = c->cfl;
-    const int lim = c->limiter, ninst = c->ninst;
-    int herr = 0;
-    // MUSCL-Hancock: one mbarrier per staging buffer for the TMA loads, and its phase
-    __shared__ uint64_t tbar[2];
-    uint32_t tph[2] = {0u, 0u};
-    bool failed = false;
-    if (SCHEME == 1) {
-        if (threadIdx.x == 0) {
-            mbar_init(&tbar[0], 1);
-            mbar_init(&tbar[1], 1);
+    double* const sU = smem;
+    __shared__ double sc[3];
+    __shared__ uint64_t bar;
+    BatchCtrl* const c = d.ctrl;
+    const BatchTile T = d.tiles[blockIdx.x];
+    const RowShape S{{T.tx, T.ty, {T.m[0], T.m[1], T.m[2]}}};
+    const int usize = 4 * (T.tx + 2 * H) * (T.ty + 2 * H);
+    double* const sW = smem + usize;
+    const int p = (int)(c->step & 1), ar = (int)(c->step % 3);
+    if (threadIdx.x == 0) {
+        if (SCHEME == 1) {
+            mbar_init(&bar, 1);
+            mbar_expect_tx(&bar, usize * 8);
+            tma_load_3d(sU, &d.maps[(size_t)p * d.ninst + T.inst], &bar, T.x0 - H, T.y0 - H, 0);
         }
+        // TimeStep::operator() for this case (timestep.cpp:29-68) from last step's maxima
+        const unsigned long long* a = d.acc + ((size_t)ar * d.ninst + T.inst) * 2;
+        const double dx = d.inst[T.inst].dx, dy = d.inst[T.inst].dy, cfl = c->cfl;
+        const double dtx = smin(1e16, div_rn(dx, bitsd(a[0])));
+        const double dty = smin(1e16, div_rn(dy, bitsd(a[1])));
+        const double dt = ((c->calls + 1 <= 10) ? 0.2 * cfl : cfl) * smin(dtx, dty);    // the step's call
+        sc[0] = dt;
+        if (SCHEME == 1) {
+            const double dtp = ((c->calls + 2 <= 10) ? 0.2 * cfl : cfl) * smin(dtx, dty);   // the predictor's
+            sc[1] = div_rn(0.5 * dtp, dx);   // muscl_hancock.cpp:248-249
+            sc[2] = div_rn(0.5 * dtp, dy);
+        }
+        if (T.x0 == 0 && T.y0 == 0) {
+            d.t[T.inst] = d.t[T.inst] + dt;
+            d.last_dt[T.inst] = dt;
+        }
+    }
+    if (SCHEME == 1) {
+        __syncthreads();   // the mbarrier is initialised
+        const bool ok = mbar_wait_bounded(&bar, 0u, kBatchWaitLimit);
+        if (__syncthreads_or(!ok || (threadIdx.x == 0 && c->err != 0))) {
+            if (!ok && threadIdx.x == 0) {
+                atomicCAS(&c->err, 0, (int)HF_DEV_TIMEOUT);
+                mbar_wait_bounded(&bar, 0u, kBatchWaitLimit);   // let the copy in flight land before exit
+            }
+            __syncthreads();
+            return;        // this step and those after it are not counted
+        }
+        mirror_halo<NT>(sU, T.tx, T.ty, T.x0, T.y0, T.n);
+    } else {
+        const double* __restrict__ base = d.U[p] + T.off;
+        const int uxy = (T.tx + 2) * (T.ty + 2);
+        for (int k = threadIdx.x; k < uxy; k += NT) {
+            const int ly = S.row2(k), lx = k - ly * (T.tx + 2);
+            const double* q = base + (size_t)mirror(T.y0 + ly - H, T.n) * T.pitch + mirror(T.x0 + lx - H, T.n);
+#pragma unroll
+            for (int v = 0; v < 4; ++v) cp_async8(sU + v * uxy + k, q + (size_t)v * T.pitch * T.n);
+        }
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
         __syncthreads();
     }
-
-    for (int s = 0; s < nsteps; ++s) {
-        const long long step = step0 + s;
-        const int p = (int)(step & 1);
-        const int ar = (int)(step % 3), aw = (int)((step + 1) % 3), az = (int)((step + 2) % 3);
-        const long long calls = calls0 + CALLS * s;
-        const double m0 = (calls + 1 <= 10) ? 0.2 * cfl : cfl;        // step TimeStep call
-        const double m1 = (calls + 2 <= 10) ? 0.2 * cfl : cfl;        // predictor call
-        for (int i = blockIdx.x * NT + threadIdx.x; i < 2 * ninst; i += gridDim.x * NT)
-            d.acc[(size_t)az * 2 * ninst + i] = 0ull;
-        const double* __restrict__ U = d.U[p];
-        double* __restrict__ Un = d.U[p ^ 1];
-        long long t = blockIdx.x;
-        if (STAGES == 2 && t < d.ntiles) {
-            if (SCHEME == 1) {
-                if (threadIdx.x == 0) tma_tile<TX, TY>(d, p, t, sUb[0], &tbar[0]);
-            } else {
-                stage_tile<SCHEME, TX, TY, NT>(d, U, t, sUb[0]);
-            }
-        }
-        int buf = 0;
-        for (; t < d.ntiles; t += gridDim.x) {
-            double* sU = sUb[STAGES == 2 ? buf : 0];
-            const int sb = STAGES == 2 ? buf : 0;   // this tile's staging buffer and mbarrier
-            if (SCHEME == 1) {
-                if (threadIdx.x == 0) {
-                    if (STAGES == 1) tma_tile<TX, TY>(d, p, t, sU, &tbar[0]);
-                    else if (t + gridDim.x < d.ntiles) tma_tile<TX, TY>(d, p, t + gridDim.x, sUb[buf ^ 1], &tbar[buf ^ 1]);
-                }
-                const bool ok = mbar_wait_bounded(&tbar[sb], tph[sb], kBatchWaitLimit);
-                if (__syncthreads_or(!ok)) {
-                    failed = true;
-                    break;
-                }
-                tph[sb] ^= 1u;
-            } else if (STAGES == 1) {
-                stage_tile<SCHEME, TX, TY, NT>(d, U, t, sU);
-                cp_async_wait<0>();
-            } else {
-                const long long tn = t + gridDim.x;
-                if (tn < d.ntiles) {
-                    stage_tile<SCHEME, TX, TY, NT>(d, U, tn, sUb[buf ^ 1]);
-                    cp_async_wait<1>();
-                } else {
-                    cp_async_wait<0>();
-                }
-            }
-            const int inst = d.tile_inst[t];
-            const int xy = d.tile_xy[t];
-            const int x0 = xy & 0xffff, y0 = xy >> 16;
-            const BatchInst I = d.inst[inst];
-            if (SCHEME == 1) mirror_halo<TX, TY, NT>(sU, x0, y0, I.n);
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                // TimeStep::operator() for this case (timestep.cpp:29-68) from last step's maxima
-                const unsigned long long* a = d.acc + ((size_t)ar * ninst + inst) * 2;
-                // (divisions on the integer pipes: the same correctly rounded quotients, without
-                // the FP64 pipe's Newton sequences on one thread while the CTA waits)
-                const double dtx = smin(1e16, div_rn(I.dx, bitsd(a[0])));
-                const double dty = smin(1e16, div_rn(I.dy, bitsd(a[1])));
-                sdt[0] = m0 * smin(dtx, dty);
-                if (SCHEME == 1) {
-                    const double dtp = m1 * smin(dtx, dty);
-                    sdt[1] = div_rn(0.5 * dtp, I.dx);   // muscl_hancock.cpp:248-249
-                    sdt[2] = div_rn(0.5 * dtp, I.dy);
-                }
-                sdt[3] = div_rn(1.0, I.dx);             // muscl_hancock.cpp:352-353, godunov.cpp:97-98
-                sdt[4] = div_rn(1.0, I.dy);
-            }
-            __syncthreads();
-            const double dt = sdt[0], hdx = sdt[1], hdy = sdt[2], one_dx = sdt[3], one_dy = sdt[4];
-            if (SCHEME == 0)
-                herr += go_tile_fluxes<NT>(BT(), sU, sW, g, g1, x0, y0, I.n, I.n);
-            else if (lim == 0)
-                herr += mh_tile_fluxes<NT, 0>(BT(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
-            else
-                herr += mh_tile_fluxes<NT, 1>(BT(), sU, sW, g, g1, hdx, hdy, x0, y0, I.n, I.n);
-            double mx = 0.0, my = 0.0;
-            double* __restrict__ out = Un + I.off;
-            const size_t plane = (size_t)I.pitch * I.n;
-            for (int it = threadIdx.x; it < TX * TY; it += NT) {
-                const int ox = it % TX, oy = it / TX;
-                const int gx = x0 + ox, gy = y0 + oy;
-                if (gx < I.n && gy < I.n) {
-                    double un[4];
-                    if (SCHEME == 0) go_update(BT(), sU, sW, ox, oy, dt, one_dx, one_dy, un);
-                    else mh_update(BT(), sU, sW, ox, oy, dt, one_dx, one_dy, un);
+    const double g = c->gamma, g1 = c->g1;
+    const int herr = SCHEME == 0 ? go_tile_fluxes<NT>(S, sU, sW, g, g1, T.x0, T.y0, T.n, T.n)
+                                 : mh_tile_fluxes<NT, LIM>(S, sU, sW, g, g1, sc[1], sc[2], T.x0, T.y0, T.n, T.n);
+    double mx = 0.0, my = 0.0;
+    const double dt = sc[0], one_dx = d.inst[T.inst].one_dx, one_dy = d.inst[T.inst].one_dy;
+    const size_t plane = (size_t)T.pitch * T.n;
+#pragma unroll 1
+    for (int it = threadIdx.x; it < T.tx * T.ty; it += NT) {
+        const int oy = S.row0(it), ox = it - oy * T.tx;
+        const int gx = T.x0 + ox, gy = T.y0 + oy;
+        if (gx >= T.n || gy >= T.n) continue;
+        double un[4];
+        if (SCHEME == 0) go_update(S, sU, sW, ox, oy, dt, one_dx, one_dy, un);
+        else mh_update(S, sU, sW, ox, oy, dt, one_dx, one_dy, un);
+        const long long at = T.off + (long long)gy * T.pitch + gx;
+        double* const out = d.U[p ^ 1] + at;
 #pragma unroll
-                    for (int v = 0; v < 4; ++v) out[v * plane + (size_t)gy * I.pitch + gx] = un[v];
-                    double sx, sy;
-                    if (!speeds(g, g1, un, sx, sy))
-                        atomicMin(&c->first_nonpos, batch_key(step, I.off + (long long)gy * I.pitch + gx));
-                    mx = nmax(mx, sx);
-                    my = nmax(my, sy);
-                }
-            }
-            unsigned long long* aw_p = d.acc + ((size_t)aw * ninst + inst) * 2;
-            block_max2_atomic<NT>(mx, my, aw_p, aw_p + 1);
-            if (x0 == 0 && y0 == 0 && threadIdx.x == 0) {
-                d.t[inst] = d.t[inst] + dt;
-                d.last_dt[inst] = dt;
-            }
-            __syncthreads();   // smem reuse by the next tile
-            buf ^= 1;
-        }
-        if (failed) {
-            if (threadIdx.x == 0) {
-                atomicCAS(&c->err, 0, (int)HF_DEV_TIMEOUT);
-                // let the copies in flight land before the CTA's shared memory goes
-                for (int k = 0; k < 2; ++k) mbar_wait_bounded(&tbar[k], tph[k], kBatchWaitLimit);
-            }
-            __syncthreads();
-            break;
-        }
-        if (!grid_barrier(c)) break;
+        for (int v = 0; v < 4; ++v) out[v * plane] = un[v];
+        double sx, sy;
+        if (!speeds(g, g1, un, sx, sy)) atomicMin(&c->first_nonpos, batch_key(c->step, at));
+        mx = nmax(mx, sx);
+        my = nmax(my, sy);
     }
+    unsigned long long* const aw = d.acc + ((size_t)(ar == 2 ? 0 : ar + 1) * d.ninst + T.inst) * 2;
+    block_max2_atomic<NT>(mx, my, aw, aw + 1);
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
-    if (blockIdx.x == 0 && threadIdx.x == 0 && c->err == 0) {
-        c->step = step0 + nsteps;
-        c->calls = calls0 + CALLS * nsteps;
+    // the last CTA ends the step: the maxima just read are cleared (the next step but one writes them)
+    __shared__ int last;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&c->tiles_done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    for (int i = threadIdx.x; i < 2 * d.ninst; i += NT) d.acc[(size_t)ar * 2 * d.ninst + i] = 0ull;
+    if (threadIdx.x == 0) {
+        c->tiles_done = 0u;
+        c->step = c->step + 1;
+        c->calls = c->calls + CALLS;
     }
 }
 
-// CFL maxima of the current state, into slot step % 3 (after an upload)
-template <int TX, int TY, int NT>
-__global__ void __launch_bounds__(NT) batch_cfl_kernel(BatchDev d) {
+// CFL maxima of the current state, into slot step % 3 (after an upload): a row of CTAs per case from
+// `first`
+constexpr int kCflThreads = 256;
+__global__ void __launch_bounds__(kCflThreads) batch_cfl_kernel(BatchDev d, int first, int count) {
     BatchCtrl* c = d.ctrl;
     const long long step = c->step;
     const int p = (int)(step & 1), ar = (int)(step % 3);
-    const long long t = blockIdx.x;
-    const int inst = d.tile_inst[t];
-    const int xy = d.tile_xy[t];
-    const int x0 = xy & 0xffff, y0 = xy >> 16;
-    const BatchInst I = d.inst[inst];
-    const double* U = d.U[p] + I.off;
-    const size_t plane = (size_t)I.pitch * I.n;
-    double mx = 0.0, my = 0.0;
-    for (int it = threadIdx.x; it < TX * TY; it += NT) {
-        const int gx = x0 + it % TX, gy = y0 + it / TX;
-        if (gx < I.n && gy < I.n) {
-            const size_t o = (size_t)gy * I.pitch + gx;
-            double sx, sy;
-            wave_terms(c->gamma, c->g1, U[o], U[plane + o], U[2 * plane + o], U[3 * plane + o], sx, sy);
-            mx = nmax(mx, sx);
-            my = nmax(my, sy);
-        }
+    const double g = c->gamma, g1 = c->g1;
+    for (int i = blockIdx.y; i < count; i += gridDim.y) {
+        const BatchInst I = d.inst[first + i];
+        const double* U = d.U[p] + I.off;
+        const size_t plane = (size_t)I.pitch * I.n;
+        double mx = 0.0, my = 0.0;
+        for (int gy = blockIdx.x; gy < I.n; gy += gridDim.x)
+            for (int gx = threadIdx.x; gx < I.n; gx += kCflThreads) {
+                const size_t o = (size_t)gy * I.pitch + gx;
+                const double u[4] = {U[o], U[plane + o], U[2 * plane + o], U[3 * plane + o]};
+                double sx, sy;
+                speeds(g, g1, u, sx, sy);
+                mx = nmax(mx, sx);
+                my = nmax(my, sy);
+            }
+        unsigned long long* a = d.acc + ((size_t)ar * c->ninst + first + i) * 2;
+        block_max2_atomic<kCflThreads>(mx, my, a, a + 1);
+        __syncthreads();   // block_max2_atomic's shared memory is used again
     }
-    unsigned long long* a = d.acc + ((size_t)ar * c->ninst + inst) * 2;
-    block_max2_atomic<NT>(mx, my, a, a + 1);
 }
 
+// A configuration's tile shape and CTA.  tx = 0: each case has its own (case_tiles), by a model that
+// counts what the rounds of a CTA's warps leave idle beside the work, or (model 1) the work alone: the first
+// was better for batches of several rounds of tiles (24 cases of 64^2 .. 385^2: 52.5 against 56.3 ms for 100
+// steps), the second for smaller ones (8 of 128^2: 9.61, 8.66; one of 256^2: 5.28, 4.68).
 struct BatchConfig {
-    int tx, ty, threads, stages, min_ctas_per_sm;
+    int tx, ty, threads, model;
 };
-
-// tile shape, threads, halo staging buffers, CTAs per SM the registers are budgeted for
-// (the last, 32x4 tiles of 128 threads at four CTAs per SM, is for batches too small to give
-// every SM several large tiles per step, such as a single 256^2 case)
-constexpr BatchConfig kConfigs[] = {{32, 14, 256, 1, 2}, {32, 14, 256, 2, 2}, {32, 19, 448, 1, 2},
-                                    {32, 12, 256, 1, 3}, {24, 25, 448, 1, 2}, {32, 4, 128, 1, 4}};
+constexpr BatchConfig kConfigs[] = {{0, 0, 448, 0},   {0, 0, 448, 1},   {32, 19, 448, 0},
+                                    {24, 25, 448, 0}, {32, 14, 256, 0}, {32, 4, 448, 0}};
 constexpr int kNumConfigs = 6;
 
-template <int SCHEME, int TX, int TY, int ST>
-size_t batch_smem() {
-    using T = BatchTile<SCHEME, TX, TY>;
-    return (size_t)(ST * T::U_SIZE + T::WORK) * 8;
-}
-
-template <int SCHEME, int TX, int TY, int NT, int ST, int MINB>
-cudaError_t launch_batch(const BatchDev& d, int nsteps, int sms, cudaStream_t s, bool cfl_only) {
-    auto k = batch_kernel<SCHEME, TX, TY, NT, ST, MINB>;
-    const size_t smem = batch_smem<SCHEME, TX, TY, ST>();
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int NT>
+cudaError_t launch_threads(int scheme, int limiter, const BatchDev& d, long long nsteps, cudaStream_t s) {
+    auto k = scheme == 0 ? batch_kernel<NT, 0, 0> : limiter == 0 ? batch_kernel<NT, 1, 0> : batch_kernel<NT, 1, 1>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes);
     if (e != cudaSuccess) return e;
-    if (cfl_only) {
-        batch_cfl_kernel<TX, TY, NT><<<(unsigned)d.ntiles, NT, 0, s>>>(d);
-        return cudaGetLastError();
+    for (long long i = 0; i < nsteps && e == cudaSuccess; ++i) {
+        k<<<(unsigned)d.ntiles, NT, kTileBytes, s>>>(d);
+        e = cudaGetLastError();
     }
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, NT, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    long long grid = (long long)per_sm * sms;
-    if (grid > d.ntiles) grid = d.ntiles;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(NT);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;   // all CTAs co-resident: the grid barrier is safe
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, d, nsteps);
+    return e;
 }
 
-template <int SCHEME>
-cudaError_t launch_scheme_config(int k, const BatchDev& d, int nsteps, int sms, cudaStream_t s, bool cfl_only) {
-    switch (k) {
-        case 0: return launch_batch<SCHEME, 32, 14, 256, 1, 2>(d, nsteps, sms, s, cfl_only);
-        case 1: return launch_batch<SCHEME, 32, 14, 256, 2, 2>(d, nsteps, sms, s, cfl_only);
-        case 2: return launch_batch<SCHEME, 32, 19, 448, 1, 2>(d, nsteps, sms, s, cfl_only);
-        case 3: return launch_batch<SCHEME, 32, 12, 256, 1, 3>(d, nsteps, sms, s, cfl_only);
-        case 4: return launch_batch<SCHEME, 24, 25, 448, 1, 2>(d, nsteps, sms, s, cfl_only);
-        default: return launch_batch<SCHEME, 32, 4, 128, 1, 4>(d, nsteps, sms, s, cfl_only);
-    }
+cudaError_t launch_batch(int k, int scheme, int limiter, const BatchDev& d, long long nsteps, cudaStream_t s) {
+    return kConfigs[k].threads == 256 ? launch_threads<256>(scheme, limiter, d, nsteps, s)
+                                      : launch_threads<448>(scheme, limiter, d, nsteps, s);
 }
 
-cudaError_t launch_batch_config(int k, int scheme, const BatchDev& d, int nsteps, int sms, cudaStream_t s,
-                                bool cfl_only) {
-    return scheme == 0 ? launch_scheme_config<0>(k, d, nsteps, sms, s, cfl_only)
-                       : launch_scheme_config<1>(k, d, nsteps, sms, s, cfl_only);
+// What a tile costs: microseconds of an SM that has enough of them (`work`), and from start to end of a
+// CTA alone on its SM (`alone`): the warp-items of its phases at their instruction counts, a time per tile,
+// and (model 0) what the rounds of the CTA's 14 warps leave idle.  Fitted to steps of many tiles and of one
+// per SM: MUSCL-Hancock tiles of 32 x 19, 16 x 16 and 32 x 4 cells take 44.5, 22.2 and 13.4 us of an SM (both
+// models within 7 %); with 32 x 14, alone, 55.5, 30.8, 18.0 and 47.5 us.
+struct TileCost {
+    double work, alone;
+};
+TileCost tile_cost(int scheme, int model, int tx, int ty) {
+    constexpr int W = kTileThreads / 32;
+    auto warps = [](int items) { return (items + 31) / 32; };
+    const int faces = warps((tx + 1) * ty) + warps(tx * (ty + 1)), cells = warps(tx * ty);
+    const int first = scheme == 0 ? warps((tx + 2) * (ty + 2)) : warps((tx + 2) * ty) + warps(tx * (ty + 2));
+    const double items = scheme == 0 ? 0.55 * first + 0.95 * faces + 0.75 * cells : 2.0 * first + 2.2 * faces + 0.8 * cells;
+    const double rounds = (scheme == 0 ? 0.35 : 1.0) * ((std::max(first, faces) + W - 1) / W);
+    return {model == 0 ? 1.9 + 0.196 * items + 2.34 * rounds : 2.5 + 0.23 * items, 3.0 + 0.165 * items + 7.2 * rounds};
+}
+
+// The tile shape of each case (sides n) by a model.  A case takes, of the shapes whose whole
+// tile is within a limit, the one whose tiles are the least work (the last row of tiles has as many rows
+// as the case has left); the limit is the one with which the tiles, dealt dearest first to the
+// 2 x sms resident CTAs, are done first.  No limit wastes the fewest lanes and halo items and suits a batch
+// of many rounds of tiles; a small batch needs more, smaller tiles.
+std::vector<TileShape> case_tiles(int scheme, int model, const std::vector<int>& n, int sms) {
+    struct Shape {
+        int tx, ty;
+        double time;   // of a whole tile beside another on its SM
+    };
+    auto shared_time = [](const TileCost& c) { return std::max(2.0 * c.work, c.alone); };
+    std::vector<Shape> shapes;
+    double lo = 0.0, hi = 0.0;
+    for (int tx = 8; tx <= 64; tx += 2)
+        for (int ty = 2; ty <= 32; ++ty) {
+            if (!tile_fits(scheme, tx, ty)) continue;
+            const double t = shared_time(tile_cost(scheme, model, tx, ty));
+            shapes.push_back({tx, ty, t});
+            lo = lo == 0.0 ? t : std::min(lo, t);
+            hi = std::max(hi, t);
+        }
+    std::vector<double> limits;
+    for (double l = hi; l > lo; l *= 0.85) limits.push_back(l);
+    limits.push_back(lo);
+    // per distinct side and limit: the best shape
+    std::map<int, std::vector<int>> best;
+    for (int side : n) {
+        if (best.count(side)) continue;
+        std::vector<int> at(limits.size(), -1);
+        std::vector<double> least(limits.size(), 0.0);
+        for (size_t k = 0; k < shapes.size(); ++k) {
+            const Shape& s = shapes[k];
+            const int rest = side % s.ty;
+            const double column = (double)(side / s.ty) * tile_cost(scheme, model, s.tx, s.ty).work +
+                                  (rest ? tile_cost(scheme, model, s.tx, rest).work : 0.0);
+            const double work = column * ((side + s.tx - 1) / s.tx);
+            for (size_t l = 0; l < limits.size() && s.time <= limits[l]; ++l)
+                if (at[l] < 0 || work < least[l]) {
+                    least[l] = work;
+                    at[l] = (int)k;
+                }
+        }
+        best.emplace(side, std::move(at));
+    }
+    size_t pick = 0;
+    double done = 0.0;
+    for (size_t l = 0; l < limits.size(); ++l) {
+        std::map<double, std::pair<long long, double>> kinds;   // shared time -> tiles, their time alone
+        double work = 0.0;
+        long long tiles = 0;
+        auto add = [&](int tx, int ty, long long k) {
+            const TileCost c = tile_cost(scheme, model, tx, ty);
+            auto& e = kinds[shared_time(c)];
+            e.first += k;
+            e.second = c.alone;
+            work += c.work * (double)k;
+            tiles += k;
+        };
+        for (int side : n) {
+            const Shape& s = shapes[best[side][l]];
+            const long long across = (side + s.tx - 1) / s.tx;
+            if (side >= s.ty) add(s.tx, s.ty, across * (side / s.ty));
+            if (side % s.ty) add(s.tx, side % s.ty, across);
+        }
+        double end = 0.0;
+        if (tiles <= sms) {
+            for (auto& e : kinds) end = std::max(end, e.second.second);
+        } else if (tiles <= 24LL * sms) {
+            std::priority_queue<double, std::vector<double>, std::greater<double>> cta;
+            for (int k = 0; k < 2 * sms; ++k) cta.push(0.0);
+            for (auto e = kinds.rbegin(); e != kinds.rend(); ++e)
+                for (long long k = 0; k < e->second.first; ++k) {
+                    const double at = cta.top() + e->first;
+                    cta.pop();
+                    cta.push(at);
+                }
+            // an SM's two CTAs: while one is done the other runs faster, but not twice as fast
+            std::vector<double> f;
+            for (; !cta.empty(); cta.pop()) f.push_back(cta.top());
+            for (int k = 0; k < sms; ++k) end = std::max(end, f[k] + 0.65 * (f[2 * sms - 1 - k] - f[k]));
+        } else {
+            end = work / sms + 0.3 * kinds.rbegin()->first;   // of many rounds: their mean and a tail
+        }
+        if (l == 0 || end < done) {
+            done = end;
+            pick = l;
+        }
+    }
+    std::vector<TileShape> out;
+    for (int side : n) {
+        const Shape& s = shapes[best[side][pick]];
+        out.push_back(tile_shape(s.tx, s.ty));
+    }
+    return out;
 }
 
 }  // namespace hf
@@ -470,10 +438,10 @@ struct hf_batch {
     double* t = nullptr;
     double* last_dt = nullptr;
     // per configuration: device tile lists
-    int* tile_inst[hf::kNumConfigs] = {};
-    int* tile_xy[hf::kNumConfigs] = {};
+    std::vector<hf::TileShape> shapes[hf::kNumConfigs];
+    hf::BatchTile* tiles[hf::kNumConfigs] = {};
     long long ntiles[hf::kNumConfigs] = {};
-    CUtensorMap* maps[hf::kNumConfigs] = {};   // MUSCL-Hancock: the TMA maps of the config's tile box
+    CUtensorMap* maps[hf::kNumConfigs] = {};   // MUSCL-Hancock: the TMA maps of the cases' tile boxes
     int config = 0;
     // graphs: key = (config, nsteps)
     struct G { int config; long long nsteps; cudaGraphExec_t exec; };
@@ -482,6 +450,8 @@ struct hf_batch {
 };
 
 namespace {
+
+constexpr long long kGraphSteps = 128;   // steps of one graph
 
 int bfail(hf_batch* b, int code, const std::string& m) {
     if (b) b->err = m;
@@ -496,32 +466,48 @@ int bfail(hf_batch* b, int code, const std::string& m) {
     } while (0)
 
 int ensure_tiles(hf_batch* b, int k) {
-    if (b->tile_inst[k]) return HF_OK;
+    if (b->tiles[k]) return HF_OK;
     const hf::BatchConfig C = hf::kConfigs[k];
-    std::vector<int> ti, txy;
-    for (size_t i = 0; i < b->inst.size(); ++i) {
-        const int n = b->inst[i].n;
-        for (int y0 = 0; y0 < n; y0 += C.ty)
-            for (int x0 = 0; x0 < n; x0 += C.tx) {
-                ti.push_back((int)i);
-                txy.push_back(x0 | (y0 << 16));
-            }
+    const size_t n = b->inst.size();
+    std::vector<int> sides(n);
+    for (size_t i = 0; i < n; ++i) sides[i] = b->inst[i].n;
+    b->shapes[k] = C.tx ? std::vector<hf::TileShape>(n, hf::tile_shape(C.tx, C.ty))
+                        : hf::case_tiles(b->scheme, C.model, sides, b->sms);
+    // rows of tiles, the dearest first
+    struct Row {
+        double time;
+        int inst, y0;
+    };
+    std::vector<Row> rows;
+    size_t ntiles = 0;
+    for (size_t i = 0; i < n; ++i) {
+        const hf::TileShape& s = b->shapes[k][i];
+        for (int y0 = 0; y0 < sides[i]; y0 += s.ty)
+            rows.push_back({hf::tile_cost(b->scheme, C.model, s.tx, std::min(s.ty, sides[i] - y0)).work, (int)i, y0});
+        ntiles += (size_t)((sides[i] + s.tx - 1) / s.tx) * ((sides[i] + s.ty - 1) / s.ty);
     }
-    BCK(cudaMalloc(&b->tile_inst[k], ti.size() * sizeof(int)));
-    BCK(cudaMalloc(&b->tile_xy[k], txy.size() * sizeof(int)));
-    b->allocs.push_back(b->tile_inst[k]);
-    b->allocs.push_back(b->tile_xy[k]);
-    BCK(cudaMemcpy(b->tile_inst[k], ti.data(), ti.size() * sizeof(int), cudaMemcpyHostToDevice));
-    BCK(cudaMemcpy(b->tile_xy[k], txy.data(), txy.size() * sizeof(int), cudaMemcpyHostToDevice));
-    b->ntiles[k] = (long long)ti.size();
+    std::stable_sort(rows.begin(), rows.end(), [](const Row& a, const Row& c) { return a.time > c.time; });
+    std::vector<hf::BatchTile> tiles;
+    tiles.reserve(ntiles);
+    for (const Row& r : rows) {
+        const hf::TileShape& s = b->shapes[k][r.inst];
+        const hf::BatchInst& I = b->inst[r.inst];
+        for (int x0 = 0; x0 < I.n; x0 += s.tx)
+            tiles.push_back({r.inst, x0, r.y0, I.n, I.pitch, s.tx, s.ty, {s.m[0], s.m[1], s.m[2]}, I.off});
+    }
+    hf::BatchTile* dt = nullptr;
+    BCK(cudaMalloc(&dt, tiles.size() * sizeof(hf::BatchTile)));
+    b->allocs.push_back(dt);
+    BCK(cudaMemcpy(dt, tiles.data(), tiles.size() * sizeof(hf::BatchTile), cudaMemcpyHostToDevice));
+    b->ntiles[k] = (long long)tiles.size();
+    b->tiles[k] = dt;
     return HF_OK;
 }
 
 // The TMA maps of configuration k (MUSCL-Hancock batches): per state parity and case, the case's
-// [4][n][pitch] state as a 3-D tensor {n, n, 4} with the box of the config's tile and its 2-cell halo.
+// [4][n][pitch] state as a 3-D tensor {n, n, 4} with the box of its tile and the 2-cell halo.
 int ensure_maps(hf_batch* b, int k) {
     if (b->scheme != 1 || b->maps[k]) return HF_OK;
-    const hf::BatchConfig C = hf::kConfigs[k];
     hf::EncodeTiledFn enc = hf::tensor_map_encoder();
     if (!enc) return bfail(b, HF_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
     const size_t n = b->inst.size();
@@ -531,7 +517,7 @@ int ensure_maps(hf_batch* b, int k) {
             const hf::BatchInst& I = b->inst[i];
             cuuint64_t dims[3] = {(cuuint64_t)I.n, (cuuint64_t)I.n, 4};
             cuuint64_t strides[2] = {(cuuint64_t)I.pitch * 8, (cuuint64_t)I.pitch * I.n * 8};
-            cuuint32_t box[3] = {(cuuint32_t)(C.tx + 4), (cuuint32_t)(C.ty + 4), 4};
+            cuuint32_t box[3] = {(cuuint32_t)(b->shapes[k][i].tx + 4), (cuuint32_t)(b->shapes[k][i].ty + 4), 4};
             cuuint32_t es[3] = {1, 1, 1};
             CUresult r = enc(&maps[par * n + i], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, b->U[par] + I.off, dims, strides,
                              box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -551,8 +537,7 @@ hf::BatchDev devview(hf_batch* b, int k) {
     d.inst = b->dinst;
     d.maps = b->maps[k];
     d.ninst = (int)b->inst.size();
-    d.tile_inst = b->tile_inst[k];
-    d.tile_xy = b->tile_xy[k];
+    d.tiles = b->tiles[k];
     d.ntiles = b->ntiles[k];
     d.U[0] = b->U[0];
     d.U[1] = b->U[1];
@@ -569,14 +554,17 @@ long long read_step(hf_batch* b) {
     return s;
 }
 
-// refresh the read slot's CFL maxima from the current state (after an upload)
-int refresh_cfl(hf_batch* b) {
-    long long step = read_step(b);
-    int ar = (int)(step % 3);
-    BCK(cudaMemsetAsync(b->acc + (size_t)ar * 2 * b->inst.size(), 0, 2 * b->inst.size() * sizeof(unsigned long long), b->stream));
-    int r = ensure_tiles(b, 0);
-    if (r) return r;
-    BCK(hf::launch_batch_config(0, b->scheme, devview(b, 0), 0, b->sms, b->stream, true));
+// refresh the read slot's CFL maxima of `count` cases from `first` on (after their upload)
+int refresh_cfl(hf_batch* b, long long step, int first, int count) {
+    const int ar = (int)(step % 3);
+    const size_t n = b->inst.size();
+    BCK(cudaMemsetAsync(b->acc + ((size_t)ar * n + first) * 2, 0, 2 * (size_t)count * sizeof(unsigned long long),
+                        b->stream));
+    int rows = 1;
+    for (int i = first; i < first + count; ++i) rows = std::max(rows, b->inst[i].n);
+    hf::batch_cfl_kernel<<<dim3((unsigned)std::min(rows, 2 * b->sms), (unsigned)std::min(count, 65535)),
+                           hf::kCflThreads, 0, b->stream>>>(devview(b, 0), first, count);
+    BCK(cudaGetLastError());
     BCK(cudaStreamSynchronize(b->stream));
     return HF_OK;
 }
@@ -643,6 +631,8 @@ int hf_batch_create(const char* manifest, size_t len, hf_batch** out) {
             b->total_doubles += 4LL * I.pitch * nx;
             I.dx = (xr - xl) / nx;   // mesh_block.cpp:227-236
             I.dy = (yt - yb) / ny;
+            I.one_dx = 1.0 / I.dx;   // muscl_hancock.cpp:352-353, godunov.cpp:97-98
+            I.one_dy = 1.0 / I.dy;
             b->inst.push_back(I);
             b->total_cells += (long long)nx * ny;
             // the centroids depend on the ghost width in floating point (mesh_block.cpp:239-257),
@@ -697,7 +687,7 @@ int hf_batch_create(const char* manifest, size_t len, hf_batch** out) {
         BCK(cudaMemcpy2D(b->U[0] + I.off, (size_t)I.pitch * 8, init[i].data(), (size_t)I.n * 8, (size_t)I.n * 8,
                          (size_t)4 * I.n, cudaMemcpyHostToDevice));
     }
-    return refresh_cfl(b);
+    return refresh_cfl(b, 0, 0, (int)n);
 }
 
 void hf_batch_destroy(hf_batch* b) {
@@ -736,7 +726,7 @@ int hf_batch_config_info(int k, int* tile_x, int* tile_y, int* threads, int* sta
     if (tile_x) *tile_x = C.tx;
     if (tile_y) *tile_y = C.ty;
     if (threads) *threads = C.threads;
-    if (stages) *stages = C.stages;
+    if (stages) *stages = 1;
     return HF_OK;
 }
 
@@ -754,25 +744,26 @@ int hf_batch_run(hf_batch* b, int64_t nsteps, int use_graph) {
     if (!r) r = ensure_maps(b, b->config);
     if (r) return r;
     hf::BatchDev d = devview(b, b->config);
-    if (!use_graph) {
-        BCK(hf::launch_batch_config(b->config, b->scheme, d, (int)nsteps, b->sms, b->stream, false));
-        return HF_OK;
+    while (use_graph && nsteps > 0) {   // graphs of up to kGraphSteps steps
+        const long long n = std::min<long long>(nsteps, kGraphSteps);
+        cudaGraphExec_t exec = nullptr;
+        for (auto& g : b->graphs)
+            if (g.config == b->config && g.nsteps == n) exec = g.exec;
+        if (!exec) {
+            cudaGraph_t graph;
+            BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+            cudaError_t e = hf::launch_batch(b->config, b->scheme, b->limiter, d, n, b->stream);
+            cudaError_t e2 = cudaStreamEndCapture(b->stream, &graph);
+            if (e != cudaSuccess) return bfail(b, HF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+            if (e2 != cudaSuccess) return bfail(b, HF_ERR_CUDA, std::string("end capture: ") + cudaGetErrorString(e2));
+            BCK(cudaGraphInstantiate(&exec, graph, 0));
+            cudaGraphDestroy(graph);
+            b->graphs.push_back({b->config, n, exec});
+        }
+        BCK(cudaGraphLaunch(exec, b->stream));
+        nsteps -= n;
     }
-    cudaGraphExec_t exec = nullptr;
-    for (auto& g : b->graphs)
-        if (g.config == b->config && g.nsteps == nsteps) exec = g.exec;
-    if (!exec) {
-        cudaGraph_t graph;
-        BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-        cudaError_t e = hf::launch_batch_config(b->config, b->scheme, d, (int)nsteps, b->sms, b->stream, false);
-        cudaError_t e2 = cudaStreamEndCapture(b->stream, &graph);
-        if (e != cudaSuccess) return bfail(b, HF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-        if (e2 != cudaSuccess) return bfail(b, HF_ERR_CUDA, std::string("end capture: ") + cudaGetErrorString(e2));
-        BCK(cudaGraphInstantiate(&exec, graph, 0));
-        cudaGraphDestroy(graph);
-        b->graphs.push_back({b->config, nsteps, exec});
-    }
-    BCK(cudaGraphLaunch(exec, b->stream));
+    BCK(hf::launch_batch(b->config, b->scheme, b->limiter, d, nsteps, b->stream));
     return HF_OK;
 }
 
@@ -808,9 +799,9 @@ int hf_batch_autotune(hf_batch* b, int steps_per_trial, int* best, double* ms_pe
         if (r) return r;
         hf::BatchDev d = devview(b, k);
         // warm (first launch pays the shared-memory opt-in), then time
-        BCK(hf::launch_batch_config(k, b->scheme, d, 1, b->sms, b->stream, false));
+        BCK(hf::launch_batch(k, b->scheme, b->limiter, d, 1, b->stream));
         cudaEventRecord(e0, b->stream);
-        BCK(hf::launch_batch_config(k, b->scheme, d, steps_per_trial, b->sms, b->stream, false));
+        BCK(hf::launch_batch(k, b->scheme, b->limiter, d, steps_per_trial, b->stream));
         cudaEventRecord(e1, b->stream);
         int er = check_device_error(b);
         if (er) return er;
@@ -849,7 +840,7 @@ int hf_batch_set_state(hf_batch* b, int i, const double* in) {
     const hf::BatchInst& I = b->inst[i];
     BCK(cudaMemcpy2D(b->U[step & 1] + I.off, (size_t)I.pitch * 8, in, (size_t)I.n * 8, (size_t)I.n * 8,
                      (size_t)4 * I.n, cudaMemcpyHostToDevice));
-    return refresh_cfl(b);
+    return refresh_cfl(b, step, i, 1);
 }
 
 int hf_batch_instance_time(hf_batch* b, int i, double* t, double* last_dt) {

@@ -519,8 +519,7 @@ __device__ __forceinline__ void store_tile(const RowShape& S, const double* sU, 
 // the tile's 42 warp-items of predictor cells are three rounds of the 14 warps, its 40 of faces too.
 // Measured at 2048^2 (Mcell-updates/s): 1973; 512 threads and 64 registers 1962, 320 threads and 32 x 18
 // tiles 1933, 256 threads and 32 x 14 1880, three CTAs of 256 threads and 32 x 12 tiles 1751.
-constexpr int kNT = 448, kTileDoubles = 13856;
-constexpr size_t kTileBytes = (size_t)kTileDoubles * 8;
+constexpr int kNT = kTileThreads;
 
 template <int LIM>
 __global__ void __launch_bounds__(kNT, 2) mh_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
@@ -911,31 +910,39 @@ TileShape tile_shape(int tx, int ty) {
     return t;
 }
 
-// The tile: of the even widths (a TMA copy starts on 16 bytes) and heights that fit a CTA's shared memory,
-// the one whose tiles take the least time by the model below -- the rounds of a CTA's 14 warps over the
-// tile's cells and faces, at their instruction counts, times the waves of the 2 x sms resident CTAs.
-// A mesh of many tiles gets the shape with the fewest wasted lanes and halo items; a small one a shape that
-// fills the GPU once: 256^2 in 32 x 19 tiles would leave 44 of 152 SMs without work.
-TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms) {
+bool tile_fits(int scheme, int tx, int ty) {
+    return (scheme == 0 ? go_tile_doubles(tx, ty) : mh_tile_doubles(tx, ty)) <= kTileDoubles;
+}
+
+// The rounds of a CTA's warps over the tile's cells and faces, at their instruction counts.
+double tile_time(int scheme, int tx, int ty) {
     constexpr int W = kNT / 32;
     auto warps = [](int items) { return (items + 31) / 32; };
     auto rounds = [](int w) { return (w + W - 1) / W; };
+    const int faces = rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))), cells = rounds(warps(tx * ty));
+    return scheme == 0
+        ? 550.0 * rounds(warps((tx + 2) * (ty + 2))) + 950.0 * faces + 750.0 * cells + 400.0
+        : 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) + 2200.0 * faces + 800.0 * cells + 600.0;
+}
+
+// The tile: of the even widths (a TMA copy starts on 16 bytes) and heights that fit a CTA's shared memory,
+// the one whose tiles take the least time (tile_time) times the waves of the 2 x sms resident CTAs.
+// A mesh of many tiles gets the shape with the fewest wasted lanes and halo items; a small one a shape that
+// fills the GPU once: 256^2 in 32 x 19 tiles would leave 44 of 152 SMs without work.
+TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms) {
     double best = 0.0;
     int bx = 8, by = 2;
     for (int tx = 8; tx <= 64; tx += 2)
         for (int ty = 2; ty <= 32; ++ty) {
-            if ((scheme == 0 ? go_tile_doubles(tx, ty) : mh_tile_doubles(tx, ty)) > kTileDoubles) continue;
+            if (!tile_fits(scheme, tx, ty)) continue;
             long long n = 0;
             for (int b = 0; b < nb; ++b) n += (long long)((nx[b] + tx - 1) / tx) * ((ny[b] + ty - 1) / ty);
-            const int faces = rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))), cells = rounds(warps(tx * ty));
-            const double tile = scheme == 0
-                ? 550.0 * rounds(warps((tx + 2) * (ty + 2))) + 950.0 * faces + 750.0 * cells + 400.0
-                : 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) + 2200.0 * faces + 800.0 * cells + 600.0;
             const long long rest = n % (2 * sms);
             // one CTA alone on its SM runs faster than beside a second one, but not twice as fast
             const double waves = (double)(n / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
-            if (best == 0.0 || tile * waves < best) {
-                best = tile * waves;
+            const double time = tile_time(scheme, tx, ty) * waves;
+            if (best == 0.0 || time < best) {
+                best = time;
                 bx = tx;
                 by = ty;
             }

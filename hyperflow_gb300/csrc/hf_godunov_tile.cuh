@@ -1,5 +1,5 @@
 // The first-order Godunov tile computation shared by the Cartesian stencils (hf_cart.cu) and the
-// batched persistent kernel (hf_batch.cu): GodunovScheme::calculate_fluxes_{x,y} +
+// batched step kernel (hf_batch.cu): GodunovScheme::calculate_fluxes_{x,y} +
 // calculate_spatial_update (src/fvm_2d_cart/scheme/godunov/godunov.cpp:27-118) with the
 // forward-Euler update (forward_euler.cpp:19-29).
 //
@@ -19,12 +19,6 @@
 
 namespace hf {
 
-template <int TX, int TY>
-struct GoTile : TileRows<TX, TY> {
-    static constexpr int UX = TX + 2, UY = TY + 2;
-    static constexpr int U_SIZE = 4 * UX * UY;                                               // doubles
-    static constexpr int WORK = 5 * UX * UY + 4 * TY * (TX + 1) + 4 * (TY + 1) * TX;
-};
 // doubles of shared memory a tile takes: the state with its halo, the cells' values, the fluxes
 inline int go_tile_doubles(int tx, int ty) {
     return 9 * (tx + 2) * (ty + 2) + 4 * ty * (tx + 1) + 4 * (ty + 1) * tx;

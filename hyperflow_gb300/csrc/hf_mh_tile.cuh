@@ -1,5 +1,5 @@
 // The MUSCL-Hancock tile computation shared by the Cartesian stencils (hf_cart.cu) and the
-// batched persistent kernel (hf_batch.cu).
+// batched step kernel (hf_batch.cu).
 //
 // Input: sU, the tile's conservative state plus a 2-cell halo in shared memory,
 // [4][ty+4][tx+4].  Output, in sA: the HLLC fluxes of the tile's x and y faces, each in the place of
@@ -21,22 +21,7 @@
 
 namespace hf {
 
-// A tile of tx x ty cells: the shape's sizes, and the row of item `it` of a list whose rows are tx, tx + 1
-// or tx + 2 long.  Of fixed size (the batch's configurations) or chosen for a block (RowShape).
-template <int TX, int TY>
-struct TileRows {
-    __device__ static constexpr int tx() { return TX; }
-    __device__ static constexpr int ty() { return TY; }
-    __device__ static constexpr int row0(int it) { return it / TX; }
-    __device__ static constexpr int row1(int it) { return it / (TX + 1); }
-    __device__ static constexpr int row2(int it) { return it / (TX + 2); }
-};
-template <int TX, int TY>
-struct MhTile : TileRows<TX, TY> {
-    static constexpr int UX = TX + 4, UY = TY + 4;
-    static constexpr int U_SIZE = 4 * UY * UX;                                  // doubles
-    static constexpr int WORK = 8 * ((TX + 2) * TY + TX * (TY + 2));
-};
+// A tile of tx x ty cells: the row of item `it` of a list whose rows are tx, tx + 1 or tx + 2 long.
 struct RowShape {
     TileShape t;
     __device__ int tx() const { return t.tx; }
@@ -132,13 +117,13 @@ __device__ __forceinline__ int mh_tile_fluxes(const S& s, const double* sU, doub
                                               double hdy, int x0, int y0, int nx, int ny,
                                               unsigned long long* first_bad = nullptr,
                                               unsigned long long key_base = 0) {
-    const int tx = s.tx(), ty = s.ty(), ux = tx + 4, plane = ux * (ty + 4);
-    const int nax = (tx + 2) * ty, nay = tx * (ty + 2);
-    double* const sY = sA + 8 * nax;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int px = (nax + 31) >> 5, pxy = px + ((nay + 31) >> 5);
 #pragma unroll 1
-    for (int w = warp; w < pxy; w += NT / 32) {
+    for (int w = warp;; w += NT / 32) {
+        const int tx = s.tx(), ty = s.ty(), ux = tx + 4, plane = ux * (ty + 4);
+        const int nax = (tx + 2) * ty, nay = tx * (ty + 2), px = (nax + 31) >> 5;
+        if (w >= px + ((nay + 31) >> 5)) break;
+        double* const sY = sA + 8 * nax;
         const bool y = w >= px;
         const int it = (y ? w - px : w) * 32 + lane, n = y ? nay : nax;
         const int row = y ? s.row0(it) : s.row2(it);
@@ -147,11 +132,13 @@ __device__ __forceinline__ int mh_tile_fluxes(const S& s, const double* sU, doub
         mh_predict<LIM>(y, sU + (cy + 2) * ux + cx + 2, plane, y ? ux : 1, g1, y ? hdy : hdx, (y ? sY : sA) + it, n);
     }
     __syncthreads();
-    const int nfx = (tx + 1) * ty, nfy = tx * (ty + 1);
-    const int fx = (nfx + 31) >> 5, fxy = fx + ((nfy + 31) >> 5);
     int herr = 0;
 #pragma unroll 1
-    for (int w = warp; w < fxy; w += NT / 32) {
+    for (int w = warp;; w += NT / 32) {
+        const int tx = s.tx(), ty = s.ty(), nfx = (tx + 1) * ty, nfy = tx * (ty + 1);
+        const int nax = (tx + 2) * ty, nay = tx * (ty + 2), fx = (nfx + 31) >> 5;
+        if (w >= fx + ((nfy + 31) >> 5)) break;
+        double* const sY = sA + 8 * nax;
         const bool y = w >= fx;
         const int it = (y ? w - fx : w) * 32 + lane, n = y ? nay : nax;
         const int row = y ? s.row0(it) : s.row1(it), col = it - row * (y ? tx : tx + 1);

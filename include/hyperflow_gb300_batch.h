@@ -4,10 +4,9 @@
  * (src/fvm_2d_cart/scheme/muscl_hancock/muscl_hancock.cpp:41-376) or Godunov step
  * (src/fvm_2d_cart/scheme/godunov/godunov.cpp:27-118), with TimeStep
  * (src/fvm_2d_cart/scheme/timestep/timestep.cpp:29-68) and ForwardEuler (forward_euler.cpp:15-33),
- * applied to every case with its own CFL dt, in one persistent cooperative kernel launch per
- * run of steps (optionally captured in a CUDA graph).  Each case's results equal what the
- * reference computes for that case alone, bit for bit.  A batch of one runs a small case's
- * whole loop in one launch.  Status codes are the HF_* codes of hyperflow_gb300.h.  States are
+ * applied to every case with its own CFL dt, in one kernel launch per step of all cases
+ * (a run of steps optionally captured in a CUDA graph).  Each case's results equal what the
+ * reference computes for that case alone, bit for bit.  Status codes are the HF_* codes of hyperflow_gb300.h.  States are
  * interior-only SoA [4][n][n].
  */
 #ifndef HYPERFLOW_GB300_BATCH_H
@@ -36,7 +35,8 @@ const char* hf_batch_last_error_message(const hf_batch* b);
 int hf_batch_sizes(const hf_batch* b, int* ninstances, int64_t* total_cells);
 int hf_batch_instance_side(const hf_batch* b, int i, int* n);
 
-/* compiled launch configurations: tile shape, threads per CTA, halo staging buffers */
+/* launch configurations: tile shape (0 x 0: each case has its own), threads per CTA, halo staging
+ * buffers */
 int hf_batch_num_configs(int* n);
 int hf_batch_config_info(int k, int* tile_x, int* tile_y, int* threads, int* stages);
 int hf_batch_set_config(hf_batch* b, int k);
@@ -45,8 +45,8 @@ int hf_batch_set_config(hf_batch* b, int k);
  * configuration) receives the timings */
 int hf_batch_autotune(hf_batch* b, int steps_per_trial, int* best, double* ms_per_step);
 
-/* nsteps steps of every case in one persistent launch; use_graph replays a captured graph of
- * that launch (captured once per (configuration, nsteps)) */
+/* nsteps steps of every case, one launch each; use_graph replays a captured graph of
+ * them (captured once per (configuration, nsteps), in pieces of up to 128 steps) */
 int hf_batch_run(hf_batch* b, int64_t nsteps, int use_graph);
 int hf_batch_sync(hf_batch* b);
 
