@@ -71,6 +71,10 @@ struct hf_ctx {
     hf::StepPlan plan{};        // the all-blocks launch (plan.nb = 0: not usable)
     hf::StepState* dstep = nullptr;
     bool solo = false;          // one block whose ghosts are interior cells' values or Dirichlet states
+    bool user_graphs = false;   // a caller has captured steps
+    int clamp = -1;             // the device's clamp switch, -1 when not known
+    hf::StepOut* out = nullptr; // a step's dt and count, in host memory the GPU maps
+    long long steps_known = -1; // steps completed, -1 when the device may have moved on
     bool clean = false;         // the step's accumulators are cleared (by the end of the last step)
     bool block_launches = false;   // hf_set_block_launches: one stencil launch per block instead
     std::vector<double*> allocs;
@@ -509,11 +513,12 @@ void ev_record(hf_ctx* ctx, int kind, bool start) {
 
 // the block updates of a step, in one launch or one per block; hout: host buffers that also take the
 // updated cells, or null.  With frames off the one launch ends the step too.
-int enqueue_blocks(hf_ctx* ctx, double* const* hout) {
+int enqueue_blocks(hf_ctx* ctx, double* const* hout, hf::StepOut* out = nullptr) {
     hf::TraceRange trace_("block stencils");
     if (step_kernel(ctx)) {
         hf::StepPlan plan = ctx->plan;
         plan.finish = ctx->ring_slots == 0;
+        plan.out = out;
         for (int b = 0; b < ctx->nblocks; ++b) plan.hout[b] = hout ? hout[b] : nullptr;
         CK(hf::launch_step(ctx->dctrl, ctx->dmesh, ctx->dstep, plan, ctx->scheme, ctx->limiter, ctx->stream));
         return HF_OK;
@@ -525,22 +530,33 @@ int enqueue_blocks(hf_ctx* ctx, double* const* hout) {
     return HF_OK;
 }
 
+// Whether a caller is capturing the stream.  A graph holds all of a step's launches, and from the first
+// capture on nothing is taken as known about the device: a replay is not seen here.
+bool capturing(hf_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const bool cap = cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+    ctx->user_graphs = ctx->user_graphs || cap;
+    return cap;
+}
+
 // the accumulators of the next step cleared, where the last step did not end normally before it
 int ensure_clean(hf_ctx* ctx) {
-    if (!ctx->clean) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-    ctx->clean = true;
+    const bool cap = capturing(ctx);
+    if (!ctx->clean || cap) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
+    ctx->clean = !cap;
     return HF_OK;
 }
 
 // A step's kernels from its ghost fill on (ensure_clean before): fill and dt, every block, the end of the
 // step -- or, for one block, one launch for all of it.  (Four launches: its start and its end were
 // kernels of one thread.)
-int enqueue_step(hf_ctx* ctx, bool profiled) {
+int enqueue_step(hf_ctx* ctx, bool profiled, hf::StepOut* out = nullptr) {
+    ctx->steps_known = -1;
     if (profiled) ev_record(ctx, 1, true);
     if (ctx->solo && ctx->ring_slots == 0 && !ctx->strict && !ctx->block_launches) {
         if (profiled) { ev_record(ctx, 1, false); ev_record(ctx, 0, true); }
         CK(hf::launch_solo(ctx->dctrl, ctx->dmesh, ctx->dstep, ctx->blocks[0].nx, ctx->blocks[0].ny, ctx->scheme,
-                           ctx->limiter, ctx->tile, &ctx->tmap[0][0], &ctx->tmap[0][1], ctx->stream));
+                           ctx->limiter, ctx->tile, &ctx->tmap[0][0], &ctx->tmap[0][1], ctx->stream, out));
         if (profiled) ev_record(ctx, 0, false);
         ctx->step_started = ctx->ghost_fresh = false;
         return HF_OK;
@@ -550,7 +566,7 @@ int enqueue_step(hf_ctx* ctx, bool profiled) {
         CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 1, ctx->dstep));
     }
     if (profiled) { ev_record(ctx, 1, false); ev_record(ctx, 0, true); }
-    int r = enqueue_blocks(ctx, nullptr);
+    int r = enqueue_blocks(ctx, nullptr, out);
     if (r != HF_OK) return r;
     if (profiled) ev_record(ctx, 0, false);
     if (ctx->ring_slots > 0) CK(hf::launch_frame_copy(ctx->dctrl, ctx->dmesh, ctx->ring, ctx->stream));
@@ -560,10 +576,33 @@ int enqueue_step(hf_ctx* ctx, bool profiled) {
 }
 
 int set_clamp(hf_ctx* ctx, int clamp) {
+    capturing(ctx);
+    if (ctx->clamp == clamp && !ctx->user_graphs) return HF_OK;
     if (clamp == 0)   // the common case needs no host memory
         CK(cudaMemsetAsync(&ctx->dctrl->clamp, 0, sizeof(int), ctx->stream));
     else
         CK(cudaMemcpyAsync(&ctx->dctrl->clamp, &clamp, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+    ctx->clamp = clamp;
+    return HF_OK;
+}
+
+// Where a step that the host waits for leaves its dt and count, or null: the launch that ends the
+// step writes them (32 steps of 100 x 5 with their upload and download: 966 us, 1320 with a copy of dt behind each).
+hf::StepOut* step_out(hf_ctx* ctx) {
+    if (ctx->ring_slots > 0 || !step_kernel(ctx) || capturing(ctx)) return nullptr;
+    if (!ctx->out && cudaMallocHost(&ctx->out, sizeof(hf::StepOut)) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->out = nullptr;
+    }
+    return ctx->out;
+}
+// the end of such a step: waits for it
+int wait_step(hf_ctx* ctx, const hf::StepOut* out, double* dt) {
+    if (!out && dt) CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (!out) return HF_OK;
+    if (dt) *dt = out->dt;
+    ctx->steps_known = ctx->user_graphs ? -1 : out->step;
     return HF_OK;
 }
 
@@ -725,6 +764,7 @@ void hf_destroy(hf_ctx* ctx) {
     if (ctx->dmesh) cudaFree(ctx->dmesh);
     if (ctx->dctrl) cudaFree(ctx->dctrl);
     if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    if (ctx->out) cudaFreeHost(ctx->out);
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     for (int b = 0; b < HF_MAXB; ++b)
         if (ctx->block_done[b]) cudaEventDestroy(ctx->block_done[b]);
@@ -881,6 +921,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         // a caller that gives dt itself may have skipped hf_time_step: start the step, and give
         // the MUSCL-Hancock predictor's TimeStep call the ghost maxima of the current fields
         ctx->clean = false;
+        ctx->steps_known = -1;
         if (!ctx->step_started) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
         if (ctx->scheme == 1 && !ctx->ghost_fresh)
             CK(hf::launch_ghost_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 0));
@@ -892,7 +933,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
         ctx->next_block = 0;
         ctx->step_started = ctx->ghost_fresh = false;
-        ctx->clean = true;
+        ctx->clean = !capturing(ctx);
     } else {
         ctx->next_block = b + 1;
     }
@@ -954,7 +995,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
         for (int b = 0; b < ctx->nblocks; ++b)
             CK(cudaEventCreateWithFlags(&ctx->block_done[b], cudaEventDisableTiming));
     }
-    const long long step = read_step(ctx);
+    const long long step = ctx->steps_known >= 0 ? ctx->steps_known : read_step(ctx);
     const int p = (int)(step & 1);
     if (blocks_mapped(ctx, in) && blocks_mapped(ctx, (const double* const*)out)) {
         // pinned host memory: the kernels read and write it over the link themselves -- one
@@ -975,13 +1016,14 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
         for (int b = 0; b < ctx->nblocks; ++b)
             CK(hf::launch_ghost_store(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].tx, ctx->blocks[b].ny, ctx->ghost,
                                       p, out[b], ctx->stream));
-        r = enqueue_blocks(ctx, out);
+        hf::StepOut* const end = step_out(ctx);
+        ctx->steps_known = -1;
+        r = enqueue_blocks(ctx, out, end);
         if (r != HF_OK) return r;
         if (ctx->ring_slots > 0 || !step_kernel(ctx)) CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
         ctx->step_started = ctx->ghost_fresh = false;
-        if (dt) CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        return strict_check(ctx);
+        r = wait_step(ctx, end, dt);
+        return r != HF_OK ? r : strict_check(ctx);
     }
     for (int b = 0; b < ctx->nblocks; ++b) {
         const BlockHost& B = ctx->blocks[b];
@@ -1007,6 +1049,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
                              (size_t)B.tx * 8, (size_t)4 * B.ty, cudaMemcpyDeviceToHost, ctx->copy_stream));
     }
     CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
+    ctx->steps_known = -1;
     ctx->step_started = ctx->ghost_fresh = false;
     if (dt) CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1021,14 +1064,11 @@ int hf_step(hf_ctx* ctx, double* dt) {
     int r = set_clamp(ctx, 0);
     if (r == HF_OK) r = ensure_clean(ctx);
     if (r != HF_OK) return r;
-    r = enqueue_step(ctx, ctx->profile);
-    if (r != HF_OK) return r;
-    if (dt) {
-        CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        return strict_check(ctx);
-    }
-    return HF_OK;
+    hf::StepOut* const out = dt ? step_out(ctx) : nullptr;
+    r = enqueue_step(ctx, ctx->profile, out);
+    if (r != HF_OK || !dt) return r;
+    r = wait_step(ctx, out, dt);
+    return r != HF_OK ? r : strict_check(ctx);
 }
 
 int hf_run(hf_ctx* ctx, int64_t n, int clamp_t_end, int use_graph, int64_t* steps_done) {
@@ -1036,6 +1076,7 @@ int hf_run(hf_ctx* ctx, int64_t n, int clamp_t_end, int use_graph, int64_t* step
     if (!ctx || n < 0) return HF_ERR_ARG;
     if (ctx->next_block != 0) return fail(ctx, HF_ERR_STATE, "run in the middle of a step");
     long long s0 = steps_done ? read_step(ctx) : 0;
+    ctx->steps_known = -1;
     int clamp = clamp_t_end ? 1 : 0;
     int r = set_clamp(ctx, clamp);
     if (r == HF_OK) r = ensure_clean(ctx);
@@ -1353,6 +1394,8 @@ int hf_checkpoint_load(hf_ctx* ctx, const void* buf, size_t bytes) {
     C.strict = cur.strict;
     ctx->drained = 0;
     ctx->step_started = ctx->ghost_fresh = ctx->clean = false;
+    ctx->clamp = -1;
+    ctx->steps_known = -1;
     for (int b = 0; b < ctx->nblocks; ++b)
         for (int k = 0; k < 2; ++k) {
             size_t n = (size_t)4 * ctx->blocks[b].ty * ctx->blocks[b].pitch * sizeof(double);

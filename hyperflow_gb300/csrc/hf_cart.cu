@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(256) frame_copy_kernel(const Ctrl* __restrict_
 
 // end of step: t += dt; the MUSCL-Hancock predictor calls advance the counter; record this
 // step's frames; flip parity; clear the next step's accumulators
-__device__ void finish_step(Ctrl* __restrict__ c) {
+__device__ void finish_step(Ctrl* __restrict__ c, StepOut* out = nullptr) {
     if (c->clamp && c->frames) {
         for (int which = 0; which < 2; ++which) {
             if (which == 0 ? !c->snap_pre : !c->snap_post) continue;
@@ -430,6 +430,10 @@ __device__ void finish_step(Ctrl* __restrict__ c) {
     const long long step = c->step + 1;
     c->step = step;
     clear_step(c, (int)(step & 1));
+    if (out) {   // (visible to the host once it has waited for the launch)
+        out->dt = c->dt;
+        out->step = step;
+    }
 }
 
 __global__ void finalize_kernel(Ctrl* c) {
@@ -595,7 +599,7 @@ __global__ void __launch_bounds__(kNT, 2) mh_kernel(Ctrl* __restrict__ c, const 
 
 // the last CTA's thread 0: the next block from b on whose predictor dt was not the reference's, its
 // scalars and records made ready; the step's end when there is none.
-__device__ void settle_step(Ctrl* __restrict__ c, StepState* __restrict__ ss, int b, int finish) {
+__device__ void settle_step(Ctrl* __restrict__ c, StepState* __restrict__ ss, int b, int finish, StepOut* out) {
     const int p = (int)(c->step & 1), nb = c->nblocks;
     for (; b < nb; ++b) {
         const double dtp = cfl_dt_fresh(c, c->calls + b, b, p, p ^ 1);
@@ -619,7 +623,7 @@ __device__ void settle_step(Ctrl* __restrict__ c, StepState* __restrict__ ss, in
         c->dt_pred[b] = ss->sc[b][4];
     }
     c->hllc_errors = c->hllc_errors + herr;
-    if (finish) finish_step(c);
+    if (finish) finish_step(c, out);
 }
 
 // this CTA's work is done; true in thread 0 of the last of the launch's CTAs
@@ -686,7 +690,7 @@ __global__ void __launch_bounds__(kNT, 2) mh_step_kernel(Ctrl* __restrict__ c, c
     int b = 0;
     while (b + 1 < plan.nb && (int)blockIdx.x >= plan.tile_start[b + 1]) ++b;
     mh_plan_tile<LIM>(c, m, ss, plan, b, blockIdx.x - plan.tile_start[b], &bar, 0u);
-    if (last_cta(&ss->tiles)) settle_step(c, ss, 1, plan.finish);
+    if (last_cta(&ss->tiles)) settle_step(c, ss, 1, plan.finish, plan.out);
 }
 
 // the block a launch before this one left to be run again, if any, on the resident CTAs
@@ -705,7 +709,7 @@ __global__ void __launch_bounds__(kNT, 2) mh_rerun_kernel(Ctrl* __restrict__ c, 
         phase ^= 1u;
         __syncthreads();   // the tile's last reads of shared memory come before the next one's load
     }
-    if (last_cta(&ss->tiles)) settle_step(c, ss, b + 1, plan.finish);
+    if (last_cta(&ss->tiles)) settle_step(c, ss, b + 1, plan.finish, plan.out);
 }
 
 // ------------------------------------------------------------------------------------
@@ -763,7 +767,7 @@ __global__ void __launch_bounds__(kNT, 2) godunov_step_kernel(Ctrl* __restrict__
     int b = 0;
     while (b + 1 < plan.nb && (int)blockIdx.x >= plan.tile_start[b + 1]) ++b;
     godunov_tile(c, m, b, blockIdx.x - plan.tile_start[b], plan.tile, &plan.tm[b][c->step & 1], plan.hout[b]);
-    if (last_cta(&ss->tiles) && plan.finish) finish_step(c);
+    if (last_cta(&ss->tiles) && plan.finish) finish_step(c, plan.out);
 }
 
 // ------------------------------------------------------------------------------------
@@ -829,7 +833,7 @@ template <int SCHEME, int LIM>
 __global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                       StepState* __restrict__ ss, const TileShape tile,
                                                       const __grid_constant__ CUtensorMap tm0,
-                                                      const __grid_constant__ CUtensorMap tm1) {
+                                                      const __grid_constant__ CUtensorMap tm1, StepOut* out) {
     constexpr int G = SCHEME == 0 ? 1 : 2;
     extern __shared__ __align__(1024) double smem[];
     __shared__ uint64_t bar;
@@ -896,7 +900,7 @@ __global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, cons
     c->dt = s_v[4];
     if (SCHEME == 1) c->dt_pred[0] = s_v[6];
     c->calls = c->calls + 1;
-    finish_step(c);
+    finish_step(c, out);
 }
 
 // ------------------------------------------------------------------------------------
@@ -980,11 +984,12 @@ cudaError_t prepare_solo(Ctrl* c, const MeshDev* m, StepState* ss, cudaStream_t 
 }
 
 cudaError_t launch_solo(Ctrl* c, const MeshDev* m, StepState* ss, int nx, int ny, int scheme, int limiter,
-                        const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s) {
+                        const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
+                        StepOut* out) {
     const int tiles = ((nx + tile.tx - 1) / tile.tx) * ((ny + tile.ty - 1) / tile.ty);
-    if (scheme == 0) solo_kernel<0, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1);
-    else if (limiter == 0) solo_kernel<1, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1);
-    else solo_kernel<1, 1><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1);
+    if (scheme == 0) solo_kernel<0, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, out);
+    else if (limiter == 0) solo_kernel<1, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, out);
+    else solo_kernel<1, 1><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, out);
     return cudaGetLastError();
 }
 

@@ -129,6 +129,11 @@ cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int b, int tx, int ny,
 // step by its last CTA (hf_cart.cu; MUSCL-Hancock: each block's predictor dt verified against the
 // reference's TimeStep call, a block whose dt differs run again by one of the launches that follow).
 // After launch_fill_cfl with ss.
+// StepOut: what a step leaves for the host, in host memory the GPU maps (null: nothing).
+struct StepOut {
+    double dt;
+    long long step;   // steps completed
+};
 constexpr int kStepMaxBlocks = 4;
 struct StepPlan {
     CUtensorMap tm[kStepMaxBlocks][2];   // per block, per state parity
@@ -138,6 +143,7 @@ struct StepPlan {
     int tile_start[kStepMaxBlocks + 1];  // prefix sums of the blocks' tile counts
     int nb;
     int finish;                          // the last CTA ends the step (else launch_finalize does)
+    StepOut* out;                        // with finish
 };
 // the tile grid of block b (nx x ny interior cells) in the plan (plan.tile set)
 void step_plan_tiles(StepPlan& plan, int b, int nx, int ny);
@@ -148,7 +154,8 @@ cudaError_t launch_step(Ctrl* c, const MeshDev* m, StepState* ss, const StepPlan
 // cell's or a Dirichlet state: no fill before it, the step ended by its last CTA.  prepare_solo once.
 cudaError_t prepare_solo(Ctrl* c, const MeshDev* m, StepState* ss, cudaStream_t s);
 cudaError_t launch_solo(Ctrl* c, const MeshDev* m, StepState* ss, int nx, int ny, int scheme, int limiter,
-                        const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s);
+                        const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
+                        StepOut* out = nullptr);
 
 // the driver's cuTensorMapEncodeTiled, or null where the driver lacks it
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
