@@ -90,7 +90,7 @@ struct hf_ctx {
     size_t coarse_n = 0;
     int next_block = 0;         // next block hf_advance_block expects
     // graphs of one step (index = clamp flag)
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[4] = {};   // of one step, without and with the clamp; of kLoopSteps
     int strict = 0;             // hf_set_strict: a zero-flux face stops the loop
     // piecewise steps: has this step been started (accumulators reset) and are the ghost
     // maxima those of the current fields (a TimeStep call since the last fill or upload)?
@@ -530,6 +530,10 @@ int enqueue_blocks(hf_ctx* ctx, double* const* hout, hf::StepOut* out = nullptr)
     return HF_OK;
 }
 
+// hf_run's graphs: of kLoopSteps steps for a mesh below kLoopCells
+constexpr int kLoopSteps = 32;
+constexpr long long kLoopCells = 1 << 20;
+
 // Whether a caller is capturing the stream.  A graph holds all of a step's launches, and from the first
 // capture on nothing is taken as known about the device: a replay is not seen here.
 bool capturing(hf_ctx* ctx) {
@@ -754,7 +758,7 @@ int hf_create(const char* case_json, size_t len, hf_ctx** out) {
 void hf_destroy(hf_ctx* ctx) {
     if (!ctx) return;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < 4; ++k) {
         if (ctx->graph[k]) cudaGraphExecDestroy(ctx->graph[k]);
         for (auto& pr : ctx->ev[k]) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
     }
@@ -1082,17 +1086,26 @@ int hf_run(hf_ctx* ctx, int64_t n, int clamp_t_end, int use_graph, int64_t* step
     if (r == HF_OK) r = ensure_clean(ctx);
     if (r != HF_OK) return r;
     if (use_graph && !ctx->profile) {
-        if (!ctx->graph[clamp]) {
-            cudaGraph_t g;
-            CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-            r = enqueue_step(ctx, false);
-            cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
-            if (r != HF_OK) return r;
-            if (e != cudaSuccess) return fail(ctx, HF_ERR_CUDA, cudaGetErrorString(e));
-            CK(cudaGraphInstantiate(&ctx->graph[clamp], g, 0));
-            cudaGraphDestroy(g);
+        // kLoopSteps steps a graph where a step is short beside the gap between graphs
+        long long cells = 0;
+        for (const BlockHost& B : ctx->blocks) cells += (long long)B.nx * B.ny;
+        const bool many = cells < kLoopCells && n >= kLoopSteps;
+        for (int64_t left = n; left > 0;) {
+            const int steps = many && left >= kLoopSteps ? kLoopSteps : 1;
+            cudaGraphExec_t& exec = ctx->graph[(steps > 1 ? 2 : 0) + clamp];
+            if (!exec) {
+                cudaGraph_t g;
+                CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+                for (int k = 0; k < steps && r == HF_OK; ++k) r = enqueue_step(ctx, false);
+                cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+                if (r != HF_OK) return r;
+                if (e != cudaSuccess) return fail(ctx, HF_ERR_CUDA, cudaGetErrorString(e));
+                CK(cudaGraphInstantiate(&exec, g, 0));
+                cudaGraphDestroy(g);
+            }
+            CK(cudaGraphLaunch(exec, ctx->stream));
+            left -= steps;
         }
-        for (int64_t k = 0; k < n; ++k) CK(cudaGraphLaunch(ctx->graph[clamp], ctx->stream));
     } else {
         for (int64_t k = 0; k < n; ++k) {
             r = enqueue_step(ctx, ctx->profile);
@@ -1139,7 +1152,7 @@ int hf_set_strict(hf_ctx* ctx, int on) {
     if (!ctx) return HF_ERR_ARG;
     if (ctx->strict != (on ? 1 : 0)) {
         CK(cudaStreamSynchronize(ctx->stream));
-        for (int k = 0; k < 2; ++k)   // the captured steps are the other mode's
+        for (int k = 0; k < 4; ++k)   // the captured steps are the other mode's
             if (ctx->graph[k]) {
                 cudaGraphExecDestroy(ctx->graph[k]);
                 ctx->graph[k] = nullptr;
@@ -1209,7 +1222,7 @@ int hf_frames_enable(hf_ctx* ctx, int ring_slots) {
         return fail(ctx, HF_ERR_ARG, "the case has no simulation.animation {duration, fps}");
     if (ctx->next_block != 0) return fail(ctx, HF_ERR_STATE, "frames_enable in the middle of a step");
     CK(cudaStreamSynchronize(ctx->stream));
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 4; ++k)
         if (ctx->graph[k]) { cudaGraphExecDestroy(ctx->graph[k]); ctx->graph[k] = nullptr; }
     if (ctx->ring.base) { CK(cudaFree(ctx->ring.base)); ctx->ring.base = nullptr; }
     ctx->ring_slots = 0;
@@ -1411,7 +1424,7 @@ int hf_set_block_launches(hf_ctx* ctx, int per_block) {
     if (ctx->next_block != 0) return fail(ctx, HF_ERR_STATE, "launch mode changed in the middle of a step");
     if (ctx->block_launches != (per_block != 0)) {
         CK(cudaStreamSynchronize(ctx->stream));
-        for (int k = 0; k < 2; ++k)   // the captured steps hold the other launch mode
+        for (int k = 0; k < 4; ++k)   // the captured steps hold the other launch mode
             if (ctx->graph[k]) {
                 cudaGraphExecDestroy(ctx->graph[k]);
                 ctx->graph[k] = nullptr;

@@ -302,24 +302,6 @@ cudaError_t launch_batch(int k, int scheme, int limiter, const BatchDev& d, long
                                       : launch_threads<448>(scheme, limiter, d, nsteps, s);
 }
 
-// What a tile costs: microseconds of an SM that has enough of them (`work`), and from start to end of a
-// CTA alone on its SM (`alone`): the warp-items of its phases at their instruction counts, a time per tile,
-// and (model 0) what the rounds of the CTA's 14 warps leave idle.  Fitted to steps of many tiles and of one
-// per SM: MUSCL-Hancock tiles of 32 x 19, 16 x 16 and 32 x 4 cells take 44.5, 22.2 and 13.4 us of an SM (both
-// models within 7 %); with 32 x 14, alone, 55.5, 30.8, 18.0 and 47.5 us.
-struct TileCost {
-    double work, alone;
-};
-TileCost tile_cost(int scheme, int model, int tx, int ty) {
-    constexpr int W = kTileThreads / 32;
-    auto warps = [](int items) { return (items + 31) / 32; };
-    const int faces = warps((tx + 1) * ty) + warps(tx * (ty + 1)), cells = warps(tx * ty);
-    const int first = scheme == 0 ? warps((tx + 2) * (ty + 2)) : warps((tx + 2) * ty) + warps(tx * (ty + 2));
-    const double items = scheme == 0 ? 0.55 * first + 0.95 * faces + 0.75 * cells : 2.0 * first + 2.2 * faces + 0.8 * cells;
-    const double rounds = (scheme == 0 ? 0.35 : 1.0) * ((std::max(first, faces) + W - 1) / W);
-    return {model == 0 ? 1.9 + 0.196 * items + 2.34 * rounds : 2.5 + 0.23 * items, 3.0 + 0.165 * items + 7.2 * rounds};
-}
-
 // The tile shape of each case (sides n) by a model.  A case takes, of the shapes whose whole
 // tile is within a limit, the one whose tiles are the least work (the last row of tiles has as many rows
 // as the case has left); the limit is the one with which the tiles, dealt dearest first to the

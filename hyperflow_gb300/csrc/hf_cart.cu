@@ -12,6 +12,7 @@
 // buffers alternating by step parity.  The stencil CTAs stage one tile plus its halo with a
 // single 3-D TMA load (box = tile + 2*ghost in x and y, all four variables) into shared
 // memory; halos come from the neighbouring tiles' cells in HBM, never from another CTA.
+#include <algorithm>
 #include <cstdio>
 
 #include "hf_cart.h"
@@ -32,8 +33,8 @@ __device__ __forceinline__ bool loop_done(const Ctrl* c) {
 }
 
 // the accumulators of a step whose starting state has parity p, cleared
-__device__ void clear_step(Ctrl* __restrict__ c, int p) {
-    for (int b = 0; b < c->nblocks; ++b) {
+__device__ void clear_step(Ctrl* __restrict__ c, int p, int nblocks) {
+    for (int b = 0; b < nblocks; ++b) {
         c->ghost_s[b][0] = c->ghost_s[b][1] = 0ull;
         c->int_s[p ^ 1][b][0] = c->int_s[p ^ 1][b][1] = 0ull;
         c->step_hllc[b] = 0;
@@ -49,7 +50,7 @@ __global__ void step_begin_kernel(Ctrl* __restrict__ c) {
     const int done = loop_done(c);
     c->done = done;
     c->snap_pre = c->snap_post = 0;
-    if (!done) clear_step(c, (int)(c->step & 1));
+    if (!done) clear_step(c, (int)(c->step & 1), c->nblocks);
 }
 
 // ------------------------------------------------------------------------------------
@@ -414,8 +415,13 @@ __global__ void __launch_bounds__(256) frame_copy_kernel(const Ctrl* __restrict_
 
 // end of step: t += dt; the MUSCL-Hancock predictor calls advance the counter; record this
 // step's frames; flip parity; clear the next step's accumulators
+// (One thread's work at the end of every step: all it reads, first, so that the loads are one latency.)
 __device__ void finish_step(Ctrl* __restrict__ c, StepOut* out = nullptr) {
-    if (c->clamp && c->frames) {
+    const int nb = c->nblocks, scheme = c->scheme;
+    const bool snap = c->clamp && c->frames;
+    const double t = c->t, dt = c->dt;
+    const long long calls = c->calls, step = c->step + 1;
+    if (snap) {
         for (int which = 0; which < 2; ++which) {
             if (which == 0 ? !c->snap_pre : !c->snap_post) continue;
             const long long slot = c->captured % c->ring_slots;
@@ -425,13 +431,12 @@ __device__ void finish_step(Ctrl* __restrict__ c, StepOut* out = nullptr) {
             c->captured = c->captured + 1;
         }
     }
-    c->t = c->t + c->dt;
-    if (c->scheme == 1) c->calls = c->calls + c->nblocks;
-    const long long step = c->step + 1;
+    c->t = t + dt;
+    if (scheme == 1) c->calls = calls + nb;
     c->step = step;
-    clear_step(c, (int)(step & 1));
+    clear_step(c, (int)(step & 1), nb);
     if (out) {   // (visible to the host once it has waited for the launch)
-        out->dt = c->dt;
+        out->dt = dt;
         out->step = step;
     }
 }
@@ -796,36 +801,30 @@ __global__ void prepare_solo_kernel(Ctrl* c, const MeshDev* m, StepState* ss) {
     ss->solo[3] = div_rn(1.0, c->dy[0]);
 }
 
-// the ghost cells in the tile's halo by the fill program, from the interior cells of U
+// The ghost cell at position it = lx + ly * ux of the tile's halo by the fill program, from the interior
+// cells of U, into u; false where there is none
 template <int G>
-__device__ __forceinline__ void tile_ghosts(double* sU, const MeshDev* __restrict__ m, const double* __restrict__ U,
-                                            int tx, int ty, int x0, int y0, int* err) {
-    const BlockDev& B = m->b[0];
-    if (x0 >= G && y0 >= G && x0 + tx + G <= B.nx && y0 + ty + G <= B.ny) return;
-    const int ux = tx + 2 * G, uy = ty + 2 * G;
-    const size_t plane = (size_t)B.ty * B.pitch;
-    for (int it = threadIdx.x; it < ux * uy; it += kNT) {
-        const int ly = it / ux, lx = it - ly * ux, i = x0 + lx, j = y0 + ly;   // in the block, ghosts included
-        if (i >= B.tx || j >= B.ty || (i >= G && i < B.tx - G && j >= G && j < B.ty - G)) continue;
-        const long long k = j < G ? (long long)j * B.tx + i
-                          : j >= B.ty - G ? (long long)(G + j - (B.ty - G)) * B.tx + i
-                          : 2LL * G * B.tx + (long long)(j - G) * (2 * G) + (i < G ? i : i - (B.tx - 2 * G));
-        const FillOp op = m->fill[k];
-        double u[4];
-        if (op.kind == 2) {
+__device__ __forceinline__ bool tile_ghost(const MeshDev* __restrict__ m, const BlockDev& B, const double* __restrict__ U,
+                                           int nx, int ny, int ux, int it, int x0, int y0, double* u, int* err) {
+    const int ly = it / ux, lx = it - ly * ux, i = x0 + lx, j = y0 + ly;   // in the block, ghosts included
+    const int bx = nx + 2 * G, by = ny + 2 * G;
+    if (i >= bx || j >= by || (i >= G && i < bx - G && j >= G && j < by - G)) return false;
+    const long long k = j < G ? (long long)j * bx + i
+                      : j >= by - G ? (long long)(G + j - (by - G)) * bx + i
+                      : 2LL * G * bx + (long long)(j - G) * (2 * G) + (i < G ? i : i - (bx - 2 * G));
+    const FillOp op = m->fill[k];
+    const size_t plane = (size_t)by * B.pitch;
+    if (op.kind == 2) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) u[v] = B.bc_state[op.side][v];
-        } else {
-            if (!hf_in(op.src, (long long)plane, err)) continue;
+        for (int v = 0; v < 4; ++v) u[v] = B.bc_state[op.side][v];
+    } else {
+        if (!hf_in(op.src, (long long)plane, err)) return false;
 #pragma unroll
-            for (int v = 0; v < 4; ++v) u[v] = U[v * plane + op.src];
-        }
-        if (op.neg & 1) u[1] = -1.0 * u[1];
-        if (op.neg & 2) u[2] = -1.0 * u[2];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) sU[v * ux * uy + it] = u[v];
+        for (int v = 0; v < 4; ++v) u[v] = U[v * plane + op.src];
     }
-    __syncthreads();
+    if (op.neg & 1) u[1] = -1.0 * u[1];
+    if (op.neg & 2) u[2] = -1.0 * u[2];
+    return true;
 }
 
 // SCHEME 0 Godunov, 1 MUSCL-Hancock with limiter LIM
@@ -833,13 +832,16 @@ template <int SCHEME, int LIM>
 __global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                       StepState* __restrict__ ss, const TileShape tile,
                                                       const __grid_constant__ CUtensorMap tm0,
-                                                      const __grid_constant__ CUtensorMap tm1, StepOut* out) {
+                                                      const __grid_constant__ CUtensorMap tm1, int nx, int ny,
+                                                      int tiles_x, StepOut* out) {
     constexpr int G = SCHEME == 0 ? 1 : 2;
     extern __shared__ __align__(1024) double smem[];
     __shared__ uint64_t bar;
     // the step's scalars live here, not in registers across the stencil: dx and dy quotients, 0.5 dtp / dx, 0.5 dtp / dy, dt, dt before its clamp, dtp
     __shared__ double s_v[7];
-    if (c->clamp && c->t == c->t_end) {   // the loop stops here
+    const int clamp = c->clamp, p = (int)(c->step & 1);
+    const double t = c->t, t_end = c->t_end;
+    if (clamp && t == t_end) {   // the loop stops here
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             c->done = 1;
             c->snap_pre = c->snap_post = 0;
@@ -847,12 +849,10 @@ __global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, cons
         return;
     }
     const RowShape S{tile};
-    const int tx = tile.tx, ty = tile.ty, usize = 4 * (tx + 2 * G) * (ty + 2 * G);
+    const int tx = tile.tx, ty = tile.ty, ux = tx + 2 * G, uxy = ux * (ty + 2 * G);
     double* sU = smem;
-    double* sW = smem + usize;
+    double* sW = smem + 4 * uxy;
     const BlockDev& B = m->b[0];
-    const int p = (int)(c->step & 1);
-    const int tiles_x = (B.nx + tx - 1) / tx;
     const int x0 = (blockIdx.x % tiles_x) * tx, y0 = (blockIdx.x / tiles_x) * ty;
     // TimeStep (timestep.cpp:29-68), its clamp (simulation.cpp:88-90) and the predictor's call
     // (muscl_hancock.cpp:246-249) while the tile is in flight; a direction's quotients per thread
@@ -860,9 +860,14 @@ __global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, cons
     const int d = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
-        mbar_expect_tx(&bar, usize * 8);
+        mbar_expect_tx(&bar, 4 * uxy * 8);
         tma_load_3d(sU, p ? &tm1 : &tm0, &bar, x0, y0, 0);
     }
+    // a ghost cell per thread of a tile on the block's edge, read while the tile is in flight
+    const bool edge = x0 < G || y0 < G || x0 + tx + G > nx || y0 + ty + G > ny;
+    double u[4];
+    const bool ghost = edge && (int)threadIdx.x < uxy &&
+                       tile_ghost<G>(m, B, B.buf[p], nx, ny, ux, threadIdx.x, x0, y0, u, &c->err);
     if (forms) s_v[d] = div_rn(d ? c->dy[0] : c->dx[0], smax(ss->solo[d], bitsd(c->int_s[p][0][d])));
     __syncthreads();
     if (forms) {
@@ -875,16 +880,25 @@ __global__ void __launch_bounds__(kNT, 2) solo_kernel(Ctrl* __restrict__ c, cons
         }
         if (d == 0) {
             const double dt = ((call + 1 <= 10) ? 0.2 * cfl : cfl) * least;
-            s_v[4] = c->clamp && c->t + dt > c->t_end ? c->t_end - c->t : dt;
+            s_v[4] = clamp && t + dt > t_end ? t_end - t : dt;
             s_v[5] = dt;
         }
     }
     if (wait_tile(&bar, c)) {
-        tile_ghosts<G>(sU, m, B.buf[p], tx, ty, x0, y0, &c->err);
+        if (edge) {
+            if (ghost)
+#pragma unroll
+                for (int v = 0; v < 4; ++v) sU[v * uxy + threadIdx.x] = u[v];
+            for (int it = threadIdx.x + kNT; it < uxy; it += kNT)
+                if (tile_ghost<G>(m, B, B.buf[p], nx, ny, ux, it, x0, y0, u, &c->err))
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) sU[v * uxy + it] = u[v];
+            __syncthreads();
+        }
         const double g = c->gamma, g1 = c->g1;
         const int herr = SCHEME == 0
-            ? go_tile_fluxes<kNT>(S, sU, sW, g, g1, x0, y0, B.nx, B.ny, &c->first_bad, face_key(c->step, 0, 0, 0, 0))
-            : mh_tile_fluxes<kNT, LIM>(S, sU, sW, g, g1, s_v[2], s_v[3], x0, y0, B.nx, B.ny, &c->first_bad,
+            ? go_tile_fluxes<kNT>(S, sU, sW, g, g1, x0, y0, nx, ny, &c->first_bad, face_key(c->step, 0, 0, 0, 0))
+            : mh_tile_fluxes<kNT, LIM>(S, sU, sW, g, g1, s_v[2], s_v[3], x0, y0, nx, ny, &c->first_bad,
                                        face_key(c->step, 0, 0, 0, 0));
         double mx = 0.0, my = 0.0;
         store_tile<kNT, G>(S, sU, sW, B, x0, y0, B.buf[p ^ 1], nullptr, s_v[4], ss->solo[2], ss->solo[3], g, g1,
@@ -918,22 +932,35 @@ bool tile_fits(int scheme, int tx, int ty) {
     return (scheme == 0 ? go_tile_doubles(tx, ty) : mh_tile_doubles(tx, ty)) <= kTileDoubles;
 }
 
-// The rounds of a CTA's warps over the tile's cells and faces, at their instruction counts.
-double tile_time(int scheme, int tx, int ty) {
+// What a tile costs: microseconds of an SM that has enough of them (`work`), and from start to end of a
+// CTA alone on its SM (`alone`): the warp-items of its phases at their instruction counts, a time per tile,
+// and (model 0) what the rounds of the CTA's 14 warps leave idle.  Fitted to steps of many tiles and of one
+// per SM: MUSCL-Hancock tiles of 32 x 19, 16 x 16 and 32 x 4 cells take 44.5, 22.2 and 13.4 us of an SM (both
+// models within 7 %); with 32 x 14, alone, 55.5, 30.8, 18.0 and 47.5 us.
+TileCost tile_cost(int scheme, int model, int tx, int ty) {
     constexpr int W = kNT / 32;
     auto warps = [](int items) { return (items + 31) / 32; };
-    auto rounds = [](int w) { return (w + W - 1) / W; };
-    const int faces = rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))), cells = rounds(warps(tx * ty));
-    return scheme == 0
-        ? 550.0 * rounds(warps((tx + 2) * (ty + 2))) + 950.0 * faces + 750.0 * cells + 400.0
-        : 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) + 2200.0 * faces + 800.0 * cells + 600.0;
+    const int faces = warps((tx + 1) * ty) + warps(tx * (ty + 1)), cells = warps(tx * ty);
+    const int first = scheme == 0 ? warps((tx + 2) * (ty + 2)) : warps((tx + 2) * ty) + warps(tx * (ty + 2));
+    const double items = scheme == 0 ? 0.55 * first + 0.95 * faces + 0.75 * cells : 2.0 * first + 2.2 * faces + 0.8 * cells;
+    const double rounds = (scheme == 0 ? 0.35 : 1.0) * ((std::max(first, faces) + W - 1) / W);
+    return {model == 0 ? 1.9 + 0.196 * items + 2.34 * rounds : 2.5 + 0.23 * items, 3.0 + 0.165 * items + 7.2 * rounds};
 }
 
 // The tile: of the even widths (a TMA copy starts on 16 bytes) and heights that fit a CTA's shared memory,
-// the one whose tiles take the least time (tile_time) times the waves of the 2 x sms resident CTAs.
-// A mesh of many tiles gets the shape with the fewest wasted lanes and halo items; a small one a shape that
-// fills the GPU once: 256^2 in 32 x 19 tiles would leave 44 of 152 SMs without work.
+// the one whose tiles are done first on the 2 x sms resident CTAs.  A mesh of many tiles gets the shape with
+// the fewest wasted lanes and halo items, by the rounds of a CTA's 14 warps over the tile's cells and faces at
+// their instruction counts; a small one, of fewer cells than one round of the largest tiles holds, a shape that
+// fills the GPU once, by tile_cost's model of the work (256^2 in 32 x 19 tiles would leave 44 of 152 SMs
+// without any).  Measured, us a step by the first and by the second: Godunov 256^2 29.1, 26.8, 512^2 69.2, 77.9;
+// MUSCL-Hancock 256^2 55.4, 49.3, 400^2 98.4, 94.6, 777 x 1000 384, 402.
 TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms) {
+    constexpr int W = kNT / 32;
+    auto warps = [](int items) { return (items + 31) / 32; };
+    auto rounds = [](int w) { return (w + W - 1) / W; };
+    long long cells = 0;
+    for (int b = 0; b < nb; ++b) cells += (long long)nx[b] * ny[b];
+    const bool small = cells < 2LL * sms * 32 * 19;
     double best = 0.0;
     int bx = 8, by = 2;
     for (int tx = 8; tx <= 64; tx += 2)
@@ -941,10 +968,20 @@ TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms)
             if (!tile_fits(scheme, tx, ty)) continue;
             long long n = 0;
             for (int b = 0; b < nb; ++b) n += (long long)((nx[b] + tx - 1) / tx) * ((ny[b] + ty - 1) / ty);
+            double shared, alone;   // a tile's time beside another one on its SM, and alone there
+            if (small) {
+                const TileCost t = tile_cost(scheme, 1, tx, ty);
+                shared = std::max(2.0 * t.work, t.alone);
+                alone = t.alone;
+            } else {
+                const int faces = rounds(warps((tx + 1) * ty) + warps(tx * (ty + 1))), own = rounds(warps(tx * ty));
+                shared = scheme == 0
+                    ? 550.0 * rounds(warps((tx + 2) * (ty + 2))) + 950.0 * faces + 750.0 * own + 400.0
+                    : 2000.0 * rounds(warps((tx + 2) * ty) + warps(tx * (ty + 2))) + 2200.0 * faces + 800.0 * own + 600.0;
+                alone = 0.6 * shared;
+            }
             const long long rest = n % (2 * sms);
-            // one CTA alone on its SM runs faster than beside a second one, but not twice as fast
-            const double waves = (double)(n / (2 * sms)) + (rest == 0 ? 0.0 : rest <= sms ? 0.6 : 1.0);
-            const double time = tile_time(scheme, tx, ty) * waves;
+            const double time = (double)(n / (2 * sms)) * shared + (rest == 0 ? 0.0 : rest <= sms ? alone : shared);
             if (best == 0.0 || time < best) {
                 best = time;
                 bx = tx;
@@ -986,10 +1023,10 @@ cudaError_t prepare_solo(Ctrl* c, const MeshDev* m, StepState* ss, cudaStream_t 
 cudaError_t launch_solo(Ctrl* c, const MeshDev* m, StepState* ss, int nx, int ny, int scheme, int limiter,
                         const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
                         StepOut* out) {
-    const int tiles = ((nx + tile.tx - 1) / tile.tx) * ((ny + tile.ty - 1) / tile.ty);
-    if (scheme == 0) solo_kernel<0, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, out);
-    else if (limiter == 0) solo_kernel<1, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, out);
-    else solo_kernel<1, 1><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, out);
+    const int across = (nx + tile.tx - 1) / tile.tx, tiles = across * ((ny + tile.ty - 1) / tile.ty);
+    if (scheme == 0) solo_kernel<0, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, nx, ny, across, out);
+    else if (limiter == 0) solo_kernel<1, 0><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, nx, ny, across, out);
+    else solo_kernel<1, 1><<<tiles, kNT, kTileBytes, s>>>(c, m, ss, tile, *tm0, *tm1, nx, ny, across, out);
     return cudaGetLastError();
 }
 

@@ -66,9 +66,12 @@ TileShape tile_shape(int tx, int ty);
 // A stencil CTA: its threads, and the doubles of shared memory a tile may take (two CTAs per SM).
 constexpr int kTileThreads = 448, kTileDoubles = 13856;
 constexpr size_t kTileBytes = (size_t)kTileDoubles * 8;
-// whether a tile of the scheme fits a CTA, and the time it takes one (arbitrary units)
+// whether a tile of the scheme fits a CTA, and what one costs by a model (hf_cart.cu)
 bool tile_fits(int scheme, int tx, int ty);
-double tile_time(int scheme, int tx, int ty);
+struct TileCost {
+    double work, alone;
+};
+TileCost tile_cost(int scheme, int model, int tx, int ty);
 // the tile for a mesh of nb blocks of nx x ny cells under the scheme, on a GPU of sms SMs
 TileShape choose_tile(int scheme, const int* nx, const int* ny, int nb, int sms);
 
