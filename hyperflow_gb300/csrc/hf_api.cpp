@@ -758,10 +758,10 @@ int hf_create(const char* case_json, size_t len, hf_ctx** out) {
 void hf_destroy(hf_ctx* ctx) {
     if (!ctx) return;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    for (int k = 0; k < 4; ++k) {
-        if (ctx->graph[k]) cudaGraphExecDestroy(ctx->graph[k]);
-        for (auto& pr : ctx->ev[k]) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
-    }
+    for (auto g : ctx->graph)
+        if (g) cudaGraphExecDestroy(g);
+    for (auto& kind : ctx->ev)
+        for (auto& pr : kind) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
     for (double* p : ctx->allocs) cudaFree(p);
     if (ctx->ring.base) cudaFree(ctx->ring.base);
     if (ctx->coarse) cudaFree(ctx->coarse);
