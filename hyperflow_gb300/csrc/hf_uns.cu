@@ -466,7 +466,7 @@ struct hf_uns {
     hf::UnsMesh dm{};
     hf::UnsCtrl* dctrl = nullptr;
     std::vector<void*> allocs;
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
+    cudaGraphExec_t graph[4] = {};      // of one step, without and with the clamp; of kUnsLoopSteps
     bool edge_mode = false;
     int strict = 0;                     // hf_uns_set_strict
     bool has_anim = false;
@@ -1013,6 +1013,9 @@ int finish_create(hf_uns* u, const Json& cfg) {
 // A step's kernels.  prep: a step of the loop, which forms its own dt; else c->dt is given.  With frames
 // on, or in strict mode (whose records change during a step), a kernel before it forms the stop flag, dt
 // and frame points, and one after it ends the step.
+constexpr int kUnsLoopSteps = 32;
+constexpr long long kUnsLoopCells = 1 << 20;
+
 int enqueue_uns_step(hf_uns* u, bool prep) {
     const int grid = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
     const bool frames = u->ring_slots > 0, fused = !frames && !u->strict;
@@ -1099,7 +1102,7 @@ int hf_uns_create_mesh(const char* case_json, size_t len, const char* mesh_text,
 void hf_uns_destroy(hf_uns* u) {
     if (!u) return;
     if (u->stream) cudaStreamSynchronize(u->stream);
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 4; ++k)
         if (u->graph[k]) cudaGraphExecDestroy(u->graph[k]);
     for (void* p : u->allocs) cudaFree(p);
     if (u->ring) cudaFree(u->ring);
@@ -1250,7 +1253,7 @@ int hf_uns_set_strict(hf_uns* u, int on) {
     if (!u || !u->dctrl) return HF_ERR_ARG;
     if (u->strict != (on ? 1 : 0)) {
         UCK(cudaStreamSynchronize(u->stream));
-        for (int k = 0; k < 2; ++k)   // the captured steps are the other mode's
+        for (int k = 0; k < 4; ++k)   // the captured steps are the other mode's
             if (u->graph[k]) { cudaGraphExecDestroy(u->graph[k]); u->graph[k] = nullptr; }
     }
     u->strict = on ? 1 : 0;
@@ -1323,17 +1326,24 @@ int hf_uns_run(hf_uns* u, int64_t n, int clamp_t_end, int use_graph, int64_t* st
     if (!u->clean) hf::uns_clean_kernel<<<1, 1, 0, u->stream>>>(u->dctrl);
     u->clean = true;
     if (use_graph) {
-        if (!u->graph[clamp]) {
-            cudaGraph_t g;
-            UCK(cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeThreadLocal));
-            r = enqueue_uns_step(u, true);
-            cudaError_t e = cudaStreamEndCapture(u->stream, &g);
-            if (r) return r;
-            if (e != cudaSuccess) return ufail(u, HF_ERR_CUDA, cudaGetErrorString(e));
-            UCK(cudaGraphInstantiate(&u->graph[clamp], g, 0));
-            cudaGraphDestroy(g);
+        // kUnsLoopSteps steps a graph where a step is short beside the gap between graphs
+        const bool many = u->ncells < kUnsLoopCells && n >= kUnsLoopSteps;
+        for (int64_t left = n; left > 0;) {
+            const int steps = many && left >= kUnsLoopSteps ? kUnsLoopSteps : 1;
+            cudaGraphExec_t& exec = u->graph[(steps > 1 ? 2 : 0) + clamp];
+            if (!exec) {
+                cudaGraph_t g;
+                UCK(cudaStreamBeginCapture(u->stream, cudaStreamCaptureModeThreadLocal));
+                for (int k = 0; k < steps && r == HF_OK; ++k) r = enqueue_uns_step(u, true);
+                cudaError_t e = cudaStreamEndCapture(u->stream, &g);
+                if (r) return r;
+                if (e != cudaSuccess) return ufail(u, HF_ERR_CUDA, cudaGetErrorString(e));
+                UCK(cudaGraphInstantiate(&exec, g, 0));
+                cudaGraphDestroy(g);
+            }
+            UCK(cudaGraphLaunch(exec, u->stream));
+            left -= steps;
         }
-        for (int64_t k = 0; k < n; ++k) UCK(cudaGraphLaunch(u->graph[clamp], u->stream));
     } else {
         for (int64_t k = 0; k < n; ++k)
             if ((r = enqueue_uns_step(u, true))) return r;
@@ -1350,7 +1360,7 @@ int hf_uns_frames_enable(hf_uns* u, int ring_slots) {
     if (ring_slots > 0 && !u->has_anim)
         return ufail(u, HF_ERR_ARG, "the case has no simulation.animation {duration, fps}");
     UCK(cudaStreamSynchronize(u->stream));
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 4; ++k)
         if (u->graph[k]) { cudaGraphExecDestroy(u->graph[k]); u->graph[k] = nullptr; }
     if (u->ring) { UCK(cudaFree(u->ring)); u->ring = nullptr; }
     u->ring_slots = 0;
@@ -1537,7 +1547,7 @@ int hf_uns_set_edge_mode(hf_uns* u, int edge_based) {
     if (!u || !u->dctrl) return HF_ERR_ARG;
     UCK(cudaStreamSynchronize(u->stream));
     u->edge_mode = edge_based != 0;
-    for (int k = 0; k < 2; ++k)
+    for (int k = 0; k < 4; ++k)
         if (u->graph[k]) { cudaGraphExecDestroy(u->graph[k]); u->graph[k] = nullptr; }
     return HF_OK;
 }

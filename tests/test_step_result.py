@@ -81,3 +81,27 @@ def test_a_captured_step_holds_all_of_itself():
     np.testing.assert_array_equal(out[1], ref[1])
     np.testing.assert_array_equal(a.state(0), b.state(0))
     assert a.time() == b.time()
+
+
+@pytest.mark.parametrize("edge", [False, True])
+def test_unstructured_loops_of_many_steps_a_graph(edge):
+    """Runs past a graph's 32 steps, clamped ones that stop inside one, and mode changes between them."""
+    from hyperflow_gb300 import UnsSolver, meshgen
+    from test_uns import load
+    g = load("tri_hole_3k")
+    case, text = g["case"], meshgen.hmsh_text(g["verts"], g["codes"])
+    first = UnsSolver(case, mesh_text=text)
+    first.run(70)
+    case["simulation"]["t_end"] = 1.6 * first.time()[0]
+    a, b = UnsSolver(case, mesh_text=text), UnsSolver(case, mesh_text=text)
+    for s in (a, b):
+        s.set_edge_mode(edge)
+    a.run(70)
+    b.run(70, graph=False)
+    np.testing.assert_array_equal(a.state(), b.state())
+    for s in (a, b):
+        s.set_edge_mode(not edge)
+    assert a.run(1000, clamp_t_end=True) == b.run(1000, clamp_t_end=True, graph=False) > 0
+    assert a.time() == b.time() and a.time()[0] == case["simulation"]["t_end"]
+    np.testing.assert_array_equal(a.state(), b.state())
+    assert a.run(40, clamp_t_end=True) == 0
