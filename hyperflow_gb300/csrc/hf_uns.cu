@@ -73,7 +73,7 @@ struct UnsMesh {
     const int* __restrict__ edge_cell;      // per unique edge: the owning cell
     const int* __restrict__ edge_nbr;       // per unique edge: the other cell
     const double* __restrict__ edge_geo;    // [5][nedges]: the owning pair's geo, edge by edge
-    double* edge_flux;                      // [4][nedges]: length x rotated-back HLLC flux
+    double2* edge_flux;                     // [nedges][2]: length x rotated-back HLLC flux, an edge's in one sector
     int nedges;
     // cells are held in a locality order (Morton order of their vertex centroids); orig[i] is
     // the mesh file's index of device cell i, used in the failure records' keys
@@ -206,6 +206,13 @@ __device__ __forceinline__ int pair_flux(const UnsMesh& m, const double* __restr
     return geo_flux(m.geo + e, (size_t)m.npairs, g, g1, cv, nb, f);
 }
 
+// the boundary pairs of edge mode, out of line
+static __device__ __noinline__ int boundary_flux(const UnsMesh& m, const double* U, size_t N, double g, double g1, int e,
+                                                 double c0, double c1, double c2, double c3, double* f, int* err) {
+    const double cv[4] = {c0, c1, c2, c3};
+    return pair_flux<true>(m, U, N, g, g1, e, cv, f, err);
+}
+
 // pair_flux of an interior edge's owning pair from the per-edge arrays (the same arithmetic):
 // the edge kernel reads its geometry once, contiguously, instead of through the pair lists
 __device__ __forceinline__ int edge_flux(const UnsMesh& m, const double* __restrict__ U, size_t N, double g,
@@ -248,8 +255,8 @@ __global__ void __launch_bounds__(kUnsNT, 6) uns_edge_flux_kernel(UnsCtrl* __res
             ++herr;
             atomicMin(&c->first_bad, uns_key(c->step, m.orig[i]));
         }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) m.edge_flux[(size_t)v * m.nedges + e] = f[v];
+        m.edge_flux[2 * (size_t)e] = make_double2(f[0], f[1]);
+        m.edge_flux[2 * (size_t)e + 1] = make_double2(f[2], f[3]);
     }
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
@@ -369,11 +376,14 @@ __global__ void uns_finalize_kernel(UnsCtrl* c) {
 // 40 FP64 instructions of 83, and no out-of-line calls.  Measured (Mcell-updates/s, 1M triangles): 1232 ->
 // 2550 with a flux per pair, 1992 -> 3450 with a flux per edge (of these two the long division alone 1650
 // and 2500).
-// MINB: CTAs per SM the registers are budgeted for -- six in edge mode (the per-cell work is a
-// gather of precomputed edge fluxes, and more warps hide its latency), four in the per-pair mode
-// (its HLLC needs the registers: 128 per thread)
+// MINB: CTAs per SM the registers are budgeted for: four in the per-pair mode (its HLLC needs the 128
+// registers per thread).  Edge mode's per-cell work is a gather of precomputed edge fluxes, bound by its
+// chains of loads: a large mesh has warps to hide them (eight CTAs, whose spills cost less), a small one does
+// not (four, nothing spilled).  us a step, both kernels, with four, six and eight: 2,000 triangles 29.7, 30.6,
+// 31.5; 120,000 53.4, 56.0, 56.4; 400,000 132, 124, 120; 1,000,000 297, 273, 261 (280 with the loads pair by
+// pair, from four planes, at six).
 template <int MINB, bool EDGES>
-__global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int mode) {
+__global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restrict__ c, const __grid_constant__ UnsMesh m, int mode) {
     if (mode & kStepForms ? uns_loop_done(c) : c->done != 0) {
         if ((mode & kStepForms) && blockIdx.x == 0 && threadIdx.x == 0) c->done = 1;
         return;
@@ -389,23 +399,57 @@ __global__ void __launch_bounds__(kUnsNT, MINB) uns_step_kernel(UnsCtrl* __restr
         double cv[4] = {U[i], U[N + i], U[2 * N + i], U[3 * N + i]};
         double acc[4] = {0.0, 0.0, 0.0, 0.0};
         const int e0 = m.pair_start[i], e1 = m.pair_start[i + 1];
-        for (int e = e0; e < e1; ++e) {
-            double f[4];
-            const int ed = EDGES && hf_in(e, m.npairs, &c->err) ? m.pair_edge[e] : -1;
-            if (ed >= 0 && hf_in(ed, m.nedges, &c->err)) {   // edge-based mode: the owner's flux, negated on the other side
-                // (a sign flip, not a multiplication by -1.0: the same value, off the FP64 pipe)
-                const bool neg = m.pair_sign[e] < 0;
+        if (EDGES) {
+            // three pairs at a time (a triangle's): their edges, then their owners' fluxes, then the sums in order
+            for (int e = e0; e < e1; e += 3) {
+                int ed[3];
+                bool neg[3];
+                double2 fa[3], fb[3];
 #pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                    const double x = m.edge_flux[(size_t)v * m.nedges + ed];
-                    f[v] = neg ? -x : x;
+                for (int k = 0; k < 3; ++k) {
+                    const bool in = e + k < e1 && hf_in(e + k, m.npairs, &c->err);
+                    ed[k] = in ? m.pair_edge[e + k] : -1;
+                    neg[k] = in && m.pair_sign[e + k] < 0;
                 }
-            } else if (pair_flux<EDGES>(m, U, N, g, g1, e, cv, f, &c->err)) {
-                ++herr;
-                atomicMin(&c->first_bad, uns_key(c->step, m.orig[i]));
-            }
 #pragma unroll
-            for (int v = 0; v < 4; ++v) acc[v] = acc[v] + f[v];
+                for (int k = 0; k < 3; ++k) {
+                    if (ed[k] >= 0 && !hf_in(ed[k], m.nedges, &c->err)) ed[k] = -1;
+                    fa[k] = fb[k] = make_double2(0.0, 0.0);
+                    if (ed[k] >= 0) {
+                        fa[k] = m.edge_flux[2 * (size_t)ed[k]];
+                        fb[k] = m.edge_flux[2 * (size_t)ed[k] + 1];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    if (e + k >= e1) break;
+                    double f[4] = {fa[k].x, fa[k].y, fb[k].x, fb[k].y};
+                    if (ed[k] < 0) {
+                        double x[4];
+                        if (boundary_flux(m, U, N, g, g1, e + k, cv[0], cv[1], cv[2], cv[3], x, &c->err)) {
+                            ++herr;
+                            atomicMin(&c->first_bad, uns_key(c->step, m.orig[i]));
+                        }
+#pragma unroll
+                        for (int v = 0; v < 4; ++v) f[v] = x[v];
+                    } else if (neg[k]) {   // the owner's flux, negated on the other side (a sign flip: off the FP64 pipe)
+#pragma unroll
+                        for (int v = 0; v < 4; ++v) f[v] = -f[v];
+                    }
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) acc[v] = acc[v] + f[v];
+                }
+            }
+        } else {
+            for (int e = e0; e < e1; ++e) {
+                double f[4];
+                if (pair_flux<false>(m, U, N, g, g1, e, cv, f, &c->err)) {
+                    ++herr;
+                    atomicMin(&c->first_bad, uns_key(c->step, m.orig[i]));
+                }
+#pragma unroll
+                for (int v = 0; v < 4; ++v) acc[v] = acc[v] + f[v];
+            }
         }
         double un[4], term;
         bool pos = true;   // the fast path's states are
@@ -976,7 +1020,7 @@ int finish_create(hf_uns* u, const Json& cfg) {
         u->dm.edge_cell = d_ec;
         u->dm.edge_nbr = d_en;
         u->dm.edge_geo = d_eg;
-        u->dm.edge_flux = d_ef;
+        u->dm.edge_flux = reinterpret_cast<double2*>(d_ef);
         u->dm.nedges = (int)ne;
     }
     u->dm.orig = org;
@@ -1013,6 +1057,8 @@ int finish_create(hf_uns* u, const Json& cfg) {
 // A step's kernels.  prep: a step of the loop, which forms its own dt; else c->dt is given.  With frames
 // on, or in strict mode (whose records change during a step), a kernel before it forms the stop flag, dt
 // and frame points, and one after it ends the step.
+// edge mode's gather: up to two rounds of four CTAs per SM it runs with their 128 registers, beyond at eight
+constexpr int kUnsFewCtas = 2 * 4 * 152;
 constexpr int kUnsLoopSteps = 32;
 constexpr long long kUnsLoopCells = 1 << 20;
 
@@ -1027,7 +1073,8 @@ int enqueue_uns_step(hf_uns* u, bool prep) {
         m.pair_sign = u->d_pair_sign;
         const int eg = (m.nedges + hf::kUnsNT - 1) / hf::kUnsNT;
         hf::uns_edge_flux_kernel<<<eg < 1 ? 1 : eg, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
-        hf::uns_step_kernel<6, true><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
+        if (grid <= kUnsFewCtas) hf::uns_step_kernel<4, true><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
+        else hf::uns_step_kernel<8, true><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
     } else {
         hf::uns_step_kernel<4, false><<<grid, hf::kUnsNT, 0, u->stream>>>(u->dctrl, m, mode);
     }
