@@ -1,12 +1,15 @@
 // Cartesian time-step kernels for sm_103a.
 //
-//   bc_fill       ghost/halo fill, Mesh::apply_bcs (src/fvm_2d_cart/mesh/mesh/mesh.cpp:31-39)
-//   ghost_cfl     TimeStep over ghost cells + the step dt (timestep.cpp:29-68)
-//   interior_cfl  TimeStep terms over interior cells (after a state upload)
+//   fill_cfl      ghost/halo fill, Mesh::apply_bcs (src/fvm_2d_cart/mesh/mesh/mesh.cpp:31-39), TimeStep over
+//                 the ghost cells and the step dt (timestep.cpp:29-68)
+//   upload,       a block's state from and into host memory the GPU maps, the upload with the TimeStep
+//   download      terms of its interior; interior_cfl: those terms after another upload
 //   godunov       fused x/y HLLC + update, GodunovScheme (godunov.cpp:27-118) + ForwardEuler
-//   muscl_hancock fused slopes/limiter/predictor/HLLC/update, MUSCLHancockScheme
+//   mh            fused slopes/limiter/predictor/HLLC/update, MUSCLHancockScheme
 //                 (muscl_hancock.cpp:41-376) + ForwardEuler, with the next step's TimeStep
 //                 terms reduced in the epilogue
+//   *_step        the same for every block of a step, a CTA per tile, the last of which ends the step
+//   solo          a whole step of a small single block, its ghosts included
 //
 // Layout: per block, SoA FP64 [var][total_y][pitch] (x contiguous), ghosts included, two
 // buffers alternating by step parity.  The stencil CTAs stage one tile plus its halo with a
@@ -526,7 +529,7 @@ __device__ __forceinline__ void store_tile(const RowShape& S, const double* sU, 
 // ------------------------------------------------------------------------------------
 // Two 448-thread CTAs per SM (72 registers; 110.9 KB of shared memory each, which a 32 x 19 tile fills):
 // the tile's 42 warp-items of predictor cells are three rounds of the 14 warps, its 40 of faces too.
-// Measured at 2048^2 (Mcell-updates/s): 1973; 512 threads and 64 registers 1962, 320 threads and 32 x 18
+// Measured at 2048^2 (Mcell-updates/s, in a persistent kernel): 1973; 512 threads and 64 registers 1962, 320 threads and 32 x 18
 // tiles 1933, 256 threads and 32 x 14 1880, three CTAs of 256 threads and 32 x 12 tiles 1751.
 constexpr int kNT = kTileThreads;
 
@@ -783,8 +786,9 @@ __global__ void __launch_bounds__(kNT, 2) godunov_step_kernel(Ctrl* __restrict__
 // interior's or of those states, so dt is known before any ghost is filled: every CTA forms it from the
 // maxima the last step left, writes the ghosts of its own tile's halo in shared memory, and stores them with
 // its update.  The fill, a chain of dependent loads, quotients and a reduction over few cells, took 9 to
-// 11 us a step beside 20 to 25 us for the stencil of a small mesh (100 x 5, 256^2).  Steps with frames,
-// strict mode (whose records change during a step) or one launch per block keep the fill.
+// 11 us a step beside 20 to 25 us for the stencil of a small mesh (100 x 5, 256^2).  A step in the loop, before
+// and now: MUSCL-Hancock 100 x 5 72 and 17.2 us, Godunov 256^2 68 and 23.7.  Steps with frames, strict mode
+// (whose records change during a step) or one launch per block keep the fill.
 __global__ void prepare_solo_kernel(Ctrl* c, const MeshDev* m, StepState* ss) {
     double mx = 0.0, my = 0.0;
     for (int side = 0; side < 4; ++side) {

@@ -238,8 +238,8 @@ static __host__ __device__ __noinline__ double div_slow(double a, double b) {
     return hw_div(a, b);
 }
 
-// Kept out of line: the stencils call it about 55 times per cell, and one shared copy keeps the
-// kernels inside the instruction cache (measured faster than inlining every call).
+// Kept out of line: one shared copy keeps the general functions inside the instruction cache (measured faster
+// than inlining every call, when the stencils made about 55 of them per cell).
 static __host__ __device__ __noinline__ double div_rn(double a, double b) {
     const uint64_t A = f64_bits(a), B = f64_bits(b);
     if (!div_fast(A, B)) return div_slow(a, b);

@@ -61,7 +61,8 @@ int hf_lc_cfl_dt(hf_lc* L, double* dt);
  * counts cells whose faces' corrections were rejected -- given, the call waits for the step and
  * reports a device error; null, the step is only enqueued on the solver's stream */
 int hf_lc_step(hf_lc* L, double dt, int use_mlp, int64_t* rejected_cells);
-/* steps with the CFL dt until t_end (dt clamped to reach it) */
+/* steps with the CFL dt until t_end (dt clamped to reach it); the dt of each step is formed on the
+ * device, the host waits once per batch of steps */
 int hf_lc_run_to(hf_lc* L, double t_end, int use_mlp, int64_t* steps, int64_t* rejected_cells);
 
 /* one Adam iteration on the pair (U0 -> T over dt) with variable weights w[4]; loss written.
