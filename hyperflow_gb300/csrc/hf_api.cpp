@@ -593,7 +593,8 @@ int set_clamp(hf_ctx* ctx, int clamp) {
 // Where a step that the host waits for leaves its dt and count, or null: the launch that ends the
 // step writes them (32 steps of 100 x 5 with their upload and download: 966 us, 1320 with a copy of dt behind each).
 hf::StepOut* step_out(hf_ctx* ctx) {
-    if (ctx->ring_slots > 0 || !step_kernel(ctx) || capturing(ctx)) return nullptr;
+    // (a strict step that stops for a failure recorded before it writes nothing)
+    if (ctx->ring_slots > 0 || ctx->strict || !step_kernel(ctx) || capturing(ctx)) return nullptr;
     if (!ctx->out && cudaMallocHost(&ctx->out, sizeof(hf::StepOut)) != cudaSuccess) {
         cudaGetLastError();
         ctx->out = nullptr;

@@ -669,7 +669,8 @@ int hf_batch_create(const char* manifest, size_t len, hf_batch** out) {
         BCK(cudaMemcpy2D(b->U[0] + I.off, (size_t)I.pitch * 8, init[i].data(), (size_t)I.n * 8, (size_t)I.n * 8,
                          (size_t)4 * I.n, cudaMemcpyHostToDevice));
     }
-    return refresh_cfl(b, 0, 0, (int)n);
+    const int r = ensure_tiles(b, 0);   // (a first run may be captured: no allocation then)
+    return r ? r : refresh_cfl(b, 0, 0, (int)n);
 }
 
 void hf_batch_destroy(hf_batch* b) {

@@ -105,3 +105,50 @@ def test_unstructured_loops_of_many_steps_a_graph(edge):
     assert a.time() == b.time() and a.time()[0] == case["simulation"]["t_end"]
     np.testing.assert_array_equal(a.state(), b.state())
     assert a.run(40, clamp_t_end=True) == 0
+
+
+def test_a_strict_stop_leaves_the_count_to_the_device():
+    """In strict mode a step that does not run, for a failure recorded before it, leaves no result; the
+    host-buffer step after it still finds the right buffers."""
+    from hyperflow_gb300 import CartSolver, HyperFlowError, cases
+    case = cases.shock_bubble_case(128, cfl=0.8)
+    a, b = CartSolver(case), CartSolver(case)
+    for s in (a, b):
+        s.step()
+        s.set_strict(True)
+        with pytest.raises(HyperFlowError, match="step 82"):
+            s.run(200)
+        with pytest.raises(HyperFlowError, match="step 82"):
+            s.step()
+        s.set_strict(False)
+        s.clear_error_cell()
+        b.set_block_launches(True)
+    assert a.time() == b.time()
+    got, ref = _host_step(a, 1), _host_step(b, 1)
+    assert got[0] == ref[0]
+    np.testing.assert_array_equal(got[1], ref[1])
+
+
+@pytest.mark.parametrize("scheme", ["Godunov", "MUSCLHancock"])
+def test_a_batch_run_may_be_captured(scheme):
+    import torch
+    from hyperflow_gb300 import BatchSolver, cases
+    spec = {"cases": [cases.quadrant_case(n, scheme=scheme, limiter="MinBee" if scheme != "Godunov" else None,
+                                          cfl=cases.CFL_2D) for n in (20, 33)]}
+    a, b = BatchSolver(spec), BatchSolver(spec)
+    if scheme != "Godunov":      # (its tensor maps are made by the first run)
+        a.run(1, graph=False), b.run(1, graph=False)
+    a.sync()
+    stream = torch.cuda.ExternalStream(a.stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        g.capture_begin(capture_error_mode="thread_local")
+        a.run(3, graph=False)
+        g.capture_end()
+        g.replay()
+        g.replay()
+    a.sync()
+    b.run(6)
+    b.sync()
+    for i in range(2):
+        np.testing.assert_array_equal(a.state(i), b.state(i))
