@@ -192,6 +192,14 @@ __device__ __forceinline__ int ghost_block(const MeshDev* __restrict__ m, long l
 // taken here: nothing it depends on changes before the last CTA forms the dt.
 __global__ void __launch_bounds__(kRedThreads) fill_cfl_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                                int form_dt, StepState* __restrict__ ss) {
+    // (a chain of loads: those that need no other's result first)
+    const long long total = m->total_ghost;
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    FillOp op{};
+    if (k < total) op = m->fill[k];
+    const int p = (int)(c->step & 1);
+    const double g = c->gamma, g1 = c->g1;
+    const int gh = m->ghost;
     if (ss ? loop_done(c) : c->done != 0) {
         if (ss && blockIdx.x == 0 && threadIdx.x == 0) {
             c->done = 1;
@@ -199,11 +207,6 @@ __global__ void __launch_bounds__(kRedThreads) fill_cfl_kernel(Ctrl* __restrict_
         }
         return;
     }
-    const int p = (int)(c->step & 1);
-    const double g = c->gamma, g1 = c->g1;
-    const int gh = m->ghost;
-    const long long total = m->total_ghost;
-    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long k0 = (long long)blockIdx.x * blockDim.x;
     const long long k1 = (k0 + blockDim.x < total ? k0 + blockDim.x : total) - 1;
     int b = -1;
@@ -213,7 +216,6 @@ __global__ void __launch_bounds__(kRedThreads) fill_cfl_kernel(Ctrl* __restrict_
         const BlockDev& B = m->b[b];
         int i, j;
         ghost_cell_ij(B, gh, k - B.ghost_off, i, j);
-        const FillOp op = m->fill[k];
         double u[4];
         if (op.kind == 2) {
             const BlockDev& S = m->b[op.block];
