@@ -824,7 +824,7 @@ int hf_set_state(hf_ctx* ctx, int b, const double* cons, int layout) {
         // pinned memory: one kernel reads it over the link into both buffers, with the TimeStep terms
         const int p = (int)(read_step(ctx) & 1);
         CK(cudaMemsetAsync(&ctx->dctrl->int_s[p][b][0], 0, 2 * sizeof(unsigned long long), ctx->stream));
-        CK(hf::launch_upload(ctx->dctrl, ctx->dmesh, b, B.tx, B.ty, p, cons, ctx->stream));
+        CK(hf::launch_upload(ctx->dctrl, ctx->dmesh, b, 1, &B.tx, &B.ty, p, {{const_cast<double*>(cons)}}, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         ctx->ghost_fresh = false;
         return HF_OK;
@@ -1010,17 +1010,20 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
         // every block's interior TimeStep maxima (int_s[p][b], contiguous over b) start at 0
         CK(cudaMemsetAsync(&ctx->dctrl->int_s[p][0][0], 0, (size_t)ctx->nblocks * 2 * sizeof(unsigned long long),
                            ctx->stream));
+        int tx[HF_MAXB], ty[HF_MAXB];
+        hf::HostBlocks hin{}, hout{};
         for (int b = 0; b < ctx->nblocks; ++b) {
-            const BlockHost& B = ctx->blocks[b];
-            CK(hf::launch_upload(ctx->dctrl, ctx->dmesh, b, B.tx, B.ty, p, in[b], ctx->stream));
+            tx[b] = ctx->blocks[b].tx;
+            ty[b] = ctx->blocks[b].ty;
+            hin.p[b] = const_cast<double*>(in[b]);
+            hout.p[b] = out[b];
         }
+        CK(hf::launch_upload(ctx->dctrl, ctx->dmesh, 0, ctx->nblocks, tx, ty, p, hin, ctx->stream));
         int r = set_clamp(ctx, 0);
         if (r == HF_OK) r = ensure_clean(ctx);
         if (r != HF_OK) return r;
         CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 1, ctx->dstep));
-        for (int b = 0; b < ctx->nblocks; ++b)
-            CK(hf::launch_ghost_store(ctx->dctrl, ctx->dmesh, b, ctx->blocks[b].tx, ctx->blocks[b].ny, ctx->ghost,
-                                      p, out[b], ctx->stream));
+        CK(hf::launch_ghost_store(ctx->dctrl, ctx->dmesh, ctx->nblocks, tx, ty, ctx->ghost, p, hout, ctx->stream));
         hf::StepOut* const end = step_out(ctx);
         ctx->steps_known = -1;
         r = enqueue_blocks(ctx, out, end);

@@ -297,8 +297,11 @@ __global__ void __launch_bounds__(kRedThreads) interior_cfl_kernel(Ctrl* __restr
 // link.  A warp takes a row's cells 32 at a time, and the next row when it has them all.
 // Bound by the link: a 4096^2 pass's upload and download (541 MB each) take about 5 ms together, where
 // the copy engine's row-by-row copies out of and into the padded rows took about 32.
+// (a row of CTAs per block from b0 on: a launch per block left the link idle between them)
 __global__ void __launch_bounds__(kRedThreads) upload_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                                             int b, int parity, const double* __restrict__ hin) {
+                                                             int b0, int parity, const HostBlocks h) {
+    const int b = b0 + blockIdx.y;
+    const double* __restrict__ hin = h.p[blockIdx.y];
     const BlockDev& B = m->b[b];
     const int g = m->ghost;
     const size_t plane = (size_t)B.ty * B.pitch, hplane = (size_t)B.ty * B.tx;
@@ -357,8 +360,9 @@ __global__ void __launch_bounds__(kRedThreads) download_kernel(Ctrl* __restrict_
 // The ghost cells filled this step into host memory the GPU maps: with the stencil's own host
 // stores of the updated cells, the whole block downloaded.
 __global__ void __launch_bounds__(256) ghost_store_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
-                                                          int b, int parity, double* __restrict__ hout) {
-    const BlockDev& B = m->b[b];
+                                                          int parity, const HostBlocks h) {
+    const BlockDev& B = m->b[blockIdx.y];
+    double* __restrict__ hout = h.p[blockIdx.y];
     const int g = m->ghost;
     const size_t plane = (size_t)B.ty * B.pitch, hplane = (size_t)B.ty * B.tx;
     const double* __restrict__ U = B.buf[parity];    // filled this step; the stencil copies them later
@@ -1144,9 +1148,11 @@ static int link_grid(int tx, int ty) {
     return (int)(want < 1 ? 1 : (want > 8 * 152 ? 8 * 152 : want));
 }
 
-cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, const double* hin,
-                          cudaStream_t s) {
-    upload_kernel<<<link_grid(tx, ty), kRedThreads, 0, s>>>(c, m, b, parity, hin);
+cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b0, int nb, const int* tx, const int* ty, int parity,
+                          const HostBlocks& h, cudaStream_t s) {
+    int grid = 1;
+    for (int k = 0; k < nb; ++k) grid = std::max(grid, link_grid(tx[k], ty[k]));
+    upload_kernel<<<dim3((unsigned)grid, (unsigned)nb), kRedThreads, 0, s>>>(c, m, b0, parity, h);
     return cudaGetLastError();
 }
 
@@ -1155,11 +1161,11 @@ cudaError_t launch_download(Ctrl* c, const MeshDev* m, int b, int tx, int ty, in
     return cudaGetLastError();
 }
 
-cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int b, int tx, int ny, int ghost, int parity,
-                               double* hout, cudaStream_t s) {
-    long long n = 2LL * ghost * (tx + ny);
-    int grid = (int)((n + 255) / 256);
-    ghost_store_kernel<<<grid < 1 ? 1 : grid, 256, 0, s>>>(c, m, b, parity, hout);
+cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int nb, const int* tx, const int* ty, int ghost, int parity,
+                               const HostBlocks& h, cudaStream_t s) {
+    long long n = 1;
+    for (int k = 0; k < nb; ++k) n = std::max(n, 2LL * ghost * (tx[k] + ty[k]));
+    ghost_store_kernel<<<dim3((unsigned)((n + 255) / 256), (unsigned)nb), 256, 0, s>>>(c, m, parity, h);
     return cudaGetLastError();
 }
 

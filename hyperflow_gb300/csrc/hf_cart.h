@@ -119,15 +119,18 @@ cudaError_t launch_frame_copy(Ctrl* c, const MeshDev* m, const FrameRing& ring, 
 cudaError_t launch_stencil(Ctrl* c, const MeshDev* m, int b, int nx, int ny, int scheme, int limiter,
                            const TileShape& tile, const CUtensorMap* tm0, const CUtensorMap* tm1, cudaStream_t s,
                            double* hout = nullptr);
-// host-buffer steps over mapped host memory: block b's state [4][total_y][total_x] into both
-// buffers with the interior TimeStep terms (int_s[parity][b] zeroed before), and, after the
-// ghost fill, the updated buffer's ghost cells back out
-cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, const double* hin,
-                          cudaStream_t s);
+// host-buffer steps over mapped host memory: the states [4][total_y][total_x] of nb blocks from b0 on
+// (total sizes tx, ty) into both buffers with the interior TimeStep terms (int_s[parity][b] zeroed
+// before), and, after the ghost fill, the ghost cells of blocks 0 to nb - 1 back out
+struct HostBlocks {
+    double* p[HF_MAXB];
+};
+cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b0, int nb, const int* tx, const int* ty, int parity,
+                          const HostBlocks& h, cudaStream_t s);
 // block b's whole state of one parity into mapped host memory [4][total_y][total_x]
 cudaError_t launch_download(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, double* hout, cudaStream_t s);
-cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int b, int tx, int ny, int ghost, int parity,
-                               double* hout, cudaStream_t s);
+cudaError_t launch_ghost_store(Ctrl* c, const MeshDev* m, int nb, const int* tx, const int* ty, int ghost, int parity,
+                               const HostBlocks& h, cudaStream_t s);
 // Every block of a step in one launch, for meshes of at most kStepMaxBlocks blocks, and the end of the
 // step by its last CTA (hf_cart.cu; MUSCL-Hancock: each block's predictor dt verified against the
 // reference's TimeStep call, a block whose dt differs run again by one of the launches that follow).
