@@ -75,7 +75,7 @@ struct hf_ctx {
     int clamp = -1;             // the device's clamp switch, -1 when not known
     hf::StepOut* out = nullptr; // a step's dt and count, in host memory the GPU maps
     long long steps_known = -1; // steps completed, -1 when the device may have moved on
-    bool clean = false;         // the step's accumulators are cleared (by the end of the last step)
+    bool clean = false;         // the end of the last step cleared the next one's accumulators (ensure_clean)
     bool block_launches = false;   // hf_set_block_launches: one stencil launch per block instead
     std::vector<double*> allocs;
     double* pinned = nullptr;   // staging for layout conversion
@@ -543,11 +543,14 @@ bool capturing(hf_ctx* ctx) {
     return cap;
 }
 
-// the accumulators of the next step cleared, where the last step did not end normally before it
+// The accumulators of the next step cleared, unless the end of the step before it did so: known only when
+// that step was enqueued by a call (which then sets `clean` again) and no graph of a caller's may have run
+// since -- the replay of a ghost fill or a TimeStep call leaves its maxima behind.
 int ensure_clean(hf_ctx* ctx) {
-    const bool cap = capturing(ctx);
-    if (!ctx->clean || cap) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-    ctx->clean = !cap;
+    capturing(ctx);
+    const bool clean = ctx->clean && !ctx->user_graphs;
+    ctx->clean = false;
+    if (!clean) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
     return HF_OK;
 }
 
@@ -890,6 +893,7 @@ int hf_apply_bcs(hf_ctx* ctx) {
     hf::TraceRange trace_("hf_apply_bcs");
     if (!ctx) return HF_ERR_ARG;
     if (ctx->next_block != 0) return fail(ctx, HF_ERR_STATE, "apply_bcs in the middle of a step");
+    capturing(ctx);
     ctx->clean = false;
     CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
     CK(hf::launch_fill_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 0));
@@ -922,6 +926,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
     hf::TraceRange trace_("hf_advance_block");
     if (!ctx || b < 0 || b >= ctx->nblocks) return HF_ERR_ARG;
     if (b != ctx->next_block) return fail(ctx, HF_ERR_STATE, "blocks must be advanced in order");
+    capturing(ctx);
     if (b == 0) {
         // a caller that gives dt itself may have skipped hf_time_step: start the step, and give
         // the MUSCL-Hancock predictor's TimeStep call the ghost maxima of the current fields
@@ -938,7 +943,7 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
         ctx->next_block = 0;
         ctx->step_started = ctx->ghost_fresh = false;
-        ctx->clean = !capturing(ctx);
+        ctx->clean = true;
     } else {
         ctx->next_block = b + 1;
     }
@@ -1029,6 +1034,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
         r = enqueue_blocks(ctx, out, end);
         if (r != HF_OK) return r;
         if (ctx->ring_slots > 0 || !step_kernel(ctx)) CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
+        ctx->clean = true;
         ctx->step_started = ctx->ghost_fresh = false;
         r = wait_step(ctx, end, dt);
         return r != HF_OK ? r : strict_check(ctx);
@@ -1057,6 +1063,7 @@ int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double*
                              (size_t)B.tx * 8, (size_t)4 * B.ty, cudaMemcpyDeviceToHost, ctx->copy_stream));
     }
     CK(hf::launch_finalize(ctx->dctrl, ctx->stream));
+    ctx->clean = true;
     ctx->steps_known = -1;
     ctx->step_started = ctx->ghost_fresh = false;
     if (dt) CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1074,7 +1081,9 @@ int hf_step(hf_ctx* ctx, double* dt) {
     if (r != HF_OK) return r;
     hf::StepOut* const out = dt ? step_out(ctx) : nullptr;
     r = enqueue_step(ctx, ctx->profile, out);
-    if (r != HF_OK || !dt) return r;
+    if (r != HF_OK) return r;
+    ctx->clean = true;
+    if (!dt) return HF_OK;
     r = wait_step(ctx, out, dt);
     return r != HF_OK ? r : strict_check(ctx);
 }
@@ -1116,6 +1125,7 @@ int hf_run(hf_ctx* ctx, int64_t n, int clamp_t_end, int use_graph, int64_t* step
             if (r != HF_OK) return r;
         }
     }
+    ctx->clean = true;
     if (steps_done) {
         *steps_done = read_step(ctx) - s0;
         return strict_check(ctx);

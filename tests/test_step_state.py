@@ -1,0 +1,52 @@
+"""What a step finds of the calls before it: the wave-speed maxima of a TimeStep call or a ghost fill that a
+caller's graph ran again, or that no step followed, are not those of the next step's fields."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _solver(n=40):
+    from hyperflow_gb300 import CartSolver, cases
+    case = cases.quadrant_case(n, scheme="MUSCLHancock", limiter="MinBee", cfl=cases.CFL_2D)
+    case["simulation"]["t_end"] = 0.01
+    return CartSolver(case)
+
+
+def _calm(U):
+    """The same pressure and density at rest: smaller wave speeds everywhere."""
+    U = U.copy()
+    U[3] -= 0.5 * (U[1] ** 2 + U[2] ** 2) / U[0]
+    U[1:3] = 0.0
+    U[3] *= 0.25
+    return U
+
+
+def _next_step(s, U):
+    s.set_state(0, U)
+    dt = s.step()
+    return [dt, s.state(0)]
+
+
+@pytest.mark.parametrize("path", ["one launch", "fill", "launch per block"])
+@pytest.mark.parametrize("call", ["hf_time_step", "hf_apply_bcs"])
+def test_a_replayed_call_leaves_no_maxima_to_the_next_step(call, path):
+    import torch
+    from hyperflow_gb300._lib import lib
+    a, b = _solver(), _solver()
+    for s in (a, b):
+        s.set_strict(path == "fill")               # (strict mode keeps the ghost fill)
+        s.set_block_launches(path == "launch per block")
+        s.run(12)
+    stream = torch.cuda.ExternalStream(a.stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        g.capture_begin(capture_error_mode="thread_local")
+        assert (lib().hf_apply_bcs(a._h) if call == "hf_apply_bcs" else lib().hf_time_step(a._h, None)) == 0
+        g.capture_end()
+        a.step(), b.step()
+        for _ in range(2):
+            g.replay()
+            U = _calm(b.state(0))
+            for x, y in zip(_next_step(a, U), _next_step(b, U)):
+                np.testing.assert_array_equal(x, y)
