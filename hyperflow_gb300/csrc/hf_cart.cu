@@ -47,13 +47,13 @@ __device__ void clear_step(Ctrl* __restrict__ c, int p, int nblocks) {
 }
 
 // Start of a step that no finished step prepared (after an upload, a restore, a ghost fill on its own): its
-// stop flag, and its accumulators cleared.  A finished step clears the next one's itself (finish_step) and
-// the fill takes the stop flag, so a loop's steps need no launch for this.
+// stop flag, and its accumulators cleared, also where the loop has ended: the step that comes next counts on
+// it.  A finished step clears the next one's itself (finish_step) and the fill takes the stop flag, so a
+// loop's steps need no launch for this.
 __global__ void step_begin_kernel(Ctrl* __restrict__ c) {
-    const int done = loop_done(c);
-    c->done = done;
+    c->done = loop_done(c);
     c->snap_pre = c->snap_post = 0;
-    if (!done) clear_step(c, (int)(c->step & 1), c->nblocks);
+    clear_step(c, (int)(c->step & 1), c->nblocks);
 }
 
 // ------------------------------------------------------------------------------------

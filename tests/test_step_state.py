@@ -50,3 +50,18 @@ def test_a_replayed_call_leaves_no_maxima_to_the_next_step(call, path):
             U = _calm(b.state(0))
             for x, y in zip(_next_step(a, U), _next_step(b, U)):
                 np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("path", ["fill", "launch per block"])
+def test_a_run_that_has_ended_leaves_no_maxima_to_the_next_step(path):
+    """At the end time: a TimeStep call, a clamped run that takes no step, then calmer fields."""
+    a, b = _solver(), _solver()
+    for s in (a, b):
+        s.set_strict(path == "fill")
+        s.set_block_launches(path == "launch per block")
+        assert s.run(1000, clamp_t_end=True) > 5 and s.time()[0] == 0.01
+    a.calculate_time_step()
+    assert a.run(3, clamp_t_end=True) == 0
+    U = _calm(b.state(0))
+    for x, y in zip(_next_step(a, U), _next_step(b, U)):
+        np.testing.assert_array_equal(x, y)
