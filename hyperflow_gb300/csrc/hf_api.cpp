@@ -72,6 +72,7 @@ struct hf_ctx {
     hf::StepState* dstep = nullptr;
     bool solo = false;          // one block whose ghosts are interior cells' values or Dirichlet states
     bool user_graphs = false;   // a caller has captured steps
+    bool caller_captures = false;   // and is capturing this call
     int clamp = -1;             // the device's clamp switch, -1 when not known
     hf::StepOut* out = nullptr; // a step's dt and count, in host memory the GPU maps
     long long steps_known = -1; // steps completed, -1 when the device may have moved on
@@ -538,9 +539,9 @@ constexpr long long kLoopCells = 1 << 20;
 // capture on nothing is taken as known about the device: a replay is not seen here.
 bool capturing(hf_ctx* ctx) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    const bool cap = cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
-    ctx->user_graphs = ctx->user_graphs || cap;
-    return cap;
+    ctx->caller_captures = cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
+    ctx->user_graphs = ctx->user_graphs || ctx->caller_captures;
+    return ctx->caller_captures;
 }
 
 // The accumulators of the next step cleared, unless the end of the step before it did so: known only when
@@ -560,7 +561,8 @@ int ensure_clean(hf_ctx* ctx) {
 int enqueue_step(hf_ctx* ctx, bool profiled, hf::StepOut* out = nullptr) {
     ctx->steps_known = -1;
     if (profiled) ev_record(ctx, 1, true);
-    if (ctx->solo && ctx->ring_slots == 0 && !ctx->strict && !ctx->block_launches) {
+    // (a caller's graph may be replayed in strict mode, whose stop the fill takes and this launch does not)
+    if (ctx->solo && ctx->ring_slots == 0 && !ctx->strict && !ctx->block_launches && !ctx->caller_captures) {
         if (profiled) { ev_record(ctx, 1, false); ev_record(ctx, 0, true); }
         CK(hf::launch_solo(ctx->dctrl, ctx->dmesh, ctx->dstep, ctx->blocks[0].nx, ctx->blocks[0].ny, ctx->scheme,
                            ctx->limiter, ctx->tile, &ctx->tmap[0][0], &ctx->tmap[0][1], ctx->stream, out));

@@ -1,5 +1,6 @@
 """What a step finds of the calls before it: the wave-speed maxima of a TimeStep call or a ghost fill that a
-caller's graph ran again, or that no step followed, are not those of the next step's fields."""
+caller's graph ran again, or that no step followed, are not those of the next step's fields; strict mode
+switched on after a step was captured stops its replays."""
 import numpy as np
 import pytest
 
@@ -65,3 +66,29 @@ def test_a_run_that_has_ended_leaves_no_maxima_to_the_next_step(path):
     U = _calm(b.state(0))
     for x, y in zip(_next_step(a, U), _next_step(b, U)):
         np.testing.assert_array_equal(x, y)
+
+
+def test_strict_mode_stops_steps_captured_before_it():
+    import torch
+    from hyperflow_gb300 import CartSolver, HyperFlowError, cases
+    from hyperflow_gb300._lib import lib
+    case = cases.shock_bubble_case(128, cfl=0.8)
+    a, b = CartSolver(case), CartSolver(case)
+    a.step(), b.step()
+    stream = torch.cuda.ExternalStream(a.stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        g.capture_begin(capture_error_mode="thread_local")
+        assert lib().hf_step(a._h, None) == 0
+        g.capture_end()
+        a.set_strict(True)
+        for _ in range(100):
+            g.replay()
+    b.set_strict(True)
+    with pytest.raises(HyperFlowError, match="step 82"):
+        b.run(100, graph=False)
+    with pytest.raises(HyperFlowError, match="step 82"):
+        a.sync()
+    assert a.time() == b.time()
+    np.testing.assert_array_equal(a.state(0), b.state(0))
+    assert a.last_nonpositive_cell() == b.last_nonpositive_cell()
