@@ -1693,16 +1693,24 @@ static int lc_pair_graph(hf_lc* L, int use_mlp) {
         return HF_OK;
     if (L->pair) cudaGraphExecDestroy(L->pair);
     L->pair = nullptr;
-    cudaGraph_t g;
+    // nothing of the state moves while its steps are only recorded, also where recording them fails
+    const int cur = L->cur;
+    const bool wp = L->wp_valid, maxs = L->maxs_valid;
+    cudaGraph_t g = nullptr;
     LCK(cudaStreamBeginCapture(L->stream, cudaStreamCaptureModeThreadLocal));
     int r = enqueue_lc_step(L, 0.0, use_mlp, L->loop);
     if (r == HF_OK) r = enqueue_lc_step(L, 0.0, use_mlp, L->loop);
-    const cudaError_t e = cudaStreamEndCapture(L->stream, &g);
+    cudaError_t e = cudaStreamEndCapture(L->stream, &g);
+    L->cur = cur;
+    L->wp_valid = wp;
+    L->maxs_valid = maxs;
+    if (r == HF_OK && e == cudaSuccess) e = cudaGraphInstantiate(&L->pair, g, 0);
+    if (g) cudaGraphDestroy(g);
     if (r) return r;
-    if (e != cudaSuccess) return lfail(L, HF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    const cudaError_t ei = cudaGraphInstantiate(&L->pair, g, 0);
-    cudaGraphDestroy(g);
-    if (ei != cudaSuccess) return lfail(L, HF_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(ei));
+    if (e != cudaSuccess) {
+        L->pair = nullptr;
+        return lfail(L, HF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+    }
     L->pair_key = key;
     return HF_OK;
 }
