@@ -129,7 +129,7 @@ __device__ __forceinline__ float slopef(int lim, float um, float u0, float up) {
 }
 
 // The run loop on the device (hf_lc_run_to): the step to take next, formed by the last CTA of the update
-// before it.  Kernels given a loop take dt and dt / dx from it and leave at once when it has ended; given
+// before it (the first one by the host).  Kernels given a loop take dt and dt / dx from it and leave at once when it has ended; given
 // none they take them as arguments.
 struct Loop {
     double t, t_end, dt, cfl_dx, dx;   // cfl_dx = cfl dx; dt: the next step's
@@ -1176,7 +1176,7 @@ __global__ void guard_kernel(const float* __restrict__ U, const float* __restric
 // the loop's next dt from the state's wave-speed maximum, or its end.  The reference's TimeStep uses 0.2 x
 // CFL for its first 10 calls; a MUSCL-Hancock step makes two (step and predictor), so the first 5
 // steps are reduced.
-__device__ void form_step(Loop* loop, float m) {
+__host__ __device__ void form_step(Loop* loop, float m) {
     loop->done = !(loop->t < loop->t_end);
     if (loop->done) return;
     double dt = loop->cfl_dx / (double)m;
@@ -1250,9 +1250,6 @@ __global__ void update_kernel(const float* __restrict__ U, const float* __restri
     if (rejected) loop->rejected = loop->rejected + (long long)*(const volatile unsigned long long*)rejected;
     form_step(loop, *(const volatile float*)maxs);
 }
-
-// the first step of a run
-__global__ void loop_begin_kernel(Loop* __restrict__ loop, const float* __restrict__ maxs) { form_step(loop, *maxs); }
 
 // dL/dY for L = (1/N) sum_cells sum_v w_v (U^{n+1}_v - T_v)^2, U^{n+1} with every correction
 __global__ void loss_grad_kernel(const float* __restrict__ Un, const float* __restrict__ T, const float* __restrict__ scale,
@@ -1345,11 +1342,11 @@ struct hf_lc {
     Out* out = nullptr;        // pinned: a training iteration's loss and the error word
     int* derr = nullptr;       // device error word (a bounded wait gave up)
     Loop* loop = nullptr;      // the device run loop
-    cudaGraphExec_t pair = nullptr;   // two steps of it, captured for the settings in pair_key
-    struct PairKey {
-        int cur, use_mlp, guard_mode, fused, ctas;
+    struct Pair {              // two steps of it, captured for these settings
+        cudaGraphExec_t exec;
+        int guard_mode, fused, ctas;
         double bound;
-    } pair_key{};
+    } pair[2][2] = {};         // [use_mlp][the current state's buffer]
     int cur = 0;
     long long steps = 0;       // steps since time 0 (TimeStep's start-up multiplier)
     long long adam_t = 0;
@@ -1565,7 +1562,9 @@ void hf_lc_destroy(hf_lc* L) {
     if (L->side) cudaStreamSynchronize(L->side);
     for (void* p : L->allocs) cudaFree(p);
     if (L->out) cudaFreeHost(L->out);
-    if (L->pair) cudaGraphExecDestroy(L->pair);
+    for (auto& of : L->pair)
+        for (auto& p : of)
+            if (p.exec) cudaGraphExecDestroy(p.exec);
     if (L->fork) cudaEventDestroy(L->fork);
     if (L->join) cudaEventDestroy(L->join);
     if (L->side) cudaStreamDestroy(L->side);
@@ -1684,15 +1683,19 @@ int hf_lc_step(hf_lc* L, double dt, int use_mlp, int64_t* rejected_cells) {
 }
 
 // Two steps of the device loop as a graph: a step is four launches on two streams with their events, and
-// the host needed 85 to 100 us for what the GPU does in 73 (512^2).  Captured once for its settings.
+// the host needed 85 to 100 us for what the GPU does in 73 (512^2).  Recorded once per network switch,
+// starting buffer and settings: with one graph for all, a run of an odd number of steps, or of the other
+// kind, had the next call record its own again.
+static bool lc_pair_ready(const hf_lc* L, int use_mlp) {
+    const hf_lc::Pair& k = L->pair[use_mlp != 0][L->cur];
+    return k.exec && k.guard_mode == L->guard_mode && k.fused == L->fused && k.ctas == L->face_ctas_per_sm &&
+           k.bound == L->bound;
+}
 static int lc_pair_graph(hf_lc* L, int use_mlp) {
-    const hf_lc::PairKey key{L->cur, use_mlp != 0, L->guard_mode, L->fused, L->face_ctas_per_sm, L->bound};
-    const hf_lc::PairKey& k = L->pair_key;
-    if (L->pair && k.cur == key.cur && k.use_mlp == key.use_mlp && k.guard_mode == key.guard_mode && k.fused == key.fused &&
-        k.ctas == key.ctas && k.bound == key.bound)
-        return HF_OK;
-    if (L->pair) cudaGraphExecDestroy(L->pair);
-    L->pair = nullptr;
+    if (lc_pair_ready(L, use_mlp)) return HF_OK;
+    hf_lc::Pair& k = L->pair[use_mlp != 0][L->cur];
+    if (k.exec) cudaGraphExecDestroy(k.exec);
+    k = hf_lc::Pair{nullptr, L->guard_mode, L->fused, L->face_ctas_per_sm, L->bound};
     // nothing of the state moves while its steps are only recorded, also where recording them fails
     const int cur = L->cur;
     const bool wp = L->wp_valid, maxs = L->maxs_valid;
@@ -1704,21 +1707,52 @@ static int lc_pair_graph(hf_lc* L, int use_mlp) {
     L->cur = cur;
     L->wp_valid = wp;
     L->maxs_valid = maxs;
-    if (r == HF_OK && e == cudaSuccess) e = cudaGraphInstantiate(&L->pair, g, 0);
+    if (r == HF_OK && e == cudaSuccess) e = cudaGraphInstantiate(&k.exec, g, 0);
     if (g) cudaGraphDestroy(g);
     if (r) return r;
     if (e != cudaSuccess) {
-        L->pair = nullptr;
+        k.exec = nullptr;
         return lfail(L, HF_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
     }
-    L->pair_key = key;
     return HF_OK;
 }
 
-// Runs until t_end with CFL dt; returns steps.  The loop is the device's: every step's update forms the
-// next dt, and a step after the end leaves its buffers alone.  The host enqueues as many steps as the
-// last dt it read suggests are left and reads the loop's state once for all of them (it read the wave-speed
-// maximum back for every step's dt: 112 us a step at 512^2 for 72 of kernels).
+// k steps of the device loop, which holds the next one, and the loop as they leave it in *S; steps past the
+// end do nothing.  Pairs from the graph where it is there or pays for its recording (50 to 60 us, and 15 to
+// 25 us less a step), else one by one.
+static int run_loop_steps(hf_lc* L, int use_mlp, int k, Loop* S) {
+    const int cur = L->cur;
+    const long long taken = S->taken;
+    int r;
+    if (k >= 4 || (k >= 2 && lc_pair_ready(L, use_mlp))) {
+        if (use_mlp && L->fused && !L->wp_valid) {   // the steps find the primitives of the state before them
+            prims_kernel<<<blocks_for(L->n * L->n, 256), 256, 0, L->stream>>>(L->U[cur], L->n, grid(L).g1, L->Wp);
+            LCK(cudaGetLastError());
+            L->wp_valid = true;
+        }
+        if ((r = lc_pair_graph(L, use_mlp))) return r;
+        for (int i = 0; i < k; i += 2) LCK(cudaGraphLaunch(L->pair[use_mlp != 0][cur].exec, L->stream));
+    } else {
+        for (int i = 0; i < k; ++i)
+            if ((r = enqueue_lc_step(L, 0.0, use_mlp, L->loop))) return r;
+    }
+    LCK(cudaMemcpyAsync(S, L->loop, sizeof *S, cudaMemcpyDeviceToHost, L->stream));
+    LCK(cudaStreamSynchronize(L->stream));
+    L->cur = cur ^ (int)((S->taken - taken) & 1);
+    // (the separate kernels form the primitives anew in every step, those past the end too)
+    L->wp_valid = use_mlp && L->fused;
+    L->maxs_valid = true;
+    L->t = S->t;
+    L->steps = S->steps;
+    return HF_OK;
+}
+
+// Runs until t_end with CFL dt; returns steps.  The first step's dt is formed here from the wave-speed
+// maximum.  From there on the loop is the device's: every step's update forms the next dt, and a step after
+// the end leaves its buffers alone.  The host enqueues as many steps as the last dt it knows suggests are
+// left and reads the loop's state once for all of them (it read the maximum back for every step's dt: 112 us
+// a step at 512^2 for 72 of kernels).  A single step left is taken with the dt the host has formed: a program
+// that advances by a step a call pays one wait for the maximum and one for the step.
 int hf_lc_run_to(hf_lc* L, double t_end, int use_mlp, int64_t* steps, int64_t* rejected_cells) {
     hf::TraceRange trace_("hf_lc_run_to");
     if (!L) return HF_ERR_ARG;
@@ -1730,37 +1764,45 @@ int hf_lc_run_to(hf_lc* L, double t_end, int use_mlp, int64_t* steps, int64_t* r
     S.cfl_dx = L->cfl * L->dx;
     S.dx = L->dx;
     S.steps = L->steps;
-    LCK(cudaMemcpyAsync(L->loop, &S, sizeof S, cudaMemcpyHostToDevice, L->stream));
-    loop_begin_kernel<<<1, 1, 0, L->stream>>>(L->loop, L->maxs);
-    LCK(cudaGetLastError());
-    const int cur = L->cur;
-    if (use_mlp && L->fused && !L->wp_valid) {   // the steps find the primitives of the state before them
-        prims_kernel<<<blocks_for(L->n * L->n, 256), 256, 0, L->stream>>>(L->U[cur], L->n, grid(L).g1, L->Wp);
-        LCK(cudaGetLastError());
-        L->wp_valid = true;
-    }
-    const bool wp = L->wp_valid;
-    if ((r = lc_pair_graph(L, use_mlp))) return r;
+    S.done = !(S.t < S.t_end);
+    bool formed = false, loaded = false, counted = true;   // the next step in S, S on the device, S.rejected whole
     for (;;) {
-        LCK(cudaMemcpyAsync(&S, L->loop, sizeof S, cudaMemcpyDeviceToHost, L->stream));
-        LCK(cudaStreamSynchronize(L->stream));
-        L->cur = cur ^ (int)(S.taken & 1);   // steps past the end did nothing
-        // (the separate kernels form the primitives anew in every step, those past the end too)
-        L->wp_valid = S.taken > 0 ? use_mlp && L->fused : wp && L->fused;
-        L->t = S.t;
-        L->steps = S.steps;
+        float m = 0.0f;
+        unsigned long long rc = 0;
+        if (!formed && !S.done) LCK(cudaMemcpyAsync(&m, L->maxs, sizeof m, cudaMemcpyDeviceToHost, L->stream));
+        if (!counted) LCK(cudaMemcpyAsync(&rc, L->rejected, sizeof rc, cudaMemcpyDeviceToHost, L->stream));
+        if (!formed) {
+            LCK(cudaStreamSynchronize(L->stream));
+            S.rejected += (long long)rc;
+            counted = true;
+            if (!S.done) form_step(&S, m);
+            formed = true;
+        }
         if (S.done) break;
         const int slow = S.steps < 5 ? (int)(5 - S.steps) : 0;   // steps at 0.2 CFL left
         const double full = slow ? 5.0 * S.dt : S.dt;
         const double left = (S.t_end - S.t - slow * S.dt) / full;
         const double want = slow + (left > 0.0 ? std::ceil(left) : 0.0);
         const int k = want < 1.0 ? 1 : (want > 64.0 ? 64 : (int)want);
-        // (pairs: the state before one is in the buffer it was captured with)
-        for (int i = 0; i < k; i += 2) LCK(cudaGraphLaunch(L->pair, L->stream));
+        if (k == 1) {
+            if ((r = enqueue_lc_step(L, S.dt, use_mlp, nullptr))) return r;
+            S.t += S.dt;
+            S.steps += 1;
+            S.taken += 1;
+            S.done = !(S.t < S.t_end);
+            L->t = S.t;
+            L->steps = S.steps;
+            formed = loaded = false;
+            counted = !use_mlp;
+        } else {
+            if (!loaded) LCK(cudaMemcpyAsync(L->loop, &S, sizeof S, cudaMemcpyHostToDevice, L->stream));
+            loaded = true;
+            if ((r = run_loop_steps(L, use_mlp, k, &S))) return r;
+        }
     }
+    if (S.failed) return lfail(L, HF_ERR_DEVICE, "coarse run stopped advancing (non-positive or non-finite dt)");
     if (steps) *steps = S.taken;
     if (rejected_cells) *rejected_cells = S.rejected;
-    if (S.failed) return lfail(L, HF_ERR_DEVICE, "coarse run stopped advancing (non-positive or non-finite dt)");
     return check_derr(L);
 }
 
