@@ -295,8 +295,8 @@ __global__ void __launch_bounds__(kRedThreads) interior_cfl_kernel(Ctrl* __restr
 // maps (pinned), written into both buffers, with the TimeStep terms of the interior cells -- the
 // upload, buffer copy and interior_cfl of a host-buffer step or a state upload in one pass over the
 // link.  A warp takes a row's cells 32 at a time, and the next row when it has them all.
-// Bound by the link: a 4096^2 pass's upload and download (541 MB each) take about 5 ms together, where
-// the copy engine's row-by-row copies out of and into the padded rows took about 32.
+// Bound by the link: 4096^2 cells (538 MB) in 2.86 ms, 188 GB/s; 3.43 with the copy engine, a device copy to the
+// other buffer and interior_cfl behind it; 1000 x 1000 in 0.20 ms, before 0.35; 300 x 8000 in 0.43, before 1.68.
 // (a row of CTAs per block from b0 on: a launch per block left the link idle between them)
 __global__ void __launch_bounds__(kRedThreads) upload_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m,
                                                              int b0, int parity, const HostBlocks h) {
@@ -335,25 +335,37 @@ __global__ void __launch_bounds__(kRedThreads) upload_kernel(Ctrl* __restrict__ 
     block_max2_atomic<kRedThreads>(mx, my, &c->int_s[parity][b][0], &c->int_s[parity][b][1]);
 }
 
-// A block's whole state into host memory the GPU maps, likewise
+// A block's whole state into host memory the GPU maps.  Bound by the link, which a store of a whole line uses
+// best: the array is taken in pieces that start on its 256-byte lines, whatever its rows' length, a warp four
+// lines at a time.  us for 1000 rows of 65, 191, 1003, 2049 cells: 37, 58, 193, 366; from each row's start 38, 64,
+// 236, 456; the copy engine 47, 61, 193, 455, with the same 191 GB/s at 4096^2 (2.82 ms) but for 4 to 10 ms in one
+// copy of ten there, and up to 20 the first time it writes an array.
+constexpr int kDownLines = 4;
 __global__ void __launch_bounds__(kRedThreads) download_kernel(Ctrl* __restrict__ c, const MeshDev* __restrict__ m, int b,
                                                                int parity, double* __restrict__ hout) {
     const BlockDev& B = m->b[b];
-    const size_t plane = (size_t)B.ty * B.pitch, hplane = (size_t)B.ty * B.tx;
+    const unsigned tx = (unsigned)B.tx;
+    const long long n = 4LL * B.ty * B.tx, all = 4LL * B.ty * B.pitch;
     const double* __restrict__ U = B.buf[parity];
-    const int segs = (B.tx + 31) >> 5, lane = threadIdx.x & 31;
-    const long long n = (long long)segs * B.ty;
-    for (long long w = (blockIdx.x * (long long)kRedThreads + threadIdx.x) >> 5; w < n;
+    const int lead = (int)(reinterpret_cast<uintptr_t>(hout) >> 3) & 31, lane = threadIdx.x & 31;
+    for (long long w = (blockIdx.x * (long long)kRedThreads + threadIdx.x) >> 5; w * 32 * kDownLines - lead < n;
          w += (long long)gridDim.x * (kRedThreads / 32)) {
-        const int j = (int)(w / segs), i = (int)(w - (long long)j * segs) * 32 + lane;
-        if (i >= B.tx) continue;
-        const size_t o = (size_t)j * B.pitch + i, h = (size_t)j * B.tx + i;
-        if (!hf_in((long long)o, (long long)plane, &c->err)) continue;
-        double u[4];
+        const long long f0 = w * 32 * kDownLines - lead, from = f0 < 0 ? 0 : f0;
+        const long long row = from / tx;                 // of the array's 4 total_y rows
+        const int col = (int)(from - row * tx);
+        double u[kDownLines];
+        bool in[kDownLines];
 #pragma unroll
-        for (int v = 0; v < 4; ++v) u[v] = U[v * plane + o];
+        for (int k = 0; k < kDownLines; ++k) {
+            const long long f = f0 + 32 * k + lane;
+            const unsigned at = (unsigned)(col + (int)(f - from)), down = at / tx;
+            const long long o = (row + down) * B.pitch + (at - down * tx);
+            in[k] = f >= 0 && f < n && hf_in(o, all, &c->err);
+            if (in[k]) u[k] = U[o];
+        }
 #pragma unroll
-        for (int v = 0; v < 4; ++v) __stcs(&hout[v * hplane + h], u[v]);
+        for (int k = 0; k < kDownLines; ++k)
+            if (in[k]) __stcs(&hout[f0 + 32 * k + lane], u[k]);
     }
 }
 
@@ -1157,7 +1169,9 @@ cudaError_t launch_upload(Ctrl* c, const MeshDev* m, int b0, int nb, const int* 
 }
 
 cudaError_t launch_download(Ctrl* c, const MeshDev* m, int b, int tx, int ty, int parity, double* hout, cudaStream_t s) {
-    download_kernel<<<link_grid(tx, ty), kRedThreads, 0, s>>>(c, m, b, parity, hout);
+    const long long want = (4LL * tx * ty + 31) / (4 * kRedThreads) + 1;   // (the array may start inside a line)
+    static_assert(kDownLines == 4, "a CTA takes 4 doubles a thread");
+    download_kernel<<<(unsigned)(want > 8 * 152 ? 8 * 152 : want), kRedThreads, 0, s>>>(c, m, b, parity, hout);
     return cudaGetLastError();
 }
 
