@@ -19,6 +19,7 @@
 
 #include "../../include/hyperflow_gb300.h"
 #include "hf_cart.h"
+#include "hf_pinned.h"
 #include "hf_trace.h"
 #include "hf_json.hpp"
 
@@ -796,19 +797,36 @@ int hf_block_dims(const hf_ctx* ctx, int b, int dims[5]) {
     return HF_OK;
 }
 
-// true when the array of len doubles is 8-byte aligned host memory that kernels may address as it is, at
-// both its ends (pinned by cudaHostAlloc / cudaHostRegister: the device pointer is the host pointer)
-static bool host_mapped(const double* p, size_t len) {
-    if (reinterpret_cast<uintptr_t>(p) % 8 != 0) return false;
-    for (const double* q : {p, p + (len - 1)}) {
-        cudaPointerAttributes a;
-        if (cudaPointerGetAttributes(&a, q) != cudaSuccess) {
+// the range of pinned host memory that holds address q, where kernels may address it as it is (the device
+// pointer is the host pointer)
+static hf::HostRange mapped_range(uintptr_t q) {
+    typedef CUresult (*PointerAttributesFn)(unsigned int, CUpointer_attribute*, void**, CUdeviceptr);
+    static const PointerAttributesFn get = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &p, 12000, cudaEnableDefault, &r) != cudaSuccess ||
+            r != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
-            return false;
+            p = nullptr;
         }
-        if (a.type != cudaMemoryTypeHost || a.devicePointer != static_cast<const void*>(q)) return false;
-    }
-    return true;
+        return reinterpret_cast<PointerAttributesFn>(p);
+    }();
+    unsigned int type = 0, managed = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* into[5] = {&type, &managed, &dev, &start, &size};
+    if (!get || get(5, what, into, (CUdeviceptr)q) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || managed ||
+        dev != (CUdeviceptr)q)
+        return {0, 0};
+    return {(uintptr_t)start, (uintptr_t)start + size};
+}
+// true when the array of len doubles is 8-byte aligned host memory that kernels may address as it is
+static bool host_mapped(const double* p, size_t len) {
+    const uintptr_t q = reinterpret_cast<uintptr_t>(p);
+    return q % 8 == 0 && hf::host_covered(q, len * sizeof(double), mapped_range);
 }
 // the same for one array per block, each a block's whole state
 static bool blocks_mapped(const hf_ctx* ctx, const double* const* p) {

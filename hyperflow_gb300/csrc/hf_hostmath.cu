@@ -1,13 +1,25 @@
 // Host build of the kernels' arithmetic (hf_device.cuh, hf_intdiv.cuh) for the CPU test
 // suite: the same source the GPU kernels compile, exposed as plain C functions so the
-// tests can compare it with the oracle and with IEEE division / sqrt without a GPU.
+// tests can compare it with the oracle and with IEEE division / sqrt without a GPU; and the walk over ranges of
+// pinned memory, on made-up ranges.
 // Built as a separate library (libhf_hostmath.so); the product library does not use it.
 #include <cstdint>
 
 #include "hf_device.cuh"
 #include "hf_fast.cuh"
+#include "hf_pinned.h"
 
 extern "C" {
+
+// host_covered over n ranges [begin[k], begin[k] + size[k])
+int hm_host_covered(const uint64_t* begin, const uint64_t* size, int n, uint64_t p, uint64_t bytes) {
+    return hf::host_covered((uintptr_t)p, (size_t)bytes, [&](uintptr_t q) {
+        for (int k = 0; k < n; ++k)
+            if (q >= begin[k] && q < begin[k] + size[k])
+                return hf::HostRange{(uintptr_t)begin[k], (uintptr_t)(begin[k] + size[k])};
+        return hf::HostRange{0, 0};
+    });
+}
 
 void hm_div(const double* a, const double* b, double* out, int64_t n) {
     for (int64_t i = 0; i < n; ++i) out[i] = hf::div_rn(a[i], b[i]);

@@ -99,7 +99,8 @@ int hf_step(hf_ctx* ctx, double* dt);
  * copied, each block's download starting as soon as its update is done. */
 int hf_step_io(hf_ctx* ctx, const double* const* in, double* const* out, double* dt);
 /* *mapped = 1 when p is 8-byte aligned host memory that the kernels address directly (pinned by
- * cudaHostAlloc / cudaHostRegister), i.e. hf_step_io's direct path applies to it. */
+ * cudaHostAlloc / cudaHostRegister).  hf_step_io's direct path, and that of hf_set_state and hf_get_state with
+ * HF_LAYOUT_SOA, applies to an array of which all is: allocations or registrations cover it without a gap. */
 int hf_host_mapped(const void* p, int* mapped);
 
 /* Simulation::solve's loop body (simulation.cpp:81-120, frame clamps excluded) run n times
