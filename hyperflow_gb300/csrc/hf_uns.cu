@@ -75,6 +75,7 @@ struct UnsMesh {
     const double* __restrict__ edge_geo;    // [5][nedges]: the owning pair's geo, edge by edge
     double2* edge_flux;                     // [nedges][2]: length x rotated-back HLLC flux, an edge's in one sector
     int nedges;
+    double* stage;                          // [4][ncells] in the mesh file's order, between steps (edge_flux's memory)
     // cells are held in a locality order (Morton order of their vertex centroids); orig[i] is
     // the mesh file's index of device cell i, used in the failure records' keys
     const int* __restrict__ orig;
@@ -261,11 +262,12 @@ __global__ void __launch_bounds__(kUnsNT, 6) uns_edge_flux_kernel(UnsCtrl* __res
     if (herr) atomicAdd(reinterpret_cast<unsigned long long*>(&c->hllc_errors), (unsigned long long)herr);
 }
 
-// a state in the mesh file's order (the other buffer) into the device's order, with its TimeStep terms
+// A state in the mesh file's order (m.stage) into the device's order, with its TimeStep terms.  (Not by way of the
+// other state buffer: a checkpoint holds both.)
 __global__ void __launch_bounds__(kUnsNT) uns_load_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int parity) {
     double mn = 1e16;
     const size_t N = (size_t)m.ncells;
-    const double* __restrict__ F = m.U[parity ^ 1];
+    const double* __restrict__ F = m.stage;
     double* __restrict__ U = m.U[parity];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.ncells; i += gridDim.x * blockDim.x) {
         const int o = m.orig[i];
@@ -279,11 +281,11 @@ __global__ void __launch_bounds__(kUnsNT) uns_load_kernel(UnsCtrl* __restrict__ 
     block_min_atomic<kUnsNT>(mn, &c->min_dt[parity]);
 }
 
-// the state into the mesh file's order, in the other buffer (the next step overwrites it)
-__global__ void __launch_bounds__(kUnsNT) uns_store_kernel(UnsCtrl* __restrict__ c, UnsMesh m, int parity) {
+// the present state into the mesh file's order, in m.stage
+__global__ void __launch_bounds__(kUnsNT) uns_store_kernel(UnsCtrl* __restrict__ c, UnsMesh m) {
     const size_t N = (size_t)m.ncells;
-    const double* __restrict__ U = m.U[parity];
-    double* __restrict__ F = m.U[parity ^ 1];
+    const double* __restrict__ U = m.U[c->step & 1];
+    double* __restrict__ F = m.stage;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.ncells; i += gridDim.x * blockDim.x) {
         const int o = m.orig[i];
         if (!hf_in(o, m.ncells, &c->err)) continue;
@@ -1012,8 +1014,9 @@ int finish_create(hf_uns* u, const Json& cfg) {
         if ((r = upload(u, &d_pe, pe)) || (r = upload(u, &d_sg, sg)) || (r = upload(u, &d_ep, ep)) ||
             (r = upload(u, &d_ec, ec)) || (r = upload(u, &d_en, en)) || (r = upload(u, &d_eg, eg)))
             return r;
-        UCK(cudaMalloc(&d_ef, 4 * (ne + 1) * sizeof(double)));
+        UCK(cudaMalloc(&d_ef, 4 * std::max(ne + 1, (size_t)n) * sizeof(double)));
         u->allocs.push_back(d_ef);
+        u->dm.stage = d_ef;
         u->d_pair_edge = d_pe;
         u->d_pair_sign = d_sg;
         u->dm.edge_pair = d_ep;
@@ -1243,8 +1246,8 @@ int hf_uns_set_state(hf_uns* u, const double* cons) {
     if (r) return r;
     int p = (int)(s & 1);
     size_t bytes = (size_t)4 * u->ncells * sizeof(double);
-    // in the file's order into the other buffer, and from there by a kernel into the device's order
-    UCK(cudaMemcpyAsync(u->dm.U[p ^ 1], cons, bytes, cudaMemcpyHostToDevice, u->stream));
+    // in the file's order into the stage, and from there by a kernel into the device's order
+    UCK(cudaMemcpyAsync(u->dm.stage, cons, bytes, cudaMemcpyHostToDevice, u->stream));
     unsigned long long init = 0;
     double big = 1e16;
     std::memcpy(&init, &big, 8);
@@ -1259,14 +1262,11 @@ int hf_uns_set_state(hf_uns* u, const double* cons) {
 
 int hf_uns_get_state(hf_uns* u, double* cons) {
     if (!u || !cons || !u->dctrl) return HF_ERR_ARG;
-    long long s;
-    int r = read_step(u, &s);
-    if (r) return r;
-    // a kernel writes it in the file's order into the other buffer; the host's scatter of 1M cells took 7 ms
-    const int p = (int)(s & 1), want = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
-    hf::uns_store_kernel<<<want > 8 * 152 ? 8 * 152 : want, hf::kUnsNT, 0, u->stream>>>(u->dctrl, u->dm, p);
+    // a kernel writes it in the file's order into the stage; the host's scatter of 1M cells took 7 ms
+    const int want = (u->ncells + hf::kUnsNT - 1) / hf::kUnsNT;
+    hf::uns_store_kernel<<<want > 8 * 152 ? 8 * 152 : want, hf::kUnsNT, 0, u->stream>>>(u->dctrl, u->dm);
     UCK(cudaGetLastError());
-    UCK(cudaMemcpyAsync(cons, u->dm.U[p ^ 1], (size_t)4 * u->ncells * sizeof(double), cudaMemcpyDeviceToHost, u->stream));
+    UCK(cudaMemcpyAsync(cons, u->dm.stage, (size_t)4 * u->ncells * sizeof(double), cudaMemcpyDeviceToHost, u->stream));
     UCK(cudaStreamSynchronize(u->stream));
     return HF_OK;
 }
