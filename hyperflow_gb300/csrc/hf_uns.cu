@@ -23,6 +23,7 @@
 #include <cstring>
 #include <fstream>
 #include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -502,7 +503,7 @@ struct hf_uns {
     std::vector<int> codes;             // per pair boundary code from the mesh file
     std::vector<int> pair_start, nbr;
     // the device holds cells in a locality order: perm[d] = file index of device cell d,
-    // iperm[f] = device index of file cell f; stage: a [4][ncells] host buffer for reordering
+    // iperm[f] = device index of file cell f; stage: a [4][ncells] host buffer for reordering frames
     std::vector<int> perm, iperm;
     std::vector<double> stage;
     long long unmatched = 0;            // pairs with a cell-index code (0: interior) and no match
@@ -1412,6 +1413,11 @@ int hf_uns_frames_enable(hf_uns* u, int ring_slots) {
     if (u->ring) { UCK(cudaFree(u->ring)); u->ring = nullptr; }
     u->ring_slots = 0;
     if (ring_slots > 0) {
+        try {
+            u->stage.resize((size_t)4 * u->ncells);
+        } catch (const std::bad_alloc&) {
+            return ufail(u, HF_ERR_TOO_LARGE, "no host memory for a frame");
+        }
         UCK(cudaMalloc(&u->ring, (size_t)ring_slots * 4 * u->ncells * sizeof(double)));
         u->ring_slots = ring_slots;
     }
@@ -1558,7 +1564,6 @@ int hf_uns_frame_pop(hf_uns* u, double* cons, double* t, int64_t* index) {
     if (C.captured == u->drained) return ufail(u, HF_ERR_STATE, "no frame pending");
     const long long slot = u->drained % u->ring_slots, len = 4LL * u->ncells;
     if (cons) {
-        u->stage.resize((size_t)len);
         UCK(cudaMemcpy(u->stage.data(), u->ring + slot * len, (size_t)len * sizeof(double), cudaMemcpyDeviceToHost));
         to_file_order(u, cons);
     }
