@@ -30,7 +30,6 @@
 #include <cstring>
 #include <map>
 #include <memory>
-#include <queue>
 #include <string>
 #include <vector>
 
@@ -311,38 +310,54 @@ std::vector<TileShape> case_tiles(int scheme, int model, const std::vector<int>&
     struct Shape {
         int tx, ty;
         double time;   // of a whole tile beside another on its SM
+        int order;
     };
     auto shared_time = [](const TileCost& c) { return std::max(2.0 * c.work, c.alone); };
+    // the model's costs, once: a case looks up a whole tile and its last row for every shape
+    std::vector<TileCost> costs(29 * 32);
+    auto cost = [&](int tx, int ty) -> TileCost& { return costs[(tx - 8) / 2 * 32 + ty - 1]; };
     std::vector<Shape> shapes;
     double lo = 0.0, hi = 0.0;
     for (int tx = 8; tx <= 64; tx += 2)
-        for (int ty = 2; ty <= 32; ++ty) {
-            if (!tile_fits(scheme, tx, ty)) continue;
-            const double t = shared_time(tile_cost(scheme, model, tx, ty));
-            shapes.push_back({tx, ty, t});
+        for (int ty = 1; ty <= 32; ++ty) {
+            cost(tx, ty) = tile_cost(scheme, model, tx, ty);
+            if (ty < 2 || !tile_fits(scheme, tx, ty)) continue;
+            const double t = shared_time(cost(tx, ty));
+            shapes.push_back({tx, ty, t, (int)shapes.size()});
             lo = lo == 0.0 ? t : std::min(lo, t);
             hi = std::max(hi, t);
         }
+    std::sort(shapes.begin(), shapes.end(),
+              [](const Shape& a, const Shape& b) { return a.time < b.time || (a.time == b.time && a.order < b.order); });
     std::vector<double> limits;
     for (double l = hi; l > lo; l *= 0.85) limits.push_back(l);
     limits.push_back(lo);
-    // per distinct side and limit: the best shape
+    // per distinct side and limit: the shape of the least work, the narrower and lower of two alike (the shapes
+    // by their time, so one pass serves every limit)
     std::map<int, std::vector<int>> best;
     for (int side : n) {
         if (best.count(side)) continue;
         std::vector<int> at(limits.size(), -1);
-        std::vector<double> least(limits.size(), 0.0);
-        for (size_t k = 0; k < shapes.size(); ++k) {
-            const Shape& s = shapes[k];
-            const int rest = side % s.ty;
-            const double column = (double)(side / s.ty) * tile_cost(scheme, model, s.tx, s.ty).work +
-                                  (rest ? tile_cost(scheme, model, s.tx, rest).work : 0.0);
-            const double work = column * ((side + s.tx - 1) / s.tx);
-            for (size_t l = 0; l < limits.size() && s.time <= limits[l]; ++l)
-                if (at[l] < 0 || work < least[l]) {
-                    least[l] = work;
-                    at[l] = (int)k;
+        int pick = -1, across[29], whole[33], rest[33];   // by tx, and by ty
+        for (int i = 0; i < 29; ++i) across[i] = (side + 7 + 2 * i) / (8 + 2 * i);
+        for (int ty = 1; ty <= 32; ++ty) {
+            whole[ty] = side / ty;
+            rest[ty] = side % ty;
+        }
+        double least = 0.0;
+        size_t k = 0;
+        for (size_t l = limits.size(); l-- > 0;) {
+            for (; k < shapes.size() && shapes[k].time <= limits[l]; ++k) {
+                const Shape& s = shapes[k];
+                const double column = (double)whole[s.ty] * cost(s.tx, s.ty).work +
+                                      (rest[s.ty] ? cost(s.tx, rest[s.ty]).work : 0.0);
+                const double work = column * across[(s.tx - 8) / 2];
+                if (pick < 0 || work < least || (work == least && s.order < shapes[pick].order)) {
+                    least = work;
+                    pick = (int)k;
                 }
+            }
+            at[l] = pick;
         }
         best.emplace(side, std::move(at));
     }
@@ -353,7 +368,7 @@ std::vector<TileShape> case_tiles(int scheme, int model, const std::vector<int>&
         double work = 0.0;
         long long tiles = 0;
         auto add = [&](int tx, int ty, long long k) {
-            const TileCost c = tile_cost(scheme, model, tx, ty);
+            const TileCost c = cost(tx, ty);
             auto& e = kinds[shared_time(c)];
             e.first += k;
             e.second = c.alone;
@@ -370,17 +385,19 @@ std::vector<TileShape> case_tiles(int scheme, int model, const std::vector<int>&
         if (tiles <= sms) {
             for (auto& e : kinds) end = std::max(end, e.second.second);
         } else if (tiles <= 24LL * sms) {
-            std::priority_queue<double, std::vector<double>, std::greater<double>> cta;
-            for (int k = 0; k < 2 * sms; ++k) cta.push(0.0);
+            // each tile to the CTA that is done first, alike ones together: end -> CTAs
+            std::map<double, long long> cta{{0.0, 2LL * sms}};
             for (auto e = kinds.rbegin(); e != kinds.rend(); ++e)
-                for (long long k = 0; k < e->second.first; ++k) {
-                    const double at = cta.top() + e->first;
-                    cta.pop();
-                    cta.push(at);
+                for (long long k = e->second.first; k > 0;) {
+                    auto first = cta.begin();
+                    const long long m = std::min(k, first->second);
+                    cta[first->first + e->first] += m;
+                    k -= m;
+                    if ((first->second -= m) == 0) cta.erase(first);
                 }
             // an SM's two CTAs: while one is done the other runs faster, but not twice as fast
             std::vector<double> f;
-            for (; !cta.empty(); cta.pop()) f.push_back(cta.top());
+            for (auto& c : cta) f.insert(f.end(), (size_t)c.second, c.first);
             for (int k = 0; k < sms; ++k) end = std::max(end, f[k] + 0.65 * (f[2 * sms - 1 - k] - f[k]));
         } else {
             end = work / sms + 0.3 * kinds.rbegin()->first;   // of many rounds: their mean and a tail
