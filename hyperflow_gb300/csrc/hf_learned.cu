@@ -1339,7 +1339,7 @@ struct hf_lc {
     unsigned long long* rejected = nullptr;
     double* loss = nullptr;
     struct Out { double loss; int derr, pad; };
-    Out* out = nullptr;        // pinned: a training iteration's loss and the error word
+    Out* out = nullptr;        // pinned, from the first training iteration on: its loss and the error word
     int* derr = nullptr;       // device error word (a bounded wait gave up)
     Loop* loop = nullptr;      // the device run loop
     struct Pair {              // two steps of it, captured for these settings
@@ -1552,7 +1552,6 @@ int hf_lc_create(int n, double dx, double gamma, double cfl, int limiter, hf_lc*
     static_assert(NPARAM % 2 == 0, "the loss follows the gradient");
     L->loss = reinterpret_cast<double*>(L->grad + NPARAM);
     L->derr = reinterpret_cast<int*>(L->loss + 1);
-    LCK(cudaMallocHost(&L->out, sizeof(hf_lc::Out)));
     return HF_OK;
 }
 
@@ -1850,6 +1849,8 @@ int hf_lc_train_step(hf_lc* L, const float* U0, const float* T, const float* w, 
     LCK(cudaMemcpyAsync(L->T, T, bytes, cudaMemcpyHostToDevice, L->side));   // beside the forward
     LCK(cudaEventRecord(L->join, L->side));
     LCK(cudaStreamWaitEvent(L->stream, L->join, 0));
+    // (not at the creation, which it made up to 150 us longer; a copy to pageable memory takes 2 us more an iteration)
+    if (!L->out) LCK(cudaMallocHost(&L->out, sizeof(hf_lc::Out)));
     const float rr = (float)(dt / L->dx);
     if (L->train_guard) {   // the guard of inference: rejected faces take the plain flux
         LCK(cudaMemsetAsync(L->ok, 1, nf, L->stream));
