@@ -663,7 +663,7 @@ int hf_create(const char* case_json, size_t len, hf_ctx** out) {
     *out = holder.release();
     CK(cudaGetDevice(&ctx->device));
     CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
-    CK(hf::stencil_prepare());
+    CK(hf::stencil_prepare(ctx->scheme, ctx->limiter));
     // device state
     hf::MeshDev& M = ctx->hmesh;
     M.nblocks = ctx->nblocks;
@@ -725,8 +725,9 @@ int hf_create(const char* case_json, size_t len, hf_ctx** out) {
     constexpr size_t step_off = (sizeof(hf::Ctrl) + 255) / 256 * 256;
     CK(cudaMalloc(&ctx->dctrl, step_off + sizeof(hf::StepState)));
     ctx->dstep = reinterpret_cast<hf::StepState*>(reinterpret_cast<char*>(ctx->dctrl) + step_off);
-    CK(cudaMemsetAsync(ctx->dstep, 0, sizeof(hf::StepState), ctx->stream));
-    CK(cudaMemcpyAsync(ctx->dctrl, &C, sizeof C, cudaMemcpyHostToDevice, ctx->stream));
+    unsigned char init[step_off + sizeof(hf::StepState)] = {};
+    std::memcpy(init, &C, sizeof C);
+    CK(cudaMemcpyAsync(ctx->dctrl, init, sizeof init, cudaMemcpyHostToDevice, ctx->stream));
     {
         int nx[HF_MAXB], ny[HF_MAXB], sms = 0;
         for (int b = 0; b < ctx->nblocks; ++b) {

@@ -1052,12 +1052,15 @@ cudaError_t launch_solo(Ctrl* c, const MeshDev* m, StepState* ss, int nx, int ny
     return cudaGetLastError();
 }
 
-cudaError_t stencil_prepare() {
-    for (const void* k : {(const void*)mh_step_kernel<0>, (const void*)mh_step_kernel<1>, (const void*)mh_rerun_kernel<0>,
-                          (const void*)mh_rerun_kernel<1>, (const void*)mh_kernel<0>, (const void*)mh_kernel<1>,
-                          (const void*)godunov_step_kernel, (const void*)godunov_kernel, (const void*)solo_kernel<0, 0>,
-                          (const void*)solo_kernel<1, 0>, (const void*)solo_kernel<1, 1>}) {
-        const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes);
+// (of the scheme's kernels alone: an opt-in costs a creation about a microsecond)
+cudaError_t stencil_prepare(int scheme, int limiter) {
+    const void* const kernels[3][4] = {
+        {(const void*)godunov_step_kernel, (const void*)godunov_kernel, (const void*)solo_kernel<0, 0>, nullptr},
+        {(const void*)mh_step_kernel<0>, (const void*)mh_rerun_kernel<0>, (const void*)mh_kernel<0>, (const void*)solo_kernel<1, 0>},
+        {(const void*)mh_step_kernel<1>, (const void*)mh_rerun_kernel<1>, (const void*)mh_kernel<1>, (const void*)solo_kernel<1, 1>}};
+    for (const void* k : kernels[scheme == 0 ? 0 : limiter == 0 ? 1 : 2]) {
+        const cudaError_t e = k ? cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileBytes)
+                                : cudaSuccess;
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

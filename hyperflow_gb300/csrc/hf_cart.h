@@ -169,7 +169,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn tensor_map_encoder();
 
-cudaError_t stencil_prepare();   // sets the large dynamic shared-memory opt-ins once
+cudaError_t stencil_prepare(int scheme, int limiter);   // the large shared-memory opt-ins of its kernels
 
 // geometry of one block as the initial condition needs it
 struct BlockGeom {
