@@ -530,6 +530,13 @@ int ensure_maps(hf_batch* b, int k) {
     return HF_OK;
 }
 
+// the tile list and maps of configuration k, from its selection on: a run allocates and copies nothing, so the
+// first one too may be captured, or made in a thread that has no context yet
+int prepare_config(hf_batch* b, int k) {
+    const int r = ensure_tiles(b, k);
+    return r ? r : ensure_maps(b, k);
+}
+
 hf::BatchDev devview(hf_batch* b, int k) {
     hf::BatchDev d{};
     d.ctrl = b->dctrl;
@@ -686,7 +693,7 @@ int hf_batch_create(const char* manifest, size_t len, hf_batch** out) {
         BCK(cudaMemcpy2D(b->U[0] + I.off, (size_t)I.pitch * 8, init[i].data(), (size_t)I.n * 8, (size_t)I.n * 8,
                          (size_t)4 * I.n, cudaMemcpyHostToDevice));
     }
-    const int r = ensure_tiles(b, 0);   // (a first run may be captured: no allocation then)
+    const int r = prepare_config(b, 0);
     return r ? r : refresh_cfl(b, 0, 0, (int)n);
 }
 
@@ -732,16 +739,16 @@ int hf_batch_config_info(int k, int* tile_x, int* tile_y, int* threads, int* sta
 
 int hf_batch_set_config(hf_batch* b, int k) {
     if (!b || k < 0 || k >= hf::kNumConfigs) return HF_ERR_ARG;
-    b->config = k;
-    return HF_OK;
+    const int r = prepare_config(b, k);
+    if (r == HF_OK) b->config = k;
+    return r;
 }
 
 int hf_batch_run(hf_batch* b, int64_t nsteps, int use_graph) {
     hf::TraceRange trace_("hf_batch_run");
     if (!b || nsteps < 0 || nsteps > (1 << 30)) return HF_ERR_ARG;
     if (nsteps == 0) return HF_OK;
-    int r = ensure_tiles(b, b->config);
-    if (!r) r = ensure_maps(b, b->config);
+    const int r = prepare_config(b, b->config);   // (there already, unless a call before failed)
     if (r) return r;
     hf::BatchDev d = devview(b, b->config);
     while (use_graph && nsteps > 0) {   // graphs of up to kGraphSteps steps
@@ -794,8 +801,7 @@ int hf_batch_autotune(hf_batch* b, int steps_per_trial, int* best, double* ms_pe
     int bestk = -1;
     double bestms = 1e300;
     for (int k = 0; k < hf::kNumConfigs; ++k) {
-        int r = ensure_tiles(b, k);
-        if (!r) r = ensure_maps(b, k);
+        int r = prepare_config(b, k);
         if (r) return r;
         hf::BatchDev d = devview(b, k);
         // warm (first launch pays the shared-memory opt-in), then time
