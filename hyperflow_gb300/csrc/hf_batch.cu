@@ -442,15 +442,13 @@ struct hf_batch {
     long long ntiles[hf::kNumConfigs] = {};
     CUtensorMap* maps[hf::kNumConfigs] = {};   // MUSCL-Hancock: the TMA maps of the cases' tile boxes
     int config = 0;
-    // graphs: key = (config, nsteps)
+    // graphs: key = (config, nsteps), a bounded number per configuration (batch_graph_steps)
     struct G { int config; long long nsteps; cudaGraphExec_t exec; };
     std::vector<G> graphs;
     std::string err;
 };
 
 namespace {
-
-constexpr long long kGraphSteps = 128;   // steps of one graph
 
 int bfail(hf_batch* b, int code, const std::string& m) {
     if (b) b->err = m;
@@ -551,6 +549,12 @@ hf::BatchDev devview(hf_batch* b, int k) {
     d.t = b->t;
     d.last_dt = b->last_dt;
     return d;
+}
+
+cudaGraphExec_t find_graph(const hf_batch* b, long long nsteps) {
+    for (const auto& g : b->graphs)
+        if (g.config == b->config && g.nsteps == nsteps) return g.exec;
+    return nullptr;
 }
 
 long long read_step(hf_batch* b) {
@@ -751,11 +755,15 @@ int hf_batch_run(hf_batch* b, int64_t nsteps, int use_graph) {
     const int r = prepare_config(b, b->config);   // (there already, unless a call before failed)
     if (r) return r;
     hf::BatchDev d = devview(b, b->config);
-    while (use_graph && nsteps > 0) {   // graphs of up to kGraphSteps steps
-        const long long n = std::min<long long>(nsteps, kGraphSteps);
-        cudaGraphExec_t exec = nullptr;
-        for (auto& g : b->graphs)
-            if (g.config == b->config && g.nsteps == n) exec = g.exec;
+    while (use_graph && nsteps > 0) {
+        long long n = std::min<long long>(nsteps, hf::kBatchGraphSteps);
+        cudaGraphExec_t exec = find_graph(b, n);
+        if (!exec) {
+            n = hf::batch_graph_steps(nsteps, (int)std::count_if(b->graphs.begin(), b->graphs.end(), [&](const hf_batch::G& g) {
+                return g.config == b->config;
+            }));
+            exec = find_graph(b, n);
+        }
         if (!exec) {
             cudaGraph_t graph;
             BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));

@@ -1,15 +1,18 @@
 // Host build of the kernels' arithmetic (hf_device.cuh, hf_intdiv.cuh) for the CPU test
 // suite: the same source the GPU kernels compile, exposed as plain C functions so the
-// tests can compare it with the oracle and with IEEE division / sqrt without a GPU; and the walk over ranges of
-// pinned memory, on made-up ranges.
+// tests can compare it with the oracle and with IEEE division / sqrt without a GPU; and the rules
+// of the host side that can be told apart there (ranges of pinned memory, the graphs of a batched run).
 // Built as a separate library (libhf_hostmath.so); the product library does not use it.
 #include <cstdint>
 
+#include "hf_cart.h"
 #include "hf_device.cuh"
 #include "hf_fast.cuh"
 #include "hf_pinned.h"
 
 extern "C" {
+
+int64_t hm_batch_graph_steps(int64_t left, int graphs) { return hf::batch_graph_steps(left, graphs); }
 
 // host_covered over n ranges [begin[k], begin[k] + size[k])
 int hm_host_covered(const uint64_t* begin, const uint64_t* size, int n, uint64_t p, uint64_t bytes) {
