@@ -73,7 +73,7 @@ struct hf_ctx {
     hf::StepState* dstep = nullptr;
     bool solo = false;          // one block whose ghosts are interior cells' values or Dirichlet states
     bool user_graphs = false;   // a caller has captured steps
-    bool caller_captures = false;   // and is capturing this call
+    unsigned long long capture = 0; // the capture this call is part of (0: none)
     int clamp = -1;             // the device's clamp switch, -1 when not known
     hf::StepOut* out = nullptr; // a step's dt and count, in host memory the GPU maps
     long long steps_known = -1; // steps completed, -1 when the device may have moved on
@@ -98,6 +98,7 @@ struct hf_ctx {
     // maxima those of the current fields (a TimeStep call since the last fill or upload)?
     bool step_started = false;
     bool ghost_fresh = false;
+    unsigned long long started_in = 0;   // the capture the call that set them was part of
     // profiling
     bool profile = false;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev[2];
@@ -540,9 +541,16 @@ constexpr long long kLoopCells = 1 << 20;
 // capture on nothing is taken as known about the device: a replay is not seen here.
 bool capturing(hf_ctx* ctx) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    ctx->caller_captures = cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone;
-    ctx->user_graphs = ctx->user_graphs || ctx->caller_captures;
-    return ctx->caller_captures;
+    unsigned long long id = 0;
+    const bool known = cudaStreamGetCaptureInfo(ctx->stream, &st, &id) == cudaSuccess;
+    ctx->capture = known && st == cudaStreamCaptureStatusNone ? 0 : (id ? id : ~0ull);
+    ctx->user_graphs = ctx->user_graphs || ctx->capture != 0;
+    return ctx->capture != 0;
+}
+// Whether step_started and ghost_fresh hold for the call being made: a captured call does its part when its
+// graph runs, so they pass on within a capture, or between calls of a context that no graph moves.
+bool pieces_known(const hf_ctx* ctx) {
+    return ctx->started_in == ctx->capture && (ctx->capture != 0 || !ctx->user_graphs);
 }
 
 // The accumulators of the next step cleared, unless the end of the step before it did so: known only when
@@ -563,7 +571,7 @@ int enqueue_step(hf_ctx* ctx, bool profiled, hf::StepOut* out = nullptr) {
     ctx->steps_known = -1;
     if (profiled) ev_record(ctx, 1, true);
     // (a caller's graph may be replayed in strict mode, whose stop the fill takes and this launch does not)
-    if (ctx->solo && ctx->ring_slots == 0 && !ctx->strict && !ctx->block_launches && !ctx->caller_captures) {
+    if (ctx->solo && ctx->ring_slots == 0 && !ctx->strict && !ctx->block_launches && ctx->capture == 0) {
         if (profiled) { ev_record(ctx, 1, false); ev_record(ctx, 0, true); }
         CK(hf::launch_solo(ctx->dctrl, ctx->dmesh, ctx->dstep, ctx->blocks[0].nx, ctx->blocks[0].ny, ctx->scheme,
                            ctx->limiter, ctx->tile, &ctx->tmap[0][0], &ctx->tmap[0][1], ctx->stream, out));
@@ -921,6 +929,7 @@ int hf_apply_bcs(hf_ctx* ctx) {
     CK(hf::launch_ghost_mirror(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
     ctx->step_started = true;
     ctx->ghost_fresh = false;
+    ctx->started_in = ctx->capture;
     return HF_OK;
 }
 
@@ -936,6 +945,7 @@ int hf_time_step(hf_ctx* ctx, double* dt) {
     CK(hf::launch_ghost_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream));
     ctx->step_started = true;
     ctx->ghost_fresh = true;
+    ctx->started_in = ctx->capture;
     if (dt) {
         CK(cudaMemcpyAsync(dt, &ctx->dctrl->dt_cfl, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
@@ -953,8 +963,9 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         // the MUSCL-Hancock predictor's TimeStep call the ghost maxima of the current fields
         ctx->clean = false;
         ctx->steps_known = -1;
-        if (!ctx->step_started) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-        if (ctx->scheme == 1 && !ctx->ghost_fresh)
+        const bool known = pieces_known(ctx);
+        if (!known || !ctx->step_started) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
+        if (ctx->scheme == 1 && !(known && ctx->ghost_fresh))
             CK(hf::launch_ghost_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 0));
         CK(hf::launch_set_dt(ctx->dctrl, dt, ctx->stream));
     }

@@ -1,6 +1,6 @@
 """What a step finds of the calls before it: the wave-speed maxima of a TimeStep call or a ghost fill that a
 caller's graph ran again, or that no step followed, are not those of the next step's fields; strict mode
-switched on after a step was captured stops its replays."""
+switched on after a step was captured stops its replays; a captured TimeStep call is not taken as made."""
 import numpy as np
 import pytest
 
@@ -92,3 +92,43 @@ def test_strict_mode_stops_steps_captured_before_it():
     assert a.time() == b.time()
     np.testing.assert_array_equal(a.state(0), b.state(0))
     assert a.last_nonpositive_cell() == b.last_nonpositive_cell()
+
+
+@pytest.mark.parametrize("scheme", ["Godunov", "MUSCLHancock"])
+@pytest.mark.parametrize("call", ["hf_time_step", "hf_apply_bcs"])
+def test_a_call_that_was_only_captured_is_not_taken_as_made(call, scheme):
+    """hf_advance after it starts the step itself, and the step after that finds its own wave speeds."""
+    import torch
+    from hyperflow_gb300 import CartSolver, cases
+    from hyperflow_gb300._lib import lib
+    case = cases.quadrant_case(40, scheme=scheme, limiter="VanLeer" if scheme == "MUSCLHancock" else None, cfl=cases.CFL_2D)
+    case["mesh"]["blocks"][0]["boundaries"]["left"] = {"type": "Dirichlet", "variables": "Primitive",
+                                                       "flow_state": [0.5, 9.0, 0.3, 4.0]}
+    a, b = CartSolver(case), CartSolver(case)
+    for s in (a, b):
+        s.run(12)
+    stream = torch.cuda.ExternalStream(a.stream())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        g.capture_begin(capture_error_mode="thread_local")
+        assert (lib().hf_apply_bcs(a._h) if call == "hf_apply_bcs" else lib().hf_time_step(a._h, None)) == 0
+        g.capture_end()
+    for s in (a, b):
+        s.advance(1e-3)
+    np.testing.assert_array_equal(a.state(0), b.state(0))
+    assert a.calculate_time_step() == b.calculate_time_step()
+    # captured together, the TimeStep call serves the advance behind it
+    h = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        h.capture_begin(capture_error_mode="thread_local")
+        assert lib().hf_apply_bcs(a._h) == 0 and lib().hf_time_step(a._h, None) == 0
+        a.advance(2e-4)
+        h.capture_end()
+        h.replay()
+        h.replay()
+    for _ in range(2):
+        b.apply_bcs()
+        b.calculate_time_step()
+        b.advance(2e-4)
+    np.testing.assert_array_equal(a.state(0), b.state(0))
+    assert a.time() == b.time()
