@@ -963,9 +963,10 @@ int hf_advance_block(hf_ctx* ctx, int b, double dt) {
         // the MUSCL-Hancock predictor's TimeStep call the ghost maxima of the current fields
         ctx->clean = false;
         ctx->steps_known = -1;
-        const bool known = pieces_known(ctx);
-        if (!known || !ctx->step_started) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
-        if (ctx->scheme == 1 && !(known && ctx->ghost_fresh))
+        // (from zero: a ghost fill before an upload has left the maxima of other fields)
+        const bool known = pieces_known(ctx), pass = ctx->scheme == 1 && !(known && ctx->ghost_fresh);
+        if (!known || !ctx->step_started || pass) CK(hf::launch_step_begin(ctx->dctrl, ctx->stream));
+        if (pass)
             CK(hf::launch_ghost_cfl(ctx->dctrl, ctx->dmesh, ctx->hmesh.total_ghost, ctx->stream, 0));
         CK(hf::launch_set_dt(ctx->dctrl, dt, ctx->stream));
     }

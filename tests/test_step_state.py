@@ -132,3 +132,17 @@ def test_a_call_that_was_only_captured_is_not_taken_as_made(call, scheme):
         b.advance(2e-4)
     np.testing.assert_array_equal(a.state(0), b.state(0))
     assert a.time() == b.time()
+
+
+def test_fields_uploaded_after_a_ghost_fill_have_their_own_predictor():
+    a, b = _solver(), _solver()
+    U = None
+    for s in (a, b):
+        s.run(12)
+        U = _calm(s.state(0)) if U is None else U
+        if s is a:
+            s.apply_bcs()
+        s.set_state(0, U)
+        s.advance(1e-3)
+    np.testing.assert_array_equal(a.state(0), b.state(0))
+    assert a.calculate_time_step() == b.calculate_time_step()
