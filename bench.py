@@ -19,7 +19,7 @@ Other workloads (`--workload`, one JSON line each, not the headline):
     square    one N x N four-quadrant block (--n, --scheme, --limiter)
     batch     512 batched Riemann problems, one launch per step of all (autotuned)
     uns       the ~1M-triangle channel, edge-based (or --uns-per-side) fluxes
-    quad256   the 256^2 Godunov problem as a batch of one (the whole run one launch)
+    quad256   the 256^2 Godunov problem as a batch of one (one launch per step)
     learned   the 512^2 learned coarse step (FP32 + the tcgen05 MLP on every face)
     learned-train  a 512^2 training iteration of the learned solver (tcgen05 forward and backward)
 """
@@ -575,6 +575,7 @@ def main():
     s.sync()
     ms = e0.elapsed_time(e1)
     stencil_ms, stencil_launches = s.kernel_time(0)
+    fill_ms, _ = s.kernel_time(1)
     s.profile(False)
     value, t_max = replica_value(ms, ws, cells, args.steps, pg)
     hllc_fallbacks = s.hllc_errors()
@@ -651,6 +652,9 @@ def main():
     tr = ncu_traffic()
     all_blocks = nb <= 4 and not args.per_block_launches
     all_mh = args.scheme == "MUSCLHancock"
+    # a small single block steps in one launch: with no ghost fill before it, the two events that bracket
+    # the fill lie side by side (a fill takes 9 us or more)
+    solo = nb == 1 and all_blocks and fill_ms / args.steps < 0.005
     per_launch = 1 if all_blocks else nb           # stencil launches per step
     if tr and tr.get("workload") == workload_name(args):
         traffic = tr["dram_bytes_per_cell_update"] * cells / per_launch
@@ -658,10 +662,14 @@ def main():
             "frac": achieved / hbm, "traffic": traffic, "peak_kind": peak_kind,
             "algorithmic_bytes_per_launch": BYTES_PER_CELL * cells / per_launch,
             "avg_launch_ms": stencil_ms / max(stencil_launches * per_launch, 1),
-            "kernel": ("mh_step_kernel (every block of the step in one launch: fused MUSCL-Hancock + HLLC + "
-                       "forward Euler + CFL epilogue)") if all_blocks else
-                      "mh_kernel (fused MUSCL-Hancock + HLLC + forward Euler + CFL epilogue)"}
-    # the bound that binds on this part: FP64 issue (2 lanes per SM per clock)
+            "kernel": ("solo_kernel (a whole step of one block, its ghosts and dt included: " if solo else
+                       ("mh_step_kernel" if all_mh else "godunov_step_kernel") +
+                       " (every block of the step in one launch: " if all_blocks else
+                       ("mh_kernel" if all_mh else "godunov_kernel") + " (") +
+                      ("fused MUSCL-Hancock + HLLC" if all_mh else "fused Godunov + HLLC") +
+                      " + forward Euler + CFL epilogue)"}
+    # the bound that binds on this part: the FP64 pipe, which an addition or product of a warp holds for 19
+    # cycles of its SM and a fused multiply-add for 16 (measured; the traffic file has the kernel's mix)
     if tr and tr.get("workload") == workload_name(args) and tr.get("fp64_ops_per_cell_update"):
         sm_mhz = 2070.0
         pk = os.path.join(ROOT, "MEASURED_PEAKS.json")
@@ -670,9 +678,10 @@ def main():
                 sm_mhz = float(json.load(f).get("sm_max_mhz", sm_mhz))
         nsm = torch.cuda.get_device_properties(local).multi_processor_count
         ops = tr["fp64_ops_per_cell_update"] * cells * args.steps / (stencil_ms / 1e3) / 1e9
-        peak_ops = 2.0 * nsm * sm_mhz / 1e3
+        cycles = float(tr.get("fp64_cycles_per_warp_instruction", 19.0))
+        peak_ops = 32.0 / cycles * nsm * sm_mhz / 1e3
         roof["fp64_pipe"] = {"achieved": ops, "peak": peak_ops, "unit": "G FP64 ops/s (FMA = 1)",
-                             "frac": ops / peak_ops,
+                             "frac": ops / peak_ops, "cycles_per_warp_instruction": cycles,
                              "ops_per_cell_update": tr["fp64_ops_per_cell_update"]}
 
     # ---- CPU baseline (rank 0, N=1): the oracle on all host cores, bounded sample ----
@@ -690,10 +699,10 @@ def main():
     if rank == 0 and ws == 1 and args.workload == "ffs" and args.cpu_seconds > 0:
         cpu_ref = reference_cpu_baseline(args.limiter)
 
-    # the ghost fill + ghost CFL + dt, then one launch for every block of a mesh of up to 4 blocks (with
-    # MUSCL-Hancock one more for each block but the first, which re-runs it where its predictor dt
-    # changed), else one per block and the step's end
-    launches_per_step = (2 + (nb - 1 if all_mh else 0)) if all_blocks else 2 + nb
+    # one launch for a small single block; else the ghost fill + ghost CFL + dt, then one launch for every
+    # block of a mesh of up to 4 blocks (with MUSCL-Hancock one more for each block but the first, which
+    # re-runs it where its predictor dt changed), or one per block and the step's end
+    launches_per_step = 1 if solo else (2 + (nb - 1 if all_mh else 0)) if all_blocks else 2 + nb
     if rank == 0:
         line = {
             "metric": "Mcell-updates/s", "value": value, "unit": "Mcell-updates/s",

@@ -3,8 +3,9 @@
 // Host side: parses the reference's case file, builds the initial state exactly as
 // the reference does (setup only), owns the device buffers, the TMA descriptors and the
 // CUDA stream, and orders the kernels of one step:
-//     bc_fill -> ghost_cfl (dt) -> stencil(block 0) ... stencil(block B-1) -> finalize
-// which is the reference's apply_bcs -> calculate_time_step -> per-block ODE sequence
+//     ghost fill and dt -> every block's update, whose last CTA ends the step (-> re-runs)
+// or, where it applies, one launch for all of that, or a launch per block and one for the end; which is the
+// reference's apply_bcs -> calculate_time_step -> per-block ODE sequence
 // (src/fvm_2d_cart/simulation/simulation/simulation.cpp:85-120).
 #include <cmath>
 #include <cstdio>
@@ -91,8 +92,7 @@ struct hf_ctx {
     float* coarse = nullptr;    // device scratch of hf_coarsen
     size_t coarse_n = 0;
     int next_block = 0;         // next block hf_advance_block expects
-    // graphs of one step (index = clamp flag)
-    cudaGraphExec_t graph[4] = {};   // of one step, without and with the clamp; of kLoopSteps
+    cudaGraphExec_t graph[4] = {};   // hf_run's: of one step without and with the clamp, of kLoopSteps likewise
     int strict = 0;             // hf_set_strict: a zero-flux face stops the loop
     // piecewise steps: has this step been started (accumulators reset) and are the ghost
     // maxima those of the current fields (a TimeStep call since the last fill or upload)?

@@ -63,8 +63,6 @@ struct BatchCtrl {
     double gamma, g1, cfl;
     long long calls;        // TimeStep calls made by every case so far
     long long step;         // steps completed
-    int limiter;
-    int scheme;             // 0 Godunov, 1 MUSCL-Hancock
     int ninst;
     int err;
     unsigned int tiles_done;           // of the running step
@@ -276,7 +274,11 @@ __global__ void __launch_bounds__(kCflThreads) batch_cfl_kernel(BatchDev d, int 
 // A configuration's tile shape and CTA.  tx = 0: each case has its own (case_tiles), by a model that
 // counts what the rounds of a CTA's warps leave idle beside the work, or (model 1) the work alone: the first
 // was better for batches of several rounds of tiles (24 cases of 64^2 .. 385^2: 52.5 against 56.3 ms for 100
-// steps), the second for smaller ones (8 of 128^2: 9.61, 8.66; one of 256^2: 5.28, 4.68).
+// steps), the second for smaller ones (8 of 128^2: 9.61, 8.66; one of 256^2: 5.28, 4.68).  Of the fixed
+// shapes, timed on 72 batches of 1 to 200 cases, the fifth beat both by up to 9 % on five (8 of 128^2, Godunov: 36.8
+// against 40.6 us a step, MUSCL-Hancock 84.6, 88.7) and the sixth by up to 15 % on three (8 of 64^2,
+// MUSCL-Hancock: 36.6, 43.1); the third and fourth by no more than 0.1 % on any: they stay for callers that
+// select a configuration by its number.
 struct BatchConfig {
     int tx, ty, threads, model;
 };
@@ -687,8 +689,6 @@ int hf_batch_create(const char* manifest, size_t len, hf_batch** out) {
     C.gamma = b->gamma;
     C.g1 = b->gamma - 1.0;
     C.cfl = b->cfl;
-    C.limiter = b->limiter;
-    C.scheme = b->scheme;
     C.ninst = (int)n;
     C.first_nonpos = ~0ull;
     BCK(cudaMemcpy(b->dctrl, &C, sizeof C, cudaMemcpyHostToDevice));

@@ -1,8 +1,8 @@
 // The MUSCL-Hancock predictor, the HLLC face and the update of ordinary states, with every product,
 // quotient and root on the integer pipes and without a branch per operation.
 //
-// What bounds the stencils is the FP64 pipe: a warp's FP64 instruction holds it for 20 cycles of the SM
-// (measured, any mix of additions and products), the time of 80 instructions on the other pipes.  With
+// What bounds the stencils is the FP64 pipe: a warp's FP64 addition or product holds it for 19 cycles of the SM
+// (measured; a fused multiply-add 16), the time of 76 instructions on the other pipes.  With
 // divisions and roots on the integer pipes the step was at that bound, two fifths of its FP64
 // instructions products; an exact product costs 29 integer instructions (prod).  A range check and a
 // branch per product cost half as much again and cut the code into pieces too short to overlap, so the
@@ -15,7 +15,7 @@
 // products, 1600 - 1700 with one checked integer product at a time or in groups, 1973 like this (2107 with
 // a CTA per tile, hf_cart.cu); Van Leer 1469 -> 1964 (2097), the developed forward-facing step 1639 -> 2038
 // (2171).  FP64 instructions a cell update 305 -> 194, all instructions 7,300 -> 11,000; issue slots 58 % busy,
-// FP64 pipe 83 % of saturation, the integer (ALU) pipe 62 %.  It is no longer the FP64 pipe alone: with 8 %
+// FP64 pipe 75 % of what it can take, the integer (ALU) pipe 62 %.  It is no longer the FP64 pipe alone: with 8 %
 // of the FP64 instructions moved too (the limiter's 1 + r and slope product, 17 and 31 integer ones each) it
 // ran between 1.5 % slower and 1 % faster, and stays as it is.
 #pragma once

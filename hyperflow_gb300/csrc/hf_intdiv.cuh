@@ -1,7 +1,7 @@
 // Correctly rounded FP64 division and square root on the integer pipes.
 //
-// GB300 issues FP64 at 2 lanes per SM per clock: a warp's FP64 instruction holds the SM's pipe for
-// 16 cycles, in which the SM can issue 64 others.  An IEEE division built from FP64 Newton steps
+// A warp's FP64 addition or product holds the SM's FP64 pipe for 19 cycles, a fused multiply-add for 16
+// (measured), in which the SM can issue 76 or 64 others.  An IEEE division built from FP64 Newton steps
 // costs about ten FP64 instructions; this one costs none, and about 60 others.  It is schoolbook
 // long division with two large digits (see Muller et al., "Handbook of Floating-Point
 // Arithmetic", the chapter on division; Moller & Granlund, "Improved division by invariant

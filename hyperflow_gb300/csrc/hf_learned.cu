@@ -786,7 +786,7 @@ size_t mlp_forward_smem() { return sizeof(TcSmem) + 1024; }
 //     operands MN-major (a face's values contiguous): D[0:64][0:64] = sum dz1^T x = dW1,
 //     D[64:128][64:128] = sum dz2^T h1 = dW2, D[:][128] = sum dz = db1, db2; the off-diagonal
 //     blocks are not used;
-//   dW3 = sum dY^T h2 and db3 on the CUDA cores from shared memory while that MMA runs.
+//   dW3 = sum dY^T h2 and db3 on the CUDA cores from shared memory, once that MMA is done.
 // The activations h1, h2 are the forward's (BF16(gelu(z)) from the saved pre-activations).
 // MN-major canonical layout without swizzle: core matrices of 8 K-rows x 8 contiguous M/N
 // elements (128 B), K-adjacent core matrices 128 B apart (the descriptor's leading offset),

@@ -105,8 +105,9 @@ int hf_host_mapped(const void* p, int* mapped);
 
 /* Simulation::solve's loop body (simulation.cpp:81-120, frame clamps excluded) run n times
  * on the device with no host round trip per step: dt stays on the device.  clamp_t_end != 0
- * applies the t_end clamp and stops at t_end like the reference.  use_graph != 0 replays a
- * captured CUDA graph of one step.  steps_done (optional) = steps actually taken. */
+ * applies the t_end clamp and stops at t_end like the reference.  use_graph != 0 replays
+ * captured CUDA graphs, of 32 steps below 2^20 cells and of one step for the rest.  steps_done (optional) =
+ * steps actually taken. */
 int hf_run(hf_ctx* ctx, int64_t n, int clamp_t_end, int use_graph, int64_t* steps_done);
 
 /* simulation time, TimeStep call count, and the dt applied by the last step */
@@ -157,7 +158,7 @@ int hf_blocks_rerun(hf_ctx* ctx, int64_t* count);
 /* per-kernel timing: when enabled, every step's stencil launches are bracketed by CUDA events on
  * the context's stream; hf_kernel_time returns the summed milliseconds and the number of
  * bracketed steps since the last reset.  kind 0 = stencil (Godunov/MUSCL-Hancock), 1 = ghost
- * fill + CFL. */
+ * fill + CFL (next to nothing for a step in one launch, whose whole is of kind 0). */
 int hf_profile(hf_ctx* ctx, int enable);
 int hf_kernel_time(hf_ctx* ctx, int kind, double* ms, int64_t* launches);
 
