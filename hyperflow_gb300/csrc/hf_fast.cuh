@@ -15,7 +15,7 @@
 // products, 1600 - 1700 with one checked integer product at a time or in groups, 1973 like this (2107 with
 // a CTA per tile, hf_cart.cu); Van Leer 1469 -> 1964 (2097), the developed forward-facing step 1639 -> 2038
 // (2171).  FP64 instructions a cell update 305 -> 194, all instructions 7,300 -> 11,000; issue slots 58 % busy,
-// FP64 pipe 75 % of what it can take, the integer (ALU) pipe 62 %.  It is no longer the FP64 pipe alone: with 8 %
+// FP64 pipe 76 % of what it can take, the integer (ALU) pipe 62 %.  It is no longer the FP64 pipe alone: with 8 %
 // of the FP64 instructions moved too (the limiter's 1 + r and slope product, 17 and 31 integer ones each) it
 // ran between 1.5 % slower and 1 % faster, and stays as it is.
 #pragma once

@@ -45,8 +45,9 @@ int hf_batch_set_config(hf_batch* b, int k);
  * configuration) receives the timings */
 int hf_batch_autotune(hf_batch* b, int steps_per_trial, int* best, double* ms_per_step);
 
-/* nsteps steps of every case, one launch each; use_graph replays a captured graph of
- * them (captured once per (configuration, nsteps), in pieces of up to 128 steps) */
+/* nsteps steps of every case, one launch each; use_graph replays captured graphs of them, of up to 128
+ * steps (the first 16 lengths of a configuration have one of their own, later ones are put together).  Without
+ * use_graph a run allocates nothing and may be captured by the caller, the first one too. */
 int hf_batch_run(hf_batch* b, int64_t nsteps, int use_graph);
 int hf_batch_sync(hf_batch* b);
 
